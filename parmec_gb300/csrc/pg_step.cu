@@ -25,9 +25,12 @@ namespace {
 constexpr int TPB = 128;
 
 // minimum resident blocks per SM asked of the FP64 particle update and of
-// the contact evaluation (register budget against warps in flight)
+// the contact evaluation (register budget against warps in flight).  The
+// particle update at 1, 4 and 5 blocks (144, 128, 96 registers): 571, 552,
+// 547 us on the 1,048,576-sphere drum and 56, 52, 48 us on 230,000 shaken
+// spheres; a warp waits for its loads while others hold the FP64 pipe.
 #ifndef PG_INTEGRATE_MINB
-#define PG_INTEGRATE_MINB 1
+#define PG_INTEGRATE_MINB 5
 #endif
 #ifndef PG_EVAL_MINB
 #define PG_EVAL_MINB 8
@@ -96,33 +99,6 @@ __device__ __forceinline__ void set_piso(const PgDev &d, int i)
   for (int k = 0; k < 6; k ++)
     iso = iso && dbits(d.inertia[off[k]][i]) == 0 && dbits(d.inverse[off[k]][i]) == 0;
   d.piso[i] = iso ? 1 : 0;
-}
-
-__device__ __forceinline__ bool finite_bits(double x) { return finite_d(x); }
-
-// p + 0*a + 0*b as the full product sums them, for finite a and b
-__device__ __forceinline__ double zero_terms(double p, double a, double b)
-{
-  const long long bp = (long long)dbits(p);
-  if ((bp << 1) != 0) return p;
-  const bool neg = bp < 0 && (long long)dbits(a) < 0 && (long long)dbits(b) < 0;
-  return __longlong_as_double(neg ? (long long)0x8000000000000000ull : 0ll);
-}
-
-// C = (j*I) B, bit for bit as nvmul with the full matrix
-__device__ __forceinline__ void iso_nvmul(double j, const double *B, double *C)
-{
-  if (finite_bits(B[0]) && finite_bits(B[1]) && finite_bits(B[2]))
-  {
-    C[0] = zero_terms(j*B[0], B[1], B[2]);
-    C[1] = zero_terms(j*B[1], B[0], B[2]);
-    C[2] = zero_terms(j*B[2], B[0], B[1]);
-  }
-  else
-  {
-    const double M[9] = {j, 0.0, 0.0, 0.0, j, 0.0, 0.0, 0.0, j};
-    nvmul(M, B, C);
-  }
 }
 
 __global__ void k_iso_flags(PgDev d, int p0, int p1)
@@ -1855,33 +1831,58 @@ __global__ void PG_LB_INTEGRATE k_integrate(PgDev d, double step, double half, d
       }
       f[0] = F[0]; f[1] = F[1]; f[2] = F[2];
       t[0] = T[0]; t[1] = T[1]; t[2] = T[2];
-      tvmul(L1, t, Tb);
-      expmap(-half*O[0], -half*O[1], -half*O[2], DL, typo);
-      if (iso) iso_nvmul(js, O, A); else nvmul(J, O, A);
-      nvmul(DL, A, B);
-      B[0] = B[0] + half*Tb[0];
-      B[1] = B[1] + half*Tb[1];
-      B[2] = B[2] + half*Tb[2];
-      if (iso) { iso_nvmul(is, B, A); iso_nvmul(js, A, B); }
-      else { nvmul(I, B, A); nvmul(J, A, B); }
-      Tb[0] -= A[1]*B[2] - A[2]*B[1];
-      Tb[1] -= A[2]*B[0] - A[0]*B[2];
-      Tb[2] -= A[0]*B[1] - A[1]*B[0];
-      Tb[0] *= step; Tb[1] *= step; Tb[2] *= step;
-      if (iso)
+      const bool free_spin = (dbits(T[0]) << 1 | dbits(T[1]) << 1 | dbits(T[2]) << 1) == 0;
+      if (iso && free_spin) Tb[0] = Tb[1] = Tb[2] = 0.0;
+      else tvmul(L1, t, Tb);
+      if (iso && gyro_settled(O, Tb, js, is, step, half))
       {
-        double IT[3];
-        iso_nvmul(is, Tb, IT);
-        O[0] = O[0] + IT[0]; O[1] = O[1] + IT[1]; O[2] = O[2] + IT[2];
+        // O + J^-1 (h Tb); unchanged, bit for bit, without a torque
+        if (!free_spin)
+        {
+          O[0] = O[0] + is*(step*Tb[0]);
+          O[1] = O[1] + is*(step*Tb[1]);
+          O[2] = O[2] + is*(step*Tb[2]);
+        }
       }
-      else nvaddmul(O, I, Tb, O);
+      else if (iso)
+      {
+        if (free_spin) tvmul(L1, t, Tb);                 // the signs of its zeros
+        spin_iso(O, Tb, js, is, step, half, typo);
+      }
+      else
+      {
+        expmap(-half*O[0], -half*O[1], -half*O[2], DL, typo);
+        nvmul(J, O, A);
+        nvmul(DL, A, B);
+        B[0] = B[0] + half*Tb[0];
+        B[1] = B[1] + half*Tb[1];
+        B[2] = B[2] + half*Tb[2];
+        nvmul(I, B, A);
+        nvmul(J, A, B);
+        Tb[0] -= A[1]*B[2] - A[2]*B[1];
+        Tb[1] -= A[2]*B[0] - A[0]*B[2];
+        Tb[2] -= A[0]*B[1] - A[1]*B[0];
+        Tb[0] *= step; Tb[1] *= step; Tb[2] *= step;
+        nvaddmul(O, I, Tb, O);
+      }
       im *= step;
       v[0] = v[0] + im*f[0];
       v[1] = v[1] + im*f[1];
       v[2] = v[2] + im*f[2];
-      expmap(hstep*O[0], hstep*O[1], hstep*O[2], DL, typo);
-      nnmul(L1, DL, L2);
-      nvmul(L2, O, o);
+      if ((dbits(O[0]) | dbits(O[1]) | dbits(O[2])) == 0 && turn_is_identity(L1, hstep))
+      {
+        // no spin: exp(0) is the identity and L stands; L O is zero, negative
+        // where all three products are
+        for (int k = 0; k < 9; k ++) L2[k] = L1[k];
+        for (int k = 0; k < 3; k ++)
+          o[k] = __longlong_as_double((long long)(dbits(L1[k]) & dbits(L1[3+k]) & dbits(L1[6+k]) & 0x8000000000000000ull));
+      }
+      else
+      {
+        expmap(hstep*O[0], hstep*O[1], hstep*O[2], DL, typo);
+        nnmul(L1, DL, L2);
+        nvmul(L2, O, o);
+      }
       x[0] += hstep*v[0];
       x[1] += hstep*v[1];
       x[2] += hstep*v[2];
@@ -1941,8 +1942,10 @@ __global__ void PG_LB_INTEGRATE k_integrate(PgDev d, double step, double half, d
       if (centre_is_position(x, L2, X, C)) { c[0] = x[0]; c[1] = x[1]; c[2] = x[2]; }
       else body_point(x, L2, X, C, c);
       d.center[0][e] = c[0]; d.center[1][e] = c[1]; d.center[2][e] = c[2];
-      double r0 = c[0] - d.cref[0][e], r1 = c[1] - d.cref[1][e], r2 = c[2] - d.cref[2][e];
-      need = gt_nonneg(r0*r0 + r1*r1 + r2*r2, d.half_skin_sq);
+      // the displacement since the rebuild, squared in FP32: its rounding
+      // (1e-6) is far inside the margin between 0.45 and 0.5 of the skin
+      const float r0 = mag32(c[0] - d.cref[0][e]), r1 = mag32(c[1] - d.cref[1][e]), r2 = mag32(c[2] - d.cref[2][e]);
+      need = r0*r0 + r1*r1 + r2*r2 > d.half_skin_sq_f;
     }
   }
   if (FUSED && d.ellnum) flag_rebuild(d, need);
