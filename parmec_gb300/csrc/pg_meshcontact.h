@@ -7,6 +7,11 @@
 
 #define PG_TT_KMAX 64             // partners one triangle may find (the search's thread-local list)
 
+// a pair whose contact a few distances decide: candidates (bits as in
+// pgtf::judge), where their results start, a bound on the smallest
+struct PgTTNear { int pair; unsigned mask; int vbase, ebase; float upper, size; };
+#define PG_TT_GEO 24
+
 struct PgTT
 {
   double r = 0.0;                 // swept radius of every mesh triangle
@@ -29,7 +34,17 @@ struct PgTT
   int cap = 0;                    // pair capacity
   int np_last = 0;                // pairs of the last step
   int *pf = nullptr, *pu = nullptr;         // [cap] finder and partner of each pair
-  int *queue = nullptr, *qn = nullptr;      // [cap] pairs that are not plainly apart, their count
+  // the narrow phase's work (pg_ttfilter.cuh): float copies of the triangles
+  // and their FP64 differences, the pairs that may touch with what decides
+  // them, the pairs that need every test, and the distances to take
+  float4 *fv = nullptr;           // [3][trinum] vertices relative to org; w of the first: error bound
+  double *geo = nullptr;          // [trinum][PG_TT_GEO] vertices, edges, squared edges, third minus first vertex
+  PgTTNear *near = nullptr;       // [cap]
+  int *full = nullptr;            // [cap]
+  unsigned *vit = nullptr, *eit = nullptr;  // [vcap], [ecap] near pair << 4 | candidate; vit then holds the region
+  double *vres = nullptr, *eres = nullptr;  // [.cap][3] squared distance and the closest points' parameters
+  int vcap = 0, ecap = 0;
+  int *qn = nullptr;              // [4] near pairs, full pairs, vertex-face and edge-edge distances
   unsigned char *act = nullptr;
   double *st[3] = {}, *f[3] = {}, *p[3] = {};   // tangential state, force on the finder's particle, point
   // the previous step's pairs (state carried by (finder, partner))

@@ -1102,9 +1102,7 @@ int tt_stage(pg_session *s, double step)
     const int cap = np + np / 2 + 1024;
     int *ppu = nullptr; unsigned char *pact = nullptr; double *pst[3] = {};
     int *pf = nullptr, *pu = nullptr; unsigned char *act = nullptr; double *st[3] = {}, *f[3] = {}, *p[3] = {};
-    int *queue = nullptr;
     TRY(dalloc(s, &pf, cap)); TRY(dalloc(s, &pu, cap)); TRY(dalloc(s, &act, cap)); TRY(dalloc(s, &ppu, cap));
-    TRY(dalloc(s, &queue, cap));
     TRY(dalloc(s, &pact, cap));
     for (int c = 0; c < 3; c ++)
     {
@@ -1118,14 +1116,23 @@ int tt_stage(pg_session *s, double step)
         CK(cudaMemcpyAsync(pst[c], g.pst[c], (size_t)g.cap * sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
     }
     CK(cudaStreamSynchronize(s->stream));
-    for (void *q : {(void *)g.pf, (void *)g.pu, (void *)g.act, (void *)g.ppu, (void *)g.pact, (void *)g.queue})
+    for (void *q : {(void *)g.pf, (void *)g.pu, (void *)g.act, (void *)g.ppu, (void *)g.pact, (void *)g.near,
+                    (void *)g.full, (void *)g.vit, (void *)g.eit, (void *)g.vres, (void *)g.eres})
       release(s, q);
     for (int c = 0; c < 3; c ++) for (void *q : {(void *)g.st[c], (void *)g.f[c], (void *)g.p[c], (void *)g.pst[c]}) release(s, q);
     release(s, g.ekeys[0]); release(s, g.ekeys[1]); release(s, g.evals[0]); release(s, g.evals[1]); release(s, g.ehist);
     TRY(dalloc(s, &g.ekeys[0], 2 * (size_t)cap)); TRY(dalloc(s, &g.ekeys[1], 2 * (size_t)cap));
     TRY(dalloc(s, &g.evals[0], 2 * (size_t)cap)); TRY(dalloc(s, &g.evals[1], 2 * (size_t)cap));
     TRY(dalloc(s, &g.ehist, pg_sort_hist_len(2 * cap)));
-    g.pf = pf; g.pu = pu; g.act = act; g.ppu = ppu; g.pact = pact; g.queue = queue;
+    // room for 2 vertex-triangle and 3 edge-edge distances a pair (the spring
+    // lattice, whose faces lie parallel, asks for 1.3 and 2.4); pairs beyond
+    // it take the whole narrow phase
+    g.vcap = (int)std::min(2LL * cap, 0x7fff0000LL);
+    g.ecap = (int)std::min(3LL * cap, 0x7fff0000LL);
+    TRY(dalloc(s, &g.near, cap)); TRY(dalloc(s, &g.full, cap));
+    TRY(dalloc(s, &g.vit, g.vcap)); TRY(dalloc(s, &g.eit, g.ecap));
+    TRY(dalloc(s, &g.vres, 3 * (size_t)g.vcap)); TRY(dalloc(s, &g.eres, 3 * (size_t)g.ecap));
+    g.pf = pf; g.pu = pu; g.act = act; g.ppu = ppu; g.pact = pact;
     for (int c = 0; c < 3; c ++) { g.st[c] = st[c]; g.f[c] = f[c]; g.p[c] = p[c]; g.pst[c] = pst[c]; }
     g.cap = cap;
   }
@@ -1690,7 +1697,9 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
     TRY(dalloc(s, &g.nch, P));
     TRY(dalloc(s, &g.choff, (size_t)P + 1));
     TRY(dalloc(s, &g.nchunks, 1));
-    TRY(dalloc(s, &g.qn, 1));
+    TRY(dalloc(s, &g.qn, 4));
+    TRY(dalloc(s, &g.fv, 3 * (size_t)T));
+    TRY(dalloc(s, &g.geo, (size_t)PG_TT_GEO * T));
     for (int c = 0; c < 3; c ++) { TRY(dalloc(s, &d.ttF[c], P)); TRY(dalloc(s, &d.ttT[c], P)); }
   }
   release(s, g.cstart);

@@ -81,8 +81,8 @@ PG_TT double clamp01(double x) { return x < 0.0 ? 0.0 : (x > 1.0 ? 1.0 : x); }
 // divides the same operands as the textbook branches do.
 // (ab = b - a and ac = c - a come with the triangle, computed once for the
 // three calls of a triangle pair that use them.)
-PG_TT void point_triangle(const double *p, const double *a, const double *b, const double *c,
-                          const double *ab, const double *ac, double *q)
+PG_TT int point_triangle_region(const double *p, const double *a, const double *b, const double *c,
+                                const double *ab, const double *ac, double *x0, double *x1)
 {
   double ap[3], bp[3], cp[3];
   sub(p, a, ap); sub(p, b, bp); sub(p, c, cp);
@@ -106,22 +106,36 @@ PG_TT void point_triangle(const double *p, const double *a, const double *b, con
   else if (region == 5) { num = e43; den = e43 + e56; }
   else if (region == 6) { num = 1.0; den = va + vb + vc; }
   const double x = num / den;
+  *x0 = region == 6 ? vb * x : x;
+  *x1 = region == 6 ? vc * x : 0.0;
+  return region;
+}
+
+// the point of a region: x0 along its edge, or x0 and x1 on the face
+PG_TT void point_triangle_at(int region, double x0, double x1, const double *a, const double *b, const double *c,
+                             const double *ab, const double *ac, double *q)
+{
   switch (region)
   {
   case 0: q[0] = a[0]; q[1] = a[1]; q[2] = a[2]; break;
   case 1: q[0] = b[0]; q[1] = b[1]; q[2] = b[2]; break;
   case 3: q[0] = c[0]; q[1] = c[1]; q[2] = c[2]; break;
-  case 2: q[0] = a[0] + x*ab[0]; q[1] = a[1] + x*ab[1]; q[2] = a[2] + x*ab[2]; break;
-  case 4: q[0] = a[0] + x*ac[0]; q[1] = a[1] + x*ac[1]; q[2] = a[2] + x*ac[2]; break;
-  case 5: q[0] = b[0] + x*(c[0]-b[0]); q[1] = b[1] + x*(c[1]-b[1]); q[2] = b[2] + x*(c[2]-b[2]); break;
+  case 2: q[0] = a[0] + x0*ab[0]; q[1] = a[1] + x0*ab[1]; q[2] = a[2] + x0*ab[2]; break;
+  case 4: q[0] = a[0] + x0*ac[0]; q[1] = a[1] + x0*ac[1]; q[2] = a[2] + x0*ac[2]; break;
+  case 5: q[0] = b[0] + x0*(c[0]-b[0]); q[1] = b[1] + x0*(c[1]-b[1]); q[2] = b[2] + x0*(c[2]-b[2]); break;
   default:
-  {
-    const double v = vb * x, w = vc * x;
-    q[0] = a[0] + ab[0]*v + ac[0]*w;
-    q[1] = a[1] + ab[1]*v + ac[1]*w;
-    q[2] = a[2] + ab[2]*v + ac[2]*w;
+    q[0] = a[0] + ab[0]*x0 + ac[0]*x1;
+    q[1] = a[1] + ab[1]*x0 + ac[1]*x1;
+    q[2] = a[2] + ab[2]*x0 + ac[2]*x1;
   }
-  }
+}
+
+PG_TT void point_triangle(const double *p, const double *a, const double *b, const double *c,
+                          const double *ab, const double *ac, double *q)
+{
+  double x0, x1;
+  const int region = point_triangle_region(p, a, b, c, ab, ac, &x0, &x1);
+  point_triangle_at(region, x0, x1, a, b, c, ab, ac, q);
 }
 
 // Closest points c1 on p1q1 and c2 on p2q2 (Ericson 5.1.9); returns |c1-c2|^2.
@@ -130,8 +144,8 @@ PG_TT void point_triangle(const double *p, const double *a, const double *b, con
 // numerator applies), so that threads of a warp share them.
 // (d1 = q1 - p1 and d2 = q2 - p2 come with the triangles' edges, a = d1.d1
 // and e = d2.d2 with them.)
-PG_TT double segment_segment(const double *p1, const double *d1, double a, const double *p2, const double *d2,
-                             double e, double *c1, double *c2)
+PG_TT void segment_params(const double *p1, const double *d1, double a, const double *p2, const double *d2,
+                          double e, double *ps, double *pt)
 {
   double r[3];
   sub(p1, p2, r);
@@ -158,9 +172,22 @@ PG_TT double segment_segment(const double *p1, const double *d1, double a, const
       }
     }
   }
-  c1[0] = p1[0] + d1[0]*s; c1[1] = p1[1] + d1[1]*s; c1[2] = p1[2] + d1[2]*s;
-  c2[0] = p2[0] + d2[0]*t; c2[1] = p2[1] + d2[1]*t; c2[2] = p2[2] + d2[2]*t;
-  double w[3];
+  *ps = s;
+  *pt = t;
+}
+
+PG_TT void segment_at(const double *p, const double *d, double s, double *c)
+{
+  c[0] = p[0] + d[0]*s; c[1] = p[1] + d[1]*s; c[2] = p[2] + d[2]*s;
+}
+
+PG_TT double segment_segment(const double *p1, const double *d1, double a, const double *p2, const double *d2,
+                             double e, double *c1, double *c2)
+{
+  double s, t, w[3];
+  segment_params(p1, d1, a, p2, d2, e, &s, &t);
+  segment_at(p1, d1, s, c1);
+  segment_at(p2, d2, t, c2);
   sub(c1, c2, w);
   return dot(w, w);
 }
@@ -277,20 +304,26 @@ PG_TT bool apart(const double *const a[3], const double *const b[3], double ra, 
   return beyond_plane(a, b, ra + rb) || beyond_plane(b, a, ra + rb);
 }
 
+// Depth, point and normal from the closest points of two triangles a
+// positive distance (squared: d2) apart
+PG_TT double contact_at(const double *pa, const double *pb, double d2, double ra, double rb, double *point,
+                        double *normal)
+{
+  point[0] = 0.5*(pa[0]+pb[0]); point[1] = 0.5*(pa[1]+pb[1]); point[2] = 0.5*(pa[2]+pb[2]);
+  const double d = sqrt(d2);
+  const double id = 1.0 / d;
+  normal[0] = (pa[0]-pb[0])*id; normal[1] = (pa[1]-pb[1])*id; normal[2] = (pa[2]-pb[2])*id;
+  return (ra + rb) - d;
+}
+
 // contact() for triangles that are not apart
 PG_TT double contact_near(const double *const a[3], const double *const b[3], double ra, double rb,
                           double *point, double *normal)
 {
   double pa[3], pb[3];
   const double d2 = triangle_triangle(a, b, pa, pb);
+  if (d2 > 0.0) return contact_at(pa, pb, d2, ra, rb, point, normal);
   point[0] = 0.5*(pa[0]+pb[0]); point[1] = 0.5*(pa[1]+pb[1]); point[2] = 0.5*(pa[2]+pb[2]);
-  if (d2 > 0.0)
-  {
-    const double d = sqrt(d2);
-    const double id = 1.0 / d;
-    normal[0] = (pa[0]-pb[0])*id; normal[1] = (pa[1]-pb[1])*id; normal[2] = (pa[2]-pb[2])*id;
-    return (ra + rb) - d;
-  }
   double e1[3], e2[3], n[3];
   sub(b[1], b[0], e1); sub(b[2], b[0], e2);
   cross(e1, e2, n);
