@@ -71,15 +71,15 @@ __device__ __forceinline__ unsigned long long hi_key(double x)
   return pgtt::nan_b(b) ? 0ULL : pgtt::okey(b);
 }
 
-// 1. boxes and cell keys
-__global__ void __launch_bounds__(TPB) k_tt_keys(PgDev d, PgTT g)
+// 1. every step: boxes, FP64 differences, float copies, and whether a vertex
+// coordinate moved by half the skin since the last search (a NaN did)
+__global__ void __launch_bounds__(TPB) k_tt_boxes(PgDev d, PgTT g)
 {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.trinum) return;
-  unsigned key = g.none;
-  if (mesh_tri(d, t))
+  bool moved = false;
+  if (t < d.trinum && mesh_tri(d, t))
   {
-    double lo[3], hi[3], v[3][3];
+    double v[3][3];
     tri_vertices(d, t, v);
     const double *vp[3] = {v[0], v[1], v[2]};
     pgtt::Tri T;
@@ -98,30 +98,63 @@ __global__ void __launch_bounds__(TPB) k_tt_keys(PgDev d, PgTT g)
       double l = a < b ? a : b, h = a > b ? a : b;
       l = l < e ? l : e;
       h = h > e ? h : e;
-      lo[c] = l - g.r;
-      hi[c] = h + g.r;
-      g.box[c][t] = lo_key(lo[c]);
-      g.box[3+c][t] = hi_key(hi[c]);
+      g.box[c][t] = lo_key(l - g.r);
+      g.box[3+c][t] = hi_key(h + g.r);
     }
-    if (g.big[t]) key = (unsigned)g.ncells;
+    const double lim = 0.4999 * g.skin;
+    for (int a = 0; a < 3; a ++)
+      for (int c = 0; c < 3; c ++) moved |= !(fabs(v[a][c] - g.ref[3*a + c][t]) <= lim);
+  }
+  if (__syncthreads_or(moved) && threadIdx.x == 0) g.moved[0] = 1;
+}
+
+// 2. a search: reference vertices, search boxes and cell keys
+__global__ void __launch_bounds__(TPB) k_tt_keys(PgDev d, PgTT g)
+{
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= d.trinum) return;
+  unsigned key = g.none;
+  PgTTBox bx;
+  bx.owner = -1;
+  bx.big = 0;
+  for (int c = 0; c < 3; c ++) bx.lo[c] = bx.hi[c] = 0.0f;
+  if (mesh_tri(d, t))
+  {
+    double v[3][3], mid[3];
+    tri_vertices(d, t, v);
+    const double w = g.r + 0.5 * g.skin;
+    for (int c = 0; c < 3; c ++)
+    {
+      const double a = v[0][c], b = v[1][c], e = v[2][c];
+      for (int k = 0; k < 3; k ++) g.ref[3*k + c][t] = v[k][c];
+      double l = a < b ? a : b, h = a > b ? a : b;
+      l = l < e ? l : e;
+      h = h > e ? h : e;
+      mid[c] = 0.5*((l - g.r) + (h + g.r));
+      bx.lo[c] = __double2float_rd(l - w);
+      bx.hi[c] = __double2float_ru(h + w);
+    }
+    bx.owner = d.triobs[t];
+    bx.big = g.big[t];
+    if (bx.big) key = (unsigned)g.ncells;
     else
     {
       int ix[3];
       for (int c = 0; c < 3; c ++)
       {
-        const double q = floor((0.5*(lo[c] + hi[c]) - g.org[c]) / g.h);
-        int k = q < 0.0 ? 0 : (q > (double)(g.dim[c]-1) ? g.dim[c]-1 : (int)q);
-        ix[c] = k;
+        const double q = floor((mid[c] - g.org[c]) / g.h);
+        ix[c] = q < 0.0 ? 0 : (q > (double)(g.dim[c]-1) ? g.dim[c]-1 : (int)q);
       }
       key = (unsigned)((ix[2]*g.dim[1] + ix[1])*g.dim[0] + ix[0]);
     }
     g.cell[t] = (int)key;
   }
+  g.sbox[t] = bx;
   g.keys[0][t] = key;
   g.vals[0][t] = t;
 }
 
-// 2. cell ranges over the sorted keys
+// cell ranges over the sorted keys
 __global__ void __launch_bounds__(TPB) k_tt_ranges(PgTT g, int n)
 {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -132,59 +165,103 @@ __global__ void __launch_bounds__(TPB) k_tt_ranges(PgTT g, int n)
   if (k == n-1 || g.keys[0][k+1] != key) g.cend[key] = k + 1;
 }
 
-// 3. partners found by triangle t, sorted by index, in cand[slot][t]
-// (sorted in a thread-local array, written once)
+// 3. partners found by triangle t, sorted by index: counted (FILL false), or
+// written to the pair list with the state carried from the previous one.
+// One warp per triangle: the lanes take the ranges of the 27 cells around
+// its own and the big range, then test 32 candidates at a time, so that 32
+// loads are in flight where one thread a triangle followed one chain of them
+// (231 us a search on 3,000 triangles, all of it latency).
+template <bool FILL>
 __global__ void __launch_bounds__(TPB) k_tt_find(PgDev d, PgTT g)
 {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr unsigned all = 0xffffffffu;
+  __shared__ int lists[TPB / 32][PG_TT_KMAX];
+  const int lane = threadIdx.x & 31;
+  int *list = lists[threadIdx.x >> 5];
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= d.trinum) return;
+  const PgTTBox me = g.sbox[t];
   int cnt = 0;
-  int loc[PG_TT_KMAX];
-  if (mesh_tri(d, t))
+  if (me.owner >= 0)
   {
-    const int owner = d.triobs[t];
-    const bool big = g.big[t] != 0;
-    unsigned long long lo[3], hi[3];
-    for (int c = 0; c < 3; c ++) { lo[c] = g.box[c][t]; hi[c] = g.box[3+c][t]; }
-    auto take = [&](int u) {
-      if (u == t || !mesh_tri(d, u) || d.triobs[u] == owner) return;
-      const bool ubig = g.big[u] != 0;
-      if (big && !ubig) return;                       // found from the small side
-      if (big == ubig && u < t) return;               // found by the lower index
-      for (int c = 0; c < 3; c ++)
-        if (!(lo[c] < g.box[3+c][u] && g.box[c][u] < hi[c])) return;
-      if (cnt >= g.kmax) { pgk::set_err(d, PG_ERR_CAPACITY, 40, t, cnt); return; }
-      // insertion in index order
-      int k = cnt ++;
-      while (k > 0 && loc[k-1] > u) { loc[k] = loc[k-1]; k --; }
-      loc[k] = u;
-    };
-    if (!big)
+    // this lane's range of sorted triangles
+    int b = 0, n = 0;
+    if (lane < 27 && !me.big)
     {
       const int cell = g.cell[t];
-      const int ix[3] = {cell % g.dim[0], (cell / g.dim[0]) % g.dim[1], cell / (g.dim[0] * g.dim[1])};
-      for (int z = ix[2]-1; z <= ix[2]+1; z ++)
+      const int x = cell % g.dim[0] + lane % 3 - 1, y = (cell / g.dim[0]) % g.dim[1] + lane / 3 % 3 - 1;
+      const int z = cell / (g.dim[0] * g.dim[1]) + lane / 9 - 1;
+      if (x >= 0 && y >= 0 && z >= 0 && x < g.dim[0] && y < g.dim[1] && z < g.dim[2])
       {
-        if (z < 0 || z >= g.dim[2]) continue;
-        for (int y = ix[1]-1; y <= ix[1]+1; y ++)
-        {
-          if (y < 0 || y >= g.dim[1]) continue;
-          for (int x = ix[0]-1; x <= ix[0]+1; x ++)
-          {
-            if (x < 0 || x >= g.dim[0]) continue;
-            const int cell = (z*g.dim[1] + y)*g.dim[0] + x;
-            for (int k = g.cstart[cell]; k < g.cend[cell]; k ++) take(g.vals[0][k]);
-          }
-        }
+        const int c = (z*g.dim[1] + y)*g.dim[0] + x;
+        b = g.cstart[c];
+        n = g.cend[c] - b;
       }
     }
-    for (int k = g.cstart[g.ncells]; k < g.cend[g.ncells]; k ++) take(g.vals[0][k]);
+    if (lane == 27) { b = g.cstart[g.ncells]; n = g.cend[g.ncells] - b; }
+    int upto = n;                                        // inclusive sums of the ranges' lengths
+    for (int o = 1; o < 32; o <<= 1)
+    {
+      const int v = __shfl_up_sync(all, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const int total = __shfl_sync(all, upto, 31);
+    for (int q0 = 0; q0 < total; q0 += 32)
+    {
+      const int q = q0 + lane;
+      int lo = 0;                                        // the first range that ends beyond q
+      for (int o = 16; o > 0; o >>= 1) if (__shfl_sync(all, upto, lo + o - 1) <= q) lo += o;
+      lo = lo < 31 ? lo : 31;
+      const int k = __shfl_sync(all, b, lo) + q - (__shfl_sync(all, upto, lo) - __shfl_sync(all, n, lo));
+      bool hit = false;
+      int u = 0;
+      if (q < total)
+      {
+        u = g.vals[0][k];
+        const PgTTBox o = g.sbox[u];
+        hit = u != t && o.owner != me.owner && (me.big == o.big ? u > t : !me.big);
+        for (int c = 0; c < 3; c ++) hit = hit && me.lo[c] < o.hi[c] && o.lo[c] < me.hi[c];
+      }
+      const unsigned m = __ballot_sync(all, hit);
+      const int at = cnt + __popc(m & ((1u << lane) - 1u));
+      if (hit && at < PG_TT_KMAX) list[at] = u;
+      cnt += __popc(m);
+    }
+    if (cnt > PG_TT_KMAX)
+    {
+      if (lane == 0) pgk::set_err(d, PG_ERR_CAPACITY, 40, t, cnt);
+      cnt = PG_TT_KMAX;
+    }
   }
-  for (int k = 0; k < cnt; k ++) g.cand[(size_t)k * d.trinum + t] = loc[k];
-  g.cnt[t] = cnt;
+  if (!FILL)
+  {
+    if (lane == 0) g.cnt[t] = cnt;
+    return;
+  }
+  __syncwarp();
+  const int o = g.off[t], pb = g.poff[t], pe = g.poff[t+1];
+  for (int a = lane; a < cnt; a += 32)
+  {
+    const int u = list[a];
+    int rank = 0;
+    for (int c = 0; c < cnt; c ++) rank += list[c] < u;
+    const int k = o + rank;
+    g.pf[k] = t;
+    g.pu[k] = u;
+    int lo = pb, hi = pe;
+    while (lo < hi)
+    {
+      const int mid = (lo + hi) >> 1;
+      if (g.ppu[mid] < u) lo = mid + 1;
+      else hi = mid;
+    }
+    const bool kept = lo < pe && g.ppu[lo] == u && g.pact[lo];
+    g.act[k] = kept;
+    for (int c = 0; c < 3; c ++) g.st[c][k] = kept ? g.pst[c][lo] : 0.0;
+  }
 }
 
-// 4a. exclusive scan of the counts in one block (off[n] = total)
+// 4. exclusive scan of the counts in one block (off[n] = total)
 __global__ void __launch_bounds__(1024) k_tt_scan(const int *in, int *out, int n, int *total)
 {
   __shared__ int part[1024];
@@ -195,29 +272,33 @@ __global__ void __launch_bounds__(1024) k_tt_scan(const int *in, int *out, int n
   for (int i = b; i < e; i ++) s += in[i];
   part[tid] = s;
   __syncthreads();
-  if (tid == 0)
+  for (int o = 1; o < 1024; o <<= 1)
   {
-    int acc = 0;
-    for (int k = 0; k < 1024; k ++) { const int v = part[k]; part[k] = acc; acc += v; }
-    out[n] = acc;
-    *total = acc;
+    const int v = tid >= o ? part[tid - o] : 0;
+    __syncthreads();
+    part[tid] += v;
+    __syncthreads();
   }
-  __syncthreads();
-  int acc = part[tid];
-  for (int i = b; i < e; i ++) { out[i] = acc; acc += in[i]; }
+  int acc = tid ? part[tid - 1] : 0;
+  for (int i = b; i < e; i ++) { const int v = in[i]; out[i] = acc; acc += v; }
+  if (tid == 1023) { out[n] = part[1023]; *total = part[1023]; }
 }
 
-// 4b. the pair list in finder order
-__global__ void __launch_bounds__(TPB) k_tt_emit(PgDev d, PgTT g)
+// the boxes of pair k overlap with positive measure this step
+__device__ __forceinline__ bool boxes_overlap(const PgTT &g, int f, int u)
 {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.trinum) return;
-  const int o = g.off[t], c = g.cnt[t];
-  for (int k = 0; k < c; k ++)
-  {
-    g.pf[o + k] = t;
-    g.pu[o + k] = g.cand[(size_t)k * d.trinum + t];
-  }
+  bool in = true;
+  for (int c = 0; c < 3; c ++) in = in && g.box[c][f] < g.box[3+c][u] && g.box[c][u] < g.box[3+c][f];
+  return in;
+}
+
+// overlapping and active pairs of the last step
+__global__ void __launch_bounds__(TPB) k_tt_counts(PgTT g, int *out2)
+{
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = __syncthreads_count(k < g.np && boxes_overlap(g, g.pf[k], g.pu[k]));
+  const int b = __syncthreads_count(k < g.np && g.act[k]);
+  if (threadIdx.x == 0) { atomicAdd(out2, a); atomicAdd(out2 + 1, b); }
 }
 
 // 5a. what each pair needs, in FP32 (pg_ttfilter.cuh): the pairs farther
@@ -241,13 +322,13 @@ __device__ __forceinline__ int warp_take(int *count, int n)
   return base + s - n;
 }
 
-__global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g, int np)
+__global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g)
 {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   int verdict = pgtf::APART;
   unsigned mask = 0;
   float upper = 0.0f, size = 0.0f;
-  if (k < np)
+  if (k < g.np)
   {
     const int f = g.pf[k], u = g.pu[k];
     const size_t T = d.trinum;
@@ -260,6 +341,8 @@ __global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g, int np)
       if (v == 0) { ea = x.w; eb = y.w; }
     }
     verdict = pgtf::judge(a, b, ea, eb, (float)(g.r + g.r), &mask, &upper, &size);
+    // (a pair whose boxes no longer overlap holds no contact)
+    if (verdict != pgtf::APART && !boxes_overlap(g, f, u)) verdict = pgtf::APART;
     if (verdict == pgtf::APART) g.act[k] = 0;
   }
   int nv = verdict == pgtf::NEAR ? __popc(mask & 63u) : 0, ne = verdict == pgtf::NEAR ? __popc(mask >> 6) : 0;
@@ -336,21 +419,11 @@ __global__ void __launch_bounds__(TPB) k_tt_edge_edge(PgTT g)
 __device__ __forceinline__ void tt_force(const PgDev &d, const PgTT &g, int k, int f, int u, double depth,
                                          const double *point, const double *normal, double step)
 {
-  const bool active = depth > 0.0;
+  const bool active = depth > 0.0, was = g.act[k] != 0;
   g.act[k] = active ? 1 : 0;
   if (!active) return;
-  double st[3] = {0.0, 0.0, 0.0}, fr[3];
-  // the pair's state of the previous step: (finder, partner) in its list
-  int lo = g.poff[f], hi = g.poff[f+1];
-  const int end = hi;
-  while (lo < hi)
-  {
-    const int mid = (lo + hi) >> 1;
-    if (g.ppu[mid] < u) lo = mid + 1;
-    else hi = mid;
-  }
-  if (lo < end && g.ppu[lo] == u && g.pact[lo])
-    for (int c = 0; c < 3; c ++) st[c] = g.pst[c][lo];
+  double st[3], fr[3];
+  for (int c = 0; c < 3; c ++) st[c] = was ? g.st[c][k] : 0.0;
   const int pa = d.triobs[f], pb = d.triobs[u];
   // contact point velocities (forces.ispc:226-246) and their difference
   double vij[3];
@@ -463,97 +536,189 @@ int resident_blocks(K k)
   return (sms > 0 ? sms : 152) * (per > 0 ? per : 4);
 }
 
-// 6a. two entries per pair, keyed by particle (inactive: the sentinel)
-__global__ void __launch_bounds__(TPB) k_tt_entries(PgDev d, PgTT g, int np)
+// 6a. with the list: two entries per pair, keyed by particle
+__global__ void __launch_bounds__(TPB) k_tt_entries(PgDev d, PgTT g)
 {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= np) return;
-  const bool on = g.act[k] != 0;
-  g.ekeys[0][2*k] = on ? (unsigned)d.triobs[g.pf[k]] : g.enone;
-  g.ekeys[0][2*k+1] = on ? (unsigned)d.triobs[g.pu[k]] : g.enone;
+  if (k >= g.np) return;
+  g.ekeys[0][2*k] = (unsigned)d.triobs[g.pf[k]];
+  g.ekeys[0][2*k+1] = (unsigned)d.triobs[g.pu[k]];
   g.evals[0][2*k] = 2*k;
   g.evals[0][2*k+1] = 2*k + 1;
 }
 
-// 6b. each particle's range of the sorted entries
+// particles with more than PG_TT_CHUNK entries, from their ranges of the
+// sorted entries (pfirst and plast, for now)
 __global__ void __launch_bounds__(TPB) k_tt_segments(PgTT g, int n)
 {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const unsigned key = g.ekeys[0][k];
-  if (key == g.enone) return;
   if (k == 0 || g.ekeys[0][k-1] != key) g.pfirst[key] = k;
   if (k == n-1 || g.ekeys[0][k+1] != key) g.plast[key] = k + 1;
 }
 
-// 6c. chunks per particle
-__global__ void __launch_bounds__(TPB) k_tt_chunks(PgDev d, PgTT g)
+__global__ void __launch_bounds__(TPB) k_tt_big(PgDev d, PgTT g)
 {
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= d.parnum) return;
-  g.nch[w] = (g.plast[w] - g.pfirst[w] + PG_TT_CHUNK - 1) / PG_TT_CHUNK;
+  const int n = g.plast[w] - g.pfirst[w];
+  if (n <= PG_TT_CHUNK) return;
+  const int b = atomicAdd(g.moved + 2, 1);
+  g.bigp[b] = w;
+  g.bigoff[b] = atomicAdd(g.moved + 3, (n + PG_TT_CHUNK - 1) / PG_TT_CHUNK);
 }
 
-// 6d. one warp per chunk: lane sums over entries lane, lane+32, ... of the
-// chunk, then the lane sums in lane order
-__global__ void __launch_bounds__(TPB) k_tt_chunk_sums(PgDev d, PgTT g)
+// which big particle a chunk belongs to (one block per big particle)
+__global__ void __launch_bounds__(TPB) k_tt_chmap(PgTT g)
 {
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  const bool on = c < *g.nchunks;
-  int w = 0;
-  if (on)
+  const int b = blockIdx.x, w = g.bigp[b];
+  const int nc = (g.plast[w] - g.pfirst[w] + PG_TT_CHUNK - 1) / PG_TT_CHUNK;
+  for (int c = threadIdx.x; c < nc; c += blockDim.x) g.chmap[g.bigoff[b] + c] = b;
+}
+
+// 6b. every step: the active entries in their order: one bit per entry and
+// their number per tile, the scan of the tiles, the selection
+constexpr int TILE_THREADS = 256;
+
+__global__ void __launch_bounds__(TILE_THREADS) k_tt_active(PgTT g)
+{
+  __shared__ int sum;
+  if (threadIdx.x == 0) sum = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, n = 2 * g.np;
+  for (int it = 0; it < PG_TT_TILE / TILE_THREADS; it ++)
   {
-    // the particle whose chunks hold c: the last w with choff[w] <= c
-    int lo = 0, hi = d.parnum - 1;
-    while (lo < hi)
+    const int e = blockIdx.x * PG_TT_TILE + it * TILE_THREADS + threadIdx.x;
+    const unsigned m = __ballot_sync(0xffffffffu, e < n && g.act[g.evals[0][e] >> 1] != 0);
+    if (lane == 0)
     {
-      const int mid = (lo + hi + 1) >> 1;
-      if (g.choff[mid] <= c) lo = mid;
-      else hi = mid - 1;
-    }
-    w = lo;
-  }
-  double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  if (on)
-  {
-    const int b = g.pfirst[w] + (c - g.choff[w]) * PG_TT_CHUNK;
-    const int e = min(b + PG_TT_CHUNK, g.plast[w]);
-    const double x[3] = {d.position[0][w], d.position[1][w], d.position[2][w]};
-    for (int q = b + lane; q < e; q += 32)
-    {
-      const int v = g.evals[0][q];
-      const int k = v >> 1;
-      double f[3] = {g.f[0][k], g.f[1][k], g.f[2][k]};
-      if (v & 1) { f[0] = -f[0]; f[1] = -f[1]; f[2] = -f[2]; }
-      const double a[3] = {g.p[0][k]-x[0], g.p[1][k]-x[1], g.p[2][k]-x[2]};
-      s[0] += f[0]; s[1] += f[1]; s[2] += f[2];
-      s[3] += a[1]*f[2] - a[2]*f[1];
-      s[4] += a[2]*f[0] - a[0]*f[2];
-      s[5] += a[0]*f[1] - a[1]*f[0];
+      g.ebits[e >> 5] = m;
+      atomicAdd(&sum, __popc(m));
     }
   }
-  __shared__ double part[TPB / 32][32][6];
-  const int wl = threadIdx.x >> 5;
-  for (int k = 0; k < 6; k ++) part[wl][lane][k] = s[k];
-  __syncwarp();
-  if (on && lane == 0)
+  __syncthreads();
+  if (threadIdx.x == 0) g.etile[blockIdx.x] = sum;
+}
+
+__global__ void __launch_bounds__(1024) k_tt_tiles(PgTT g, int tiles)
+{
+  __shared__ int part[1024];
+  pgk::block_scan_seq(g.etile, tiles, part);
+}
+
+__global__ void __launch_bounds__(TILE_THREADS) k_tt_select(PgTT g)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = 2 * g.np;
+  // the tile's 32 words, one a lane: active entries before each
+  const unsigned word = g.ebits[blockIdx.x * (PG_TT_TILE / 32) + lane];
+  int before = __popc(word);
+  for (int o = 1; o < 32; o <<= 1)
   {
-    double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int L = 0; L < 32; L ++)
-      for (int k = 0; k < 6; k ++) acc[k] += part[wl][L][k];
-    for (int k = 0; k < 6; k ++) g.csum[k][c] = acc[k];
+    const int v = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += v;
+  }
+  before += g.etile[blockIdx.x] - __popc(word);
+  for (int it = 0; it < PG_TT_TILE / TILE_THREADS; it ++)
+  {
+    const int wd = it * (TILE_THREADS / 32) + warp;
+    const int e = blockIdx.x * PG_TT_TILE + wd * 32 + lane;
+    const unsigned m = __shfl_sync(0xffffffffu, word, wd);
+    const int rank = __shfl_sync(0xffffffffu, before, wd) + __popc(m & ((1u << lane) - 1u));
+    if (e >= n) continue;
+    const int on = m >> lane & 1u;
+    const unsigned p = g.ekeys[0][e];
+    if (on) g.elist[rank] = g.evals[0][e];
+    if (e == 0 || g.ekeys[0][e-1] != p) g.pfirst[p] = rank;
+    if (e == n-1 || g.ekeys[0][e+1] != p) g.plast[p] = rank + on;
   }
 }
 
-// 6e. one thread per particle: its chunk sums in chunk order
+// 6c. sums of entries [b, e) of elist, e - b <= PG_TT_CHUNK, by one warp: lane
+// sums over entries lane, lane+32, ..., then the lane sums in lane order, the
+// six components by a lane each; the totals in s of lanes 0 to 5.  Four
+// entries' loads are issued before the first is added.
+__device__ __forceinline__ double chunk_sum(const PgTT &g, const double *x, int b, int e, double (*part)[6])
+{
+  const int lane = threadIdx.x & 31;
+  double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int q0 = b + lane; q0 < e; q0 += 128)
+  {
+    double f[4][3], p[4][3];
+    int v[4];
+    #pragma unroll
+    for (int j = 0; j < 4; j ++) v[j] = q0 + 32*j < e ? g.elist[q0 + 32*j] : -1;
+    #pragma unroll
+    for (int j = 0; j < 4; j ++)
+    {
+      const int k = v[j] >= 0 ? v[j] >> 1 : 0;
+      for (int c = 0; c < 3; c ++) { f[j][c] = g.f[c][k]; p[j][c] = g.p[c][k]; }
+    }
+    #pragma unroll
+    for (int j = 0; j < 4; j ++)
+    {
+      if (v[j] < 0) break;
+      if (v[j] & 1) { f[j][0] = -f[j][0]; f[j][1] = -f[j][1]; f[j][2] = -f[j][2]; }
+      const double a[3] = {p[j][0]-x[0], p[j][1]-x[1], p[j][2]-x[2]};
+      s[0] += f[j][0]; s[1] += f[j][1]; s[2] += f[j][2];
+      s[3] += a[1]*f[j][2] - a[2]*f[j][1];
+      s[4] += a[2]*f[j][0] - a[0]*f[j][2];
+      s[5] += a[0]*f[j][1] - a[1]*f[j][0];
+    }
+  }
+  for (int k = 0; k < 6; k ++) part[lane][k] = s[k];
+  __syncwarp();
+  double acc = 0.0;
+  if (lane < 6) for (int L = 0; L < 32; L ++) acc += part[L][lane];
+  return acc;
+}
+
+// one warp per particle of at most one chunk of active entries
 __global__ void __launch_bounds__(TPB) k_tt_sums(PgDev d, PgTT g)
 {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double part[TPB / 32][32][6];
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= d.parnum) return;
-  double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int c = g.choff[w]; c < g.choff[w+1]; c ++)
-    for (int k = 0; k < 6; k ++) acc[k] += g.csum[k][c];
-  for (int k = 0; k < 3; k ++) { d.ttF[k][w] = acc[k]; d.ttT[k][w] = acc[3+k]; }
+  const int b = g.pfirst[w], e = g.plast[w];
+  if (e - b > PG_TT_CHUNK) return;
+  double acc = 0.0;
+  if (e > b)
+  {
+    const double x[3] = {d.position[0][w], d.position[1][w], d.position[2][w]};
+    acc += chunk_sum(g, x, b, e, part[threadIdx.x >> 5]);
+  }
+  if (lane < 3) d.ttF[lane][w] = acc;
+  else if (lane < 6) d.ttT[lane - 3][w] = acc;
+}
+
+// the others: one warp per chunk, then one thread per component, the chunk
+// sums in chunk order
+__global__ void __launch_bounds__(TPB) k_tt_chunk_sums(PgDev d, PgTT g)
+{
+  __shared__ double part[TPB / 32][32][6];
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (c >= g.nchunks) return;
+  const int q = g.chmap[c], w = g.bigp[q];
+  const int b = g.pfirst[w] + (c - g.bigoff[q]) * PG_TT_CHUNK, e = min(b + PG_TT_CHUNK, g.plast[w]);
+  if (b >= e) return;
+  const double x[3] = {d.position[0][w], d.position[1][w], d.position[2][w]};
+  const double acc = chunk_sum(g, x, b, e, part[threadIdx.x >> 5]);
+  if (lane < 6) g.csum[lane][c] = acc;
+}
+
+__global__ void __launch_bounds__(TPB) k_tt_totals(PgDev d, PgTT g)
+{
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) / 6, k = (blockIdx.x * blockDim.x + threadIdx.x) % 6;
+  if (q >= g.nbig) return;
+  const int w = g.bigp[q], n = g.plast[w] - g.pfirst[w];
+  if (n <= PG_TT_CHUNK) return;
+  const double *s = g.csum[k] + g.bigoff[q];
+  const int nc = (n + PG_TT_CHUNK - 1) / PG_TT_CHUNK;
+  double acc = 0.0;
+  #pragma unroll 8
+  for (int c = 0; c < nc; c ++) acc += s[c];
+  if (k < 3) d.ttF[k][w] = acc;
+  else d.ttT[k - 3][w] = acc;
 }
 
 } // namespace
@@ -565,7 +730,14 @@ int pg_tt_key_bits(int ncells)
   return b;
 }
 
-void pg_tt_find(const PgDev &d, PgTT &g, cudaStream_t s)
+void pg_tt_prepare(const PgDev &d, PgTT &g, cudaStream_t s)
+{
+  if (d.trinum <= 0) return;
+  cudaMemsetAsync(g.moved, 0, 4 * sizeof(int), s);
+  k_tt_boxes<<<nblk(d.trinum), TPB, 0, s>>>(d, g);
+}
+
+void pg_tt_search(const PgDev &d, PgTT &g, cudaStream_t s)
 {
   const int T = d.trinum;
   if (T <= 0) return;
@@ -574,46 +746,64 @@ void pg_tt_find(const PgDev &d, PgTT &g, cudaStream_t s)
   cudaMemsetAsync(g.cstart, 0, (size_t)(g.ncells + 1) * sizeof(int), s);
   cudaMemsetAsync(g.cend, 0, (size_t)(g.ncells + 1) * sizeof(int), s);
   k_tt_ranges<<<nblk(T), TPB, 0, s>>>(g, T);
-  k_tt_find<<<nblk(T), TPB, 0, s>>>(d, g);
-  k_tt_scan<<<1, 1024, 0, s>>>(g.cnt, g.off, T, g.np_dev);
+  k_tt_find<false><<<nblk(32LL * T), TPB, 0, s>>>(d, g);
+  k_tt_scan<<<1, 1024, 0, s>>>(g.cnt, g.off, T, g.moved + 1);
 }
 
-void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, int np, double step)
+void pg_tt_list(const PgDev &d, PgTT &g, cudaStream_t s)
 {
-  const int T = d.trinum;
-  if (np > 0)
+  cudaMemsetAsync(g.pfirst, 0, (size_t)d.parnum * sizeof(int), s);
+  cudaMemsetAsync(g.plast, 0, (size_t)d.parnum * sizeof(int), s);
+  if (g.np <= 0) return;
+  k_tt_find<true><<<nblk(32LL * d.trinum), TPB, 0, s>>>(d, g);
+  k_tt_entries<<<nblk(g.np), TPB, 0, s>>>(d, g);
+  pg_launch_radix_sort(g.ekeys[0], g.evals[0], g.ekeys[1], g.evals[1], g.ehist, 2 * g.np, g.epasses, nullptr, s);
+  k_tt_segments<<<nblk(2LL * g.np), TPB, 0, s>>>(g, 2 * g.np);
+  k_tt_big<<<nblk(d.parnum), TPB, 0, s>>>(d, g);
+}
+
+void pg_tt_chunk_map(PgTT &g, cudaStream_t s)
+{
+  if (g.nbig > 0) k_tt_chmap<<<g.nbig, TPB, 0, s>>>(g);
+}
+
+void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, double step)
+{
+  if (g.np > 0)
   {
-    k_tt_emit<<<nblk(T), TPB, 0, s>>>(d, g);
     static const int bv = resident_blocks(k_tt_vertex_face), be = resident_blocks(k_tt_edge_edge),
                      bn = resident_blocks(k_tt_near), bf = resident_blocks(k_tt_full);
     auto upto = [](int most, long long n) { const int b = nblk(n); return b < most ? b : most; };
+    const int tiles = (2 * g.np + PG_TT_TILE - 1) / PG_TT_TILE;
     cudaMemsetAsync(g.qn, 0, 4 * sizeof(int), s);
-    k_tt_judge<<<nblk(np), TPB, 0, s>>>(d, g, np);
-    k_tt_vertex_face<<<upto(bv, 6LL * np), TPB, 0, s>>>(g);
-    k_tt_edge_edge<<<upto(be, 9LL * np), TPB, 0, s>>>(g);
-    k_tt_near<<<upto(bn, np), TPB, 0, s>>>(d, g, step);
-    k_tt_full<<<upto(bf, np), TPB, 0, s>>>(d, g, step);
-    k_tt_entries<<<nblk(np), TPB, 0, s>>>(d, g, np);
-    pg_launch_radix_sort(g.ekeys[0], g.evals[0], g.ekeys[1], g.evals[1], g.ehist, 2*np, g.epasses, nullptr, s);
+    k_tt_judge<<<nblk(g.np), TPB, 0, s>>>(d, g);
+    k_tt_vertex_face<<<upto(bv, 6LL * g.np), TPB, 0, s>>>(g);
+    k_tt_edge_edge<<<upto(be, 9LL * g.np), TPB, 0, s>>>(g);
+    k_tt_near<<<upto(bn, g.np), TPB, 0, s>>>(d, g, step);
+    k_tt_full<<<upto(bf, g.np), TPB, 0, s>>>(d, g, step);
+    k_tt_active<<<tiles, TILE_THREADS, 0, s>>>(g);
+    k_tt_tiles<<<1, 1024, 0, s>>>(g, tiles);
+    k_tt_select<<<tiles, TILE_THREADS, 0, s>>>(g);
   }
-  cudaMemsetAsync(g.pfirst, 0, (size_t)d.parnum * sizeof(int), s);
-  cudaMemsetAsync(g.plast, 0, (size_t)d.parnum * sizeof(int), s);
-  if (np > 0) k_tt_segments<<<nblk(2*(long long)np), TPB, 0, s>>>(g, 2*np);
-  k_tt_chunks<<<nblk(d.parnum), TPB, 0, s>>>(d, g);
-  k_tt_scan<<<1, 1024, 0, s>>>(g.nch, g.choff, d.parnum, g.nchunks);
-  k_tt_chunk_sums<<<nblk(32LL * pg_tt_max_chunks(d.parnum, np)), TPB, 0, s>>>(d, g);
-  k_tt_sums<<<nblk(d.parnum), TPB, 0, s>>>(d, g);
+  k_tt_sums<<<nblk(32LL * d.parnum), TPB, 0, s>>>(d, g);
+  if (g.nbig > 0)
+  {
+    k_tt_chunk_sums<<<nblk(32LL * g.nchunks), TPB, 0, s>>>(d, g);
+    k_tt_totals<<<nblk(6LL * g.nbig), TPB, 0, s>>>(d, g);
+  }
 }
 
-long long pg_tt_max_chunks(int parnum, int np)
+void pg_tt_count(const PgDev &d, const PgTT &g, int *out2, cudaStream_t s)
 {
-  // each particle's entries fill its chunks but the last: at most parnum
-  // partial chunks beside 2 np / PG_TT_CHUNK full ones
-  return (long long)parnum + (2LL * np) / PG_TT_CHUNK + 1;
+  cudaMemsetAsync(out2, 0, 2 * sizeof(int), s);
+  if (d.trinum > 0 && g.np > 0) k_tt_counts<<<nblk(g.np), TPB, 0, s>>>(g, out2);
 }
 
-// kernels of one step's mesh-contact stage
-int pg_tt_kernel_count(const PgTT &g, int trinum, int np)
+// kernels of a search and its list, and of one step's contacts and sums
+int pg_tt_search_kernels(const PgTT &g, int trinum)
 {
-  return 5 + pg_sort_kernel_count(trinum, g.passes) + (np > 0 ? 8 + pg_sort_kernel_count(2 * np, g.epasses) : 0) + 4;
+  return 4 + pg_sort_kernel_count(trinum, g.passes) +
+         (g.np > 0 ? 4 + pg_sort_kernel_count(2 * g.np, g.epasses) + (g.nbig > 0 ? 1 : 0) : 0);
 }
+
+int pg_tt_step_kernels(const PgTT &g) { return 2 + (g.np > 0 ? 8 : 0) + (g.nbig > 0 ? 2 : 0); }

@@ -5,34 +5,42 @@
 #include <cuda_runtime.h>
 #include "pg_state.h"
 
-#define PG_TT_KMAX 64             // partners one triangle may find (the search's thread-local list)
+#define PG_TT_KMAX 256            // partners one triangle may find (a warp's list in the search)
 
 // a pair whose contact a few distances decide: candidates (bits as in
 // pgtf::judge), where their results start, a bound on the smallest
 struct PgTTNear { int pair; unsigned mask; int vbase, ebase; float upper, size; };
 #define PG_TT_GEO 24
 
+// a triangle's box at a search, widened by r and half the skin (rounded
+// outwards), its particle (-1: not of a mesh) and whether it is big
+struct PgTTBox { float lo[3], hi[3]; int owner, big; };
+
 struct PgTT
 {
   double r = 0.0;                 // swept radius of every mesh triangle
   double h = 0.0, org[3] = {0, 0, 0};
   int dim[3] = {1, 1, 1}, ncells = 1;
-  unsigned none = 0, enone = 0;   // sentinel keys (above every cell / particle)
+  unsigned none = 0;              // sentinel key (above every cell)
   int passes = 2, epasses = 2;    // radix-sort passes of the two sorts
-  int kmax = PG_TT_KMAX;          // partners one triangle may find
   unsigned char *big = nullptr;   // [trinum] 1: larger than a cell
-  // [trinum] box widened by r, as keys whose unsigned order is the IEEE
-  // order of the coordinates (-0 = +0): min xyz (NaN: above every key),
-  // max xyz (NaN: 0), so that a NaN fails every overlap test
+  // [trinum] this step's box widened by r, as keys whose unsigned order is
+  // the IEEE order of the coordinates (-0 = +0): min xyz (NaN: above every
+  // key), max xyz (NaN: 0), so that a NaN fails every overlap test
   unsigned long long *box[6] = {};
+  // the pair list: every pair of triangles whose boxes, widened by half the
+  // skin, overlapped at the last search, in (finder, partner) order; valid
+  // while no vertex coordinate has moved by half the skin since
+  double skin = 0.0;
+  int valid = 0;
+  int *moved = nullptr;           // [4]: a vertex moved, pairs found, big particles, their chunks
+  double *ref[9] = {};            // [trinum] vertices at the last search
+  PgTTBox *sbox = nullptr;        // [trinum] search boxes
   int *cell = nullptr;            // [trinum] grid cell of a small triangle's box centre
   unsigned *keys[2] = {}; int *vals[2] = {}; unsigned *hist = nullptr;
   int *cstart = nullptr, *cend = nullptr;   // [ncells + 1]: the last range holds the big triangles
-  int *cand = nullptr;            // [kmax][trinum] partners found, sorted
   int *cnt = nullptr, *off = nullptr;       // [trinum], [trinum + 1]
-  int *np_dev = nullptr;          // pairs of this step
-  int cap = 0;                    // pair capacity
-  int np_last = 0;                // pairs of the last step
+  int cap = 0, np = 0;            // pair capacity and pairs
   int *pf = nullptr, *pu = nullptr;         // [cap] finder and partner of each pair
   // the narrow phase's work (pg_ttfilter.cuh): float copies of the triangles
   // and their FP64 differences, the pairs that may touch with what decides
@@ -45,25 +53,37 @@ struct PgTT
   double *vres = nullptr, *eres = nullptr;  // [.cap][3] squared distance and the closest points' parameters
   int vcap = 0, ecap = 0;
   int *qn = nullptr;              // [4] near pairs, full pairs, vertex-face and edge-edge distances
-  unsigned char *act = nullptr;
+  unsigned char *act = nullptr;   // [cap] in contact
   double *st[3] = {}, *f[3] = {}, *p[3] = {};   // tangential state, force on the finder's particle, point
-  // the previous step's pairs (state carried by (finder, partner))
+  // the previous list (state carried by (finder, partner) at a search)
   int *poff = nullptr, *ppu = nullptr;
   unsigned char *pact = nullptr;
   double *pst[3] = {};
+  // the pairs' two entries sorted by particle (ekeys[0]: particle, evals[0]:
+  // 2 pair + side), made with the list; each step takes the active ones, in
+  // that order, into elist
   unsigned *ekeys[2] = {}; int *evals[2] = {}; unsigned *ehist = nullptr;
-  int *pfirst = nullptr, *plast = nullptr;  // [parnum] each particle's entries
-  // sums in chunks of PG_TT_CHUNK entries: chunks per particle, their
-  // offsets (an exclusive scan), the chunk sums (force, torque)
-  int *nch = nullptr, *choff = nullptr, *nchunks = nullptr;
-  double *csum[6] = {};
-  long long ccap = 0;             // chunk-sum capacity
+  unsigned *ebits = nullptr;      // active entries, one bit each
+  int *etile = nullptr;           // active entries before each tile of PG_TT_TILE
+  int *elist = nullptr;
+  int *pfirst = nullptr, *plast = nullptr;  // [parnum] each particle's range of elist
+  // particles with more than PG_TT_CHUNK entries in the list: their chunks
+  int nbig = 0, nchunks = 0;
+  int *bigp = nullptr, *bigoff = nullptr;   // [cap / PG_TT_CHUNK + 1] particle, first chunk
+  int *chmap = nullptr;           // [ccap] chunk -> big particle's place
+  double *csum[6] = {};           // [ccap] chunk sums (force, torque)
+  int ccap = 0;
 };
 
 #define PG_TT_CHUNK 1024          // entries one warp sums into one chunk sum
+#define PG_TT_TILE 1024           // entries of one tile of the selection of active entries
 
 int pg_tt_key_bits(int ncells);
-void pg_tt_find(const PgDev &d, PgTT &g, cudaStream_t s);                 // steps 1-4a; total in g.np_dev
-void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, int np, double step);   // steps 4b-6
-int pg_tt_kernel_count(const PgTT &g, int trinum, int np);
-long long pg_tt_max_chunks(int parnum, int np);   // chunk sums a step can need
+void pg_tt_prepare(const PgDev &d, PgTT &g, cudaStream_t s);              // boxes and geometry; sets moved[0]
+void pg_tt_search(const PgDev &d, PgTT &g, cudaStream_t s);               // pairs of each triangle; total in moved[1]
+void pg_tt_list(const PgDev &d, PgTT &g, cudaStream_t s);                 // the list of g.np pairs and its entry order
+void pg_tt_chunk_map(PgTT &g, cudaStream_t s);                            // chunks of the big particles
+void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, double step);  // contacts and per-particle sums
+void pg_tt_count(const PgDev &d, const PgTT &g, int *out2, cudaStream_t s);   // overlapping and active pairs
+int pg_tt_search_kernels(const PgTT &g, int trinum);
+int pg_tt_step_kernels(const PgTT &g);

@@ -54,6 +54,7 @@ struct pg_session
   int adapt_ready = 0, hrec_cap = 0, sbig_ad_cap = 0;
   // mesh-mesh contact (pg_meshcontact.cu); steps then run without graphs
   PgTT tt;
+  int *tt_host = nullptr;                  // page-locked: what a step reads back
   // a pool's live extents (pg_session_set_live): the steps cover particles,
   // spheres and triangles below them; 0: the whole arrays
   int plive = 0, elive = 0, tlive = 0;
@@ -1084,63 +1085,87 @@ void enqueue_step(pg_session *s, double step)
   pg_launch_obstacles_tail(d, s->stream, step);
 }
 
-// the mesh-contact stage of one step: pairs, forces and per-particle sums;
-// it reads the pair count back (one host wait per step), so steps with mesh
-// contact are not captured in graphs
-int tt_stage(pg_session *s, double step)
+// room for np pairs: the list arrays and the narrow phase's work are made
+// anew, the previous list (pnp pairs), whose state the new one takes, moved
+int tt_pair_buffers(pg_session *s, int np, int pnp)
+{
+  PgTT &g = s->tt;
+  const int cap = np + np / 2 + 1024;
+  int *ppu = nullptr; unsigned char *pact = nullptr; double *pst[3] = {};
+  TRY(dalloc(s, &ppu, cap)); TRY(dalloc(s, &pact, cap));
+  for (int c = 0; c < 3; c ++) TRY(dalloc(s, &pst[c], cap));
+  if (pnp > 0)
+  {
+    CK(cudaMemcpyAsync(ppu, g.ppu, (size_t)pnp * sizeof(int), cudaMemcpyDeviceToDevice, s->stream));
+    CK(cudaMemcpyAsync(pact, g.pact, (size_t)pnp, cudaMemcpyDeviceToDevice, s->stream));
+    for (int c = 0; c < 3; c ++)
+      CK(cudaMemcpyAsync(pst[c], g.pst[c], (size_t)pnp * sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
+  }
+  CK(cudaStreamSynchronize(s->stream));
+  for (void *q : {(void *)g.pf, (void *)g.pu, (void *)g.act, (void *)g.ppu, (void *)g.pact, (void *)g.near,
+                  (void *)g.full, (void *)g.vit, (void *)g.eit, (void *)g.vres, (void *)g.eres, (void *)g.ekeys[0],
+                  (void *)g.ekeys[1], (void *)g.evals[0], (void *)g.evals[1], (void *)g.ehist, (void *)g.ebits,
+                  (void *)g.etile, (void *)g.elist, (void *)g.bigp, (void *)g.bigoff})
+    release(s, q);
+  for (int c = 0; c < 3; c ++) for (void *q : {(void *)g.st[c], (void *)g.f[c], (void *)g.p[c], (void *)g.pst[c]}) release(s, q);
+  g.ppu = ppu; g.pact = pact;
+  TRY(dalloc(s, &g.pf, cap)); TRY(dalloc(s, &g.pu, cap)); TRY(dalloc(s, &g.act, cap));
+  for (int c = 0; c < 3; c ++)
+  {
+    g.pst[c] = pst[c];
+    TRY(dalloc(s, &g.st[c], cap)); TRY(dalloc(s, &g.f[c], cap)); TRY(dalloc(s, &g.p[c], cap));
+  }
+  // room for 2 vertex-triangle and 3 edge-edge distances a pair (the spring
+  // lattice, whose faces lie parallel, asks for 1.3 and 2.4); pairs beyond
+  // it take the whole narrow phase
+  g.vcap = (int)std::min(2LL * cap, 0x7fff0000LL);
+  g.ecap = (int)std::min(3LL * cap, 0x7fff0000LL);
+  TRY(dalloc(s, &g.near, cap)); TRY(dalloc(s, &g.full, cap));
+  TRY(dalloc(s, &g.vit, g.vcap)); TRY(dalloc(s, &g.eit, g.ecap));
+  TRY(dalloc(s, &g.vres, 3 * (size_t)g.vcap)); TRY(dalloc(s, &g.eres, 3 * (size_t)g.ecap));
+  const size_t E = 2 * (size_t)cap, tiles = (E + PG_TT_TILE - 1) / PG_TT_TILE;
+  for (int k = 0; k < 2; k ++) { TRY(dalloc(s, &g.ekeys[k], E)); TRY(dalloc(s, &g.evals[k], E)); }
+  TRY(dalloc(s, &g.ehist, pg_sort_hist_len((int)E)));
+  TRY(dalloc(s, &g.ebits, tiles * (PG_TT_TILE / 32)));
+  TRY(dalloc(s, &g.etile, tiles));
+  TRY(dalloc(s, &g.elist, E));
+  TRY(dalloc(s, &g.bigp, E / PG_TT_CHUNK + 1)); TRY(dalloc(s, &g.bigoff, E / PG_TT_CHUNK + 1));
+  g.cap = cap;
+  return PG_OK;
+}
+
+// a new pair list: its pairs, the state of the previous list's, the entry
+// order of the sums.  The host waits twice, for the pair count and for the
+// number of particles with long sums.
+int tt_search(pg_session *s)
 {
   PgDev &d = s->d;
   PgTT &g = s->tt;
-  pg_tt_find(d, g, s->stream);
-  int np = 0;
-  TRY(d2h(s, &np, g.np_dev, 1));
+  const int pnp = g.valid ? g.np : 0;
+  std::swap(g.off, g.poff);
+  std::swap(g.pu, g.ppu);
+  std::swap(g.act, g.pact);
+  for (int c = 0; c < 3; c ++) std::swap(g.st[c], g.pst[c]);
+  g.valid = 0;
+  if (!pnp) CK(cudaMemsetAsync(g.poff, 0, ((size_t)d.trinum + 1) * sizeof(int), s->stream));
+  pg_tt_search(d, g, s->stream);
+  CK(cudaMemcpyAsync(s->tt_host, g.moved, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
-  if (np > g.cap)
+  const int np = s->tt_host[1];
+  if (np > 0x3fffffff) return PG_ERR_CAPACITY;
+  if (np > g.cap || !g.pf) TRY(tt_pair_buffers(s, np, pnp));
+  g.np = np;
+  pg_tt_list(d, g, s->stream);
+  CK(cudaMemcpyAsync(s->tt_host, g.moved, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaStreamSynchronize(s->stream));
+  g.nbig = s->tt_host[2];
+  g.nchunks = s->tt_host[3];
+  if (g.nchunks > g.ccap)
   {
-    // room for the pairs of this step (and the next): both pair lists grow
-    // together, the previous step's list keeping its entries
-    const int cap = np + np / 2 + 1024;
-    int *ppu = nullptr; unsigned char *pact = nullptr; double *pst[3] = {};
-    int *pf = nullptr, *pu = nullptr; unsigned char *act = nullptr; double *st[3] = {}, *f[3] = {}, *p[3] = {};
-    TRY(dalloc(s, &pf, cap)); TRY(dalloc(s, &pu, cap)); TRY(dalloc(s, &act, cap)); TRY(dalloc(s, &ppu, cap));
-    TRY(dalloc(s, &pact, cap));
-    for (int c = 0; c < 3; c ++)
-    {
-      TRY(dalloc(s, &st[c], cap)); TRY(dalloc(s, &f[c], cap)); TRY(dalloc(s, &p[c], cap)); TRY(dalloc(s, &pst[c], cap));
-    }
-    if (g.cap > 0)
-    {
-      CK(cudaMemcpyAsync(ppu, g.ppu, (size_t)g.cap * sizeof(int), cudaMemcpyDeviceToDevice, s->stream));
-      CK(cudaMemcpyAsync(pact, g.pact, (size_t)g.cap, cudaMemcpyDeviceToDevice, s->stream));
-      for (int c = 0; c < 3; c ++)
-        CK(cudaMemcpyAsync(pst[c], g.pst[c], (size_t)g.cap * sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
-    }
-    CK(cudaStreamSynchronize(s->stream));
-    for (void *q : {(void *)g.pf, (void *)g.pu, (void *)g.act, (void *)g.ppu, (void *)g.pact, (void *)g.near,
-                    (void *)g.full, (void *)g.vit, (void *)g.eit, (void *)g.vres, (void *)g.eres})
-      release(s, q);
-    for (int c = 0; c < 3; c ++) for (void *q : {(void *)g.st[c], (void *)g.f[c], (void *)g.p[c], (void *)g.pst[c]}) release(s, q);
-    release(s, g.ekeys[0]); release(s, g.ekeys[1]); release(s, g.evals[0]); release(s, g.evals[1]); release(s, g.ehist);
-    TRY(dalloc(s, &g.ekeys[0], 2 * (size_t)cap)); TRY(dalloc(s, &g.ekeys[1], 2 * (size_t)cap));
-    TRY(dalloc(s, &g.evals[0], 2 * (size_t)cap)); TRY(dalloc(s, &g.evals[1], 2 * (size_t)cap));
-    TRY(dalloc(s, &g.ehist, pg_sort_hist_len(2 * cap)));
-    // room for 2 vertex-triangle and 3 edge-edge distances a pair (the spring
-    // lattice, whose faces lie parallel, asks for 1.3 and 2.4); pairs beyond
-    // it take the whole narrow phase
-    g.vcap = (int)std::min(2LL * cap, 0x7fff0000LL);
-    g.ecap = (int)std::min(3LL * cap, 0x7fff0000LL);
-    TRY(dalloc(s, &g.near, cap)); TRY(dalloc(s, &g.full, cap));
-    TRY(dalloc(s, &g.vit, g.vcap)); TRY(dalloc(s, &g.eit, g.ecap));
-    TRY(dalloc(s, &g.vres, 3 * (size_t)g.vcap)); TRY(dalloc(s, &g.eres, 3 * (size_t)g.ecap));
-    g.pf = pf; g.pu = pu; g.act = act; g.ppu = ppu; g.pact = pact;
-    for (int c = 0; c < 3; c ++) { g.st[c] = st[c]; g.f[c] = f[c]; g.p[c] = p[c]; g.pst[c] = pst[c]; }
-    g.cap = cap;
-  }
-  const long long chunks = pg_tt_max_chunks(d.parnum, np);
-  if (chunks > g.ccap)
-  {
-    const long long cap = chunks + chunks / 2;
-    CK(cudaStreamSynchronize(s->stream));
+    const int cap = g.nchunks + g.nchunks / 2;
+    release(s, g.chmap);
+    g.chmap = nullptr;
+    TRY(dalloc(s, &g.chmap, (size_t)cap));
     for (int c = 0; c < 6; c ++)
     {
       release(s, g.csum[c]);
@@ -1149,14 +1174,27 @@ int tt_stage(pg_session *s, double step)
     }
     g.ccap = cap;
   }
-  pg_tt_forces(d, g, s->stream, np, step);
-  s->launches += pg_tt_kernel_count(g, d.trinum, np);
-  // this step's pairs become the previous step's
-  g.np_last = np;
-  std::swap(g.off, g.poff);
-  std::swap(g.pu, g.ppu);
-  std::swap(g.act, g.pact);
-  for (int c = 0; c < 3; c ++) std::swap(g.st[c], g.pst[c]);
+  pg_tt_chunk_map(g, s->stream);
+  s->launches += pg_tt_search_kernels(g, d.trinum);
+  g.valid = 1;
+  return PG_OK;
+}
+
+// the mesh-contact stage of one step: boxes, a new pair list when a triangle
+// left its neighbourhood, contacts and per-particle sums.  It reads back
+// whether a list is due (one host wait per step), so steps with mesh contact
+// are not captured in graphs.
+int tt_stage(pg_session *s, double step)
+{
+  PgDev &d = s->d;
+  PgTT &g = s->tt;
+  if (!s->tt_host) CK(cudaMallocHost((void **)&s->tt_host, 4 * sizeof(int)));
+  pg_tt_prepare(d, g, s->stream);
+  CK(cudaMemcpyAsync(s->tt_host, g.moved, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaStreamSynchronize(s->stream));
+  if (!g.valid || s->tt_host[0]) TRY(tt_search(s));
+  pg_tt_forces(d, g, s->stream, step);
+  s->launches += pg_tt_step_kernels(g);
   CK(cudaGetLastError());
   return PG_OK;
 }
@@ -1372,6 +1410,7 @@ int pg_session_destroy(pg_session *s)
   if (s->stream) cudaStreamSynchronize(s->stream);
   drop_graph(s);
   for (void *p : s->allocs) cudaFree(p);
+  if (s->tt_host) cudaFreeHost(s->tt_host);
   for (auto &e : s->ring) if (e) cudaEventDestroy(e);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
@@ -1654,7 +1693,12 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
         hi[c] = std::max(hi[c], x);
       }
   }
-  double h = cell;
+  // the pair list serves until a vertex coordinate has moved by half the
+  // skin: a fifth of the radius adds few pairs (0.1 r a side), and where the
+  // radius is small against the triangles a part of their size keeps the
+  // searches rare
+  g.skin = std::max(0.2 * radius, 0.005 * cell);
+  double h = cell + g.skin;
   for (int c = 0; c < 3; c ++) if (!(hi[c] >= lo[c])) { lo[c] = 0.0; hi[c] = 0.0; }
   long long cells = 0;
   int dim[3];
@@ -1678,7 +1722,6 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
   g.passes = pg_sort_passes_bits(kb);
   int pb = 1;
   while ((1u << pb) <= (unsigned)P) pb ++;
-  g.enone = (1u << pb) - 1u;
   g.epasses = pg_sort_passes_bits(pb);
   if (!g.big)
   {
@@ -1687,16 +1730,14 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
     TRY(dalloc(s, &g.cell, T));
     for (int k = 0; k < 2; k ++) { TRY(dalloc(s, &g.keys[k], T)); TRY(dalloc(s, &g.vals[k], T)); }
     TRY(dalloc(s, &g.hist, pg_sort_hist_len(T)));
-    TRY(dalloc(s, &g.cand, (size_t)g.kmax * T));
+    for (int c = 0; c < 9; c ++) TRY(dalloc(s, &g.ref[c], T));
+    TRY(dalloc(s, &g.sbox, T));
+    TRY(dalloc(s, &g.moved, 4));
     TRY(dalloc(s, &g.cnt, T));
     TRY(dalloc(s, &g.off, (size_t)T + 1));
     TRY(dalloc(s, &g.poff, (size_t)T + 1));
-    TRY(dalloc(s, &g.np_dev, 1));
     TRY(dalloc(s, &g.pfirst, P));
     TRY(dalloc(s, &g.plast, P));
-    TRY(dalloc(s, &g.nch, P));
-    TRY(dalloc(s, &g.choff, (size_t)P + 1));
-    TRY(dalloc(s, &g.nchunks, 1));
     TRY(dalloc(s, &g.qn, 4));
     TRY(dalloc(s, &g.fv, 3 * (size_t)T));
     TRY(dalloc(s, &g.geo, (size_t)PG_TT_GEO * T));
@@ -1708,7 +1749,7 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
   TRY(dalloc(s, &g.cend, (size_t)g.ncells + 1));
   TRY(h2d(s, g.big, big, T));
   // no pairs carried into the first step
-  CK(cudaMemsetAsync(g.poff, 0, ((size_t)T + 1) * sizeof(int), s->stream));
+  g.valid = 0;
   CK(cudaStreamSynchronize(s->stream));
   d.tt_on = 1;
   return PG_OK;
@@ -1747,16 +1788,14 @@ int pg_session_set_live(pg_session *s, int particles, int spheres, int triangles
 int pg_session_mesh_contact_stats(pg_session *s, int *pairs, int *active)
 {
   if (!s || !pairs || !active) return PG_ERR_ARGUMENT;
-  PgTT &g = s->tt;
-  *pairs = s->d.tt_on ? g.np_last : 0;
-  *active = 0;
-  if (*pairs > 0)
-  {
-    std::vector<unsigned char> a(*pairs);
-    TRY(d2h(s, a.data(), g.pact, a.size()));
-    CK(cudaStreamSynchronize(s->stream));
-    for (unsigned char v : a) *active += v ? 1 : 0;
-  }
+  *pairs = *active = 0;
+  if (!s->d.tt_on || !s->tt.valid) return PG_OK;
+  int n[2] = {0, 0};
+  pg_tt_count(s->d, s->tt, s->tt.qn, s->stream);         // (the step's counters are free between steps)
+  TRY(d2h(s, n, s->tt.qn, 2));
+  CK(cudaStreamSynchronize(s->stream));
+  *pairs = n[0];
+  *active = n[1];
   return PG_OK;
 }
 
