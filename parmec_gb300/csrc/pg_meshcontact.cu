@@ -87,7 +87,8 @@ __global__ void __launch_bounds__(TPB) k_tt_boxes(PgDev d, PgTT g)
     double *o = g.geo + (size_t)PG_TT_GEO * t;
     for (int a = 0; a < 3; a ++)
       for (int c = 0; c < 3; c ++) { o[3*a + c] = v[a][c]; o[9 + 3*a + c] = T.e[a][c]; }
-    for (int a = 0; a < 3; a ++) { o[18 + a] = T.l2[a]; o[21 + a] = T.ac[a]; }
+    for (int a = 0; a < 3; a ++) { o[18 + a] = T.l2[a]; o[21 + a] = T.ac[a]; o[24 + a] = T.n[a]; }
+    o[27] = (g.r + g.r) * sqrt(pgtt::dot(T.n, T.n));
     float f[3][3];
     const float err = pgtf::float_triangle(v, T.n, T.l2, g.org, f);
     for (int a = 0; a < 3; a ++)
@@ -324,11 +325,32 @@ __device__ __forceinline__ int warp_take(int *count, int n)
 
 __global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g)
 {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  // the block's pairs whose boxes overlap, on its first threads
+  __shared__ int some[TPB], warps[TPB / 32];
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  bool in = false;
+  if (q < g.np)
+  {
+    in = boxes_overlap(g, g.pf[q], g.pu[q]);
+    if (!in) g.act[q] = 0;
+  }
+  const unsigned m0 = __ballot_sync(0xffffffffu, in);
+  if (lane == 0) warps[warp] = __popc(m0);
+  __syncthreads();
+  int at = __popc(m0 & ((1u << lane) - 1u)), count = 0;
+  for (int w = 0; w < TPB / 32; w ++)
+  {
+    if (w < warp) at += warps[w];
+    count += warps[w];
+  }
+  if (in) some[at] = q;
+  __syncthreads();
+  if (warp * 32 >= count) return;
+  const int k = threadIdx.x < count ? some[threadIdx.x] : -1;
   int verdict = pgtf::APART;
   unsigned mask = 0;
   float upper = 0.0f, size = 0.0f;
-  if (k < g.np)
+  if (k >= 0)
   {
     const int f = g.pf[k], u = g.pu[k];
     const size_t T = d.trinum;
@@ -341,14 +363,12 @@ __global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g)
       if (v == 0) { ea = x.w; eb = y.w; }
     }
     verdict = pgtf::judge(a, b, ea, eb, (float)(g.r + g.r), &mask, &upper, &size);
-    // (a pair whose boxes no longer overlap holds no contact)
-    if (verdict != pgtf::APART && !boxes_overlap(g, f, u)) verdict = pgtf::APART;
     if (verdict == pgtf::APART) g.act[k] = 0;
   }
   int nv = verdict == pgtf::NEAR ? __popc(mask & 63u) : 0, ne = verdict == pgtf::NEAR ? __popc(mask >> 6) : 0;
   const int vb = warp_take(g.qn + 2, nv), eb = warp_take(g.qn + 3, ne);
   if (verdict == pgtf::NEAR && (vb + nv > g.vcap || eb + ne > g.ecap)) verdict = pgtf::FULL;   // no room for its items
-  const int q = warp_take(g.qn, verdict == pgtf::NEAR), z = warp_take(g.qn + 1, verdict == pgtf::FULL);
+  const int np = warp_take(g.qn, verdict == pgtf::NEAR), z = warp_take(g.qn + 1, verdict == pgtf::FULL);
   // (items of a pair that found no room in the other list name no pair)
   if (nv + ne && verdict == pgtf::FULL)
   {
@@ -357,11 +377,11 @@ __global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g)
   }
   if (verdict == pgtf::FULL) g.full[z] = k;
   if (verdict != pgtf::NEAR) return;
-  g.near[q] = {k, mask, vb, eb, upper, size};
+  g.near[np] = {k, mask, vb, eb, upper, size};
   int j = vb;
-  for (unsigned m = mask & 63u; m; m &= m - 1) g.vit[j ++] = (unsigned)q << 4 | (unsigned)(__ffs(m) - 1);
+  for (unsigned m = mask & 63u; m; m &= m - 1) g.vit[j ++] = (unsigned)np << 4 | (unsigned)(__ffs(m) - 1);
   j = eb;
-  for (unsigned m = mask >> 6; m; m &= m - 1) g.eit[j ++] = (unsigned)q << 4 | (unsigned)(__ffs(m) - 1);
+  for (unsigned m = mask >> 6; m; m &= m - 1) g.eit[j ++] = (unsigned)np << 4 | (unsigned)(__ffs(m) - 1);
 }
 
 // 5b. the vertex-triangle and the edge-edge distances asked for, one thread
@@ -504,7 +524,7 @@ __global__ void __launch_bounds__(TPB) k_tt_near(PgDev d, PgTT g, double step)
       if (depth > 0.0 && !(depth > 1e-9 * (double)e.size))
       {
         const double *Av[3] = {A, A + 3, A + 6}, *Bv[3] = {B, B + 3, B + 6};
-        if (pgtt::apart(Av, Bv, g.r, g.r)) depth = -1.0;
+        if (pgtt::beyond_plane_of(A, A + 24, A[27], Bv) || pgtt::beyond_plane_of(B, B + 24, B[27], Av)) depth = -1.0;
       }
     }
     tt_force(d, g, k, f, u, depth, point, normal, step);
@@ -634,50 +654,66 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tt_select(PgTT g)
   }
 }
 
-// 6c. sums of entries [b, e) of elist, e - b <= PG_TT_CHUNK, by one warp: lane
-// sums over entries lane, lane+32, ..., then the lane sums in lane order, the
-// six components by a lane each; the totals in s of lanes 0 to 5.  Four
-// entries' loads are issued before the first is added.
+// 6c. sums of entries [b, e) of elist, e - b <= PG_TT_CHUNK: lane sums over
+// entries lane, lane+32, ..., then the lane sums in lane order, one lane per
+// component.  Four entries' loads are issued before the first is added.
+// One warp sums all six components (18 FP64 instructions an entry, 64 clocks
+// each); with SPLIT four warps of a block share them, the force by warp 0 and
+// a component of the torque by each other (a chain of 6 an entry, but four
+// times the lane sums): for the long sums of few particles, where the chip
+// waits for the chain (a chunk 57 -> 34 us), not for thousands of short ones
+// (4,097 particles 35 -> 73 us).  Returns component `lane` (warp 0: force;
+// without SPLIT all six) or, in lane 0, torque component warp - 1.
+template <bool SPLIT>
 __device__ __forceinline__ double chunk_sum(const PgTT &g, const double *x, int b, int e, double (*part)[6])
 {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = SPLIT ? threadIdx.x >> 5 : 0;
+  const int c1 = warp % 3, c2 = (warp + 1) % 3;          // torque component warp-1: a[c1] f[c2] - a[c2] f[c1]
+  const bool force = !SPLIT || warp == 0;
   double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   for (int q0 = b + lane; q0 < e; q0 += 128)
   {
-    double f[4][3], p[4][3];
     int v[4];
     #pragma unroll
     for (int j = 0; j < 4; j ++) v[j] = q0 + 32*j < e ? g.elist[q0 + 32*j] : -1;
+    double f[4][3], p[4][3];
     #pragma unroll
     for (int j = 0; j < 4; j ++)
     {
       const int k = v[j] >= 0 ? v[j] >> 1 : 0;
-      for (int c = 0; c < 3; c ++) { f[j][c] = g.f[c][k]; p[j][c] = g.p[c][k]; }
+      if (force) for (int c = 0; c < 3; c ++) f[j][c] = g.f[c][k];
+      if (!SPLIT) for (int c = 0; c < 3; c ++) p[j][c] = g.p[c][k];
+      else if (!force) { f[j][0] = g.f[c1][k]; f[j][1] = g.f[c2][k]; f[j][2] = 0.0; p[j][0] = g.p[c1][k]; p[j][1] = g.p[c2][k]; }
     }
     #pragma unroll
     for (int j = 0; j < 4; j ++)
     {
       if (v[j] < 0) break;
       if (v[j] & 1) { f[j][0] = -f[j][0]; f[j][1] = -f[j][1]; f[j][2] = -f[j][2]; }
-      const double a[3] = {p[j][0]-x[0], p[j][1]-x[1], p[j][2]-x[2]};
-      s[0] += f[j][0]; s[1] += f[j][1]; s[2] += f[j][2];
-      s[3] += a[1]*f[j][2] - a[2]*f[j][1];
-      s[4] += a[2]*f[j][0] - a[0]*f[j][2];
-      s[5] += a[0]*f[j][1] - a[1]*f[j][0];
+      if (force) { s[0] += f[j][0]; s[1] += f[j][1]; s[2] += f[j][2]; }
+      if (!SPLIT)
+      {
+        const double a[3] = {p[j][0]-x[0], p[j][1]-x[1], p[j][2]-x[2]};
+        s[3] += a[1]*f[j][2] - a[2]*f[j][1];
+        s[4] += a[2]*f[j][0] - a[0]*f[j][2];
+        s[5] += a[0]*f[j][1] - a[1]*f[j][0];
+      }
+      else if (!force) s[0] += (p[j][0]-x[c1])*f[j][1] - (p[j][1]-x[c2])*f[j][0];
     }
   }
-  for (int k = 0; k < 6; k ++) part[lane][k] = s[k];
+  for (int c = 0; c < 6; c ++) part[lane][c] = s[c];
   __syncwarp();
   double acc = 0.0;
-  if (lane < 6) for (int L = 0; L < 32; L ++) acc += part[L][lane];
+  if (lane < (!SPLIT ? 6 : force ? 3 : 1)) for (int L = 0; L < 32; L ++) acc += part[L][lane];
   return acc;
 }
 
-// one warp per particle of at most one chunk of active entries
+// particles of at most one chunk of active entries, one warp each
 __global__ void __launch_bounds__(TPB) k_tt_sums(PgDev d, PgTT g)
 {
   __shared__ double part[TPB / 32][32][6];
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= d.parnum) return;
   const int b = g.pfirst[w], e = g.plast[w];
   if (e - b > PG_TT_CHUNK) return;
@@ -685,25 +721,25 @@ __global__ void __launch_bounds__(TPB) k_tt_sums(PgDev d, PgTT g)
   if (e > b)
   {
     const double x[3] = {d.position[0][w], d.position[1][w], d.position[2][w]};
-    acc += chunk_sum(g, x, b, e, part[threadIdx.x >> 5]);
+    acc += chunk_sum<false>(g, x, b, e, part[threadIdx.x >> 5]);
   }
   if (lane < 3) d.ttF[lane][w] = acc;
   else if (lane < 6) d.ttT[lane - 3][w] = acc;
 }
 
-// the others: one warp per chunk, then one thread per component, the chunk
+// the others: one block per chunk, then one thread per component, the chunk
 // sums in chunk order
 __global__ void __launch_bounds__(TPB) k_tt_chunk_sums(PgDev d, PgTT g)
 {
   __shared__ double part[TPB / 32][32][6];
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (c >= g.nchunks) return;
+  const int c = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int q = g.chmap[c], w = g.bigp[q];
   const int b = g.pfirst[w] + (c - g.bigoff[q]) * PG_TT_CHUNK, e = min(b + PG_TT_CHUNK, g.plast[w]);
   if (b >= e) return;
   const double x[3] = {d.position[0][w], d.position[1][w], d.position[2][w]};
-  const double acc = chunk_sum(g, x, b, e, part[threadIdx.x >> 5]);
-  if (lane < 6) g.csum[lane][c] = acc;
+  const double acc = chunk_sum<true>(g, x, b, e, part[warp]);
+  if (warp == 0) { if (lane < 3) g.csum[lane][c] = acc; }
+  else if (lane == 0) g.csum[2 + warp][c] = acc;
 }
 
 __global__ void __launch_bounds__(TPB) k_tt_totals(PgDev d, PgTT g)
@@ -785,10 +821,10 @@ void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, double step)
     k_tt_tiles<<<1, 1024, 0, s>>>(g, tiles);
     k_tt_select<<<tiles, TILE_THREADS, 0, s>>>(g);
   }
-  k_tt_sums<<<nblk(32LL * d.parnum), TPB, 0, s>>>(d, g);
+  if (d.parnum > 0) k_tt_sums<<<nblk(32LL * d.parnum), TPB, 0, s>>>(d, g);
   if (g.nbig > 0)
   {
-    k_tt_chunk_sums<<<nblk(32LL * g.nchunks), TPB, 0, s>>>(d, g);
+    k_tt_chunk_sums<<<g.nchunks, TPB, 0, s>>>(d, g);
     k_tt_totals<<<nblk(6LL * g.nbig), TPB, 0, s>>>(d, g);
   }
 }

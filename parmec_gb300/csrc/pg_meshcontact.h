@@ -10,7 +10,7 @@
 // a pair whose contact a few distances decide: candidates (bits as in
 // pgtf::judge), where their results start, a bound on the smallest
 struct PgTTNear { int pair; unsigned mask; int vbase, ebase; float upper, size; };
-#define PG_TT_GEO 24
+#define PG_TT_GEO 28
 
 // a triangle's box at a search, widened by r and half the skin (rounded
 // outwards), its particle (-1: not of a mesh) and whether it is big
@@ -46,7 +46,7 @@ struct PgTT
   // and their FP64 differences, the pairs that may touch with what decides
   // them, the pairs that need every test, and the distances to take
   float4 *fv = nullptr;           // [3][trinum] vertices relative to org; w of the first: error bound
-  double *geo = nullptr;          // [trinum][PG_TT_GEO] vertices, edges, squared edges, third minus first vertex
+  double *geo = nullptr;          // [trinum][PG_TT_GEO] vertices, edges, squared edges, third minus first vertex, normal, 2r |normal|
   PgTTNear *near = nullptr;       // [cap]
   int *full = nullptr;            // [cap]
   unsigned *vit = nullptr, *eit = nullptr;  // [vcap], [ecap] near pair << 4 | candidate; vit then holds the region

@@ -72,7 +72,31 @@ PG_TT bool lt_neg(double x, double y)
   const unsigned long long a = bits(x), b = bits(y) ^ 0x8000000000000000ULL;
   return !nan_b(a) && !nan_b(b) && okey(a) < okey(b);
 }
-PG_TT double clamp01(double x) { return x < 0.0 ? 0.0 : (x > 1.0 ? 1.0 : x); }
+// x <= 0, x >= 0 and x <= y for the region tests of the distances that the
+// device takes one thread each (there a test on the integer pipe costs a
+// tenth of one on the FP64 pipe)
+#ifdef __CUDA_ARCH__
+PG_TT bool le0(double x) { const unsigned long long b = bits(x); return (b << 1) == 0 || b - 0x8000000000000000ULL <= 0x7ff0000000000000ULL; }
+PG_TT bool ge0(double x) { const unsigned long long b = bits(x); return (b << 1) == 0 || b <= 0x7ff0000000000000ULL; }
+PG_TT bool le(double x, double y)
+{
+  const unsigned long long a = bits(x), b = bits(y);
+  return !nan_b(a) && !nan_b(b) && okey(a) <= okey(b);
+}
+#else
+PG_TT bool le0(double x) { return x <= 0.0; }
+PG_TT bool ge0(double x) { return x >= 0.0; }
+PG_TT bool le(double x, double y) { return x <= y; }
+#endif
+// x < 0 and x > 1 (false for NaN)
+#ifdef __CUDA_ARCH__
+PG_TT bool lt0(double x) { return bits(x) - 0x8000000000000001ULL < 0x7ff0000000000000ULL; }
+PG_TT bool gt1(double x) { return bits(x) - 0x3ff0000000000001ULL < 0x4000000000000000ULL; }
+#else
+PG_TT bool lt0(double x) { return x < 0.0; }
+PG_TT bool gt1(double x) { return x > 1.0; }
+#endif
+PG_TT double clamp01(double x) { return lt0(x) ? 0.0 : (gt1(x) ? 1.0 : x); }
 
 // Closest point q of triangle (a, b, c) to p: the Voronoi-region method
 // (Ericson, Real-Time Collision Detection, 5.1.5).  The region is found
@@ -94,12 +118,12 @@ PG_TT int point_triangle_region(const double *p, const double *a, const double *
   const double va = d3*d6 - d5*d4;
   const double e43 = d4 - d3, e56 = d5 - d6;
   // 0: vertex a, 1: vertex b, 2: edge ab, 3: vertex c, 4: edge ac, 5: edge bc, 6: face
-  const int region = (d1 <= 0.0 && d2 <= 0.0) ? 0 :
-                     (d3 >= 0.0 && d4 <= d3) ? 1 :
-                     (vc <= 0.0 && d1 >= 0.0 && d3 <= 0.0) ? 2 :
-                     (d6 >= 0.0 && d5 <= d6) ? 3 :
-                     (vb <= 0.0 && d2 >= 0.0 && d6 <= 0.0) ? 4 :
-                     (va <= 0.0 && e43 >= 0.0 && e56 >= 0.0) ? 5 : 6;
+  const int region = (le0(d1) && le0(d2)) ? 0 :
+                     (ge0(d3) && le(d4, d3)) ? 1 :
+                     (le0(vc) && ge0(d1) && le0(d3)) ? 2 :
+                     (ge0(d6) && le(d5, d6)) ? 3 :
+                     (le0(vb) && ge0(d2) && le0(d6)) ? 4 :
+                     (le0(va) && ge0(e43) && ge0(e56)) ? 5 : 6;
   double num = 0.0, den = 1.0;
   if (region == 2) { num = d1; den = d1 - d3; }
   else if (region == 4) { num = d2; den = d2 - d6; }
@@ -151,20 +175,21 @@ PG_TT void segment_params(const double *p1, const double *d1, double a, const do
   sub(p1, p2, r);
   const double f = dot(d2, r);
   double s, t;
-  if (a <= 0.0 && e <= 0.0) { s = 0.0; t = 0.0; }
-  else if (a <= 0.0) { s = 0.0; t = clamp01(f / e); }
+  if (le0(a) && le0(e)) { s = 0.0; t = 0.0; }
+  else if (le0(a)) { s = 0.0; t = clamp01(f / e); }
   else
   {
     const double c = dot(d1, r);
-    if (e <= 0.0) { t = 0.0; s = clamp01(-c / a); }
+    if (le0(e)) { t = 0.0; s = clamp01(-c / a); }
     else
     {
       const double b = dot(d1, d2);
       const double den = a*e - b*b;
-      const double s0 = (b*f - c*e) / (den != 0.0 ? den : 1.0);
-      s = den != 0.0 ? clamp01(s0) : 0.0;
+      const bool skew = (bits(den) << 1) != 0;            // den != 0
+      const double s0 = (b*f - c*e) / (skew ? den : 1.0);
+      s = skew ? clamp01(s0) : 0.0;
       t = (b*s + f) / e;
-      const bool low = t < 0.0, high = t > 1.0;
+      const bool low = lt0(t), high = gt1(t);
       if (low || high)
       {
         s = clamp01((low ? -c : b - c) / a);
@@ -280,22 +305,26 @@ PG_TT double triangle_triangle(const double *const a[3], const double *const b[3
 
 // Are Q's vertices all farther than s from P's plane, on one side?  (The
 // plane normal is left unnormalised: distances are compared with s |n|.)
-PG_TT bool beyond_plane(const double *const P[3], const double *const Q[3], double s)
+PG_TT bool beyond_plane_of(const double *P0, const double *n, double lim, const double *const Q[3])
 {
-  double e1[3], e2[3], n[3];
-  sub(P[1], P[0], e1); sub(P[2], P[0], e2);
-  cross(e1, e2, n);
-  const double lim = s * sqrt(dot(n, n));
   int above = 0, below = 0;
   for (int k = 0; k < 3; k ++)
   {
     double w[3];
-    sub(Q[k], P[0], w);
+    sub(Q[k], P0, w);
     const double h = dot(n, w);
     above += gt(h, lim) ? 1 : 0;
     below += lt_neg(h, lim) ? 1 : 0;
   }
   return above == 3 || below == 3;
+}
+
+PG_TT bool beyond_plane(const double *const P[3], const double *const Q[3], double s)
+{
+  double e1[3], e2[3], n[3];
+  sub(P[1], P[0], e1); sub(P[2], P[0], e2);
+  cross(e1, e2, n);
+  return beyond_plane_of(P[0], n, s * sqrt(dot(n, n)), Q);
 }
 
 // Triangles with one wholly beyond the other's plane by ra + rb are apart.

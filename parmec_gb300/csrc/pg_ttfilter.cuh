@@ -31,6 +31,24 @@ PG_TF float dot(const float *a, const float *b) { return a[0]*b[0] + a[1]*b[1] +
 PG_TF float mn(float a, float b) { return a < b ? a : b; }
 PG_TF float mx(float a, float b) { return a > b ? a : b; }
 PG_TF float clamp01(float x) { return x < 0.0f ? 0.0f : (x > 1.0f ? 1.0f : x); }
+// quotient and inverse root to a few units in the last place: the points and
+// directions they give serve whatever their error, the bounds have room for it
+PG_TF float quot(float a, float b)
+{
+#ifdef __CUDA_ARCH__
+  return __fdividef(a, b);
+#else
+  return a / b;
+#endif
+}
+PG_TF float iroot(float x)
+{
+#ifdef __CUDA_ARCH__
+  return rsqrtf(x);
+#else
+  return 1.0f / sqrtf(x);
+#endif
+}
 
 // closest point of triangle (v[0], v[1], v[2]) to p, in FP32 (any point of
 // the triangle serves)
@@ -42,23 +60,21 @@ PG_TF void vertex_face(const float *p, const float v[3][3], float *q)
   const float d1 = dot(ab, ap), d2 = dot(ac, ap);
   const float d3 = d1 - g11, d4 = d2 - g12, d5 = d1 - g12, d6 = d2 - g22;
   const float vc = d1*d4 - d3*d2, vb = d5*d2 - d1*d6, va = d3*d6 - d5*d4;
-  float s, t;                                            // q = a + s ab + t ac
-  if (d1 <= 0.0f && d2 <= 0.0f) { s = 0.0f; t = 0.0f; }
-  else if (d3 >= 0.0f && d4 <= d3) { s = 1.0f; t = 0.0f; }
-  else if (vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f) { s = d1 / (d1 - d3); t = 0.0f; }
-  else if (d6 >= 0.0f && d5 <= d6) { s = 0.0f; t = 1.0f; }
-  else if (vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f) { s = 0.0f; t = d2 / (d2 - d6); }
-  else if (va <= 0.0f && d4 - d3 >= 0.0f && d5 - d6 >= 0.0f)
-  {
-    t = (d4 - d3) / ((d4 - d3) + (d5 - d6));
-    s = 1.0f - t;
-  }
-  else
-  {
-    const float x = 1.0f / (va + vb + vc);
-    s = vb * x;
-    t = vc * x;
-  }
+  // the region's parameters by selection, with one division (q = a + s ab + t ac)
+  const float e43 = d4 - d3, e56 = d5 - d6;
+  const bool r0 = d1 <= 0.0f && d2 <= 0.0f, r1 = d3 >= 0.0f && d4 <= d3, r2 = vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f,
+             r3 = d6 >= 0.0f && d5 <= d6, r4 = vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f,
+             r5 = va <= 0.0f && e43 >= 0.0f && e56 >= 0.0f;
+  const float num = r2 ? d1 : r4 ? d2 : r5 ? e43 : 1.0f;
+  const float den = r2 ? d1 - d3 : r4 ? d2 - d6 : r5 ? e43 + e56 : va + vb + vc;
+  const float x = quot(num, den);
+  float s = vb * x, t = vc * x;
+  if (r5) { s = 1.0f - x; t = x; }
+  if (r4) { s = 0.0f; t = x; }
+  if (r3) { s = 0.0f; t = 1.0f; }
+  if (r2) { s = x; t = 0.0f; }
+  if (r1) { s = 1.0f; t = 0.0f; }
+  if (r0) { s = 0.0f; t = 0.0f; }
   for (int k = 0; k < 3; k ++) q[k] = v[0][k] + s*ab[k] + t*ac[k];
 }
 
@@ -69,10 +85,11 @@ PG_TF void edge_edge(const float *p1, const float *q1, const float *p2, const fl
   for (int k = 0; k < 3; k ++) { d1[k] = q1[k] - p1[k]; d2[k] = q2[k] - p2[k]; r[k] = p1[k] - p2[k]; }
   const float a = dot(d1, d1), e = dot(d2, d2), f = dot(d2, r), c = dot(d1, r), b = dot(d1, d2);
   const float den = a*e - b*b;
-  float s = den > 1e-6f*a*e ? clamp01((b*f - c*e) / den) : 0.0f;
-  float t = (b*s + f) / e;
-  if (t < 0.0f) { t = 0.0f; s = clamp01(-c / a); }
-  else if (t > 1.0f) { t = 1.0f; s = clamp01((b - c) / a); }
+  float s = den > 1e-6f*a*e ? clamp01(quot(b*f - c*e, den)) : 0.0f;
+  float t = quot(b*s + f, e);
+  const bool low = t < 0.0f, high = t > 1.0f;
+  if (low || high) s = clamp01(quot(low ? -c : b - c, a));
+  t = clamp01(t);
   for (int k = 0; k < 3; k ++) w[k] = (p1[k] + s*d1[k]) - (p2[k] + t*d2[k]);
 }
 
@@ -130,14 +147,14 @@ PG_TF int judge(const float a[3][3], const float b[3][3], float ea, float eb, fl
       lo = mn(dot(w, A[m]), dot(w, A[m1])) - mx(dot(w, B[n]), dot(w, B[n1]));
     }
     const float w2 = dot(w, w);
-    lb[i] = w2 > 1e-36f ? lo / sqrtf(w2) : 0.0f;
+    lb[i] = w2 > 1e-36f ? lo * iroot(w2) : 0.0f;
     if (w2 < best) { best = w2; for (int k = 0; k < 3; k ++) bw[k] = w[k]; }
   }
   if (!(best < 3e38f)) return FULL;
-  const float d = sqrtf(best);
-  float la = mn(mn(dot(bw, A[0]), dot(bw, A[1])), dot(bw, A[2]));
+  const float d = best > 1e-36f ? best * iroot(best) : 0.0f;
+  const float la = mn(mn(dot(bw, A[0]), dot(bw, A[1])), dot(bw, A[2]));
   const float hb = mx(mx(dot(bw, B[0]), dot(bw, B[1])), dot(bw, B[2]));
-  const float gap = best > 1e-36f ? (la - hb) / d : 0.0f;
+  const float gap = best > 1e-36f ? (la - hb) * iroot(best) : 0.0f;
   if (gap - tol > reach * 1.000001f) return APART;
   if (!(gap > tol)) return FULL;
   const float up = d * 1.000001f + tol;
