@@ -726,6 +726,12 @@ template <typename T>
 __device__ bool grid_scan(const PgDev &d, T *a, int n, T *bs, T *sh)
 {
   const int tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+  if (tiles <= 4)
+  {
+    // one block scans a few tiles in less than two grid barriers take
+    if (blockIdx.x == 0) block_scan_seq(a, n, sh);
+    return grid_barrier(d);
+  }
   for (int t = blockIdx.x; t < tiles; t += gridDim.x)
   {
     const T s = scan_tile_sum(a, n, t, sh);
@@ -760,7 +766,9 @@ template <int B, class Hook>
 __device__ bool rebuild_all(const PgDev &d, int passes, int epasses, RebuildSmem<B> &sm, Hook hook)
 {
   const int gsz = gridDim.x * B;
-  const int g0 = blockIdx.x * B + threadIdx.x;
+  // warps are dealt to the blocks in turn, so that a small scene's spheres
+  // spread over the grid (one warp a block) instead of filling its first blocks
+  const int g0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
   const int E = d.ellnum, P = d.parnum, T = d.trinum;
   for (int s = g0; s < E; s += gsz) { rb_clear_item(d, s); hook(d, s); }
   for (int t = g0; t < T; t += gsz) rb_tref_item(d, t);
@@ -776,6 +784,21 @@ __device__ bool rebuild_all(const PgDev &d, int passes, int epasses, RebuildSmem
   }
   if (!grid_barrier(d)) return false;
   const int nb = d.nsortblocks;
+  if (nb == 1)
+  {
+    // one tile: one block sorts it without grid barriers
+    if (blockIdx.x == 0)
+      for (int p = 0; p < passes; p ++)
+      {
+        unsigned *ks = (p & 1) ? d.keys[1] : d.keys[0], *kd = (p & 1) ? d.keys[0] : d.keys[1];
+        int *vs = (p & 1) ? d.vals[1] : d.vals[0], *vd = (p & 1) ? d.vals[0] : d.vals[1];
+        sort_hist_tile(ks, E, d.hist, 1, 8 * p, 0, sm.h);
+        block_scan_seq(d.hist, 256, sm.part);
+        sort_scatter_tile(ks, vs, kd, vd, E, d.hist, 1, 8 * p, 0, sm.sc.wcnt, sm.sc.goff);
+      }
+    if (!grid_barrier(d)) return false;
+  }
+  else
   for (int p = 0; p < passes; p ++)
   {
     unsigned *ks = (p & 1) ? d.keys[1] : d.keys[0], *kd = (p & 1) ? d.keys[0] : d.keys[1];
@@ -950,6 +973,63 @@ __device__ __forceinline__ void tail_item(const PgDev &d, double step, int use_r
     *d.stepno = row + 1;
     *d.gstep = gs + 1;
   }
+}
+
+// The end of a step: the tail, and the work queue of the FP64 contacts emptied
+// for the next one.  In a grid of one wave of blocks it runs inside the
+// particle update's launch: every block calls step_done, and the last one (a
+// counter that it resets) runs it, after every block has read the step
+// counter, the scene gravity and the old obstacle points; that saves a launch
+// (3 us a step).  In a larger grid the blocks' fences cost more (5% of the
+// update over 810,000 shaken spheres) and it has its own launch.
+// (Calls out of line: the update's registers and its straight line of
+// instructions stay its own.)
+static __device__ __noinline__ bool obstacles_front(const PgDev &d, int t, double step)
+{
+  return obstacles_item(d, t, step, 1);
+}
+
+static __device__ __noinline__ void step_end(const PgDev &d, double step)
+{
+  *d.obs_done = 0;
+  if (d.cwork_n) *d.cwork_n = 0;
+  if (d.hs)
+  {
+    // adaptive: the obstacles move by (step0 + step1)/2; step1 is recorded
+    // for the host and becomes the next step's step0
+    const double h1 = d.hs[1];
+    const double st = 0.5*(d.hs[0] + h1);
+    d.hrec[*d.stepno] = h1;
+    tail_item(d, st, 1);
+    d.hs[0] = h1;
+    return;
+  }
+  tail_item(d, step, 1);
+}
+
+__device__ __forceinline__ void step_done(const PgDev &d, double step, int last)
+{
+  if (!last) return;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(d.obs_done, 1) != (int)gridDim.x - 1) return;
+  __threadfence();
+  step_end(d, step);
+}
+
+// The scene gravities of a step, taken by the first blocks of its first
+// kernel (`blocks` of them, beside the kernel's own work, which does not read
+// them): true when the block is one of them.  Saves k_excite's launch, and
+// the chain of sines of a pool's excitation (12 us) runs beside the contacts.
+static __device__ __noinline__ void excite_scene(const PgDev &d, int sc, double step) { excite_item(d, sc, step); }
+
+__device__ __forceinline__ bool excite_front(const PgDev &d, int blocks, double step)
+{
+  if ((int)blockIdx.x >= blocks) return false;
+  const int sc = blockIdx.x * blockDim.x + threadIdx.x;
+  if (sc < d.nscene) excite_scene(d, sc, step);
+  return true;
 }
 
 } // namespace pgk

@@ -10,9 +10,9 @@ void pg_launch_iso_flags(const PgDev &d, cudaStream_t s, int p0, int p1);   // i
 void pg_launch_euler(const PgDev &d, cudaStream_t s, double step);
 void pg_launch_shapes(const PgDev &d, cudaStream_t s, bool skip_analytical);
 void pg_launch_obstacles_state(const PgDev &d, cudaStream_t s, double step);   // velocities from obsang/obslin
-void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step);
+void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_step = false);
 int pg_contacts_kernel_count(const PgDev &d);   // launches of one contact evaluation (either form)
-void pg_launch_springs(const PgDev &d, cudaStream_t s, double step);
+void pg_launch_springs(const PgDev &d, cudaStream_t s, double step, bool in_step = false);
 void pg_launch_spring_runs(const PgDev &d, cudaStream_t s);     // sums of the long flush runs
 void pg_launch_unspring(const PgDev &d, cudaStream_t s);        // UNSPRING rules, after the springs
 void pg_launch_torsion(const PgDev &d, cudaStream_t s, double step);   // torsion springs, before the force sums
@@ -32,18 +32,18 @@ void pg_launch_eqm_one(const PgDev &d, cudaStream_t s, int part2, const double *
 void pg_launch_restrain_velocities(const PgDev &d, cudaStream_t s);   // once per DEM call
 void pg_launch_restrain_forces(const PgDev &d, cudaStream_t s);       // drop-in export (fused steps do it in k_integrate)
 void pg_launch_mesh(const PgDev &d, cudaStream_t s);
-void pg_launch_obstacles_row(const PgDev &d, cudaStream_t s, double step);     // velocities from the step table
-void pg_launch_tail(const PgDev &d, cudaStream_t s, double step);
-void pg_launch_obstacles_tail(const PgDev &d, cudaStream_t s, double step);  // both, one launch when it can
-int pg_obstacles_kernel_count(const PgDev &d);
+void pg_launch_obstacles_tail(const PgDev &d, cudaStream_t s, double step);  // of a step without particles
 void pg_launch_excite(const PgDev &d, cudaStream_t s, double step);
 int  pg_step_kernel_count(const PgDev &d);
+void pg_launch_step_end(const PgDev &d, cudaStream_t s, double step);   // where the integration's launch does not
+// whether the integration's launch ends the step: a grid of one wave
+#define PG_MX_BLOCKS 8
+static inline int pg_ends_step(int blocks, int per_sm) { return blocks <= 152 * per_sm; }
 
 // pg_mixed.cu
 void pg_launch_mx_from64(const PgDev &d, cudaStream_t s, int p0 = 0, int p1 = -1, int e0 = 0, int e1 = -1);
 void pg_launch_mx_inertia(const PgDev &d, cudaStream_t s);
 void pg_launch_mx_to64(const PgDev &d, cudaStream_t s, int p0 = 0, int p1 = -1);
-void pg_launch_mx_centres(const PgDev &d, cudaStream_t s);   // before a due rebuild
 void pg_launch_contacts_mx(const PgDev &d, cudaStream_t s, double step);
 void pg_launch_integrate_mx(const PgDev &d, cudaStream_t s, double step);
 // the persistent fused step of the mixed form: shape index into the kernel

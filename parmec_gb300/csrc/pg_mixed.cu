@@ -32,7 +32,7 @@ inline int nblk(int n) { return (n + TPB - 1) / TPB; }
 // contact and integration kernels (latency-bound gathers: more resident
 // warps keep more loads in flight)
 #ifndef PG_MX_MIN_BLOCKS
-#define PG_MX_MIN_BLOCKS 8
+#define PG_MX_MIN_BLOCKS PG_MX_BLOCKS
 #endif
 
 __device__ __forceinline__ void set_err(const PgDev &d, int code, int site, int index, int value)
@@ -179,28 +179,6 @@ __global__ void k_mx_inertia(PgDev d)
   d.mass_f[i] = (float)d.mass[i];
   d.invm_f[i] = (float)d.invm[i];
   set_iso(d, i);
-}
-
-// sphere centres (FP64, for the rebuild's keys and distance tests) and their
-// FP32 reference copies, from the particle position pairs; only when a
-// rebuild is due -- between rebuilds the mixed step never reads them
-__device__ __forceinline__ void mx_centres_item(const PgDev &d, int e)
-{
-  const int p = d.part[e];
-  for (int c = 0; c < 3; c ++)
-  {
-    d.center[c][e] = df_to({d.xh[c][p], d.xl[c][p]});
-    d.cref_f[c][e] = d.xh[c][p];
-  }
-}
-
-// launched every step and idle unless a rebuild is due: a grid-stride loop
-// over a grid of a few blocks per SM, so that the idle launch is short
-__global__ void k_mx_centres(PgDev d)
-{
-  if (!*d.rebuild) return;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < d.ellnum; e += gridDim.x * blockDim.x)
-    mx_centres_item(d, e);
 }
 
 __global__ void k_mx_to64(PgDev d, int p0, int p1)
@@ -400,9 +378,10 @@ __device__ __forceinline__ bool mx_contacts_item(const PgDev &d, int i, double s
 // the sphere partners of every sphere; spheres whose lists go on with
 // triangles are queued for k_tri_mx (queue order does not matter: each
 // sphere's triangles are evaluated by one thread, in list order)
-__global__ void __launch_bounds__(TPB, PG_MX_MIN_BLOCKS) k_contacts_mx(PgDev d, double step_d)
+__global__ void __launch_bounds__(TPB, PG_MX_MIN_BLOCKS) k_contacts_mx(PgDev d, double step_d, int xblocks)
 {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pgk::excite_front(d, xblocks, step_d)) return;
+  int i = (blockIdx.x - xblocks) * blockDim.x + threadIdx.x;
   bool more = false;
   if (i < d.ellnum) more = mx_contacts_item<MX_SPHERES>(d, i, step_d);
   pgk::tri_queue_push(d, more, i);
@@ -568,12 +547,23 @@ __device__ __forceinline__ bool mx_integrate_item(const PgDev &d, int i, double 
   return need;
 }
 
-__global__ void __launch_bounds__(TPB, PG_MX_MIN_BLOCKS) k_integrate_mx(PgDev d, double step_d)
+__global__ void __launch_bounds__(TPB, PG_MX_MIN_BLOCKS) k_integrate_mx(PgDev d, double step_d, int oblocks, int last)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // the first blocks move the obstacle triangles; `last`: the last block to
+  // finish ends the step
   bool need = false;
-  if (i < d.parnum) need = mx_integrate_item(d, i, step_d);
+  if ((int)blockIdx.x < oblocks)
+  {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < d.trinum) need = pgk::obstacles_front(d, t, step_d);
+  }
+  else
+  {
+    const int i = (blockIdx.x - oblocks) * blockDim.x + threadIdx.x;
+    if (i < d.parnum) need = mx_integrate_item(d, i, step_d);
+  }
   if (d.ellnum) flag_rebuild(d, need);
+  pgk::step_done(d, step_d, last);
 }
 
 // ------------------------------------------------------------ fused step
@@ -668,8 +658,7 @@ cudaError_t pg_launch_fused_mx(const PgDev &d, cudaStream_t s, double step, int 
   cfg.numAttrs = 1;
   for (int k = 0; k < nsteps; k ++)
   {
-    // the rebuild, when flagged (both return at once otherwise)
-    pg_launch_mx_centres(d, s);
+    // the rebuild, when flagged (it returns at once otherwise)
     pg_launch_rebuild(d, s);
     cudaError_t e = cudaMemsetAsync(d.gbar, 0, 4 * sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
@@ -698,29 +687,19 @@ void pg_launch_mx_to64(const PgDev &d, cudaStream_t s, int p0, int p1)
   if (p1 > p0) k_mx_to64<<<nblk(p1 - p0), TPB, 0, s>>>(d, p0, p1);
 }
 
-void pg_launch_mx_centres(const PgDev &d, cudaStream_t s)
-{
-  static int cap = 0;
-  if (!cap)
-  {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cap = 4 * (sms > 0 ? sms : 152);
-  }
-  const int nb = nblk(d.ellnum);
-  if (d.ellnum) k_mx_centres<<<nb < cap ? nb : cap, TPB, 0, s>>>(d);
-}
-
 void pg_launch_contacts_mx(const PgDev &d, cudaStream_t s, double step)
 {
-  if (!d.ellnum) return;
-  k_contacts_mx<<<nblk(d.ellnum), TPB, 0, s>>>(d, step);
-  const int nb = nblk(d.ellnum);
+  if (!d.ellnum) { pg_launch_excite(d, s, step); return; }
+  const int nb = nblk(d.ellnum), xb = nblk(d.nscene);
+  k_contacts_mx<<<xb + nb, TPB, 0, s>>>(d, step, xb);
   k_tri_mx<<<nb < pgk::TRI_PASS_BLOCKS ? nb : pgk::TRI_PASS_BLOCKS, TPB, 0, s>>>(d, step);
 }
 
 void pg_launch_integrate_mx(const PgDev &d, cudaStream_t s, double step)
 {
-  if (d.parnum) k_integrate_mx<<<nblk(d.parnum), TPB, 0, s>>>(d, step);
+  if (!d.parnum) { pg_launch_obstacles_tail(d, s, step); return; }
+  const int ob = d.obsnum ? nblk(d.trinum) : 0;
+  const int nb = ob + nblk(d.parnum), last = pg_ends_step(nb, PG_MX_BLOCKS);
+  k_integrate_mx<<<nb, TPB, 0, s>>>(d, step, ob, last);
+  if (!last) pg_launch_step_end(d, s, step);
 }

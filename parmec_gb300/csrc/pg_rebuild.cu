@@ -23,6 +23,7 @@
 #include <cmath>
 #include "pg_state.h"
 #include "pg_math.cuh"
+#include "pg_df.cuh"
 #include "pg_launch.h"
 #include "pg_items.cuh"
 #include "../../include/parmec_gb300.h"
@@ -35,6 +36,23 @@ inline int nblk(int n) { return (n + TPB - 1) / TPB; }
 
 using namespace pgk;
 
+// Mixed form: sphere centres (FP64, for the keys and distance tests) and
+// their FP32 reference copies from the particle position pairs; between
+// rebuilds the mixed step never reads them
+struct Centres
+{
+  __device__ void operator()(const PgDev &d, int e) const
+  {
+    if (d.form != PG_FORM_MIXED) return;
+    const int p = d.part[e];
+    for (int c = 0; c < 3; c ++)
+    {
+      d.center[c][e] = pg::df_to({d.xh[c][p], d.xl[c][p]});
+      d.cref_f[c][e] = d.xh[c][p];
+    }
+  }
+};
+
 // the whole rebuild as one cooperative launch; returns at once (one empty
 // launch per step) unless a rebuild is due
 template <int B>
@@ -42,7 +60,7 @@ __global__ void __launch_bounds__(B) k_rebuild_coop(PgDev d, int passes, int epa
 {
   __shared__ RebuildSmem<B> sm;
   if (!d.ellnum || !*(volatile int *)d.rebuild) return;
-  rebuild_all<B>(d, passes, epasses, sm, NoHook());
+  rebuild_all<B>(d, passes, epasses, sm, Centres());
 }
 
 // self-test of the bounded grid barrier: the host presets the arrival count
@@ -158,8 +176,12 @@ cudaError_t pg_launch_barrier_probe(const PgDev &d, cudaStream_t s, int blocks)
 void pg_launch_rebuild(const PgDev &d, cudaStream_t s)
 {
   if (!d.ellnum) return;
+  // no more blocks than there are warps of spheres, particles or triangles:
+  // the launch is idle unless a rebuild is due, and a rebuild's grid barriers
+  // are shorter with fewer blocks
+  const int n = d.ellnum > d.parnum ? d.ellnum : d.parnum, m = n > d.trinum ? n : d.trinum, w = (m + 31) / 32;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(rebuild_grid());
+  cfg.gridDim = dim3(w < rebuild_grid() ? w : rebuild_grid());
   cfg.blockDim = dim3(RB_THREADS);
   cfg.stream = s;
   cudaLaunchAttribute at[1];

@@ -924,11 +924,11 @@ void drop_graph(pg_session *s)
 
 // the fused kernel for 'n' steps, as a captured graph of 'chunk' steps per
 // replay when capture works, else as direct cooperative launches
-// kernels one fused step launches: the gated centre conversion and rebuild
-// (with spheres), then the fused step kernel
+// kernels one fused step launches: the gated rebuild (with spheres), then the
+// fused step kernel
 PgDev live_view(const pg_session *s);
 
-static int fused_kernels_per_step(const PgDev &d) { return d.ellnum ? 3 : 1; }
+static int fused_kernels_per_step(const PgDev &d) { return d.ellnum ? 2 : 1; }
 
 int run_fused(pg_session *s, double step, int n, int chunk)
 {
@@ -1064,25 +1064,23 @@ PgDev live_view(const pg_session *s)
 void enqueue_step(pg_session *s, double step)
 {
   const PgDev d = live_view(s);
-  if (d.form == PG_FORM_MIXED) pg_launch_mx_centres(d, s->stream);
+  // the scene gravities are taken beside the first of these that runs, the
+  // obstacles and the step's tail in the integration's launch
   pg_launch_rebuild(d, s->stream);
-  pg_launch_excite(d, s->stream, step);
   if (d.form == PG_FORM_MIXED)
   {
     pg_launch_contacts_mx(d, s->stream, step);
     pg_launch_integrate_mx(d, s->stream, step);
-    pg_launch_obstacles_tail(d, s->stream, step);
     return;
   }
-  pg_launch_contacts(d, s->stream, step);
-  pg_launch_springs(d, s->stream, step);
+  pg_launch_contacts(d, s->stream, step, true);
+  pg_launch_springs(d, s->stream, step, true);
   pg_launch_spring_runs(d, s->stream);
   pg_launch_torsion(d, s->stream, step);
   pg_launch_unspring(d, s->stream);
   if (d.tt_on) tt_stage(s, step);
   pg_launch_integrate(d, s->stream, step);
   pg_launch_mesh(d, s->stream);
-  pg_launch_obstacles_tail(d, s->stream, step);
 }
 
 // room for np pairs: the list arrays and the narrow phase's work are made
@@ -1287,9 +1285,8 @@ void enqueue_step_adaptive(pg_session *s)
 {
   const PgDev &d = s->d;
   pg_launch_rebuild(d, s->stream);
-  pg_launch_excite(d, s->stream, 0.0);
-  pg_launch_contacts(d, s->stream, 0.0);
-  pg_launch_springs(d, s->stream, 0.0);
+  pg_launch_contacts(d, s->stream, 0.0, true);
+  pg_launch_springs(d, s->stream, 0.0, true);
   pg_launch_spring_runs(d, s->stream);
   pg_launch_torsion(d, s->stream, 0.0);
   pg_launch_unspring(d, s->stream);
@@ -1297,19 +1294,17 @@ void enqueue_step_adaptive(pg_session *s)
   pg_launch_adapt_step(d, s->stream);
   pg_launch_dynamics_fused(d, s->stream);
   pg_launch_mesh(d, s->stream);
-  pg_launch_obstacles_tail(d, s->stream, 0.0);
 }
 
 int adaptive_kernel_count(const PgDev &d)
 {
-  int n = pg_rebuild_kernel_count(d) + 2 + 1;     // excite, select, tail
-  if (d.ellnum) n += 1;
+  int n = pg_rebuild_kernel_count(d) + 1 + pg_contacts_kernel_count(d);   // the step's selection
+  if (!d.ellnum && !d.sprnum) n += 1;             // excite
   if (d.sprnum) n += 1 + (d.nbig > 0 ? 4 : 0) + (d.unsprnum ? 1 : 0);
   if (d.trqsprnum) n += 1;
-  if (d.parnum) n += 3;                           // force sums, minimum, dynamics
+  n += d.parnum ? 3 : 1;                          // force sums, minimum, dynamics with obstacles and tail
   if (d.nodnum) n += 1;
   if (d.facnum) n += 1;
-  if (d.obsnum && d.trinum) n += 1;
   return n;
 }
 
@@ -1505,7 +1500,7 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
     if (wait) CK(cudaStreamSynchronize(s->stream));
     return PG_OK;
   }
-  const int per_step = pg_rebuild_kernel_count(d) + pg_step_kernel_count(d) + (d.form == PG_FORM_MIXED ? 1 : 0);
+  const int per_step = pg_rebuild_kernel_count(d) + pg_step_kernel_count(d);
   if (!s->profile && s->use_graph && !d.tt_on)
   {
     TRY(capture_step(s, step));
@@ -1523,7 +1518,8 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
   }
   else
   {
-    // groups: 0 rebuild, 1 contacts, 2 springs, 3 integrate, 4 mesh, 5 obstacles + tail
+    // groups: 0 rebuild, 1 contacts, 2 springs, 3 integrate (with the obstacles
+    // and the tail), 4 mesh, 5 nothing any more
     const PgDev d = live_view(s);
     const int G = 6;
     s->ring.resize((size_t)n * (G + 1));
@@ -1532,16 +1528,14 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
     {
       cudaEvent_t *ev = &s->ring[(size_t)k * (G + 1)];
       CK(cudaEventRecord(ev[0], s->stream));
-      if (d.form == PG_FORM_MIXED) pg_launch_mx_centres(d, s->stream);
       pg_launch_rebuild(d, s->stream);
-      pg_launch_excite(d, s->stream, step);
       CK(cudaEventRecord(ev[1], s->stream));
       if (d.form == PG_FORM_MIXED) pg_launch_contacts_mx(d, s->stream, step);
-      else pg_launch_contacts(d, s->stream, step);
+      else pg_launch_contacts(d, s->stream, step, true);
       CK(cudaEventRecord(ev[2], s->stream));
       if (d.form != PG_FORM_MIXED)
       {
-        pg_launch_springs(d, s->stream, step);
+        pg_launch_springs(d, s->stream, step, true);
         pg_launch_spring_runs(d, s->stream);
         pg_launch_torsion(d, s->stream, step);
         pg_launch_unspring(d, s->stream);
@@ -1553,12 +1547,11 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
       CK(cudaEventRecord(ev[4], s->stream));
       pg_launch_mesh(d, s->stream);
       CK(cudaEventRecord(ev[5], s->stream));
-      pg_launch_obstacles_tail(d, s->stream, step);
       CK(cudaEventRecord(ev[6], s->stream));
     }
     CK(cudaStreamSynchronize(s->stream));
     const int counts[6] = {pg_rebuild_kernel_count(d), pg_contacts_kernel_count(d), d.sprnum ? 1 : 0, d.parnum ? 1 : 0,
-                           (d.nodnum ? 1 : 0) + (d.facnum ? 1 : 0), pg_obstacles_kernel_count(d)};
+                           (d.nodnum ? 1 : 0) + (d.facnum ? 1 : 0), 0};
     for (int k = 0; k < n; k ++)
     {
       cudaEvent_t *ev = &s->ring[(size_t)k * (G + 1)];

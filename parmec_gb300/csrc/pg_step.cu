@@ -35,11 +35,6 @@ constexpr int TPB = 128;
 #ifndef PG_EVAL_MINB
 #define PG_EVAL_MINB 8
 #endif
-#if PG_INTEGRATE_MINB
-#define PG_LB_INTEGRATE __launch_bounds__(TPB, PG_INTEGRATE_MINB)
-#else
-#define PG_LB_INTEGRATE __launch_bounds__(TPB)
-#endif
 #if PG_EVAL_MINB
 #define PG_LB_EVAL __launch_bounds__(TPB, PG_EVAL_MINB)
 #else
@@ -47,6 +42,10 @@ constexpr int TPB = 128;
 #endif
 
 inline int nblk(int n) { return (n + TPB - 1) / TPB; }
+
+// spheres or particles up to which a launch leaves SMs idle at 32 a warp and
+// one warp a scheduler (152 SMs of four)
+#define PG_SMALL_SCENE (152 * 4 * 32)
 
 // record the first error with where it happened (site), the index and a value
 __device__ __forceinline__ void set_err(const PgDev &d, int code, int site, int index, int value)
@@ -223,67 +222,37 @@ __global__ void k_faces(PgDev d)
 }
 
 // ---------------------------------------------------------------- obstacles (obstacles.ispc:28-78)
-// velocities: row of the step table (use_row) or the current obsang/obslin state
-__global__ void k_obstacles(PgDev d, double step, int use_row)
+// with the current obsang/obslin state
+__global__ void k_obstacles(PgDev d, double step)
 {
-  if (d.hs) step = 0.5*(d.hs[0] + d.hs[1]);
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   bool need = false;
-  if (t < d.trinum) need = pgk::obstacles_item(d, t, step, use_row);
+  if (t < d.trinum) need = pgk::obstacles_item(d, t, step, 0);
   if (d.ellnum) flag_rebuild(d, need);
 }
 
-// obstacle points (after every triangle used the old point), obstacle
-// velocity state, and the step counter
-__global__ void k_tail(PgDev d, double step, int use_row)
+// obstacle points of the state-mode update, after every triangle used the old ones
+__global__ void k_tail(PgDev d, double step)
 {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (d.hs)
-  {
-    // adaptive: the obstacles move by (step0 + step1)/2; step1 is recorded
-    // for the host and becomes the next step's step0
-    const double h1 = d.hs[1];
-    step = 0.5*(d.hs[0] + h1);
-    d.hrec[use_row ? *d.stepno : 0] = h1;
-    pgk::tail_item(d, step, use_row);
-    d.hs[0] = h1;
-    return;
-  }
-  pgk::tail_item(d, step, use_row);
+  pgk::tail_item(d, step, 0);
 }
 
-// The row-mode obstacle update with the tail in the same launch: the last
-// block to finish (a counter that it resets) runs the tail, after every
-// block has read the old obstacle points and the step pair.
+// The obstacle update and tail of a step without particles (with particles
+// they run in k_integrate's launch)
 __global__ void k_obstacles_tail(PgDev d, double step)
 {
-  const double step0 = step;
-  if (d.hs) step = 0.5*(d.hs[0] + d.hs[1]);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   bool need = false;
-  if (t < d.trinum) need = pgk::obstacles_item(d, t, step, 1);
+  if (d.obsnum && t < d.trinum) need = pgk::obstacles_item(d, t, d.hs ? 0.5*(d.hs[0] + d.hs[1]) : step, 1);
   if (d.ellnum) flag_rebuild(d, need);
-  __shared__ int last;
-  __syncthreads();
-  if (threadIdx.x == 0)
-  {
-    __threadfence();
-    last = atomicAdd(d.obs_done, 1) == (int)gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last || threadIdx.x != 0) return;
-  __threadfence();
-  *d.obs_done = 0;
-  if (d.hs)
-  {
-    const double h1 = d.hs[1];
-    const double st = 0.5*(d.hs[0] + h1);
-    d.hrec[*d.stepno] = h1;
-    pgk::tail_item(d, st, 1);
-    d.hs[0] = h1;
-    return;
-  }
-  pgk::tail_item(d, step0, 1);
+  pgk::step_done(d, step, 1);
+}
+
+// the end of a step in a launch of its own
+__global__ void k_step_end(PgDev d, double step)
+{
+  if (threadIdx.x == 0) pgk::step_end(d, step);
 }
 
 using pgk::pairing;
@@ -542,7 +511,8 @@ __global__ void __launch_bounds__(TPB) k_contacts(PgDev d, double step)
 //   k_contacts_probe  one thread per sphere: the squared-distance test of
 //                     every sphere candidate; a candidate clearly apart is
 //                     settled there (an existing contact ends), every other
-//                     slot goes to the work queue (one atomic per warp);
+//                     slot goes to the work queue (one atomic per warp
+//                     and four slots);
 //   k_contacts_eval   one thread per queued slot (a grid-stride loop over
 //                     the queue): geometry, the creation/persistence rule,
 //                     contact velocities and the granular law, written to
@@ -555,20 +525,10 @@ __global__ void __launch_bounds__(TPB) k_contacts(PgDev d, double step)
 // Every slot takes the same operations as in k_contacts and the sums the
 // same order, so the results are the same bits; the queue's order plays no
 // part.
-__device__ __forceinline__ void queue_push(int *work, int *count, bool push, int idx)
+__global__ void __launch_bounds__(TPB) k_contacts_probe(PgDev d, int xblocks, double step)
 {
-  const unsigned m = __ballot_sync(__activemask(), push);
-  if (!m) return;
-  const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-  int base = 0;
-  if (lane == leader) base = atomicAdd(count, __popc(m));
-  base = __shfl_sync(__activemask(), base, leader);
-  if (push) work[base + __popc(m & ((1u << lane) - 1u))] = idx;
-}
-
-__global__ void __launch_bounds__(TPB) k_contacts_probe(PgDev d)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pgk::excite_front(d, xblocks, step)) return;
+  const int i = (blockIdx.x - xblocks) * blockDim.x + threadIdx.x;
   const int cnt = i < d.ellnum ? d.ncnt[i] : 0;
   double c[3] = {0.0, 0.0, 0.0}, ri = 0.0;
   if (cnt > 0)
@@ -583,23 +543,36 @@ __global__ void __launch_bounds__(TPB) k_contacts_probe(PgDev d)
     const int other = __shfl_xor_sync(0xffffffffu, kmax, o);
     kmax = other > kmax ? other : kmax;
   }
-  for (int k = 0; k < kmax; k ++)
+  // four candidates at a time: their codes, then their centres and radii,
+  // are loaded together, and one atomic takes their places in the queue
+  constexpr int W = 4;
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  for (int k0 = 0; k0 < kmax; k0 += W)
   {
-    bool push = false;
-    size_t idx = 0;
-    if (k < cnt)
-    {
-      idx = (size_t)k * d.estride + i;
-      const int code = d.ncode[idx];
-      push = true;
-      if (code >= 0)
+    int code[W];
+    double q[W][3], rj[W];
+    #pragma unroll
+    for (int j = 0; j < W; j ++) code[j] = k0 + j < cnt ? d.ncode[(size_t)(k0 + j) * d.estride + i] : -1;
+    #pragma unroll
+    for (int j = 0; j < W; j ++)
+      if (code[j] >= 0)
       {
-        double q[3];
-        q[0] = c[0]-d.center[0][code];
-        q[1] = c[1]-d.center[1][code];
-        q[2] = c[2]-d.center[2][code];
-        const double d2 = dot3(q, q);
-        const double sr = ri+d.radii[0][code];
+        for (int c1 = 0; c1 < 3; c1 ++) q[j][c1] = d.center[c1][code[j]];
+        rj[j] = d.radii[0][code[j]];
+      }
+    unsigned vote[W];
+    #pragma unroll
+    for (int j = 0; j < W; j ++)
+    {
+      const int k = k0 + j;
+      bool push = k < cnt;
+      const size_t idx = (size_t)k * d.estride + i;
+      if (code[j] >= 0)
+      {
+        const double w[3] = {c[0]-q[j][0], c[1]-q[j][1], c[2]-q[j][2]};
+        const double d2 = dot3(w, w);
+        const double sr = ri+rj[j];
         if (gt_nonneg(d2, (sr*sr) * (1.0 + 1e-12)))
         {
           push = false;
@@ -610,8 +583,18 @@ __global__ void __launch_bounds__(TPB) k_contacts_probe(PgDev d)
           }
         }
       }
+      vote[j] = __ballot_sync(all, push);
     }
-    queue_push(d.cwork, d.cwork_n, push, (int)idx);
+    int base = 0;
+    if (lane == 0) base = atomicAdd(d.cwork_n, __popc(vote[0]) + __popc(vote[1]) + __popc(vote[2]) + __popc(vote[3]));
+    base = __shfl_sync(all, base, 0);
+    #pragma unroll
+    for (int j = 0; j < W; j ++)
+    {
+      if (vote[j] >> lane & 1u)
+        d.cwork[base + __popc(vote[j] & ((1u << lane) - 1u))] = (int)((size_t)(k0 + j) * d.estride + i);
+      base += __popc(vote[j]);
+    }
   }
 }
 
@@ -942,9 +925,10 @@ __device__ double eqm(const PgDev &d, int part1, const double *point1, int part2
 // force is zero.  The k arm is taken in the k particle's frame (the reference
 // rotates it with the j particle's rotation, forces.ispc:1341).
 template <bool ADAPT>
-__global__ void __launch_bounds__(TPB) k_springs(PgDev d, double step)
+__global__ void __launch_bounds__(TPB) k_springs(PgDev d, double step, int xblocks)
 {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pgk::excite_front(d, xblocks, step)) return;
+  int i = (blockIdx.x - xblocks) * blockDim.x + threadIdx.x;
   if (i >= d.sprnum) return;
   if (ADAPT) step = d.hs[0];
   const double time = d.t_curtime[*d.stepno];
@@ -1506,13 +1490,31 @@ __device__ __forceinline__ double add_times_zero(double F, double m, double g)
 
 // half = step/2 and hstep = (step + step1)/2 come from the host (the same
 // IEEE operations), except where the step is chosen on the device
-template <int MODE>
-__global__ void PG_LB_INTEGRATE k_integrate(PgDev d, double step, double half, double hstep)
+// WIDE: contact entries whose loads are in flight together, and the blocks
+// asked for per SM.  A scene whose particles fill less than two blocks an SM
+// waits for its chain of loads (flag, then force and point, of one entry
+// after another): it takes four entries at a time in 2 x 24 more registers.
+// Larger ones hide one warp's loads behind the others' FP64 work and need the
+// warps: one entry at a time in 96 registers.
+template <int MODE, int WIDE>
+__global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integrate(PgDev d, double step, double half, double hstep, int oblocks, int last)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // fused modes: the first blocks move the obstacle triangles; `last`: the last
+  // block to finish ends the step
+  const int i = ((int)blockIdx.x - oblocks) * (int)blockDim.x + (int)threadIdx.x;
   bool need = false;
   constexpr bool ADAPT = MODE == INT_FORCES_ADAPT;
   constexpr bool FUSED = MODE == INT_FUSED || MODE == INT_DYN_FUSED;
+  const double step0 = step;
+  if (FUSED && i < 0)
+  {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const double st = d.hs ? 0.5*(d.hs[0] + d.hs[1]) : step;
+    if (t < d.trinum) need = pgk::obstacles_front(d, t, st);
+    if (d.ellnum) flag_rebuild(d, need);
+    pgk::step_done(d, step0, last);
+    return;
+  }
   if (MODE == INT_FORCES_ADAPT || MODE == INT_DYN_FUSED)
   {
     step = d.hs[0];
@@ -1557,16 +1559,29 @@ __global__ void PG_LB_INTEGRATE k_integrate(PgDev d, double step, double half, d
       // as k_contacts_sum sums them into fm and tm in the adaptive mode
       double fs[3] = {0.0, 0.0, 0.0}, ts[3] = {0.0, 0.0, 0.0};
       const int cnt = d.ncnt[e];
-      for (int k = 0; k < cnt; k ++)
+      for (int k0 = 0; k0 < cnt; k0 += WIDE)
       {
-        const size_t idx = (size_t)k * d.estride + e;
-        if (!d.nflag[idx]) continue;
-        const double f[3] = {d.nfrc[0][idx], d.nfrc[1][idx], d.nfrc[2][idx]};
-        const double a[3] = {d.npnt[0][idx]-po[0], d.npnt[1][idx]-po[1], d.npnt[2][idx]-po[2]};
-        fs[0] += f[0]; fs[1] += f[1]; fs[2] += f[2];
-        ts[0] += a[1]*f[2] - a[2]*f[1];
-        ts[1] += a[2]*f[0] - a[0]*f[2];
-        ts[2] += a[0]*f[1] - a[1]*f[0];
+        bool on[WIDE];
+        double f[WIDE][3], p[WIDE][3];
+        #pragma unroll
+        for (int j = 0; j < WIDE; j ++) on[j] = k0 + j < cnt && d.nflag[(size_t)(k0 + j) * d.estride + e] != 0;
+        #pragma unroll
+        for (int j = 0; j < WIDE; j ++)
+          if (on[j])
+          {
+            const size_t idx = (size_t)(k0 + j) * d.estride + e;
+            for (int c = 0; c < 3; c ++) { f[j][c] = d.nfrc[c][idx]; p[j][c] = d.npnt[c][idx]; }
+          }
+        #pragma unroll
+        for (int j = 0; j < WIDE; j ++)
+          if (on[j])
+          {
+            const double a[3] = {p[j][0]-po[0], p[j][1]-po[1], p[j][2]-po[2]};
+            fs[0] += f[j][0]; fs[1] += f[j][1]; fs[2] += f[j][2];
+            ts[0] += a[1]*f[j][2] - a[2]*f[j][1];
+            ts[1] += a[2]*f[j][0] - a[0]*f[j][2];
+            ts[2] += a[0]*f[j][1] - a[1]*f[j][0];
+          }
       }
       F[0] = fs[0]; F[1] = fs[1]; F[2] = fs[2];
       T[0] = ts[0]; T[1] = ts[1]; T[2] = ts[2];
@@ -1582,12 +1597,25 @@ __global__ void PG_LB_INTEGRATE k_integrate(PgDev d, double step, double half, d
     if (E)
     {
       const int rb = d.soff[i], re = d.soff[i+1];
-      for (int r = rb; r < re; r ++)
+      for (int r0 = rb; r0 < re; r0 += WIDE)
       {
-        const int ref = d.rref[r];
-        if (!d.nflag[ref]) continue;
-        double f[3] = {-d.nfrc[0][ref], -d.nfrc[1][ref], -d.nfrc[2][ref]};
-        double a[3] = {d.npnt[0][ref]-po[0], d.npnt[1][ref]-po[1], d.npnt[2][ref]-po[2]};
+      int refs[WIDE];
+      bool on[WIDE];
+      double fr[WIDE][3], pr[WIDE][3];
+      #pragma unroll
+      for (int j = 0; j < WIDE; j ++) refs[j] = r0 + j < re ? d.rref[r0 + j] : -1;
+      #pragma unroll
+      for (int j = 0; j < WIDE; j ++) on[j] = refs[j] >= 0 && d.nflag[refs[j]] != 0;
+      #pragma unroll
+      for (int j = 0; j < WIDE; j ++)
+        if (on[j]) for (int c = 0; c < 3; c ++) { fr[j][c] = d.nfrc[c][refs[j]]; pr[j][c] = d.npnt[c][refs[j]]; }
+      #pragma unroll
+      for (int j = 0; j < WIDE; j ++)
+      {
+        if (!on[j]) continue;
+        const int ref = refs[j];
+        double f[3] = {-fr[j][0], -fr[j][1], -fr[j][2]};
+        double a[3] = {pr[j][0]-po[0], pr[j][1]-po[1], pr[j][2]-po[2]};
         F[0] += f[0]; F[1] += f[1]; F[2] += f[2];
         T[0] += a[1]*f[2] - a[2]*f[1];
         T[1] += a[2]*f[0] - a[0]*f[2];
@@ -1620,6 +1648,7 @@ __global__ void PG_LB_INTEGRATE k_integrate(PgDev d, double step, double half, d
           nvmul(Li, a, A);
           krot_add(krot, A);
         }
+      }
       }
     }
     F[0] = add_times_zero(F[0], ma, grav[0]);
@@ -1949,6 +1978,7 @@ __global__ void PG_LB_INTEGRATE k_integrate(PgDev d, double step, double half, d
     }
   }
   if (FUSED && d.ellnum) flag_rebuild(d, need);
+  if (FUSED) pgk::step_done(d, step0, last);
 }
 
 // ---------------------------------------------------------------- torsion springs
@@ -2478,8 +2508,8 @@ void pg_launch_shapes(const PgDev &d, cudaStream_t s, bool skip_analytical)
 
 void pg_launch_obstacles_state(const PgDev &d, cudaStream_t s, double step)
 {
-  if (d.obsnum && d.trinum) k_obstacles<<<(d.trinum + 31) / 32, 32, 0, s>>>(d, step, 0);
-  if (d.obsnum) k_tail<<<1, 32, 0, s>>>(d, step, 0);
+  if (d.obsnum && d.trinum) k_obstacles<<<(d.trinum + 31) / 32, 32, 0, s>>>(d, step);
+  if (d.obsnum) k_tail<<<1, 32, 0, s>>>(d, step);
 }
 
 // the grid of the queue pass: resident blocks over every SM
@@ -2497,15 +2527,18 @@ static int eval_blocks()
   return nb;
 }
 
-void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step)
+// in_step: a session's step, whose end empties the work queue and whose scene
+// gravities (nothing else having taken them) the probe's first blocks take
+void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_step)
 {
   if (!d.ellnum) return;
   if (d.cwork && d.cwork_n)
   {
     // three passes (probe, queued evaluation, sums; the sums in k_integrate
     // unless adaptive): the same bits as k_contacts
-    cudaMemsetAsync(d.cwork_n, 0, sizeof(int), s);
-    k_contacts_probe<<<nblk(d.ellnum), TPB, 0, s>>>(d);
+    if (!in_step) cudaMemsetAsync(d.cwork_n, 0, sizeof(int), s);
+    const int B = d.ellnum <= PG_SMALL_SCENE ? 32 : TPB, xb = in_step ? (d.nscene + B - 1) / B : 0;
+    k_contacts_probe<<<xb + (d.ellnum + B - 1) / B, B, 0, s>>>(d, xb, step);
     const int nb = eval_blocks();
     if (d.hs)
     {
@@ -2521,6 +2554,7 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step)
     }
     return;
   }
+  if (in_step) pg_launch_excite(d, s, step);
   if (d.hs)
   {
     if (d.record_geometry) k_contacts<true, true><<<nblk(d.ellnum), TPB, 0, s>>>(d, step);
@@ -2540,11 +2574,18 @@ int pg_contacts_kernel_count(const PgDev &d)
   return (d.cwork && d.cwork_n) ? (d.hs ? 3 : 2) : 1;
 }
 
-void pg_launch_springs(const PgDev &d, cudaStream_t s, double step)
+// in_step: a session's step; without spheres its scene gravities are taken here
+void pg_launch_springs(const PgDev &d, cudaStream_t s, double step, bool in_step)
 {
-  if (!d.sprnum) return;
-  if (d.hs) k_springs<true><<<nblk(d.sprnum), TPB, 0, s>>>(d, step);
-  else k_springs<false><<<nblk(d.sprnum), TPB, 0, s>>>(d, step);
+  const bool excite = in_step && !d.ellnum;
+  if (!d.sprnum)
+  {
+    if (excite) pg_launch_excite(d, s, step);
+    return;
+  }
+  const int xb = excite ? nblk(d.nscene) : 0;
+  if (d.hs) k_springs<true><<<xb + nblk(d.sprnum), TPB, 0, s>>>(d, step, xb);
+  else k_springs<false><<<xb + nblk(d.sprnum), TPB, 0, s>>>(d, step, xb);
 }
 
 void pg_launch_torsion(const PgDev &d, cudaStream_t s, double step)
@@ -2576,24 +2617,46 @@ void pg_launch_spring_runs(const PgDev &d, cudaStream_t s)
   }
 }
 
+void pg_launch_step_end(const PgDev &d, cudaStream_t s, double step) { k_step_end<<<1, 32, 0, s>>>(d, step); }
+
+// a scene of few particles takes the latency-bound form in blocks of one
+// warp, so that its warps spread over the SMs
+template <int MODE>
+static void launch_integrate(const PgDev &d, cudaStream_t s, double step, double half, double hstep)
+{
+  constexpr bool fused = MODE == INT_FUSED || MODE == INT_DYN_FUSED;
+  if (!d.parnum)
+  {
+    if (fused) pg_launch_obstacles_tail(d, s, step);
+    return;
+  }
+  const bool few = d.parnum <= PG_SMALL_SCENE;
+  const int B = few ? 32 : TPB;
+  const int ob = fused && d.obsnum ? (d.trinum + B - 1) / B : 0, nb = (d.parnum + B - 1) / B;
+  const int last = pg_ends_step(ob + nb, few ? 16 : PG_INTEGRATE_MINB);
+  if (few) k_integrate<MODE, 4><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
+  else k_integrate<MODE, 1><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
+  if (fused && !last) pg_launch_step_end(d, s, step);
+}
+
 void pg_launch_integrate(const PgDev &d, cudaStream_t s, double step)
 {
-  if (d.parnum) k_integrate<INT_FUSED><<<nblk(d.parnum), TPB, 0, s>>>(d, step, 0.5*step, 0.5*(step+step));
+  launch_integrate<INT_FUSED>(d, s, step, 0.5*step, 0.5*(step+step));
 }
 
 void pg_launch_force_sums(const PgDev &d, cudaStream_t s)
 {
-  if (d.parnum) k_integrate<INT_FORCES><<<nblk(d.parnum), TPB, 0, s>>>(d, 0.0, 0.0, 0.0);
+  launch_integrate<INT_FORCES>(d, s, 0.0, 0.0, 0.0);
 }
 
 void pg_launch_dynamics(const PgDev &d, cudaStream_t s, double step0, double step1)
 {
-  if (d.parnum) k_integrate<INT_DYNAMICS><<<nblk(d.parnum), TPB, 0, s>>>(d, step0, 0.5*step0, 0.5*(step0+step1));
+  launch_integrate<INT_DYNAMICS>(d, s, step0, 0.5*step0, 0.5*(step0+step1));
 }
 
 void pg_launch_force_sums_adapt(const PgDev &d, cudaStream_t s)
 {
-  if (d.parnum) k_integrate<INT_FORCES_ADAPT><<<nblk(d.parnum), TPB, 0, s>>>(d, 0.0, 0.0, 0.0);
+  launch_integrate<INT_FORCES_ADAPT>(d, s, 0.0, 0.0, 0.0);
 }
 
 void pg_launch_adapt_step(const PgDev &d, cudaStream_t s)
@@ -2621,7 +2684,7 @@ void pg_launch_eqm_one(const PgDev &d, cudaStream_t s, int part2, const double *
 
 void pg_launch_dynamics_fused(const PgDev &d, cudaStream_t s)
 {
-  if (d.parnum) k_integrate<INT_DYN_FUSED><<<nblk(d.parnum), TPB, 0, s>>>(d, 0.0, 0.0, 0.0);
+  launch_integrate<INT_DYN_FUSED>(d, s, 0.0, 0.0, 0.0);
 }
 
 void pg_launch_restrain_velocities(const PgDev &d, cudaStream_t s)
@@ -2640,49 +2703,29 @@ void pg_launch_mesh(const PgDev &d, cudaStream_t s)
   if (d.facnum) k_faces<<<nblk(d.facnum), TPB, 0, s>>>(d);
 }
 
-void pg_launch_obstacles_row(const PgDev &d, cudaStream_t s, double step)
-{
-  // one warp per block: a few thousand triangles then spread over most SMs,
-  // each triangle's update being a chain of FP64 work
-  if (d.obsnum && d.trinum) k_obstacles<<<(d.trinum + 31) / 32, 32, 0, s>>>(d, step, 1);
-}
-
 void pg_launch_excite(const PgDev &d, cudaStream_t s, double step)
 {
   k_excite<<<nblk(d.nscene), TPB, 0, s>>>(d, step);
 }
 
-void pg_launch_tail(const PgDev &d, cudaStream_t s, double step)
-{
-  k_tail<<<1, 32, 0, s>>>(d, step, 1);
-}
-
-// the obstacle update and the tail of a step: one launch when the session
-// has the completion counter, else the two kernels
 void pg_launch_obstacles_tail(const PgDev &d, cudaStream_t s, double step)
 {
-  if (d.obsnum && d.trinum && d.obs_done) k_obstacles_tail<<<(d.trinum + 31) / 32, 32, 0, s>>>(d, step);
-  else
-  {
-    pg_launch_obstacles_row(d, s, step);
-    pg_launch_tail(d, s, step);
-  }
+  const int nb = d.obsnum ? (d.trinum + 31) / 32 : 0;
+  k_obstacles_tail<<<nb > 0 ? nb : 1, 32, 0, s>>>(d, step);
 }
 
-int pg_obstacles_kernel_count(const PgDev &d)
-{
-  return 1 + ((d.obsnum && d.trinum && !d.obs_done) ? 1 : 0);
-}
-
+// launches of a session's step beside the rebuild's
 int pg_step_kernel_count(const PgDev &d)
 {
-  int n = 1;                                   // excite
-  n += pg_contacts_kernel_count(d);            // contacts: sphere and triangle passes
+  int n = pg_contacts_kernel_count(d);         // contacts: sphere and triangle passes
+  // the scene gravities have a launch of their own only without both
+  if (!d.ellnum && !d.sprnum) n += 1;
   if (d.sprnum) n += 1 + (d.nbig > 0 ? 2 : 0) + (d.unsprnum ? 1 : 0);
   if (d.trqsprnum) n += 1;                     // torsion springs
-  if (d.parnum) n += 1;                        // integrate
+  n += 1;                                      // integrate, obstacles and (in small scenes) the step's end
+  const int nb = nblk(d.parnum) + (d.obsnum ? nblk(d.trinum) : 0);
+  if (d.parnum > PG_SMALL_SCENE && !pg_ends_step(nb, d.form == PG_FORM_MIXED ? PG_MX_BLOCKS : PG_INTEGRATE_MINB)) n += 1;
   if (d.nodnum) n += 1;
   if (d.facnum) n += 1;
-  n += pg_obstacles_kernel_count(d);           // obstacles and tail
   return n;
 }
