@@ -748,6 +748,7 @@ void forces(int, master_conpnt master[], slave_conpnt[], int parnum, double *ang
          grow(d.sbig_grp, 32 * 12 * std::max<size_t>(1, big.size()));
     if (adaptive) ok = ok && grow(d.sbig_ad, 11 * std::max<size_t>(1, big.size()));
     d.nbig = (int)big.size();
+    d.nbig_groups = pg_spring_run_groups(big);
   }
   const int Q = std::max(trqsprnum, 0);
   if (Q)

@@ -55,6 +55,7 @@ cudaError_t pg_launch_fused_mx(const PgDev &d, cudaStream_t s, double step, int 
 // pg_session.cu
 // spring flush runs longer than this are summed by k_spring_runs
 #define PG_SPRING_RUN_LONG 64
+int  pg_spring_run_groups(const std::vector<int4> &big);         // PgDev.nbig_groups
 void pg_spring_events(int P, int S, const int *sj, const int *sk, std::vector<int> &first, std::vector<int4> &ev,
                       std::vector<int4> &big);
 

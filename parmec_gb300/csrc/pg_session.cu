@@ -395,6 +395,7 @@ int upload_static(pg_session *s, const pg_scene *sc)
     TRY(h2d(s, d.sev_first, first.data(), P + 1));
     TRY(h2d(s, d.sev, evv.data(), evv.size()));
     d.nbig = (int)big.size();
+    d.nbig_groups = pg_spring_run_groups(big);
     TRY(dalloc(s, &d.sbig, std::max<size_t>(1, big.size())));
     TRY(dalloc(s, &d.sbig_sum, 6 * std::max<size_t>(1, big.size())));
     TRY(dalloc(s, &d.sbig_grp, 32 * 12 * std::max<size_t>(1, big.size())));

@@ -59,7 +59,7 @@ struct PgDev
   int4 *sbig;               // [nbig] the long runs
   double *sbig_sum;         // [nbig][6] their force and torque sums
   double *sbig_grp;         // [nbig][32][12] group partials of the long-run sums
-  int nbig;
+  int nbig, nbig_groups;    // long runs, groups of the longest
 
   // ---- adaptive time step (parmec.ispc:275-420, forces.ispc:453-596, 1248-1345)
   double *hs;               // [3]: step0, step1, factor (null: fixed step, from the kernel arguments)

@@ -12,6 +12,7 @@
 // All sums run in a fixed order (master list in partner order, then slave
 // list in master order), so results repeat bit for bit from run to run.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include "pg_state.h"
 #include "pg_math.cuh"
 #include "pg_launch.h"
@@ -1237,10 +1238,10 @@ __global__ void __launch_bounds__(TPB) k_springs(PgDev d, double step, int xbloc
 // chunks of springs in spring order (first element assigned), groups of 32
 // chunk sums in order, then the group sums in order (the first-run rule
 // applied to them).  Chunks hold 64 springs, doubled until there are at most
-// 1,024.  k_spring_run_groups runs one warp per group (grid: groups x runs):
-// lane l sums chunk 32 g + l, loading four springs at a time, and the warp
-// sums its chunk sums in lane order through shuffles; k_spring_run_totals
-// sums each run's group partials in order.  A dependent FP64 add costs tens
+// 1,024.  k_spring_run_groups runs a warp per group and value (grid: runs x
+// groups x 6): lane l sums chunk 32 g + l and the warp sums its chunk sums in
+// lane order through shuffles; k_spring_run_totals sums each run's group
+// partials in order.  A dependent FP64 add costs tens
 // of ns on this part, so the sequential depth stays near 64 + 32 + 32 adds
 // for any run length, and the groups of a run spread over the SMs.
 constexpr int RUN_GROUP = 32;
@@ -1248,7 +1249,7 @@ constexpr int RUN_MAXCHUNKS = 1024;
 constexpr int RUN_GROUPS = RUN_MAXCHUNKS / RUN_GROUP;
 constexpr int RUN_SLOT = 12;                   // doubles per group partial: 11 values, has-flag
 
-__device__ __forceinline__ int run_chunk(int len)
+__host__ __device__ __forceinline__ int run_chunk(int len)
 {
   int c = 64;
   while ((len + c - 1) / c > RUN_MAXCHUNKS) c *= 2;
@@ -1264,50 +1265,46 @@ __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups(PgDev d)
   const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch;
   if (g * RUN_GROUP >= nc) return;
   const int c = g * RUN_GROUP + lane;
-  double a[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  constexpr int W = 16;
+  double a = 0.0;
   int any = 0;
   if (c < nc)
   {
     const int b = v.y + c * ch, e = min(b + ch, v.z);
-    for (int s0 = b; s0 < e; s0 += 4)
+    for (int s0 = b; s0 < e; s0 += W)
     {
-      double x[4][6];
-      bool ok[4];
+      double x[W];
+      bool ok[W];
       #pragma unroll
-      for (int u = 0; u < 4; u ++)
+      for (int u = 0; u < W; u ++)
       {
         const int sp = s0 + u < e ? s0 + u : b;
         ok[u] = s0 + u < e && !(type == 1 && d.sprpart[1][sp] < 0);
-        x[u][0] = d.spr_out[0][sp]; x[u][1] = d.spr_out[1][sp]; x[u][2] = d.spr_out[2][sp];
-        x[u][3] = d.spr_out[off][sp]; x[u][4] = d.spr_out[off+1][sp]; x[u][5] = d.spr_out[off+2][sp];
+        x[u] = value[sp];
       }
       #pragma unroll
-      for (int u = 0; u < 4; u ++)
+      for (int u = 0; u < W; u ++)
         if (ok[u])
         {
-          if (!any) for (int k = 0; k < 6; k ++) a[k] = x[u][k];
-          else for (int k = 0; k < 6; k ++) a[k] = a[k] + x[u][k];
+          a = any ? a + x[u] : x[u];
           any = 1;
         }
     }
   }
-  double gs[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  double gs = 0.0;
   int gany = 0;
   for (int l = 0; l < RUN_GROUP; l ++)
   {
-    const int la = __shfl_sync(full, any, l);
-    double x[6];
-    for (int k = 0; k < 6; k ++) x[k] = __shfl_sync(full, a[k], l);
-    if (!la) continue;
-    if (!gany) for (int k = 0; k < 6; k ++) gs[k] = x[k];
-    else for (int k = 0; k < 6; k ++) gs[k] = gs[k] + x[k];
+    const double x = __shfl_sync(full, a, l);
+    if (!(has >> l & 1u)) continue;
+    gs = gany ? gs + x : x;
     gany = 1;
   }
   if (lane == 0)
   {
     double *o = d.sbig_grp + ((size_t)run * RUN_GROUPS + g) * RUN_SLOT;
-    for (int k = 0; k < 6; k ++) o[k] = gs[k];
-    o[11] = gany ? 1.0 : 0.0;
+    o[q] = gs;
+    if (q == 0) o[11] = gany ? 1.0 : 0.0;
   }
 }
 
@@ -1317,18 +1314,24 @@ __global__ void k_spring_run_totals(PgDev d)
   if (run >= d.nbig) return;
   const int4 v = d.sbig[run];
   const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch, ng = (nc + RUN_GROUP - 1) / RUN_GROUP;
-  double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  const double *o = d.sbig_grp + (size_t)run * RUN_GROUPS * RUN_SLOT;
+  double acc = 0.0;
   bool started = false;
-  for (int q = 0; q < ng; q ++)
+  #pragma unroll 8
+  for (int g = 0; g < ng; g ++)
   {
-    const double *o = d.sbig_grp + ((size_t)run * RUN_GROUPS + q) * RUN_SLOT;
-    if (o[11] == 0.0) continue;
-    if (!started && !v.w) for (int k = 0; k < 6; k ++) acc[k] = o[k];
-    else for (int k = 0; k < 6; k ++) acc[k] = acc[k] + o[k];
+    const double x = o[g * RUN_SLOT + q], has = o[g * RUN_SLOT + 11];
+    if (has == 0.0) continue;
+    acc = !started && !v.w ? x : acc + x;
     started = true;
   }
-  for (int k = 0; k < 6; k ++) d.sbig_sum[6*run + k] = acc[k];
+  d.sbig_sum[6*run + q] = acc;
 }
+// One of the six sums a block (grid z): the adds of a warp hold the FP64 pipe
+// for 64 clocks each, so a lane that sums all six values of its chunk takes
+// 384 of them in a row, and the warp 192 more for the group; with one value a
+// warp it is 64 and 32, and 16 loads are in flight (32.6 -> 8 us for the 9,216
+// springs of the 96x96 lattice's plate).
 
 // Adaptive stiffness partials of the long runs, in the levels of the force
 // sums: each chunk sums its springs' terms from zero in spring order (maxima
@@ -1337,7 +1340,8 @@ __global__ void k_spring_run_totals(PgDev d)
 __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups_adapt(PgDev d)
 {
   const unsigned full = 0xffffffffu;
-  const int run = blockIdx.x, g = blockIdx.y, lane = threadIdx.x;
+  const double *value = d.spr_out[q < 3 ? q : off + q - 3];
+  const int run = blockIdx.x, g = blockIdx.y, q = blockIdx.z, lane = threadIdx.x;
   const int4 v = d.sbig[run];
   const int type = v.x & 1, off = type == 0 ? 5 : 11;
   const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch;
@@ -1367,6 +1371,8 @@ __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups_adapt(PgDev d)
     gq[9] = x[9] > gq[9] ? x[9] : gq[9];
     gq[10] = x[10] > gq[10] ? x[10] : gq[10];
   }
+  const unsigned has = __ballot_sync(full, any);
+  #pragma unroll
   if (lane == 0)
   {
     double *o = d.sbig_grp + ((size_t)run * RUN_GROUPS + g) * RUN_SLOT;
@@ -1376,7 +1382,7 @@ __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups_adapt(PgDev d)
 
 __global__ void k_spring_run_totals_adapt(PgDev d)
 {
-  const int run = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, run = t / 6, q = t % 6;
   if (run >= d.nbig) return;
   const int4 v = d.sbig[run];
   const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch, ng = (nc + RUN_GROUP - 1) / RUN_GROUP;
@@ -1385,6 +1391,7 @@ __global__ void k_spring_run_totals_adapt(PgDev d)
   {
     const double *o = d.sbig_grp + ((size_t)run * RUN_GROUPS + r) * RUN_SLOT;
     for (int k = 0; k < 9; k ++) p[k] = p[k] + o[k];
+// one thread per run and value
     km = o[9] > km ? o[9] : km;
     em = o[10] > em ? o[10] : em;
   }
@@ -2558,6 +2565,18 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
   if (d.hs)
   {
     if (d.record_geometry) k_contacts<true, true><<<nblk(d.ellnum), TPB, 0, s>>>(d, step);
+// groups of the longest of the long runs, at least 1
+int pg_spring_run_groups(const std::vector<int4> &big)
+{
+  int most = 1;
+  for (const int4 &v : big)
+  {
+    const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch;
+    most = std::max(most, (nc + RUN_GROUP - 1) / RUN_GROUP);
+  }
+  return most;
+}
+
     else k_contacts<false, true><<<nblk(d.ellnum), TPB, 0, s>>>(d, step);
   }
   else if (d.record_geometry) k_contacts<true, false><<<nblk(d.ellnum), TPB, 0, s>>>(d, step);
@@ -2606,10 +2625,10 @@ void pg_launch_unspring(const PgDev &d, cudaStream_t s)
 void pg_launch_spring_runs(const PgDev &d, cudaStream_t s)
 {
   if (!(d.sprnum && d.nbig > 0)) return;
-  const dim3 grid(d.nbig, RUN_GROUPS);      // runs on x: no 65,535 limit on their count
+  const dim3 grid(d.nbig, d.nbig_groups);   // runs on x: no 65,535 limit on their count
   const int tb = (d.nbig + 127) / 128;
-  k_spring_run_groups<<<grid, RUN_GROUP, 0, s>>>(d);
-  k_spring_run_totals<<<tb, 128, 0, s>>>(d);
+  k_spring_run_groups<<<dim3(d.nbig, d.nbig_groups, 6), RUN_GROUP, 0, s>>>(d);
+  k_spring_run_totals<<<(6*d.nbig + 127) / 128, 128, 0, s>>>(d);
   if (d.hs)
   {
     k_spring_run_groups_adapt<<<grid, RUN_GROUP, 0, s>>>(d);
