@@ -599,6 +599,196 @@ __global__ void __launch_bounds__(TPB) k_contacts_probe(PgDev d, int xblocks, do
   }
 }
 
+// geometry, the creation/persistence rule, contact velocities and the granular
+// law of one candidate entry, written to its slot
+template <bool GEOM, bool ADAPT>
+__device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double step, bool obsc)
+{
+  const size_t idx = (size_t)idx0;
+  const int i = idx0 % d.estride;
+  const int pi = d.part[i];
+  double x[3], v[3], oi[3], c[3];
+  for (int k = 0; k < 3; k ++)
+  {
+    x[k] = d.position[k][pi];
+    v[k] = d.linear[k][pi];
+    oi[k] = d.angular[3+k][pi];
+    c[k] = d.center[k][i];
+  }
+  const double ri = d.radii[0][i];
+  const int coli = d.ellcol[i];
+  const double invmi = d.invm[pi], massi = d.mass[pi];
+  const int code = d.ncode[idx];
+  const bool existing = d.nflag[idx] != 0;
+  double point[3], normal[3], depth = 0.0, q[3], len = 0.0;
+  int pj, colj;
+  bool apart;
+  bool sphere = code >= 0;
+  double cj[3];
+  if (sphere)
+  {
+    const int j = code;
+    pj = d.part[j];
+    colj = d.ellcol[j];
+    cj[0] = d.center[0][j]; cj[1] = d.center[1][j]; cj[2] = d.center[2][j];
+    q[0] = c[0]-cj[0];
+    q[1] = c[1]-cj[1];
+    q[2] = c[2]-cj[2];
+    const double d2 = dot3(q, q);
+    const double sr = ri+d.radii[0][j];
+    apart = gt_nonneg(d2, (sr*sr) * (1.0 + 1e-12));
+    if (!apart)
+    {
+      len = sqrt(d2);
+      depth = sr - len;
+    }
+  }
+  else
+  {
+    const int t = -code-1;
+    double A[3], B[3], C[3];
+    for (int kk = 0; kk < 3; kk ++) { A[kk] = d.tri[kk][t]; B[kk] = d.tri[3+kk][t]; C[kk] = d.tri[6+kk][t]; }
+    triangle_closest(A, B, C, c, point, (d.compat & PG_COMPAT_TRIEDGE) != 0);
+    q[0] = c[0]-point[0];
+    q[1] = c[1]-point[1];
+    q[2] = c[2]-point[2];
+    const double d2 = dot3(q, q);
+    apart = gt_nonneg(d2, (ri*ri) * (1.0 + 1e-12));
+    if (!apart)
+    {
+      len = sqrt(d2);
+      depth = ri - len;
+    }
+    pj = d.triobs[t];
+    colj = d.tricol[t];
+  }
+  const bool active = !apart && (existing ? !lt_zero_d(depth) : gt_zero_d(depth));
+  if (!active)
+  {
+    if (existing)
+    {
+      d.nflag[idx] = 0;
+      d.nstate[0][idx] = 0.0; d.nstate[1][idx] = 0.0; d.nstate[2][idx] = 0.0;
+    }
+    return;
+  }
+  if (sphere)
+  {
+    double ilen = existing ? 1.0/len : (gt_zero_d(len) ? 1.0/len : 1.0);
+    point[0] = 0.5*(c[0]+cj[0]);
+    point[1] = 0.5*(c[1]+cj[1]);
+    point[2] = 0.5*(c[2]+cj[2]);
+    normal[0] = ilen*q[0];
+    normal[1] = ilen*q[1];
+    normal[2] = ilen*q[2];
+  }
+  else
+  {
+    double ilen = 1.0/len;
+    normal[0] = ilen*q[0];
+    normal[1] = ilen*q[1];
+    normal[2] = ilen*q[2];
+  }
+
+  // contact point velocities (forces.ispc:226-279)
+  double z[3], vi[3], vj[3], oj[3], vij[3];
+  z[0] = point[0]-x[0]; z[1] = point[1]-x[1]; z[2] = point[2]-x[2];
+  vi[0] = oi[1]*z[2]-oi[2]*z[1] + v[0];
+  vi[1] = oi[2]*z[0]-oi[0]*z[2] + v[1];
+  vi[2] = oi[0]*z[1]-oi[1]*z[0] + v[2];
+  if (pj >= 0)
+  {
+    z[0] = point[0]-d.position[0][pj];
+    z[1] = point[1]-d.position[1][pj];
+    z[2] = point[2]-d.position[2][pj];
+    oj[0] = d.angular[3][pj]; oj[1] = d.angular[4][pj]; oj[2] = d.angular[5][pj];
+    vj[0] = oj[1]*z[2]-oj[2]*z[1] + d.linear[0][pj];
+    vj[1] = oj[2]*z[0]-oj[0]*z[2] + d.linear[1][pj];
+    vj[2] = oj[0]*z[1]-oj[1]*z[0] + d.linear[2][pj];
+  }
+  else
+  {
+    int l = -pj-2;
+    if (obsc && l >= 0) l = l+1;
+    if (l >= 0 && l < d.obsnum)
+    {
+      z[0] = point[0]-d.obspnt[3*l];
+      z[1] = point[1]-d.obspnt[3*l+1];
+      z[2] = point[2]-d.obspnt[3*l+2];
+      oj[0] = d.obsang[3*l]; oj[1] = d.obsang[3*l+1]; oj[2] = d.obsang[3*l+2];
+      vj[0] = oj[1]*z[2]-oj[2]*z[1] + d.obslin[3*l];
+      vj[1] = oj[2]*z[0]-oj[0]*z[2] + d.obslin[3*l+1];
+      vj[2] = oj[0]*z[1]-oj[1]*z[0] + d.obslin[3*l+2];
+    }
+    else
+    {
+      vj[0] = vj[1] = vj[2] = 0.0;
+    }
+  }
+  vij[0] = vj[0] - vi[0];
+  vij[1] = vj[1] - vi[1];
+  vij[2] = vj[2] - vi[2];
+
+  const int ij = pairing(d, coli, colj);
+  if (d.ikind[ij] != 0) set_err(d, PG_ERR_UNSUPPORTED, 4, i, ij);
+
+  // granular force (forces.ispc:125-192)
+  double state[3];
+  if (existing) { state[0] = d.nstate[0][idx]; state[1] = d.nstate[1][idx]; state[2] = d.nstate[2][idx]; }
+  else { state[0] = 0.0; state[1] = 0.0; state[2] = 0.0; }
+  double kn = d.iparam[0][ij];
+  double en;
+  if (d.nen) en = d.nen[idx];
+  else
+  {
+    double ma = pj >= 0 ? 1.0 / (invmi + d.invm[pj]) : massi;
+    en = d.iparam[1][ij] * 2.0 * sqrt(kn*ma);
+  }
+  double vn = dot3(vij, normal);
+  double fn = kn*depth + en*vn;
+  double f[3];
+  f[0] = fn*normal[0];
+  f[1] = fn*normal[1];
+  f[2] = fn*normal[2];
+  double kskn = d.iparam[6][ij];
+  double kt = kn * kskn;
+  double et = en * kskn;
+  double mus = d.iparam[2][ij];
+  double mud = d.iparam[3][ij];
+  double vt[3], ft[3];
+  vt[0] = vij[0] - vn*normal[0];
+  vt[1] = vij[1] - vn*normal[1];
+  vt[2] = vij[2] - vn*normal[2];
+  state[0] += step*vt[0];
+  state[1] += step*vt[1];
+  state[2] += step*vt[2];
+  ft[0] = kt*state[0] + et*vt[0];
+  ft[1] = kt*state[1] + et*vt[1];
+  ft[2] = kt*state[2] + et*vt[2];
+  double flen = sqrt(dot3(ft, ft));
+  double lim = mus*fn;
+  if (gt_d(flen, lim))
+  {
+    lim = mud*fn/flen;
+    ft[0] *= lim;
+    ft[1] *= lim;
+    ft[2] *= lim;
+  }
+  f[0] += ft[0];
+  f[1] += ft[1];
+  f[2] += ft[2];
+
+  d.nflag[idx] = 1;
+  d.nstate[0][idx] = state[0]; d.nstate[1][idx] = state[1]; d.nstate[2][idx] = state[2];
+  d.nfrc[0][idx] = f[0]; d.nfrc[1][idx] = f[1]; d.nfrc[2][idx] = f[2];
+  d.npnt[0][idx] = point[0]; d.npnt[1][idx] = point[1]; d.npnt[2][idx] = point[2];
+  if (GEOM || ADAPT)
+  {
+    d.nnrm[0][idx] = normal[0]; d.nnrm[1][idx] = normal[1]; d.nnrm[2][idx] = normal[2];
+  }
+  if (GEOM) d.ndep[idx] = depth;
+}
+
 template <bool GEOM, bool ADAPT>
 __global__ void PG_LB_EVAL k_contacts_eval(PgDev d, double step)
 {
@@ -606,191 +796,75 @@ __global__ void PG_LB_EVAL k_contacts_eval(PgDev d, double step)
   const int n = *d.cwork_n;
   const bool obsc = (d.compat & PG_COMPAT_OBSIDX) != 0;
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
+    contact_entry<GEOM, ADAPT>(d, d.cwork[w], step, obsc);
+}
+
+// Probe and evaluation in one launch for a scene that leaves SMs idle: one
+// warp a block takes S spheres (8, 16 or 32: as many as keep one warp a
+// scheduler over the chip), 32/S lanes testing slots of the same sphere at a
+// time, and evaluates the entries that are not apart 32 at a time from its own
+// list.  The queue's atomics, its round trip through memory and a launch are
+// saved; each warp's chain of loads is what bounds these scenes.  (216
+// spheres: 23 -> 15 us, 4,096: 26 -> 16 us for the contacts of a step.)  The
+// operations of an entry are those of the two passes.
+template <bool GEOM, bool ADAPT>
+__global__ void __launch_bounds__(32) k_contacts_few(PgDev d, double step, int S, int xblocks)
+{
+  if (pgk::excite_front(d, xblocks, step)) return;
+  constexpr unsigned all = 0xffffffffu;
+  __shared__ int list[64];
+  if (ADAPT) step = d.hs[0];
+  const bool obsc = (d.compat & PG_COMPAT_OBSIDX) != 0;
+  const int lane = threadIdx.x, i = (blockIdx.x - xblocks) * S + lane % S, per = 32 / S;
+  const int cnt = i < d.ellnum ? d.ncnt[i] : 0;
+  double c[3] = {0.0, 0.0, 0.0}, ri = 0.0;
+  if (cnt > 0)
   {
-    const int idx0 = d.cwork[w];
-    const size_t idx = (size_t)idx0;
-    const int i = idx0 % d.estride;
-    const int pi = d.part[i];
-    double x[3], v[3], oi[3], c[3];
-    for (int k = 0; k < 3; k ++)
+    c[0] = d.center[0][i]; c[1] = d.center[1][i]; c[2] = d.center[2][i];
+    ri = d.radii[0][i];
+  }
+  const int kmax = __reduce_max_sync(all, cnt);
+  int k = lane / S, k0 = 0, have = 0;                    // this lane's slot, the round's first, entries in the list
+  for (;;)
+  {
+    while (have < 32 && k0 < kmax)
     {
-      x[k] = d.position[k][pi];
-      v[k] = d.linear[k][pi];
-      oi[k] = d.angular[3+k][pi];
-      c[k] = d.center[k][i];
-    }
-    const double ri = d.radii[0][i];
-    const int coli = d.ellcol[i];
-    const double invmi = d.invm[pi], massi = d.mass[pi];
-    const int code = d.ncode[idx];
-    const bool existing = d.nflag[idx] != 0;
-    double point[3], normal[3], depth = 0.0, q[3], len = 0.0;
-    int pj, colj;
-    bool apart;
-    bool sphere = code >= 0;
-    double cj[3];
-    if (sphere)
-    {
-      const int j = code;
-      pj = d.part[j];
-      colj = d.ellcol[j];
-      cj[0] = d.center[0][j]; cj[1] = d.center[1][j]; cj[2] = d.center[2][j];
-      q[0] = c[0]-cj[0];
-      q[1] = c[1]-cj[1];
-      q[2] = c[2]-cj[2];
-      const double d2 = dot3(q, q);
-      const double sr = ri+d.radii[0][j];
-      apart = gt_nonneg(d2, (sr*sr) * (1.0 + 1e-12));
-      if (!apart)
+      bool push = k < cnt;
+      const size_t idx = (size_t)k * d.estride + i;
+      if (push)
       {
-        len = sqrt(d2);
-        depth = sr - len;
+        const int code = d.ncode[idx];
+        if (code >= 0)
+        {
+          const double w[3] = {c[0]-d.center[0][code], c[1]-d.center[1][code], c[2]-d.center[2][code]};
+          const double d2 = dot3(w, w);
+          const double sr = ri+d.radii[0][code];
+          if (gt_nonneg(d2, (sr*sr) * (1.0 + 1e-12)))
+          {
+            push = false;
+            if (d.nflag[idx])
+            {
+              d.nflag[idx] = 0;
+              d.nstate[0][idx] = 0.0; d.nstate[1][idx] = 0.0; d.nstate[2][idx] = 0.0;
+            }
+          }
+        }
       }
+      const unsigned m = __ballot_sync(all, push);
+      if (push) list[have + __popc(m & ((1u << lane) - 1u))] = (int)idx;
+      have += __popc(m);
+      k += per;
+      k0 += per;
     }
-    else
-    {
-      const int t = -code-1;
-      double A[3], B[3], C[3];
-      for (int kk = 0; kk < 3; kk ++) { A[kk] = d.tri[kk][t]; B[kk] = d.tri[3+kk][t]; C[kk] = d.tri[6+kk][t]; }
-      triangle_closest(A, B, C, c, point, (d.compat & PG_COMPAT_TRIEDGE) != 0);
-      q[0] = c[0]-point[0];
-      q[1] = c[1]-point[1];
-      q[2] = c[2]-point[2];
-      const double d2 = dot3(q, q);
-      apart = gt_nonneg(d2, (ri*ri) * (1.0 + 1e-12));
-      if (!apart)
-      {
-        len = sqrt(d2);
-        depth = ri - len;
-      }
-      pj = d.triobs[t];
-      colj = d.tricol[t];
-    }
-    const bool active = !apart && (existing ? !lt_zero_d(depth) : gt_zero_d(depth));
-    if (!active)
-    {
-      if (existing)
-      {
-        d.nflag[idx] = 0;
-        d.nstate[0][idx] = 0.0; d.nstate[1][idx] = 0.0; d.nstate[2][idx] = 0.0;
-      }
-      continue;
-    }
-    if (sphere)
-    {
-      double ilen = existing ? 1.0/len : (gt_zero_d(len) ? 1.0/len : 1.0);
-      point[0] = 0.5*(c[0]+cj[0]);
-      point[1] = 0.5*(c[1]+cj[1]);
-      point[2] = 0.5*(c[2]+cj[2]);
-      normal[0] = ilen*q[0];
-      normal[1] = ilen*q[1];
-      normal[2] = ilen*q[2];
-    }
-    else
-    {
-      double ilen = 1.0/len;
-      normal[0] = ilen*q[0];
-      normal[1] = ilen*q[1];
-      normal[2] = ilen*q[2];
-    }
-
-    // contact point velocities (forces.ispc:226-279)
-    double z[3], vi[3], vj[3], oj[3], vij[3];
-    z[0] = point[0]-x[0]; z[1] = point[1]-x[1]; z[2] = point[2]-x[2];
-    vi[0] = oi[1]*z[2]-oi[2]*z[1] + v[0];
-    vi[1] = oi[2]*z[0]-oi[0]*z[2] + v[1];
-    vi[2] = oi[0]*z[1]-oi[1]*z[0] + v[2];
-    if (pj >= 0)
-    {
-      z[0] = point[0]-d.position[0][pj];
-      z[1] = point[1]-d.position[1][pj];
-      z[2] = point[2]-d.position[2][pj];
-      oj[0] = d.angular[3][pj]; oj[1] = d.angular[4][pj]; oj[2] = d.angular[5][pj];
-      vj[0] = oj[1]*z[2]-oj[2]*z[1] + d.linear[0][pj];
-      vj[1] = oj[2]*z[0]-oj[0]*z[2] + d.linear[1][pj];
-      vj[2] = oj[0]*z[1]-oj[1]*z[0] + d.linear[2][pj];
-    }
-    else
-    {
-      int l = -pj-2;
-      if (obsc && l >= 0) l = l+1;
-      if (l >= 0 && l < d.obsnum)
-      {
-        z[0] = point[0]-d.obspnt[3*l];
-        z[1] = point[1]-d.obspnt[3*l+1];
-        z[2] = point[2]-d.obspnt[3*l+2];
-        oj[0] = d.obsang[3*l]; oj[1] = d.obsang[3*l+1]; oj[2] = d.obsang[3*l+2];
-        vj[0] = oj[1]*z[2]-oj[2]*z[1] + d.obslin[3*l];
-        vj[1] = oj[2]*z[0]-oj[0]*z[2] + d.obslin[3*l+1];
-        vj[2] = oj[0]*z[1]-oj[1]*z[0] + d.obslin[3*l+2];
-      }
-      else
-      {
-        vj[0] = vj[1] = vj[2] = 0.0;
-      }
-    }
-    vij[0] = vj[0] - vi[0];
-    vij[1] = vj[1] - vi[1];
-    vij[2] = vj[2] - vi[2];
-
-    const int ij = pairing(d, coli, colj);
-    if (d.ikind[ij] != 0) set_err(d, PG_ERR_UNSUPPORTED, 4, i, ij);
-
-    // granular force (forces.ispc:125-192)
-    double state[3];
-    if (existing) { state[0] = d.nstate[0][idx]; state[1] = d.nstate[1][idx]; state[2] = d.nstate[2][idx]; }
-    else { state[0] = 0.0; state[1] = 0.0; state[2] = 0.0; }
-    double kn = d.iparam[0][ij];
-    double en;
-    if (d.nen) en = d.nen[idx];
-    else
-    {
-      double ma = pj >= 0 ? 1.0 / (invmi + d.invm[pj]) : massi;
-      en = d.iparam[1][ij] * 2.0 * sqrt(kn*ma);
-    }
-    double vn = dot3(vij, normal);
-    double fn = kn*depth + en*vn;
-    double f[3];
-    f[0] = fn*normal[0];
-    f[1] = fn*normal[1];
-    f[2] = fn*normal[2];
-    double kskn = d.iparam[6][ij];
-    double kt = kn * kskn;
-    double et = en * kskn;
-    double mus = d.iparam[2][ij];
-    double mud = d.iparam[3][ij];
-    double vt[3], ft[3];
-    vt[0] = vij[0] - vn*normal[0];
-    vt[1] = vij[1] - vn*normal[1];
-    vt[2] = vij[2] - vn*normal[2];
-    state[0] += step*vt[0];
-    state[1] += step*vt[1];
-    state[2] += step*vt[2];
-    ft[0] = kt*state[0] + et*vt[0];
-    ft[1] = kt*state[1] + et*vt[1];
-    ft[2] = kt*state[2] + et*vt[2];
-    double flen = sqrt(dot3(ft, ft));
-    double lim = mus*fn;
-    if (gt_d(flen, lim))
-    {
-      lim = mud*fn/flen;
-      ft[0] *= lim;
-      ft[1] *= lim;
-      ft[2] *= lim;
-    }
-    f[0] += ft[0];
-    f[1] += ft[1];
-    f[2] += ft[2];
-
-    d.nflag[idx] = 1;
-    d.nstate[0][idx] = state[0]; d.nstate[1][idx] = state[1]; d.nstate[2][idx] = state[2];
-    d.nfrc[0][idx] = f[0]; d.nfrc[1][idx] = f[1]; d.nfrc[2][idx] = f[2];
-    d.npnt[0][idx] = point[0]; d.npnt[1][idx] = point[1]; d.npnt[2][idx] = point[2];
-    if (GEOM || ADAPT)
-    {
-      d.nnrm[0][idx] = normal[0]; d.nnrm[1][idx] = normal[1]; d.nnrm[2][idx] = normal[2];
-    }
-    if (GEOM) d.ndep[idx] = depth;
+    if (have == 0) return;
+    __syncwarp();
+    const int n = have < 32 ? have : 32;
+    const int idx = lane < n ? list[lane] : -1, rest = lane < have - n ? list[32 + lane] : -1;
+    __syncwarp();
+    if (rest >= 0) list[lane] = rest;
+    have -= n;
+    if (idx >= 0) contact_entry<GEOM, ADAPT>(d, idx, step, obsc);
+    __syncwarp();
   }
 }
 
@@ -1256,14 +1330,20 @@ __host__ __device__ __forceinline__ int run_chunk(int len)
   return c;
 }
 
+// One of the six sums a block (grid z): the adds of a warp hold the FP64 pipe
+// for 64 clocks each, so a lane that sums all six values of its chunk takes
+// 384 of them in a row, and the warp 192 more for the group; with one value a
+// warp it is 64 and 32, and 16 loads are in flight (32.6 -> 8 us for the 9,216
+// springs of the 96x96 lattice's plate).
 __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups(PgDev d)
 {
   const unsigned full = 0xffffffffu;
-  const int run = blockIdx.x, g = blockIdx.y, lane = threadIdx.x;
+  const int run = blockIdx.x, g = blockIdx.y, q = blockIdx.z, lane = threadIdx.x;
   const int4 v = d.sbig[run];
   const int type = v.x & 1, off = type == 0 ? 3 : 6;
   const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch;
   if (g * RUN_GROUP >= nc) return;
+  const double *value = d.spr_out[q < 3 ? q : off + q - 3];
   const int c = g * RUN_GROUP + lane;
   constexpr int W = 16;
   double a = 0.0;
@@ -1293,6 +1373,8 @@ __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups(PgDev d)
   }
   double gs = 0.0;
   int gany = 0;
+  const unsigned has = __ballot_sync(full, any);
+  #pragma unroll
   for (int l = 0; l < RUN_GROUP; l ++)
   {
     const double x = __shfl_sync(full, a, l);
@@ -1308,9 +1390,10 @@ __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups(PgDev d)
   }
 }
 
+// one thread per run and value
 __global__ void k_spring_run_totals(PgDev d)
 {
-  const int run = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, run = t / 6, q = t % 6;
   if (run >= d.nbig) return;
   const int4 v = d.sbig[run];
   const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch, ng = (nc + RUN_GROUP - 1) / RUN_GROUP;
@@ -1327,11 +1410,6 @@ __global__ void k_spring_run_totals(PgDev d)
   }
   d.sbig_sum[6*run + q] = acc;
 }
-// One of the six sums a block (grid z): the adds of a warp hold the FP64 pipe
-// for 64 clocks each, so a lane that sums all six values of its chunk takes
-// 384 of them in a row, and the warp 192 more for the group; with one value a
-// warp it is 64 and 32, and 16 loads are in flight (32.6 -> 8 us for the 9,216
-// springs of the 96x96 lattice's plate).
 
 // Adaptive stiffness partials of the long runs, in the levels of the force
 // sums: each chunk sums its springs' terms from zero in spring order (maxima
@@ -1340,8 +1418,7 @@ __global__ void k_spring_run_totals(PgDev d)
 __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups_adapt(PgDev d)
 {
   const unsigned full = 0xffffffffu;
-  const double *value = d.spr_out[q < 3 ? q : off + q - 3];
-  const int run = blockIdx.x, g = blockIdx.y, q = blockIdx.z, lane = threadIdx.x;
+  const int run = blockIdx.x, g = blockIdx.y, lane = threadIdx.x;
   const int4 v = d.sbig[run];
   const int type = v.x & 1, off = type == 0 ? 5 : 11;
   const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch;
@@ -1371,8 +1448,6 @@ __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups_adapt(PgDev d)
     gq[9] = x[9] > gq[9] ? x[9] : gq[9];
     gq[10] = x[10] > gq[10] ? x[10] : gq[10];
   }
-  const unsigned has = __ballot_sync(full, any);
-  #pragma unroll
   if (lane == 0)
   {
     double *o = d.sbig_grp + ((size_t)run * RUN_GROUPS + g) * RUN_SLOT;
@@ -1382,7 +1457,7 @@ __global__ void __launch_bounds__(RUN_GROUP) k_spring_run_groups_adapt(PgDev d)
 
 __global__ void k_spring_run_totals_adapt(PgDev d)
 {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, run = t / 6, q = t % 6;
+  const int run = blockIdx.x * blockDim.x + threadIdx.x;
   if (run >= d.nbig) return;
   const int4 v = d.sbig[run];
   const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch, ng = (nc + RUN_GROUP - 1) / RUN_GROUP;
@@ -1391,7 +1466,6 @@ __global__ void k_spring_run_totals_adapt(PgDev d)
   {
     const double *o = d.sbig_grp + ((size_t)run * RUN_GROUPS + r) * RUN_SLOT;
     for (int k = 0; k < 9; k ++) p[k] = p[k] + o[k];
-// one thread per run and value
     km = o[9] > km ? o[9] : km;
     em = o[10] > em ? o[10] : em;
   }
@@ -2491,6 +2565,18 @@ __global__ void k_adapt_select(PgDev d)
 } // namespace
 
 // ================================================================ launchers
+// groups of the longest of the long runs, at least 1
+int pg_spring_run_groups(const std::vector<int4> &big)
+{
+  int most = 1;
+  for (const int4 &v : big)
+  {
+    const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch;
+    most = std::max(most, (nc + RUN_GROUP - 1) / RUN_GROUP);
+  }
+  return most;
+}
+
 void pg_launch_invert(const PgDev &d, cudaStream_t s)
 {
   if (d.parnum) k_invert<<<nblk(d.parnum), TPB, 0, s>>>(d);
@@ -2543,9 +2629,20 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
   {
     // three passes (probe, queued evaluation, sums; the sums in k_integrate
     // unless adaptive): the same bits as k_contacts
+    if (d.ellnum <= PG_SMALL_SCENE)
+    {
+      const int S = d.ellnum <= PG_SMALL_SCENE / 4 ? 8 : d.ellnum <= PG_SMALL_SCENE / 2 ? 16 : 32;
+      const int xb = in_step ? (d.nscene + 31) / 32 : 0, nb = xb + (d.ellnum + S - 1) / S;
+      if (d.hs && d.record_geometry) k_contacts_few<true, true><<<nb, 32, 0, s>>>(d, step, S, xb);
+      else if (d.hs) k_contacts_few<false, true><<<nb, 32, 0, s>>>(d, step, S, xb);
+      else if (d.record_geometry) k_contacts_few<true, false><<<nb, 32, 0, s>>>(d, step, S, xb);
+      else k_contacts_few<false, false><<<nb, 32, 0, s>>>(d, step, S, xb);
+      if (d.hs) k_contacts_sum<true><<<nblk(d.ellnum), TPB, 0, s>>>(d);
+      return;
+    }
     if (!in_step) cudaMemsetAsync(d.cwork_n, 0, sizeof(int), s);
-    const int B = d.ellnum <= PG_SMALL_SCENE ? 32 : TPB, xb = in_step ? (d.nscene + B - 1) / B : 0;
-    k_contacts_probe<<<xb + (d.ellnum + B - 1) / B, B, 0, s>>>(d, xb, step);
+    const int xb = in_step ? nblk(d.nscene) : 0;
+    k_contacts_probe<<<xb + nblk(d.ellnum), TPB, 0, s>>>(d, xb, step);
     const int nb = eval_blocks();
     if (d.hs)
     {
@@ -2565,18 +2662,6 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
   if (d.hs)
   {
     if (d.record_geometry) k_contacts<true, true><<<nblk(d.ellnum), TPB, 0, s>>>(d, step);
-// groups of the longest of the long runs, at least 1
-int pg_spring_run_groups(const std::vector<int4> &big)
-{
-  int most = 1;
-  for (const int4 &v : big)
-  {
-    const int len = v.z - v.y, ch = run_chunk(len), nc = (len + ch - 1) / ch;
-    most = std::max(most, (nc + RUN_GROUP - 1) / RUN_GROUP);
-  }
-  return most;
-}
-
     else k_contacts<false, true><<<nblk(d.ellnum), TPB, 0, s>>>(d, step);
   }
   else if (d.record_geometry) k_contacts<true, false><<<nblk(d.ellnum), TPB, 0, s>>>(d, step);
@@ -2590,7 +2675,8 @@ int pg_contacts_kernel_count(const PgDev &d)
 {
   if (!d.ellnum) return 0;
   if (d.form == PG_FORM_MIXED) return 2;
-  return (d.cwork && d.cwork_n) ? (d.hs ? 3 : 2) : 1;
+  if (!d.cwork || !d.cwork_n) return 1;
+  return (d.ellnum <= PG_SMALL_SCENE ? 1 : 2) + (d.hs ? 1 : 0);
 }
 
 // in_step: a session's step; without spheres its scene gravities are taken here
