@@ -138,6 +138,34 @@ __device__ __forceinline__ void cell_keys_item(int i, const double *x, const dou
   if (rx) { rx[i] = c[0]; ry[i] = c[1]; rz[i] = c[2]; }
 }
 
+// Cell key of sphere i for the rebuild's own grid.  The cell is taken with a
+// product by the reciprocal of a cell 2^-40 larger instead of three divisions
+// (26 FP64 instructions of 42 a sphere): two spheres within a cell's length
+// still lie in adjacent cells, the products being off by less than 2^-43, and
+// the exact tests of the search decide every candidate.
+__device__ __forceinline__ double rb_cell_inverse(const PgDev &d) { return (1.0 - 0x1p-40) / d.cell; }
+
+__device__ __forceinline__ void rb_key_item(const PgDev &d, int i, double inv)
+{
+  const double c[3] = {d.center[0][i], d.center[1][i], d.center[2][i]};
+  const int sc = d.escene[i];
+  unsigned key = 0xffffffffu;              // an entry of no scene: sorts last, owns no cell
+  if (sc >= 0)
+  {
+    unsigned u[3];
+    for (int k = 0; k < 3; k ++)
+    {
+      int f = __double2int_rd((c[k] - d.sorg[k][sc]) * inv);
+      f = f < 0 ? 0 : f;
+      u[k] = (unsigned)(f > d.dim[k] - 1 ? d.dim[k] - 1 : f);
+    }
+    key = ((unsigned)sc << (3 * d.bits)) | morton(u[0], u[1], u[2]);
+  }
+  d.keys[0][i] = d.ekey[i] = key;          // the sort reorders keys[]; the search reads its own cell in ekey[]
+  d.vals[0][i] = i;
+  for (int k = 0; k < 3; k ++) d.cref[k][i] = c[k];
+}
+
 // ---- exclusive scans over tiles of SCAN_TILE elements (block-level
 // helpers: every thread of the block calls them; blockDim divides SCAN_TILE)
 constexpr int SCAN_TILE = 1024;
@@ -388,6 +416,14 @@ __device__ __forceinline__ void rb_ranges_item(const PgDev &d, int s)
   if (s == n-1 || d.keys[0][s+1] != key) d.cend[key] = s + 1;
 }
 
+// margin of the float distance test (see rb_verlet_item), and whether the
+// FP64 test is to follow it
+__device__ __forceinline__ float rb_tolerance(const PgDev &d, const float *c)
+{
+  return 9.5367431640625e-7f * (fmaxf(fmaxf(fabsf(c[0]), fabsf(c[1])), fabsf(c[2])) + 2.0f * (float)d.cell);
+}
+__device__ __forceinline__ bool rb_exact(const PgDev &d, float tol) { return !(tol < 0.02f * (float)d.skin); }
+
 // 4. candidate list of sphere i with carried contact state
 // Every lane of the warp calls it (valid: i is a sphere index): the triangle
 // scan is shared by the warp.
@@ -423,8 +459,12 @@ __device__ __forceinline__ void rb_verlet_item(const PgDev &d, int i, bool valid
     // for partners within a cell.
     const float cif[3] = {(float)c[0], (float)c[1], (float)c[2]};
     const float rsf = (float)ri + (float)d.skin;
-    const float tol = 9.5367431640625e-7f *
-                      (fmaxf(fmaxf(fabsf(cif[0]), fabsf(cif[1])), fabsf(cif[2])) + 2.0f * (float)d.cell);
+    const float tol = rb_tolerance(d, cif);
+    // where tol is small against the skin the float test's few extra
+    // candidates cost less than the FP64 test, which holds the warp's FP64
+    // pipe for every lane's neighbour in turn (a candidate beyond the limit
+    // is never in contact: the lists decide nothing)
+    const bool exact = rb_exact(d, tol);
     for (int dz = -1; dz <= 1; dz ++)
       for (int dy = -1; dy <= 1; dy ++)
         for (int dx = -1; dx <= 1; dx ++)
@@ -442,6 +482,12 @@ __device__ __forceinline__ void rb_verlet_item(const PgDev &d, int i, bool valid
             if (d.pfs[s] <= pi) continue;
             int j = d.vals[0][s];
             if ((unsigned)j >= (unsigned)E) continue;
+            if (!exact)
+            {
+              if (n < d.kn) codes[n ++] = j;
+              else { over = true; nover ++; }
+              continue;
+            }
             double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
             double lim = ri + d.radii[0][j] + d.skin;
             if (q0*q0 + q1*q1 + q2*q2 < lim*lim)
@@ -532,8 +578,16 @@ __device__ __forceinline__ void rb_verlet_item(const PgDev &d, int i, bool valid
   if (!live) return;
   if (over) set_err(d, PG_ERR_CAPACITY, 1, i, n + nover);
 
-  // merge with the previous list (both in partner order)
+  // merge with the previous list (both in partner order); a list that did not
+  // change keeps its entries where they are
   const int nold = d.ncnt[i];
+  bool same = n == nold;
+  for (int k = 0; k < n && same; k ++) same = d.ncode[(size_t)k * d.estride + i] == codes[k];
+  if (same)
+  {
+    if (d.nen) for (int k = 0; k < n; k ++) d.nen[(size_t)k * d.estride + i] = pair_en(d, i, codes[k]);
+    return;
+  }
   int ocode[MAXKN];
   unsigned char oflag[MAXKN];
   double ost[3][MAXKN];
@@ -565,6 +619,185 @@ __device__ __forceinline__ void rb_verlet_item(const PgDev &d, int i, bool valid
     }
   }
   d.ncnt[i] = n;
+}
+
+// The same list by RB_GROUP lanes a sphere, for a scene that leaves SMs idle:
+// the lanes share the 27 cells, the ordering, the triangles and the merge,
+// each of which one thread walked as a chain of loads and FP64 tests (76 us
+// of a rebuild on 216 spheres, 67 on 4,096).  Every lane of the warp calls
+// it; codes and olds: RB_GROUP_KN ints of shared memory per group.
+constexpr int RB_GROUP = 8, RB_GROUP_KN = 32;
+
+__device__ __forceinline__ void rb_verlet_group(const PgDev &d, int i, bool valid, int *codes, int *olds)
+{
+  constexpr unsigned all = 0xffffffffu;
+  constexpr int W = RB_GROUP_KN / RB_GROUP;              // list entries of a lane
+  const int lane = threadIdx.x & 31, l = lane % RB_GROUP, g0 = lane - l;
+  const unsigned before = ((1u << l) - 1u) << g0, group = ((1u << RB_GROUP) - 1u) << g0;
+  double c[3] = {0.0, 0.0, 0.0}, ri = 0.0;
+  int pi = 0, sc = -1;
+  if (valid)
+  {
+    for (int k = 0; k < 3; k ++) c[k] = d.center[k][i];
+    ri = d.radii[0][i];
+    pi = d.part[i];
+    sc = d.escene[i];
+  }
+  const bool live = sc >= 0 && d.sactive[sc] != 0;
+  const int kn = d.kn;
+  int n = 0;                                             // entries found (the group's lanes agree)
+  auto append = [&](bool hit, int code) {
+    const unsigned m = __ballot_sync(all, hit);
+    const int at = n + __popc(m & before);
+    if (hit && at < kn) codes[at] = code;
+    n += __popc(m & group);
+  };
+  {
+    const unsigned prefix = (unsigned)sc << (3 * d.bits);
+    const unsigned cm = live ? d.ekey[i] & ((1u << (3 * d.bits)) - 1u) : 0u;
+    const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
+    const float cif[3] = {(float)c[0], (float)c[1], (float)c[2]};
+    const float rsf = (float)ri + (float)d.skin, tol = rb_tolerance(d, cif);
+    const bool exact = rb_exact(d, tol);
+    int b[(27 + RB_GROUP - 1) / RB_GROUP], e[(27 + RB_GROUP - 1) / RB_GROUP];
+    #pragma unroll
+    for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
+    {
+      const int k = l + RB_GROUP * q, x = u[0] + k % 3 - 1, y = u[1] + k / 3 % 3 - 1, z = u[2] + k / 9 - 1;
+      b[q] = e[q] = 0;
+      if (live && k < 27 && x >= 0 && y >= 0 && z >= 0 && x < d.dim[0] && y < d.dim[1] && z < d.dim[2])
+      {
+        const unsigned key = prefix | morton(x, y, z);
+        b[q] = d.cstart[key];
+        e[q] = d.cend[key];
+      }
+    }
+    #pragma unroll
+    for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
+    {
+      const int m = __reduce_max_sync(all, e[q] - b[q]);
+      for (int t = 0; t < m; t ++)
+      {
+        const int s = b[q] + t;
+        bool hit = s < e[q];
+        int j = 0;
+        if (hit)
+        {
+          const float4 o = d.cfs[s];
+          const float f0 = cif[0] - o.x, f1 = cif[1] - o.y, f2 = cif[2] - o.z, lf = rsf + o.w + tol;
+          hit = !(f0*f0 + f1*f1 + f2*f2 >= lf*lf) && d.pfs[s] > pi;
+          if (hit) j = d.vals[0][s];
+          hit = hit && (unsigned)j < (unsigned)d.ellnum;
+          if (hit && exact)
+          {
+            const double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
+            const double lim = ri + d.radii[0][j] + d.skin;
+            hit = q0*q0 + q1*q1 + q2*q2 < lim*lim;
+          }
+        }
+        append(hit, j);
+      }
+    }
+  }
+  // the sphere partners in index order
+  __syncwarp();
+  const int ns = n < kn ? n : kn;
+  int v[W], rank[W];
+  #pragma unroll
+  for (int q = 0; q < W; q ++)
+  {
+    const int a = l + RB_GROUP * q;
+    v[q] = a < ns ? codes[a] : 0;
+    rank[q] = 0;
+    if (a < ns) for (int o = 0; o < ns; o ++) rank[q] += codes[o] < v[q];
+  }
+  __syncwarp();
+  #pragma unroll
+  for (int q = 0; q < W; q ++) if (l + RB_GROUP * q < ns) codes[rank[q]] = v[q];
+  // triangles of the sphere's scene, in triangle order
+  const float inf = __int_as_float(0x7f800000);
+  float clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
+  if (live)
+  {
+    const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
+    for (int k = 0; k < 3; k ++) { clo[k] = __double2float_rd(c[k]) - rr; chi[k] = __double2float_ru(c[k]) + rr; }
+  }
+  const int T = d.trinum;
+  auto near = [&](int t) {
+    if (d.tbox[t] > chi[0] || d.tbox[(size_t)3 * T + t] < clo[0] ||
+        d.tbox[(size_t)T + t] > chi[1] || d.tbox[(size_t)4 * T + t] < clo[1] ||
+        d.tbox[(size_t)2 * T + t] > chi[2] || d.tbox[(size_t)5 * T + t] < clo[2]) return false;
+    double A[3], B[3], C[3], pnt[3], nrm[3];
+    for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
+    const double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
+    return depth > -d.skin || depth != depth;
+  };
+  const int tb = live ? d.stbeg[sc] : 0, te = live ? d.stend[sc] : 0;
+  const int before_t = n;
+  const int most = __reduce_max_sync(all, te - tb);
+  for (int t0 = 0; t0 < most; t0 += RB_GROUP)
+  {
+    const int t = tb + t0 + l;
+    append(t < te && near(t), -(t + 1));
+  }
+  // statistics: one atomic per warp
+  const int cmax = __reduce_max_sync(all, live ? n : 0), tmax = __reduce_max_sync(all, live ? n - before_t : 0);
+  if (lane == 0)
+  {
+    if (cmax > 0) atomicMax(&d.stats[1], cmax);
+    if (tmax > 0) atomicMax(&d.stats[3], tmax);
+  }
+  if (live && n > kn && l == 0) set_err(d, PG_ERR_CAPACITY, 1, i, n);
+  const int nn = n < kn ? n : kn;
+  // the previous entries of the same partners
+  const int nold = live ? d.ncnt[i] : 0;
+  for (int k = l; k < nold; k += RB_GROUP) olds[k] = d.ncode[(size_t)k * d.estride + i];
+  __syncwarp();
+  const bool mixed = d.form == PG_FORM_MIXED;
+  unsigned char flag[W];
+  double st[W][3];
+  #pragma unroll
+  for (int q = 0; q < W; q ++)
+  {
+    const int k = l + RB_GROUP * q;
+    v[q] = 0;
+    flag[q] = 0;
+    for (int a = 0; a < 3; a ++) st[q][a] = 0.0;
+    if (!live || k >= nn) continue;
+    v[q] = codes[k];
+    int o = 0;
+    while (o < nold && olds[o] != v[q]) o ++;
+    if (o == nold) continue;
+    const size_t idx = (size_t)o * d.estride + i;
+    flag[q] = d.nflag[idx];
+    for (int a = 0; a < 3; a ++) st[q][a] = mixed ? (double)d.nstate_f[a][idx] : d.nstate[a][idx];
+  }
+  __syncwarp();                                          // every lane has read before any writes
+  #pragma unroll
+  for (int q = 0; q < W; q ++)
+  {
+    const int k = l + RB_GROUP * q;
+    if (!live || k >= nn) continue;
+    const size_t idx = (size_t)k * d.estride + i;
+    d.ncode[idx] = v[q];
+    if (d.nen) d.nen[idx] = pair_en(d, i, v[q]);
+    d.nflag[idx] = flag[q];
+    for (int a = 0; a < 3; a ++)
+    {
+      if (mixed) d.nstate_f[a][idx] = (float)st[q][a];
+      else d.nstate[a][idx] = st[q][a];
+    }
+  }
+  if (live && l == 0) d.ncnt[i] = nn;
+  __syncwarp();
+}
+
+// whether the groups take a scene's lists: its spheres at RB_GROUP lanes each
+// fill no more than a warp a scheduler four times over (152 SMs of four), its
+// lists fit, and its triangles are few (many are scanned better by the warp)
+__device__ __forceinline__ bool rb_grouped(const PgDev &d)
+{
+  return d.ellnum <= 152 * 4 * 32 && d.kn <= RB_GROUP_KN && d.trinum <= 256 * d.nscene;
 }
 
 // 5. slave lists (CSR): count entries per sphere in particle order, emit
@@ -672,6 +905,8 @@ __device__ __forceinline__ unsigned long long global_ns()
   return t;
 }
 
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 // barrier of all blocks of a cooperative grid.  d.gbar = {arrivals,
 // generation, abort}.  A block that waits more than 2 s records
 // PG_ERR_TIMEOUT and raises abort; every block then leaves its kernel
@@ -682,10 +917,13 @@ static __device__ __noinline__ bool grid_barrier(const PgDev &d)
   __syncthreads();
   if (threadIdx.x == 0)
   {
+    // the fences make the block's writes, ordered before this thread by the
+    // block barrier, visible before its arrival, and everyone's after it; the
+    // wait polls one word and looks at the clock, slow to read, every 256 polls
     volatile unsigned *b = d.gbar;
     int ok = 1;
     const unsigned gen = b[1];
-    __threadfence();
+    fence_gpu();
     if (b[2] != 0u) ok = 0;
     else
     {
@@ -693,27 +931,29 @@ static __device__ __noinline__ bool grid_barrier(const PgDev &d)
       if (arrived == gridDim.x)
       {
         atomicExch(d.gbar, 0u);
-        __threadfence();
+        fence_gpu();
         atomicAdd(d.gbar + 1, 1u);
       }
       else
       {
-        const unsigned long long t0 = global_ns();
-        while (b[1] == gen)
+        unsigned long long t0 = 0;
+        for (unsigned polls = 1; b[1] == gen; polls ++)
         {
+          if (polls & 255u) continue;
           if (b[2] != 0u) { ok = 0; break; }
-          if (global_ns() - t0 > 2000000000ull)
+          const unsigned long long now = global_ns();
+          if (!t0) t0 = now;
+          if (now - t0 > 2000000000ull)
           {
             atomicExch(d.gbar + 2, 1u);
             set_err(d, PG_ERR_TIMEOUT, 20, blockIdx.x, 0);
             ok = 0;
             break;
           }
-          __nanosleep(32);
         }
       }
     }
-    __threadfence();
+    fence_gpu();
     ok_s = ok;
   }
   __syncthreads();
@@ -750,6 +990,7 @@ union RebuildSmem
   unsigned h[256];
   struct { unsigned wcnt[SORT_THREADS / 32][256]; unsigned goff[256]; } sc;
   unsigned part[B];
+  struct { int codes[B / RB_GROUP][RB_GROUP_KN], olds[B / RB_GROUP][RB_GROUP_KN]; } group;
 };
 
 struct NoHook
@@ -773,15 +1014,8 @@ __device__ bool rebuild_all(const PgDev &d, int passes, int epasses, RebuildSmem
   for (int s = g0; s < E; s += gsz) { rb_clear_item(d, s); hook(d, s); }
   for (int t = g0; t < T; t += gsz) rb_tref_item(d, t);
   if (!grid_barrier(d)) return false;
-  Grid g;
-  for (int k = 0; k < 3; k ++) { g.org[k] = 0.0; g.dim[k] = d.dim[k]; }
-  g.cell = d.cell;
-  for (int i = g0; i < E; i += gsz)
-  {
-    cell_keys_item(i, d.center[0], d.center[1], d.center[2], g, d.escene, d.sorg[0], d.sorg[1], d.sorg[2],
-                   3 * d.bits, d.keys[0], d.vals[0], d.cref[0], d.cref[1], d.cref[2]);
-    d.ekey[i] = d.keys[0][i];        // the sort reorders keys[]; the search reads its own cell here
-  }
+  const double inv = rb_cell_inverse(d);
+  for (int i = g0; i < E; i += gsz) rb_key_item(d, i, inv);
   if (!grid_barrier(d)) return false;
   const int nb = d.nsortblocks;
   if (nb == 1)
@@ -812,6 +1046,17 @@ __device__ bool rebuild_all(const PgDev &d, int passes, int epasses, RebuildSmem
   }
   for (int s = g0; s < E; s += gsz) rb_ranges_item(d, s);
   if (!grid_barrier(d)) return false;
+  if (rb_grouped(d))
+  {
+    constexpr int PER = 32 / RB_GROUP;                   // spheres a warp
+    const int lane = threadIdx.x & 31, slot = threadIdx.x / RB_GROUP;
+    for (int q = g0 >> 5; q * PER < E; q += gsz >> 5)
+    {
+      const int i = q * PER + lane / RB_GROUP;
+      rb_verlet_group(d, i, i < E, sm.group.codes[slot], sm.group.olds[slot]);
+    }
+  }
+  else
   for (int i = g0; i - (int)(threadIdx.x & 31) < E; i += gsz) rb_verlet_item(d, i, i < E);
   if (!grid_barrier(d)) return false;
   for (int p = g0; p < P; p += gsz) rb_rzero_item(d, p);
