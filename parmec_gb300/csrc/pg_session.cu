@@ -832,6 +832,7 @@ int mixed_buffers(pg_session *s)
     TRY(dalloc(s, &d.J_f[k], P)); TRY(dalloc(s, &d.I_f[k], P));
   }
   TRY(dalloc(s, &d.mass_f, P)); TRY(dalloc(s, &d.invm_f, P));
+  TRY(dalloc(s, &d.pushed, P)); TRY(dalloc(s, &d.touched, P)); TRY(dalloc(s, &d.still, P));
   TRY(dalloc(s, &d.rh, E)); TRY(dalloc(s, &d.rl, E));
   TRY(dalloc(s, &d.twork, std::max<size_t>(E, 1)));   // triangle queue of the contact passes
   TRY(dalloc(s, &d.tcnt, 2));

@@ -194,7 +194,10 @@ struct PgDev
   float *mass_f, *invm_f, *J_f[9], *I_f[9];
   float *F_f[3], *T_f[3];
   float *nstate_f[3], *nfrc_f[3], *narm_f[3];   // per candidate entry; arm = point - slave position
-  float *fm_f[3], *tm_f[3];
+  float *fm_f[3], *tm_f[3]; // master-side sums, where pushed
+  unsigned char *pushed;    // [parnum] the particle's sphere has master contacts this step
+  unsigned char *touched;   // [parnum] the particle has slave contacts this step (cleared when read)
+  unsigned char *still;     // [parnum] the last update with rotation left no spin
   int *twork;               // [ellnum] spheres with triangle candidates this step
   int *tcnt;                // [2] length of twork, blocks of the triangle pass done
   float *iparam_f[7];       // [pairnum] surface pair parameters in FP32
