@@ -1141,33 +1141,71 @@ __device__ bool rebuild_all(const PgDev &d, int passes, int epasses, RebuildSmem
 // local time t = (global step - start step) * step.  Written with explicit
 // round-to-nearest operations: the same bits whether or not the compiler
 // contracts multiply-adds.
-__device__ __forceinline__ void excite_item(const PgDev &d, int sc, double step)
+// One term of the sum, and what the scene's gravity (and in FP32 with it, the
+// damping row) becomes with the sum.
+__device__ __forceinline__ int excite_terms(const double *e)
 {
-  const double *tab = d.t_gravity + 3*(size_t)(*d.stepno);
+  const int nk = (int)e[6];
+  return nk > 8 ? 8 : nk;
+}
+
+__device__ __forceinline__ double excite_term(const PgDev &d, const double *e, int sc, int k, double step)
+{
+  const double t = __dmul_rn((double)(*d.gstep - d.sstart[sc]), step);
+  const double two_pi = 2.0 * 3.14159265358979323846;
+  return __dmul_rn(e[8+3*k], sin(__dadd_rn(__dmul_rn(__dmul_rn(two_pi, e[9+3*k]), t), e[10+3*k])));
+}
+
+__device__ __forceinline__ void excite_store(const PgDev &d, int sc, double sum)
+{
+  const double *tab = d.t_gravity + 3*(size_t)(*d.stepno), *e = d.sexc + (size_t)PG_EXC_LEN * sc;
+  const bool on = d.sexc_on[sc] != 0;
   if (sc == 0 && d.damp_f)
   {
     const double *damp = d.t_damping + 6*(size_t)(*d.stepno);
     for (int k = 0; k < 6; k ++) d.damp_f[k] = (float)damp[k];
   }
-  if (!d.sexc_on[sc])
+  for (int k = 0; k < 3; k ++)
   {
-    d.sgrav[3*sc] = tab[0]; d.sgrav[3*sc+1] = tab[1]; d.sgrav[3*sc+2] = tab[2];
-    if (d.sgrav_f) { d.sgrav_f[3*sc] = (float)tab[0]; d.sgrav_f[3*sc+1] = (float)tab[1]; d.sgrav_f[3*sc+2] = (float)tab[2]; }
-    return;
+    const double g = on ? __dadd_rn(e[k], __dmul_rn(e[3+k], sum)) : tab[k];
+    d.sgrav[3*sc+k] = g;
+    if (d.sgrav_f) d.sgrav_f[3*sc+k] = (float)g;
   }
-  const double *e = d.sexc + (size_t)PG_EXC_LEN * sc;
-  const double t = __dmul_rn((double)(*d.gstep - d.sstart[sc]), step);
-  int nk = (int)e[6];
-  if (nk > 8) nk = 8;
-  const double two_pi = 2.0 * 3.14159265358979323846;
+}
+
+__device__ __forceinline__ void excite_item(const PgDev &d, int sc, double step)
+{
   double sum = 0.0;
-  for (int k = 0; k < nk; k ++)
-    sum = __dadd_rn(sum, __dmul_rn(e[8+3*k], sin(__dadd_rn(__dmul_rn(__dmul_rn(two_pi, e[9+3*k]), t), e[10+3*k]))));
-  d.sgrav[3*sc] = __dadd_rn(e[0], __dmul_rn(e[3], sum));
-  d.sgrav[3*sc+1] = __dadd_rn(e[1], __dmul_rn(e[4], sum));
-  d.sgrav[3*sc+2] = __dadd_rn(e[2], __dmul_rn(e[5], sum));
-  if (d.sgrav_f)
-    for (int k = 0; k < 3; k ++) d.sgrav_f[3*sc+k] = (float)d.sgrav[3*sc+k];
+  if (d.sexc_on[sc])
+  {
+    const double *e = d.sexc + (size_t)PG_EXC_LEN * sc;
+    const int nk = excite_terms(e);
+    for (int k = 0; k < nk; k ++) sum = __dadd_rn(sum, excite_term(d, e, sc, k, step));
+  }
+  excite_store(d, sc, sum);
+}
+
+// the same by eight lanes a scene, one a term (a chain of eight sines takes
+// 10 us); every lane of the warp calls it, t counts the lanes
+constexpr int EXCITE_LANES = 8;
+
+static __device__ __noinline__ void excite_lanes(const PgDev &d, int t, double step)
+{
+  const int sc = t / EXCITE_LANES, k = t % EXCITE_LANES, lane = threadIdx.x & 31;
+  double term = 0.0, sum = 0.0;
+  int nk = 0;
+  if (sc < d.nscene && d.sexc_on[sc])
+  {
+    const double *e = d.sexc + (size_t)PG_EXC_LEN * sc;
+    nk = excite_terms(e);
+    if (k < nk) term = excite_term(d, e, sc, k, step);
+  }
+  for (int q = 0; q < EXCITE_LANES; q ++)
+  {
+    const double v = __shfl_sync(0xffffffffu, term, (lane & ~(EXCITE_LANES - 1)) + q);
+    if (q < nk) sum = __dadd_rn(sum, v);
+  }
+  if (k == 0 && sc < d.nscene) excite_store(d, sc, sum);
 }
 
 // obstacle triangle t moved by its obstacle's velocities (obstacles.ispc:28-78):
@@ -1299,15 +1337,12 @@ __device__ __forceinline__ void step_done(const PgDev &d, double step, int last)
 
 // The scene gravities of a step, taken by the first blocks of its first
 // kernel (`blocks` of them, beside the kernel's own work, which does not read
-// them): true when the block is one of them.  Saves k_excite's launch, and
-// the chain of sines of a pool's excitation (12 us) runs beside the contacts.
-static __device__ __noinline__ void excite_scene(const PgDev &d, int sc, double step) { excite_item(d, sc, step); }
-
+// them): true when the block is one of them.  Saves k_excite's launch (12 us
+// with a pool's sines).
 __device__ __forceinline__ bool excite_front(const PgDev &d, int blocks, double step)
 {
   if ((int)blockIdx.x >= blocks) return false;
-  const int sc = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sc < d.nscene) excite_scene(d, sc, step);
+  excite_lanes(d, blockIdx.x * blockDim.x + threadIdx.x, step);
   return true;
 }
 

@@ -38,6 +38,9 @@ int  pg_step_kernel_count(const PgDev &d);
 void pg_launch_step_end(const PgDev &d, cudaStream_t s, double step);   // where the integration's launch does not
 // whether the integration's launch ends the step: a grid of one wave
 #define PG_MX_BLOCKS 8
+// spheres up to which the mixed contacts take one launch: two warps of 32 a
+// scheduler (152 SMs of four)
+#define PG_MX_FEW (2 * 152 * 4 * 32)
 static inline int pg_ends_step(int blocks, int per_sm) { return blocks <= 152 * per_sm; }
 
 // pg_mixed.cu

@@ -204,10 +204,12 @@ __global__ void k_mx_to64(PgDev d, int p0, int p1)
 // A sphere's candidate list holds its sphere partners first, then its
 // triangles (order_key).  PASS selects the entries one call evaluates:
 //   MX_SPHERES   the sphere partners; returns whether triangles follow;
-//   MX_TRIANGLES the triangles, continuing the sums the sphere pass stored.
+//   MX_TRIANGLES the triangles, continuing the sums the sphere pass stored;
+//   MX_ALL       both, one after the other (scenes that leave SMs idle, where
+//                a second launch costs more than diverged triangle code).
 // The force and torque sums take the FP32 additions of a single pass over
 // the list, in the same order.
-constexpr int MX_SPHERES = 1, MX_TRIANGLES = 2;
+constexpr int MX_SPHERES = 1, MX_TRIANGLES = 2, MX_ALL = 3;
 
 // what a contact of sphere i reads of its own particle beside the position,
 // loaded at the first candidate that is not clearly apart: most of a shaken
@@ -412,7 +414,13 @@ __device__ __forceinline__ bool mx_contacts_item(const PgDev &d, int i, double s
       {
         const size_t idx = (size_t)k * d.estride + i;
         const int code = d.ncode[idx];
-        if (code < 0) { more = true; break; }
+        if (code < 0)
+        {
+          if (PASS == MX_SPHERES) { more = true; break; }
+          if (!have) { have = true; me.load(d, i, pi); }
+          mx_entry(d, i, pi, idx, code, x, ri, step, obsc, etypo, me, fs, ts, any);
+          continue;
+        }
         const int pj = d.part[code];
         const float q[3] = {d.xh[0][pj], d.xh[1][pj], d.xh[2][pj]};
         const float m = mi + fabsf(q[0]) + fabsf(q[1]) + fabsf(q[2]);
@@ -429,7 +437,7 @@ __device__ __forceinline__ bool mx_contacts_item(const PgDev &d, int i, double s
     }
   }
   if (any) for (int c = 0; c < 3; c ++) { d.fm_f[c][pi] = fs[c]; d.tm_f[c][pi] = ts[c]; }
-  if (PASS == MX_SPHERES) d.pushed[pi] = any;
+  if (PASS != MX_TRIANGLES) d.pushed[pi] = any;
   else if (any) d.pushed[pi] = 1;
   return more;
 }
@@ -444,6 +452,14 @@ __global__ void __launch_bounds__(TPB, PG_MX_MIN_BLOCKS) k_contacts_mx(PgDev d, 
   bool more = false;
   if (i < d.ellnum) more = mx_contacts_item<MX_SPHERES>(d, i, step_d);
   pgk::tri_queue_push(d, more, i);
+}
+
+// every candidate of a scene of few spheres, blocks of one warp
+__global__ void __launch_bounds__(32) k_contacts_mx_few(PgDev d, double step_d, int xblocks)
+{
+  if (pgk::excite_front(d, xblocks, step_d)) return;
+  const int i = (blockIdx.x - xblocks) * 32 + threadIdx.x;
+  if (i < d.ellnum) mx_contacts_item<MX_ALL>(d, i, step_d);
 }
 
 // the triangle candidates of the queued spheres, one thread per sphere; the
@@ -776,7 +792,13 @@ void pg_launch_mx_to64(const PgDev &d, cudaStream_t s, int p0, int p1)
 void pg_launch_contacts_mx(const PgDev &d, cudaStream_t s, double step)
 {
   if (!d.ellnum) { pg_launch_excite(d, s, step); return; }
-  const int nb = nblk(d.ellnum), xb = nblk(d.nscene);
+  if (d.ellnum <= PG_MX_FEW)
+  {
+    const int xb = (pgk::EXCITE_LANES * d.nscene + 31) / 32;
+    k_contacts_mx_few<<<xb + (d.ellnum + 31) / 32, 32, 0, s>>>(d, step, xb);
+    return;
+  }
+  const int nb = nblk(d.ellnum), xb = nblk(pgk::EXCITE_LANES * d.nscene);
   k_contacts_mx<<<xb + nb, TPB, 0, s>>>(d, step, xb);
   k_tri_mx<<<nb < pgk::TRI_PASS_BLOCKS ? nb : pgk::TRI_PASS_BLOCKS, TPB, 0, s>>>(d, step);
 }

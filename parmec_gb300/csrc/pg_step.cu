@@ -78,8 +78,7 @@ __device__ __forceinline__ void scene_gravity(const PgDev &d, int sc, double, co
 // local time t = (global step - start step) * step
 __global__ void k_excite(PgDev d, double step)
 {
-  const int sc = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sc < d.nscene) pgk::excite_item(d, sc, step);
+  pgk::excite_lanes(d, blockIdx.x * blockDim.x + threadIdx.x, step);
 }
 
 // ---------------------------------------------------------------- isotropic bodies
@@ -2632,7 +2631,7 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
     if (d.ellnum <= PG_SMALL_SCENE)
     {
       const int S = d.ellnum <= PG_SMALL_SCENE / 4 ? 8 : d.ellnum <= PG_SMALL_SCENE / 2 ? 16 : 32;
-      const int xb = in_step ? (d.nscene + 31) / 32 : 0, nb = xb + (d.ellnum + S - 1) / S;
+      const int xb = in_step ? (pgk::EXCITE_LANES * d.nscene + 31) / 32 : 0, nb = xb + (d.ellnum + S - 1) / S;
       if (d.hs && d.record_geometry) k_contacts_few<true, true><<<nb, 32, 0, s>>>(d, step, S, xb);
       else if (d.hs) k_contacts_few<false, true><<<nb, 32, 0, s>>>(d, step, S, xb);
       else if (d.record_geometry) k_contacts_few<true, false><<<nb, 32, 0, s>>>(d, step, S, xb);
@@ -2641,7 +2640,7 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
       return;
     }
     if (!in_step) cudaMemsetAsync(d.cwork_n, 0, sizeof(int), s);
-    const int xb = in_step ? nblk(d.nscene) : 0;
+    const int xb = in_step ? nblk(pgk::EXCITE_LANES * d.nscene) : 0;
     k_contacts_probe<<<xb + nblk(d.ellnum), TPB, 0, s>>>(d, xb, step);
     const int nb = eval_blocks();
     if (d.hs)
@@ -2674,7 +2673,7 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
 int pg_contacts_kernel_count(const PgDev &d)
 {
   if (!d.ellnum) return 0;
-  if (d.form == PG_FORM_MIXED) return 2;
+  if (d.form == PG_FORM_MIXED) return d.ellnum <= PG_MX_FEW ? 1 : 2;
   if (!d.cwork || !d.cwork_n) return 1;
   return (d.ellnum <= PG_SMALL_SCENE ? 1 : 2) + (d.hs ? 1 : 0);
 }
@@ -2688,7 +2687,7 @@ void pg_launch_springs(const PgDev &d, cudaStream_t s, double step, bool in_step
     if (excite) pg_launch_excite(d, s, step);
     return;
   }
-  const int xb = excite ? nblk(d.nscene) : 0;
+  const int xb = excite ? nblk(pgk::EXCITE_LANES * d.nscene) : 0;
   if (d.hs) k_springs<true><<<xb + nblk(d.sprnum), TPB, 0, s>>>(d, step, xb);
   else k_springs<false><<<xb + nblk(d.sprnum), TPB, 0, s>>>(d, step, xb);
 }
@@ -2810,7 +2809,7 @@ void pg_launch_mesh(const PgDev &d, cudaStream_t s)
 
 void pg_launch_excite(const PgDev &d, cudaStream_t s, double step)
 {
-  k_excite<<<nblk(d.nscene), TPB, 0, s>>>(d, step);
+  k_excite<<<nblk(pgk::EXCITE_LANES * d.nscene), TPB, 0, s>>>(d, step);
 }
 
 void pg_launch_obstacles_tail(const PgDev &d, cudaStream_t s, double step)
