@@ -18,9 +18,16 @@ inline double __longlong_as_double(long long i) { double x; memcpy(&x, &i, 8); r
 inline void sincos(double x, double *s, double *c) { *s = sin(x); *c = cos(x); }
 #endif
 
+#include "pg_f64.cuh"
+
 namespace pg {
 
+// The products and the particle update below take double or f64 (pg_f64.cuh):
+// the same expressions, the same bits.
 PG_DEV double dot3(const double *a, const double *b) { return a[0]*b[0] + a[1]*b[1] + a[2]*b[2]; }
+#ifdef __CUDACC__
+PG_DEV f64 dot3(const f64 *a, const f64 *b) { return a[0]*b[0] + a[1]*b[1] + a[2]*b[2]; }
+#endif
 
 // Comparisons on the integer pipe.  GB300 issues FP64 instructions, DSETP
 // included, at 2 lanes per clock per SM; these give the truth values of the
@@ -81,28 +88,32 @@ PG_DEV float mag32(double x)
 PG_DEV float pow2_floor(float x) { return __int_as_float(__float_as_int(x) & 0x7f800000); }
 
 // NVMUL: C = A*B, A column-major 3x3
-PG_DEV void nvmul(const double *A, const double *B, double *C)
+template <class TA, class TB, class TC>
+PG_DEV void nvmul(const TA *A, const TB *B, TC *C)
 {
   C[0] = A[0]*B[0]+A[3]*B[1]+A[6]*B[2];
   C[1] = A[1]*B[0]+A[4]*B[1]+A[7]*B[2];
   C[2] = A[2]*B[0]+A[5]*B[1]+A[8]*B[2];
 }
 // TVMUL: C = A^T*B
-PG_DEV void tvmul(const double *A, const double *B, double *C)
+template <class TA, class TB, class TC>
+PG_DEV void tvmul(const TA *A, const TB *B, TC *C)
 {
   C[0] = A[0]*B[0]+A[1]*B[1]+A[2]*B[2];
   C[1] = A[3]*B[0]+A[4]*B[1]+A[5]*B[2];
   C[2] = A[6]*B[0]+A[7]*B[1]+A[8]*B[2];
 }
 // NVADDMUL: D = C + A*B
-PG_DEV void nvaddmul(const double *C, const double *A, const double *B, double *D)
+template <class TC, class TA, class TB, class TD>
+PG_DEV void nvaddmul(const TC *C, const TA *A, const TB *B, TD *D)
 {
   D[0] = C[0] + (A[0]*B[0]+A[3]*B[1]+A[6]*B[2]);
   D[1] = C[1] + (A[1]*B[0]+A[4]*B[1]+A[7]*B[2]);
   D[2] = C[2] + (A[2]*B[0]+A[5]*B[1]+A[8]*B[2]);
 }
 // NNMUL: C = A*B
-PG_DEV void nnmul(const double *A, const double *B, double *C)
+template <class TA, class TB, class TC>
+PG_DEV void nnmul(const TA *A, const TB *B, TC *C)
 {
   C[0] = A[0]*B[0]+A[3]*B[1]+A[6]*B[2];
   C[1] = A[1]*B[0]+A[4]*B[1]+A[7]*B[2];
@@ -143,9 +154,10 @@ PG_DEV bool sum_settled(double p)
 }
 
 // sin(x)/x and (1 - cos(x))/x^2 from angsq = x^2
-PG_DEV void exp_series(double angsq, double *psx, double *pcx)
+template <class R>
+PG_DEV void exp_series(R angsq, R *psx, R *pcx)
 {
-  double sx, cx;
+  R sx, cx;
   if (gt_nonneg(3.0461741978671E-02, angsq))
   {
     sx = 1.0 +
@@ -175,12 +187,11 @@ PG_DEV void exp_series(double angsq, double *psx, double *pcx)
   }
   else
   {
-    double t = angsq;
-    angsq = sqrt(angsq);
+    const double t = angsq, x = sqrt(t);
     double s, c;
-    sincos(angsq, &s, &c);
-    sx = s / angsq;
-    cx = (1.0 - c) / t;
+    sincos(x, &s, &c);
+    sx = like(angsq, s / x);
+    cx = like(angsq, (1.0 - c) / t);
   }
   *psx = sx;
   *pcx = cx;
@@ -193,12 +204,13 @@ PG_DEV void exp_series(double angsq, double *psx, double *pcx)
 // holds its pipe for 64 clocks a warp; this takes 8 of them instead of 24,
 // for two integer tests.  A lane is not settled about once in
 // 1/(170 angsq) and then takes the series.
-PG_DEV void exp_terms(double angsq, double *psx, double *pcx)
+template <class R>
+PG_DEV void exp_terms(R angsq, R *psx, R *pcx)
 {
   if (dbits(angsq) < 0x3ed0000000000000ULL)
   {
-    const double ps = (-1.666666666666667E-1 + 8.333333333333333E-3 * angsq) * angsq;
-    const double pc = (-4.166666666666667E-2 + 1.388888888888889E-3 * angsq) * angsq;
+    const R ps = (-1.666666666666667E-1 + 8.333333333333333E-3 * angsq) * angsq;
+    const R pc = (-4.166666666666667E-2 + 1.388888888888889E-3 * angsq) * angsq;
     if (sum_settled<53>(ps) && sum_settled<54>(pc))
     {
       *psx = 1.0 + ps;
@@ -213,9 +225,10 @@ PG_DEV void exp_terms(double angsq, double *psx, double *pcx)
 // degrees it uses the truncated series sin(x)/x and (1-cos(x))/x^2 in x^2; the
 // coefficients are the Taylor coefficients 1/(2k+1)! and 1/(2k+2)!.
 // 'typo' reproduces the reference's v02 = O2*O3 (macros.h:1505).
-PG_DEV void expmap(double O1, double O2, double O3, double *L, bool typo)
+template <class R>
+PG_DEV void expmap(R O1, R O2, R O3, R *L, bool typo)
 {
-  double angsq, sx, cx, v0, v1, v2, v01, v02, v12, s0, s1, s2;
+  R angsq, sx, cx, v0, v1, v2, v01, v02, v12, s0, s1, s2;
   v0 = O1 * O1;
   v1 = O2 * O2;
   v2 = O3 * O3;
@@ -248,16 +261,18 @@ PG_DEV void expmap(double O1, double O2, double O3, double *L, bool typo)
 }
 
 // p + 0*a + 0*b as the full product sums them, for finite a and b
-PG_DEV double zero_terms(double p, double a, double b)
+template <class R>
+PG_DEV R zero_terms(R p, double a, double b)
 {
   const long long bp = (long long)dbits(p);
   if ((bp << 1) != 0) return p;
   const bool neg = bp < 0 && (long long)dbits(a) < 0 && (long long)dbits(b) < 0;
-  return __longlong_as_double(neg ? (long long)0x8000000000000000ull : 0ll);
+  return like(p, __longlong_as_double(neg ? (long long)0x8000000000000000ull : 0ll));
 }
 
 // C = (j*I) B, bit for bit as nvmul with the full matrix
-PG_DEV void iso_nvmul(double j, const double *B, double *C)
+template <class R>
+PG_DEV void iso_nvmul(double j, const R *B, R *C)
 {
   if (finite_d(B[0]) && finite_d(B[1]) && finite_d(B[2]))
   {
@@ -275,9 +290,10 @@ PG_DEV void iso_nvmul(double j, const double *B, double *C)
 // The referential angular velocity O of an isotropic body (J = j*I, inverse
 // i*I) over one step, with the torque Tb in the body frame
 // (dynamics.ispc:86-117)
-PG_DEV void spin_iso(double *O, double *Tb, double js, double is, double step, double half, bool typo)
+template <class R>
+PG_DEV void spin_iso(R *O, R *Tb, double js, double is, double step, double half, bool typo)
 {
-  double DL[9], A[3], B[3], IT[3];
+  R DL[9], A[3], B[3], IT[3];
   expmap(-half*O[0], -half*O[1], -half*O[2], DL, typo);
   iso_nvmul(js, O, A);
   nvmul(DL, A, B);
@@ -310,7 +326,8 @@ PG_DEV void spin_iso(double *O, double *Tb, double js, double is, double step, d
 // rotations k_integrate takes 207 FP64 instructions a warp instead of 298:
 // 697 -> 547 us on the 1,048,576-sphere drum, 121 -> 48 us on 230,000
 // spheres of shaken boxes (most of them not turning yet).
-PG_DEV bool gyro_settled(const double *O, const double *Tb, double js, double is, double step,
+template <class R>
+PG_DEV bool gyro_settled(const R *O, const R *Tb, double js, double is, double step,
                                              double half)
 {
   const float tiny = 1.2e-38f, up = 1.000001f;
@@ -331,9 +348,9 @@ PG_DEV bool gyro_settled(const double *O, const double *Tb, double js, double is
     a[k] = (of[k] * up + tiny) * 1.0001f + om * (th * th + 1e-6f) + qh * (tf[k] * up + tiny);
   for (int k = 0; k < 3; k ++)
   {
-    const float P = jf * up * a[(k+1)%3] * a[(k+2)%3], R = 4.6e-16f * P;
+    const float P = jf * up * a[(k+1)%3] * a[(k+2)%3], r = 4.6e-16f * P;
     const bool torque = tf[k] > 1e-20f && q * tf[k] > 1e-37f && (dbits(Tb[k]) & 0xfffffffffffffull) != 0 &&
-                        R <= 1.1e-16f * pow2_floor(tf[k]);
+                        r <= 1.1e-16f * pow2_floor(tf[k]);
     const bool spin = q * (tf[k] * up + tiny) + (q * 4.6e-16f) * P * up + 1e-36f <= 5.5e-17f * pow2_floor(of[k]);
     ok = ok && (torque || spin);
   }
@@ -342,14 +359,16 @@ PG_DEV bool gyro_settled(const double *O, const double *Tb, double js, double is
 
 // exp(h 0) L is L, bit for bit: h finite and not negative, L finite without a
 // negative zero (a negative zero plus the zero products would turn positive)
-PG_DEV bool turn_is_identity(const double *L, double h)
+template <class R>
+PG_DEV bool turn_is_identity(const R *L, double h)
 {
   bool ok = finite_d(h) && (long long)dbits(h) >= 0;
   for (int k = 0; k < 9; k ++) ok = ok && finite_d(L[k]) && dbits(L[k]) != 0x8000000000000000ull;
   return ok;
 }
 
-PG_DEV double clampd(double a, double b, double c) { return a < b ? b : a > c ? c : a; }
+template <class R>
+PG_DEV R clampd(R a, double b, double c) { return a < b ? like(a, b) : a > c ? like(a, c) : a; }
 
 // Closest point of triangle (a,b,c) to sphere centre p, by Voronoi regions of
 // the (s,t) parameter plane (condet.ispc:294-400).  Writes the point and the
@@ -357,35 +376,36 @@ PG_DEV double clampd(double a, double b, double c) { return a < b ? b : a > c ? 
 // 'edge_typo' reproduces the reference's -e/c in the s >= 0, t < 0 region
 // beyond edge bc (condet.ispc:373); otherwise the ab-edge parameter -d/a.
 // closest point of triangle (A, Bv, Cv) to p (condet.ispc:312-388 regions)
-PG_DEV void triangle_closest(const double *A, const double *Bv, const double *Cv, const double *p,
-                             double *point, bool edge_typo)
+template <class R>
+PG_DEV void triangle_closest(const R *A, const R *Bv, const R *Cv, const R *p, R *point, bool edge_typo)
 {
-  double edge0[3] = {Bv[0]-A[0], Bv[1]-A[1], Bv[2]-A[2]};
-  double edge1[3] = {Cv[0]-A[0], Cv[1]-A[1], Cv[2]-A[2]};
-  double v0[3] = {A[0]-p[0], A[1]-p[1], A[2]-p[2]};
-  double a = dot3(edge0, edge0);
-  double b = dot3(edge0, edge1);
-  double c = dot3(edge1, edge1);
-  double d = dot3(edge0, v0);
-  double e = dot3(edge1, v0);
-  double det = a*c - b*b;
-  double s = b*e - c*d;
-  double t = b*d - a*e;
+  const R zero = like(A[0], 0.0);
+  R edge0[3] = {Bv[0]-A[0], Bv[1]-A[1], Bv[2]-A[2]};
+  R edge1[3] = {Cv[0]-A[0], Cv[1]-A[1], Cv[2]-A[2]};
+  R v0[3] = {A[0]-p[0], A[1]-p[1], A[2]-p[2]};
+  R a = dot3(edge0, edge0);
+  R b = dot3(edge0, edge1);
+  R c = dot3(edge1, edge1);
+  R d = dot3(edge0, v0);
+  R e = dot3(edge1, v0);
+  R det = a*c - b*b;
+  R s = b*e - c*d;
+  R t = b*d - a*e;
   if (s + t < det)
   {
     if (s < 0.0)
     {
       if (t < 0.0)
       {
-        if (d < 0.0) { s = clampd(-d/a, 0.0, 1.0); t = 0.0; }
-        else { s = 0.0; t = clampd(-e/c, 0.0, 1.0); }
+        if (d < 0.0) { s = clampd(-d/a, 0.0, 1.0); t = zero; }
+        else { s = zero; t = clampd(-e/c, 0.0, 1.0); }
       }
-      else { s = 0.0; t = clampd(-e/c, 0.0, 1.0); }
+      else { s = zero; t = clampd(-e/c, 0.0, 1.0); }
     }
-    else if (t < 0.0) { s = clampd(-d/a, 0.0, 1.0); t = 0.0; }
+    else if (t < 0.0) { s = clampd(-d/a, 0.0, 1.0); t = zero; }
     else
     {
-      double invDet = 1.0 / det;
+      R invDet = 1.0 / det;
       s *= invDet;
       t *= invDet;
     }
@@ -394,32 +414,32 @@ PG_DEV void triangle_closest(const double *A, const double *Bv, const double *Cv
   {
     if (s < 0.0)
     {
-      double tmp0 = b+d;
-      double tmp1 = c+e;
+      R tmp0 = b+d;
+      R tmp1 = c+e;
       if (tmp1 > tmp0)
       {
-        double numer = tmp1 - tmp0;
-        double denom = a-2*b+c;
+        R numer = tmp1 - tmp0;
+        R denom = a-2*b+c;
         s = clampd(numer/denom, 0.0, 1.0);
         t = 1-s;
       }
-      else { t = clampd(-e/c, 0.0, 1.0); s = 0.0; }
+      else { t = clampd(-e/c, 0.0, 1.0); s = zero; }
     }
     else if (t < 0.0)
     {
       if (a+d > b+e)
       {
-        double numer = c+e-b-d;
-        double denom = a-2*b+c;
+        R numer = c+e-b-d;
+        R denom = a-2*b+c;
         s = clampd(numer/denom, 0.0, 1.0);
         t = 1-s;
       }
-      else { s = edge_typo ? clampd(-e/c, 0.0, 1.0) : clampd(-d/a, 0.0, 1.0); t = 0.0; }
+      else { s = edge_typo ? clampd(-e/c, 0.0, 1.0) : clampd(-d/a, 0.0, 1.0); t = zero; }
     }
     else
     {
-      double numer = c+e-b-d;
-      double denom = a-2*b+c;
+      R numer = c+e-b-d;
+      R denom = a-2*b+c;
       s = clampd(numer/denom, 0.0, 1.0);
       t = 1.0 - s;
     }

@@ -388,6 +388,7 @@ __global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g)
 // each, so that a warp runs one kind on all its lanes
 __global__ void __launch_bounds__(TPB) k_tt_vertex_face(PgTT g)
 {
+  const pg::Num<pg::f64> N;
   const int n = min(g.qn[2], g.vcap);
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
   {
@@ -396,10 +397,10 @@ __global__ void __launch_bounds__(TPB) k_tt_vertex_face(PgTT g)
     const int k = g.near[it >> 4].pair, i = it & 15u;
     const int tp = i < 3 ? g.pf[k] : g.pu[k], tt = i < 3 ? g.pu[k] : g.pf[k], vi = i < 3 ? i : i - 3;
     const double *P = g.geo + (size_t)PG_TT_GEO * tp + 3*vi, *T = g.geo + (size_t)PG_TT_GEO * tt;
-    const double p[3] = {P[0], P[1], P[2]};
-    double v[9], ab[3], ac[3], q[3], h[3], x0, x1;
-    for (int c = 0; c < 9; c ++) v[c] = T[c];
-    for (int c = 0; c < 3; c ++) { ab[c] = T[9 + c]; ac[c] = T[21 + c]; }
+    const pg::f64 p[3] = {N(P[0]), N(P[1]), N(P[2])};
+    pg::f64 v[9], ab[3], ac[3], q[3], h[3], x0, x1;
+    for (int c = 0; c < 9; c ++) v[c] = N(T[c]);
+    for (int c = 0; c < 3; c ++) { ab[c] = N(T[9 + c]); ac[c] = N(T[21 + c]); }
     const int region = pgtt::point_triangle_region(p, v, v + 3, v + 6, ab, ac, &x0, &x1);
     pgtt::point_triangle_at(region, x0, x1, v, v + 3, v + 6, ab, ac, q);
     if (i < 3) pgtt::sub(p, q, h);
@@ -414,6 +415,7 @@ __global__ void __launch_bounds__(TPB) k_tt_vertex_face(PgTT g)
 
 __global__ void __launch_bounds__(TPB) k_tt_edge_edge(PgTT g)
 {
+  const pg::Num<pg::f64> N;
   const int n = min(g.qn[3], g.ecap);
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
   {
@@ -421,10 +423,13 @@ __global__ void __launch_bounds__(TPB) k_tt_edge_edge(PgTT g)
     if (it == ~0u) continue;
     const int k = g.near[it >> 4].pair, i = (it & 15u) / 3u, j = (it & 15u) % 3u;
     const double *A = g.geo + (size_t)PG_TT_GEO * g.pf[k], *B = g.geo + (size_t)PG_TT_GEO * g.pu[k];
-    const double p1[3] = {A[3*i], A[3*i+1], A[3*i+2]}, d1[3] = {A[9+3*i], A[10+3*i], A[11+3*i]};
-    const double p2[3] = {B[3*j], B[3*j+1], B[3*j+2]}, d2[3] = {B[9+3*j], B[10+3*j], B[11+3*j]};
-    double s, t, c1[3], c2[3], h[3];
-    pgtt::segment_params(p1, d1, A[18+i], p2, d2, B[18+j], &s, &t);
+    pg::f64 p1[3], d1[3], p2[3], d2[3], s, t, c1[3], c2[3], h[3];
+    for (int c = 0; c < 3; c ++)
+    {
+      p1[c] = N(A[3*i + c]); d1[c] = N(A[9 + 3*i + c]);
+      p2[c] = N(B[3*j + c]); d2[c] = N(B[9 + 3*j + c]);
+    }
+    pgtt::segment_params(p1, d1, N(A[18+i]), p2, d2, N(B[18+j]), &s, &t);
     pgtt::segment_at(p1, d1, s, c1);
     pgtt::segment_at(p2, d2, t, c2);
     pgtt::sub(c1, c2, h);

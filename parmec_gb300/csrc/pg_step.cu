@@ -13,6 +13,7 @@
 // list in master order), so results repeat bit for bit from run to run.
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <type_traits>
 #include "pg_state.h"
 #include "pg_math.cuh"
 #include "pg_launch.h"
@@ -144,8 +145,8 @@ __global__ void k_euler(PgDev d, double step)
 }
 
 // ---------------------------------------------------------------- shapes (shapes.ispc:29-211)
-__device__ __forceinline__ void body_point(const double *x, const double *L, const double *X,
-                                           const double *C0, double *c)
+template <class R>
+__device__ __forceinline__ void body_point(const R *x, const R *L, const double *X, const double *C0, R *c)
 {
   double C[3] = {C0[0], C0[1], C0[2]};
   C[0] -= X[0]; C[1] -= X[1]; C[2] -= X[2];     // SCC (X, C)
@@ -158,8 +159,8 @@ __device__ __forceinline__ void body_point(const double *x, const double *L, con
 // (x + 0 = x).  That is every SPHERE particle, whose sphere centre is its
 // reference point; the test runs on the integer pipe and saves the 21 FP64
 // instructions of body_point.
-__device__ __forceinline__ bool centre_is_position(const double *x, const double *L, const double *X,
-                                                   const double *C)
+template <class R>
+__device__ __forceinline__ bool centre_is_position(const R *x, const R *L, const double *X, const double *C)
 {
   bool ok = true;
   for (int k = 0; k < 3; k ++)
@@ -530,11 +531,12 @@ __global__ void __launch_bounds__(TPB) k_contacts_probe(PgDev d, int xblocks, do
   if (pgk::excite_front(d, xblocks, step)) return;
   const int i = (blockIdx.x - xblocks) * blockDim.x + threadIdx.x;
   const int cnt = i < d.ellnum ? d.ncnt[i] : 0;
-  double c[3] = {0.0, 0.0, 0.0}, ri = 0.0;
+  const Num<f64> N;
+  f64 c[3] = {N(0.0), N(0.0), N(0.0)}, ri = N(0.0);
   if (cnt > 0)
   {
-    c[0] = d.center[0][i]; c[1] = d.center[1][i]; c[2] = d.center[2][i];
-    ri = d.radii[0][i];
+    for (int k = 0; k < 3; k ++) c[k] = N(d.center[k][i]);
+    ri = N(d.radii[0][i]);
   }
   // every lane of the warp takes part in each round's vote
   int kmax = cnt;
@@ -570,9 +572,9 @@ __global__ void __launch_bounds__(TPB) k_contacts_probe(PgDev d, int xblocks, do
       const size_t idx = (size_t)k * d.estride + i;
       if (code[j] >= 0)
       {
-        const double w[3] = {c[0]-q[j][0], c[1]-q[j][1], c[2]-q[j][2]};
-        const double d2 = dot3(w, w);
-        const double sr = ri+rj[j];
+        const f64 w[3] = {c[0]-q[j][0], c[1]-q[j][1], c[2]-q[j][2]};
+        const f64 d2 = dot3(w, w);
+        const f64 sr = ri+rj[j];
         if (gt_nonneg(d2, (sr*sr) * (1.0 + 1e-12)))
         {
           push = false;
@@ -600,62 +602,62 @@ __global__ void __launch_bounds__(TPB) k_contacts_probe(PgDev d, int xblocks, do
 
 // geometry, the creation/persistence rule, contact velocities and the granular
 // law of one candidate entry, written to its slot
-template <bool GEOM, bool ADAPT>
-__device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double step, bool obsc)
+template <bool GEOM, bool ADAPT, class R>
+__device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double step, bool obsc, const Num<R> &N)
 {
   const size_t idx = (size_t)idx0;
   const int i = idx0 % d.estride;
   const int pi = d.part[i];
-  double x[3], v[3], oi[3], c[3];
+  R x[3], v[3], oi[3], c[3];
   for (int k = 0; k < 3; k ++)
   {
-    x[k] = d.position[k][pi];
-    v[k] = d.linear[k][pi];
-    oi[k] = d.angular[3+k][pi];
-    c[k] = d.center[k][i];
+    x[k] = N(d.position[k][pi]);
+    v[k] = N(d.linear[k][pi]);
+    oi[k] = N(d.angular[3+k][pi]);
+    c[k] = N(d.center[k][i]);
   }
-  const double ri = d.radii[0][i];
+  const R ri = N(d.radii[0][i]);
   const int coli = d.ellcol[i];
   const double invmi = d.invm[pi], massi = d.mass[pi];
   const int code = d.ncode[idx];
   const bool existing = d.nflag[idx] != 0;
-  double point[3], normal[3], depth = 0.0, q[3], len = 0.0;
+  R point[3], normal[3], depth = N(0.0), q[3], len = N(0.0);
   int pj, colj;
   bool apart;
   bool sphere = code >= 0;
-  double cj[3];
+  R cj[3];
   if (sphere)
   {
     const int j = code;
     pj = d.part[j];
     colj = d.ellcol[j];
-    cj[0] = d.center[0][j]; cj[1] = d.center[1][j]; cj[2] = d.center[2][j];
+    for (int k = 0; k < 3; k ++) cj[k] = N(d.center[k][j]);
     q[0] = c[0]-cj[0];
     q[1] = c[1]-cj[1];
     q[2] = c[2]-cj[2];
-    const double d2 = dot3(q, q);
-    const double sr = ri+d.radii[0][j];
+    const R d2 = dot3(q, q);
+    const R sr = ri+d.radii[0][j];
     apart = gt_nonneg(d2, (sr*sr) * (1.0 + 1e-12));
     if (!apart)
     {
-      len = sqrt(d2);
+      len = N(sqrt((double)d2));
       depth = sr - len;
     }
   }
   else
   {
     const int t = -code-1;
-    double A[3], B[3], C[3];
-    for (int kk = 0; kk < 3; kk ++) { A[kk] = d.tri[kk][t]; B[kk] = d.tri[3+kk][t]; C[kk] = d.tri[6+kk][t]; }
+    R A[3], B[3], C[3];
+    for (int kk = 0; kk < 3; kk ++) { A[kk] = N(d.tri[kk][t]); B[kk] = N(d.tri[3+kk][t]); C[kk] = N(d.tri[6+kk][t]); }
     triangle_closest(A, B, C, c, point, (d.compat & PG_COMPAT_TRIEDGE) != 0);
     q[0] = c[0]-point[0];
     q[1] = c[1]-point[1];
     q[2] = c[2]-point[2];
-    const double d2 = dot3(q, q);
+    const R d2 = dot3(q, q);
     apart = gt_nonneg(d2, (ri*ri) * (1.0 + 1e-12));
     if (!apart)
     {
-      len = sqrt(d2);
+      len = N(sqrt((double)d2));
       depth = ri - len;
     }
     pj = d.triobs[t];
@@ -673,7 +675,7 @@ __device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double s
   }
   if (sphere)
   {
-    double ilen = existing ? 1.0/len : (gt_zero_d(len) ? 1.0/len : 1.0);
+    const double ilen = existing ? 1.0/len : (gt_zero_d(len) ? 1.0/len : 1.0);
     point[0] = 0.5*(c[0]+cj[0]);
     point[1] = 0.5*(c[1]+cj[1]);
     point[2] = 0.5*(c[2]+cj[2]);
@@ -683,14 +685,15 @@ __device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double s
   }
   else
   {
-    double ilen = 1.0/len;
+    const double ilen = 1.0/len;
     normal[0] = ilen*q[0];
     normal[1] = ilen*q[1];
     normal[2] = ilen*q[2];
   }
 
   // contact point velocities (forces.ispc:226-279)
-  double z[3], vi[3], vj[3], oj[3], vij[3];
+  R z[3], vi[3], vj[3], vij[3];
+  double oj[3];
   z[0] = point[0]-x[0]; z[1] = point[1]-x[1]; z[2] = point[2]-x[2];
   vi[0] = oi[1]*z[2]-oi[2]*z[1] + v[0];
   vi[1] = oi[2]*z[0]-oi[0]*z[2] + v[1];
@@ -721,7 +724,7 @@ __device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double s
     }
     else
     {
-      vj[0] = vj[1] = vj[2] = 0.0;
+      vj[0] = vj[1] = vj[2] = N(0.0);
     }
   }
   vij[0] = vj[0] - vi[0];
@@ -732,9 +735,8 @@ __device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double s
   if (d.ikind[ij] != 0) set_err(d, PG_ERR_UNSUPPORTED, 4, i, ij);
 
   // granular force (forces.ispc:125-192)
-  double state[3];
-  if (existing) { state[0] = d.nstate[0][idx]; state[1] = d.nstate[1][idx]; state[2] = d.nstate[2][idx]; }
-  else { state[0] = 0.0; state[1] = 0.0; state[2] = 0.0; }
+  R state[3];
+  for (int k = 0; k < 3; k ++) state[k] = N(existing ? d.nstate[k][idx] : 0.0);
   double kn = d.iparam[0][ij];
   double en;
   if (d.nen) en = d.nen[idx];
@@ -743,18 +745,18 @@ __device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double s
     double ma = pj >= 0 ? 1.0 / (invmi + d.invm[pj]) : massi;
     en = d.iparam[1][ij] * 2.0 * sqrt(kn*ma);
   }
-  double vn = dot3(vij, normal);
-  double fn = kn*depth + en*vn;
-  double f[3];
+  const R vn = dot3(vij, normal);
+  const R fn = kn*depth + en*vn;
+  R f[3];
   f[0] = fn*normal[0];
   f[1] = fn*normal[1];
   f[2] = fn*normal[2];
   double kskn = d.iparam[6][ij];
-  double kt = kn * kskn;
-  double et = en * kskn;
+  const double kt = N(kn) * kskn;
+  const double et = N(en) * kskn;
   double mus = d.iparam[2][ij];
   double mud = d.iparam[3][ij];
-  double vt[3], ft[3];
+  R vt[3], ft[3];
   vt[0] = vij[0] - vn*normal[0];
   vt[1] = vij[1] - vn*normal[1];
   vt[2] = vij[2] - vn*normal[2];
@@ -764,7 +766,7 @@ __device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double s
   ft[0] = kt*state[0] + et*vt[0];
   ft[1] = kt*state[1] + et*vt[1];
   ft[2] = kt*state[2] + et*vt[2];
-  double flen = sqrt(dot3(ft, ft));
+  const double flen = sqrt((double)dot3(ft, ft));
   double lim = mus*fn;
   if (gt_d(flen, lim))
   {
@@ -791,11 +793,12 @@ __device__ __forceinline__ void contact_entry(const PgDev &d, int idx0, double s
 template <bool GEOM, bool ADAPT>
 __global__ void PG_LB_EVAL k_contacts_eval(PgDev d, double step)
 {
+  const Num<f64> N;
   if (ADAPT) step = d.hs[0];
   const int n = *d.cwork_n;
   const bool obsc = (d.compat & PG_COMPAT_OBSIDX) != 0;
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
-    contact_entry<GEOM, ADAPT>(d, d.cwork[w], step, obsc);
+    contact_entry<GEOM, ADAPT>(d, d.cwork[w], step, obsc, N);
 }
 
 // Probe and evaluation in one launch for a scene that leaves SMs idle: one
@@ -862,7 +865,7 @@ __global__ void __launch_bounds__(32) k_contacts_few(PgDev d, double step, int S
     __syncwarp();
     if (rest >= 0) list[lane] = rest;
     have -= n;
-    if (idx >= 0) contact_entry<GEOM, ADAPT>(d, idx, step, obsc);
+    if (idx >= 0) contact_entry<GEOM, ADAPT>(d, idx, step, obsc, Num<double>());
     __syncwarp();
   }
 }
@@ -1480,12 +1483,13 @@ __global__ void k_spring_run_totals_adapt(PgDev d)
 // dynamics.ispc:30-169, with h = step and h-bar = (step + step1)/2).
 // RESTRAIN (restrain.ispc:30-133): v loses its components along the three
 // direction rows of restraint q, in order (SUBMUL (v, DOT (v, l), l, v))
-__device__ __forceinline__ void restrain_vec(double *v, double *const dir[9], int q)
+template <class R>
+__device__ __forceinline__ void restrain_vec(R *v, double *const dir[9], int q)
 {
   for (int k = 0; k < 3; k ++)
   {
-    const double l[3] = {dir[3*k][q], dir[3*k+1][q], dir[3*k+2][q]};
-    const double dt = dot3(v, l);
+    const R l[3] = {like(v[0], dir[3*k][q]), like(v[0], dir[3*k+1][q]), like(v[0], dir[3*k+2][q])};
+    const R dt = dot3(v, l);
     v[0] = v[0] - dt*l[0];
     v[1] = v[1] - dt*l[1];
     v[2] = v[2] - dt*l[2];
@@ -1558,14 +1562,15 @@ enum { INT_FUSED = 0, INT_FORCES = 1, INT_DYNAMICS = 2, INT_FORCES_ADAPT = 3, IN
 // is then a zero of sign sign(m) xor sign(g), and F plus a zero is F, except
 // that two zeros sum to -0 only when both are -0 (the gravity components of
 // a scene that are zero)
-__device__ __forceinline__ double add_times_zero(double F, double m, double g)
+template <class R>
+__device__ __forceinline__ R add_times_zero(R F, double m, double g)
 {
   const unsigned long long bg = dbits(g);
-  if ((bg << 1) != 0 || !finite_d(m) || !finite_d(F)) return F + m*g;
+  if ((bg << 1) != 0 || !finite_d(m) || !finite_d(F)) return F + like(F, m)*g;
   const unsigned long long bF = dbits(F);
   if ((bF << 1) != 0) return F;
   const bool neg = (bF >> 63) && ((dbits(m) ^ bg) >> 63);
-  return __longlong_as_double(neg ? (long long)0x8000000000000000ull : 0ll);
+  return like(F, __longlong_as_double(neg ? (long long)0x8000000000000000ull : 0ll));
 }
 
 // half = step/2 and hstep = (step + step1)/2 come from the host (the same
@@ -1581,6 +1586,9 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
 {
   // fused modes: the first blocks move the obstacle triangles; `last`: the last
   // block to finish ends the step
+  // one warp an SM gains nothing from f64
+  typedef typename std::conditional<(WIDE > 1), double, f64>::type R;
+  const Num<R> N;
   const int i = ((int)blockIdx.x - oblocks) * (int)blockDim.x + (int)threadIdx.x;
   bool need = false;
   constexpr bool ADAPT = MODE == INT_FORCES_ADAPT;
@@ -1607,8 +1615,8 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
     const double *damping = d.t_damping + 6*(size_t)row;
     const bool typo = (d.compat & PG_COMPAT_EXPMAP) != 0;
     const int E = d.ellnum;
-    double po[3] = {d.position[0][i], d.position[1][i], d.position[2][i]};
-    double F[3], T[3];
+    const R po[3] = {N(d.position[0][i]), N(d.position[1][i]), N(d.position[2][i])};
+    R F[3], T[3];
     const int e = d.pell ? d.pell[i] : -1;
     const double ma = d.mass[i];
     double kact[3] = {0.0, 0.0, 0.0}, krot[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, kmax = 0.0, emax = 0.0;
@@ -1626,8 +1634,7 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
     }
     if (MODE == INT_DYNAMICS || MODE == INT_DYN_FUSED)
     {
-      F[0] = d.force[0][i]; F[1] = d.force[1][i]; F[2] = d.force[2][i];
-      T[0] = d.torque[0][i]; T[1] = d.torque[1][i]; T[2] = d.torque[2][i];
+      for (int k = 0; k < 3; k ++) { F[k] = N(d.force[k][i]); T[k] = N(d.torque[k][i]); }
     }
     else
     {
@@ -1637,7 +1644,7 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
     {
       // the master side of the sphere's contacts, summed here in slot order
       // as k_contacts_sum sums them into fm and tm in the adaptive mode
-      double fs[3] = {0.0, 0.0, 0.0}, ts[3] = {0.0, 0.0, 0.0};
+      R fs[3] = {N(0.0), N(0.0), N(0.0)}, ts[3] = {N(0.0), N(0.0), N(0.0)};
       const int cnt = d.ncnt[e];
       for (int k0 = 0; k0 < cnt; k0 += WIDE)
       {
@@ -1656,7 +1663,7 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
         for (int j = 0; j < WIDE; j ++)
           if (on[j])
           {
-            const double a[3] = {p[j][0]-po[0], p[j][1]-po[1], p[j][2]-po[2]};
+            const R a[3] = {p[j][0]-po[0], p[j][1]-po[1], p[j][2]-po[2]};
             fs[0] += f[j][0]; fs[1] += f[j][1]; fs[2] += f[j][2];
             ts[0] += a[1]*f[j][2] - a[2]*f[j][1];
             ts[1] += a[2]*f[j][0] - a[0]*f[j][2];
@@ -1668,10 +1675,9 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
     }
     else if (e >= 0)
     {
-      F[0] = d.fm[0][i]; F[1] = d.fm[1][i]; F[2] = d.fm[2][i];
-      T[0] = d.tm[0][i]; T[1] = d.tm[1][i]; T[2] = d.tm[2][i];
+      for (int k = 0; k < 3; k ++) { F[k] = N(d.fm[k][i]); T[k] = N(d.tm[k][i]); }
     }
-    else { F[0] = F[1] = F[2] = 0.0; T[0] = T[1] = T[2] = 0.0; }
+    else for (int k = 0; k < 3; k ++) F[k] = T[k] = N(0.0);
 
     // slave contacts, in master order (forces.ispc:539-569)
     if (E)
@@ -1694,8 +1700,8 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
       {
         if (!on[j]) continue;
         const int ref = refs[j];
-        double f[3] = {-fr[j][0], -fr[j][1], -fr[j][2]};
-        double a[3] = {pr[j][0]-po[0], pr[j][1]-po[1], pr[j][2]-po[2]};
+        const double f[3] = {-fr[j][0], -fr[j][1], -fr[j][2]};
+        const R a[3] = {pr[j][0]-po[0], pr[j][1]-po[1], pr[j][2]-po[2]};
         F[0] += f[0]; F[1] += f[1]; F[2] += f[2];
         T[0] += a[1]*f[2] - a[2]*f[1];
         T[1] += a[2]*f[0] - a[0]*f[2];
@@ -1725,7 +1731,8 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
           kmax = kc > kmax ? kc : kmax;
           emax = ec > emax ? ec : emax;
           double A[3];
-          nvmul(Li, a, A);
+          const double arm[3] = {a[0], a[1], a[2]};
+          nvmul(Li, arm, A);
           krot_add(krot, A);
         }
       }
@@ -1892,36 +1899,37 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
       const double *ang = d.t_prs_ang + (size_t)row * d.tab_prs_stride + 3*q;
       if (d.prslin[q] && d.linkind[q] == 1)
       {
-        F[0] = ma * lin[0]; F[1] = ma * lin[1]; F[2] = ma * lin[2];
+        for (int k = 0; k < 3; k ++) F[k] = N(ma * lin[k]);
       }
       else if (d.prslin[q] && d.linkind[q] == 0)
       {
-        F[0] = 0.0; F[1] = 0.0; F[2] = 0.0;
+        F[0] = F[1] = F[2] = N(0.0);
       }
       if (d.prsang[q] && d.angkind[q] == 1)
       {
-        double in[9], acc[3] = {ang[0], ang[1], ang[2]};
+        double in[9];
+        const R acc[3] = {N(ang[0]), N(ang[1]), N(ang[2])};
         for (int k = 0; k < 9; k ++) in[k] = d.inertia[k][i];
         nvmul(in, acc, T);
       }
       else if (d.prsang[q] && d.angkind[q] == 0)
       {
-        T[0] = 0.0; T[1] = 0.0; T[2] = 0.0;
+        T[0] = T[1] = T[2] = N(0.0);
       }
     }
 
     // dynamics_task (dynamics.ispc:30-169)
-    double O[3], o[3], v[3], L1[9], J[9], I[9], im, f[3], t[3], Tb[3], DL[9], L2[9], A[3], B[3];
-    double x[3] = {po[0], po[1], po[2]};
+    R O[3], o[3], v[3], L1[9], J[9], I[9], im, f[3], t[3], Tb[3], DL[9], L2[9], A[3], B[3];
+    R x[3] = {po[0], po[1], po[2]};
     if (!(d.flags[i] & PG_FLAG_SKIP))
     {
-      for (int k = 0; k < 3; k ++) { O[k] = d.angular[k][i]; v[k] = d.linear[k][i]; }
+      for (int k = 0; k < 3; k ++) { O[k] = N(d.angular[k][i]); v[k] = N(d.linear[k][i]); }
       const bool iso = d.piso && d.piso[i];
       const double js = iso ? d.inertia[0][i] : 0.0, is = iso ? d.inverse[0][i] : 0.0;
-      for (int k = 0; k < 9; k ++) L1[k] = d.rotation[k][i];
+      for (int k = 0; k < 9; k ++) L1[k] = N(d.rotation[k][i]);
       if (!iso)
-        for (int k = 0; k < 9; k ++) { J[k] = d.inertia[k][i]; I[k] = d.inverse[k][i]; }
-      im = d.invm[i];
+        for (int k = 0; k < 9; k ++) { J[k] = N(d.inertia[k][i]); I[k] = N(d.inverse[k][i]); }
+      im = N(d.invm[i]);
       if (nonzero_d(damping[0]) || nonzero_d(damping[1]) || nonzero_d(damping[2]))
       {
         F[0] -= ma * damping[0] * v[0];
@@ -1930,9 +1938,7 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
       }
       if (nonzero_d(damping[3]) || nonzero_d(damping[4]) || nonzero_d(damping[5]))
       {
-        o[0] = damping[3]*d.angular[3][i];
-        o[1] = damping[4]*d.angular[4][i];
-        o[2] = damping[5]*d.angular[5][i];
+        for (int k = 0; k < 3; k ++) o[k] = N(damping[3+k]*d.angular[3+k][i]);
         tvmul(L1, o, t);
         if (iso) iso_nvmul(js, t, Tb); else nvmul(J, t, Tb);
         nvmul(L1, Tb, t);
@@ -1941,7 +1947,7 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
       f[0] = F[0]; f[1] = F[1]; f[2] = F[2];
       t[0] = T[0]; t[1] = T[1]; t[2] = T[2];
       const bool free_spin = (dbits(T[0]) << 1 | dbits(T[1]) << 1 | dbits(T[2]) << 1) == 0;
-      if (iso && free_spin) Tb[0] = Tb[1] = Tb[2] = 0.0;
+      if (iso && free_spin) Tb[0] = Tb[1] = Tb[2] = N(0.0);
       else tvmul(L1, t, Tb);
       if (iso && gyro_settled(O, Tb, js, is, step, half))
       {
@@ -1984,7 +1990,7 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
         // where all three products are
         for (int k = 0; k < 9; k ++) L2[k] = L1[k];
         for (int k = 0; k < 3; k ++)
-          o[k] = __longlong_as_double((long long)(dbits(L1[k]) & dbits(L1[3+k]) & dbits(L1[6+k]) & 0x8000000000000000ull));
+          o[k] = N(__longlong_as_double((long long)(dbits(L1[k]) & dbits(L1[3+k]) & dbits(L1[6+k]) & 0x8000000000000000ull)));
       }
       else
       {
@@ -2002,10 +2008,10 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
         const int q = d.prs_list[pp];
         const double *lin = d.t_prs_lin + (size_t)row * d.tab_prs_stride + 3*q;
         const double *ang = d.t_prs_ang + (size_t)row * d.tab_prs_stride + 3*q;
-        if (d.prslin[q] && d.linkind[q] == 0) { v[0] = lin[0]; v[1] = lin[1]; v[2] = lin[2]; }
+        if (d.prslin[q] && d.linkind[q] == 0) for (int k = 0; k < 3; k ++) v[k] = N(lin[k]);
         if (d.prsang[q] && d.angkind[q] == 0)
         {
-          double oo[3] = {ang[0], ang[1], ang[2]};
+          const R oo[3] = {N(ang[0]), N(ang[1]), N(ang[2])};
           tvmul(L2, oo, O);
           o[0] = oo[0]; o[1] = oo[1]; o[2] = oo[2];
         }
@@ -2038,7 +2044,7 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
           for (int k = 0; k < 3; k ++) { d.angular[k][i] = Oc[k]; d.angular[3+k][i] = oo[k]; }
         }
       }
-      for (int k = 0; k < 9; k ++) L2[k] = d.rotation[k][i];
+      for (int k = 0; k < 9; k ++) L2[k] = N(d.rotation[k][i]);
     }
     d.force[0][i] = F[0]; d.force[1][i] = F[1]; d.force[2][i] = F[2];
     d.torque[0][i] = T[0]; d.torque[1][i] = T[1]; d.torque[2][i] = T[2];
@@ -2047,7 +2053,8 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
     if (FUSED && e >= 0)
     {
       double X[3] = {d.position[3][i], d.position[4][i], d.position[5][i]};
-      double C[3] = {d.center[3][e], d.center[4][e], d.center[5][e]}, c[3];
+      double C[3] = {d.center[3][e], d.center[4][e], d.center[5][e]};
+      R c[3];
       if (centre_is_position(x, L2, X, C)) { c[0] = x[0]; c[1] = x[1]; c[2] = x[2]; }
       else body_point(x, L2, X, C, c);
       d.center[0][e] = c[0]; d.center[1][e] = c[1]; d.center[2][e] = c[2];

@@ -18,6 +18,7 @@
 #pragma once
 #include <math.h>
 #include <string.h>
+#include "pg_f64.cuh"
 
 #ifdef __CUDACC__
 #define PG_TT __host__ __device__ __forceinline__
@@ -27,8 +28,12 @@
 
 namespace pgtt {
 
-PG_TT double dot(const double *a, const double *b) { return a[0]*b[0] + a[1]*b[1] + a[2]*b[2]; }
-PG_TT void sub(const double *a, const double *b, double *c) { c[0] = a[0]-b[0]; c[1] = a[1]-b[1]; c[2] = a[2]-b[2]; }
+using pg::like;
+
+// The distances take double or, on the device, f64 (pg_f64.cuh): the same
+// expressions, the same bits.
+template <class R> PG_TT R dot(const R *a, const R *b) { return a[0]*b[0] + a[1]*b[1] + a[2]*b[2]; }
+template <class R> PG_TT void sub(const R *a, const R *b, R *c) { c[0] = a[0]-b[0]; c[1] = a[1]-b[1]; c[2] = a[2]-b[2]; }
 PG_TT void cross(const double *a, const double *b, double *c)
 {
   c[0] = a[1]*b[2] - a[2]*b[1];
@@ -96,7 +101,7 @@ PG_TT bool gt1(double x) { return bits(x) - 0x3ff0000000000001ULL < 0x4000000000
 PG_TT bool lt0(double x) { return x < 0.0; }
 PG_TT bool gt1(double x) { return x > 1.0; }
 #endif
-PG_TT double clamp01(double x) { return lt0(x) ? 0.0 : (gt1(x) ? 1.0 : x); }
+template <class R> PG_TT R clamp01(R x) { return lt0(x) ? like(x, 0.0) : (gt1(x) ? like(x, 1.0) : x); }
 
 // Closest point q of triangle (a, b, c) to p: the Voronoi-region method
 // (Ericson, Real-Time Collision Detection, 5.1.5).  The region is found
@@ -105,18 +110,18 @@ PG_TT double clamp01(double x) { return lt0(x) ? 0.0 : (gt1(x) ? 1.0 : x); }
 // divides the same operands as the textbook branches do.
 // (ab = b - a and ac = c - a come with the triangle, computed once for the
 // three calls of a triangle pair that use them.)
-PG_TT int point_triangle_region(const double *p, const double *a, const double *b, const double *c,
-                                const double *ab, const double *ac, double *x0, double *x1)
+template <class R>
+PG_TT int point_triangle_region(const R *p, const R *a, const R *b, const R *c, const R *ab, const R *ac, R *x0, R *x1)
 {
-  double ap[3], bp[3], cp[3];
+  R ap[3], bp[3], cp[3];
   sub(p, a, ap); sub(p, b, bp); sub(p, c, cp);
-  const double d1 = dot(ab, ap), d2 = dot(ac, ap);
-  const double d3 = dot(ab, bp), d4 = dot(ac, bp);
-  const double d5 = dot(ab, cp), d6 = dot(ac, cp);
-  const double vc = d1*d4 - d3*d2;
-  const double vb = d5*d2 - d1*d6;
-  const double va = d3*d6 - d5*d4;
-  const double e43 = d4 - d3, e56 = d5 - d6;
+  const R d1 = dot(ab, ap), d2 = dot(ac, ap);
+  const R d3 = dot(ab, bp), d4 = dot(ac, bp);
+  const R d5 = dot(ab, cp), d6 = dot(ac, cp);
+  const R vc = d1*d4 - d3*d2;
+  const R vb = d5*d2 - d1*d6;
+  const R va = d3*d6 - d5*d4;
+  const R e43 = d4 - d3, e56 = d5 - d6;
   // 0: vertex a, 1: vertex b, 2: edge ab, 3: vertex c, 4: edge ac, 5: edge bc, 6: face
   const int region = (le0(d1) && le0(d2)) ? 0 :
                      (ge0(d3) && le(d4, d3)) ? 1 :
@@ -124,20 +129,20 @@ PG_TT int point_triangle_region(const double *p, const double *a, const double *
                      (ge0(d6) && le(d5, d6)) ? 3 :
                      (le0(vb) && ge0(d2) && le0(d6)) ? 4 :
                      (le0(va) && ge0(e43) && ge0(e56)) ? 5 : 6;
-  double num = 0.0, den = 1.0;
+  R num = like(d1, 0.0), den = like(d1, 1.0);
   if (region == 2) { num = d1; den = d1 - d3; }
   else if (region == 4) { num = d2; den = d2 - d6; }
   else if (region == 5) { num = e43; den = e43 + e56; }
-  else if (region == 6) { num = 1.0; den = va + vb + vc; }
-  const double x = num / den;
+  else if (region == 6) { num = like(d1, 1.0); den = va + vb + vc; }
+  const R x = num / den;
   *x0 = region == 6 ? vb * x : x;
-  *x1 = region == 6 ? vc * x : 0.0;
+  *x1 = region == 6 ? vc * x : like(x, 0.0);
   return region;
 }
 
 // the point of a region: x0 along its edge, or x0 and x1 on the face
-PG_TT void point_triangle_at(int region, double x0, double x1, const double *a, const double *b, const double *c,
-                             const double *ab, const double *ac, double *q)
+template <class R>
+PG_TT void point_triangle_at(int region, R x0, R x1, const R *a, const R *b, const R *c, const R *ab, const R *ac, R *q)
 {
   switch (region)
   {
@@ -168,32 +173,32 @@ PG_TT void point_triangle(const double *p, const double *a, const double *b, con
 // numerator applies), so that threads of a warp share them.
 // (d1 = q1 - p1 and d2 = q2 - p2 come with the triangles' edges, a = d1.d1
 // and e = d2.d2 with them.)
-PG_TT void segment_params(const double *p1, const double *d1, double a, const double *p2, const double *d2,
-                          double e, double *ps, double *pt)
+template <class R>
+PG_TT void segment_params(const R *p1, const R *d1, R a, const R *p2, const R *d2, R e, R *ps, R *pt)
 {
-  double r[3];
+  R r[3];
   sub(p1, p2, r);
-  const double f = dot(d2, r);
-  double s, t;
-  if (le0(a) && le0(e)) { s = 0.0; t = 0.0; }
-  else if (le0(a)) { s = 0.0; t = clamp01(f / e); }
+  const R f = dot(d2, r), zero = like(f, 0.0);
+  R s, t;
+  if (le0(a) && le0(e)) { s = zero; t = zero; }
+  else if (le0(a)) { s = zero; t = clamp01(f / e); }
   else
   {
-    const double c = dot(d1, r);
-    if (le0(e)) { t = 0.0; s = clamp01(-c / a); }
+    const R c = dot(d1, r);
+    if (le0(e)) { t = zero; s = clamp01(-c / a); }
     else
     {
-      const double b = dot(d1, d2);
-      const double den = a*e - b*b;
+      const R b = dot(d1, d2);
+      const R den = a*e - b*b;
       const bool skew = (bits(den) << 1) != 0;            // den != 0
-      const double s0 = (b*f - c*e) / (skew ? den : 1.0);
-      s = skew ? clamp01(s0) : 0.0;
+      const R s0 = (b*f - c*e) / (skew ? den : like(den, 1.0));
+      s = skew ? clamp01(s0) : zero;
       t = (b*s + f) / e;
       const bool low = lt0(t), high = gt1(t);
       if (low || high)
       {
         s = clamp01((low ? -c : b - c) / a);
-        t = low ? 0.0 : 1.0;
+        t = low ? zero : like(zero, 1.0);
       }
     }
   }
@@ -201,7 +206,8 @@ PG_TT void segment_params(const double *p1, const double *d1, double a, const do
   *pt = t;
 }
 
-PG_TT void segment_at(const double *p, const double *d, double s, double *c)
+template <class R>
+PG_TT void segment_at(const R *p, const R *d, R s, R *c)
 {
   c[0] = p[0] + d[0]*s; c[1] = p[1] + d[1]*s; c[2] = p[2] + d[2]*s;
 }
