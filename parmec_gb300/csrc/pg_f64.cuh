@@ -54,8 +54,9 @@ template <> struct Num<f64>
   double one, nz;
   __device__ __forceinline__ Num()
   {
-    // zero, as far as anyone can tell: the first lane's thread index is below 1,024
-    const unsigned z = __shfl_sync(0xffffffffu, threadIdx.x, 0) >> 20;
+    // zero (the neighbour's thread index is below 1,024), but to the compiler a
+    // value of its own in every lane, which keeps it out of the uniform registers
+    const unsigned z = __shfl_xor_sync(0xffffffffu, threadIdx.x, 1) >> 20;
     one = __hiloint2double(0x3ff00000 | z, z);
     nz = __hiloint2double(0x80000000 | z, z);
   }
