@@ -441,29 +441,30 @@ __global__ void __launch_bounds__(TPB) k_tt_edge_edge(PgTT g)
 }
 
 // granular force of pair k with the contact found (depth > 0: active)
-__device__ __forceinline__ void tt_force(const PgDev &d, const PgTT &g, int k, int f, int u, double depth,
-                                         const double *point, const double *normal, double step)
+template <class R>
+__device__ __forceinline__ void tt_force(const PgDev &d, const PgTT &g, const pg::Num<R> &N, int k, int f, int u,
+                                         R depth, const R *point, const R *normal, double step)
 {
   const bool active = depth > 0.0, was = g.act[k] != 0;
   g.act[k] = active ? 1 : 0;
   if (!active) return;
-  double st[3], fr[3];
-  for (int c = 0; c < 3; c ++) st[c] = was ? g.st[c][k] : 0.0;
+  R st[3], fr[3];
+  for (int c = 0; c < 3; c ++) st[c] = N(was ? g.st[c][k] : 0.0);
   const int pa = d.triobs[f], pb = d.triobs[u];
   // contact point velocities (forces.ispc:226-246) and their difference
-  double vij[3];
-  const double za[3] = {point[0]-d.position[0][pa], point[1]-d.position[1][pa], point[2]-d.position[2][pa]};
-  const double zb[3] = {point[0]-d.position[0][pb], point[1]-d.position[1][pb], point[2]-d.position[2][pb]};
+  R vij[3];
+  const R za[3] = {point[0]-d.position[0][pa], point[1]-d.position[1][pa], point[2]-d.position[2][pa]};
+  const R zb[3] = {point[0]-d.position[0][pb], point[1]-d.position[1][pb], point[2]-d.position[2][pb]};
   for (int c = 0; c < 3; c ++)
   {
     const int c1 = (c+1)%3, c2 = (c+2)%3;
-    const double vi = d.angular[3+c1][pa]*za[c2] - d.angular[3+c2][pa]*za[c1] + d.linear[c][pa];
-    const double vj = d.angular[3+c1][pb]*zb[c2] - d.angular[3+c2][pb]*zb[c1] + d.linear[c][pb];
+    const R vi = d.angular[3+c1][pa]*za[c2] - d.angular[3+c2][pa]*za[c1] + d.linear[c][pa];
+    const R vj = d.angular[3+c1][pb]*zb[c2] - d.angular[3+c2][pb]*zb[c1] + d.linear[c][pb];
     vij[c] = vj - vi;
   }
   const int ij = pgk::pairing(d, d.tricol[f], d.tricol[u]);
   if (d.ikind[ij] != 0) pgk::set_err(d, PG_ERR_UNSUPPORTED, 41, k, ij);
-  const double ma = 1.0 / (d.invm[pa] + d.invm[pb]);
+  const R ma = 1.0 / (N(d.invm[pa]) + d.invm[pb]);
   pgtt::granular(d.iparam[0][ij], d.iparam[1][ij], d.iparam[6][ij], d.iparam[2][ij], d.iparam[3][ij], ma,
                  normal, vij, depth, step, st, fr);
   for (int c = 0; c < 3; c ++)
@@ -488,8 +489,12 @@ __device__ __noinline__ double tt_contact(const PgDev &d, const PgTT &g, int f, 
 // as the full search keeps it; then the granular force.  The plane test,
 // which calls a pair apart that the distances would call touching only
 // within its rounding, is taken for depths below 1e-9 of the pair's size.
-__global__ void __launch_bounds__(TPB) k_tt_near(PgDev d, PgTT g, double step)
+// Bound by FP64 issue and by the gathers before it: four blocks an SM hide
+// more of them than three or five (a step of a 48x48 lattice pressed together
+// 898 us against 910 and 904; 926 with constants as operands and three).
+__global__ void __launch_bounds__(TPB, 4) k_tt_near(PgDev d, PgTT g, double step)
 {
+  const pg::Num<pg::f64> N;
   const int n = g.qn[0];
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
   {
@@ -504,35 +509,43 @@ __global__ void __launch_bounds__(TPB) k_tt_near(PgDev d, PgTT g, double step)
       const double d2 = i < 6 ? g.vres[3*(size_t)slot] : g.eres[3*(size_t)slot];
       if (d2 < best) { best = d2; at = slot; cand = i; }
     }
-    double point[3], normal[3], depth;
+    pg::f64 point[3], normal[3], depth;
     if (at < 0 || !(best > 0.0) || !(best <= (double)e.upper * (double)e.upper))
-      depth = tt_contact(d, g, f, u, point, normal);
+    {
+      double po[3], no[3];
+      depth = N(tt_contact(d, g, f, u, po, no));
+      for (int c = 0; c < 3; c ++) { point[c] = N(po[c]); normal[c] = N(no[c]); }
+    }
     else
     {
       const double *A = g.geo + (size_t)PG_TT_GEO * f, *B = g.geo + (size_t)PG_TT_GEO * u;
-      double pa[3], pb[3];
+      pg::f64 pa[3], pb[3], v[9], x[3], y[3];
       if (cand < 6)
       {
         const double *P = (cand < 3 ? A : B) + 3 * (cand < 3 ? cand : cand - 3), *T = cand < 3 ? B : A;
-        double q[3];
-        pgtt::point_triangle_at((int)g.vit[at], g.vres[3*(size_t)at+1], g.vres[3*(size_t)at+2], T, T + 3, T + 6, T + 9,
-                                T + 21, q);
-        for (int c = 0; c < 3; c ++) { pa[c] = cand < 3 ? P[c] : q[c]; pb[c] = cand < 3 ? q[c] : P[c]; }
+        pg::f64 q[3];
+        for (int c = 0; c < 9; c ++) v[c] = N(T[c]);
+        for (int c = 0; c < 3; c ++) { x[c] = N(T[9 + c]); y[c] = N(T[21 + c]); }
+        pgtt::point_triangle_at((int)g.vit[at], N(g.vres[3*(size_t)at+1]), N(g.vres[3*(size_t)at+2]), v, v + 3, v + 6,
+                                x, y, q);
+        for (int c = 0; c < 3; c ++) { pa[c] = cand < 3 ? N(P[c]) : q[c]; pb[c] = cand < 3 ? q[c] : N(P[c]); }
       }
       else
       {
         const int i = (cand - 6) / 3, j = (cand - 6) % 3;
-        pgtt::segment_at(A + 3*i, A + 9 + 3*i, g.eres[3*(size_t)at+1], pa);
-        pgtt::segment_at(B + 3*j, B + 9 + 3*j, g.eres[3*(size_t)at+2], pb);
+        for (int c = 0; c < 3; c ++) { x[c] = N(A[3*i + c]); y[c] = N(A[9 + 3*i + c]); }
+        pgtt::segment_at(x, y, N(g.eres[3*(size_t)at+1]), pa);
+        for (int c = 0; c < 3; c ++) { x[c] = N(B[3*j + c]); y[c] = N(B[9 + 3*j + c]); }
+        pgtt::segment_at(x, y, N(g.eres[3*(size_t)at+2]), pb);
       }
-      depth = pgtt::contact_at(pa, pb, best, g.r, g.r, point, normal);
+      depth = pgtt::contact_at(pa, pb, N(best), g.r, g.r, point, normal);
       if (depth > 0.0 && !(depth > 1e-9 * (double)e.size))
       {
         const double *Av[3] = {A, A + 3, A + 6}, *Bv[3] = {B, B + 3, B + 6};
-        if (pgtt::beyond_plane_of(A, A + 24, A[27], Bv) || pgtt::beyond_plane_of(B, B + 24, B[27], Av)) depth = -1.0;
+        if (pgtt::beyond_plane_of(A, A + 24, A[27], Bv) || pgtt::beyond_plane_of(B, B + 24, B[27], Av)) depth = N(-1.0);
       }
     }
-    tt_force(d, g, k, f, u, depth, point, normal, step);
+    tt_force(d, g, N, k, f, u, depth, point, normal, step);
   }
 }
 
@@ -546,7 +559,7 @@ __global__ void __launch_bounds__(TPB) k_tt_full(PgDev d, PgTT g, double step)
     const int k = g.full[w], f = g.pf[k], u = g.pu[k];
     double point[3], normal[3];
     const double depth = tt_contact(d, g, f, u, point, normal);
-    tt_force(d, g, k, f, u, depth, point, normal, step);
+    tt_force(d, g, pg::Num<double>(), k, f, u, depth, point, normal, step);
   }
 }
 

@@ -341,12 +341,12 @@ PG_TT bool apart(const double *const a[3], const double *const b[3], double ra, 
 
 // Depth, point and normal from the closest points of two triangles a
 // positive distance (squared: d2) apart
-PG_TT double contact_at(const double *pa, const double *pb, double d2, double ra, double rb, double *point,
-                        double *normal)
+template <class R>
+PG_TT R contact_at(const R *pa, const R *pb, R d2, double ra, double rb, R *point, R *normal)
 {
   point[0] = 0.5*(pa[0]+pb[0]); point[1] = 0.5*(pa[1]+pb[1]); point[2] = 0.5*(pa[2]+pb[2]);
-  const double d = sqrt(d2);
-  const double id = 1.0 / d;
+  const R d = like(d2, sqrt(d2));
+  const R id = 1.0 / d;
   normal[0] = (pa[0]-pb[0])*id; normal[1] = (pa[1]-pb[1])*id; normal[2] = (pa[2]-pb[2])*id;
   return (ra + rb) - d;
 }
@@ -395,18 +395,19 @@ PG_TT double contact(const double *const a[3], const double *const b[3], double 
 // partner towards the master), relative velocity vij = v_partner - v_master,
 // depth, pair parameters and reduced mass: the force f on the master, and
 // the tangential spring state advanced by step * the tangential velocity.
-PG_TT void granular(double kn, double damper, double kskn, double mus, double mud, double ma,
-                    const double *n, const double *vij, double depth, double step, double *state, double *f)
+template <class R>
+PG_TT void granular(double kn, double damper, double kskn, double mus, double mud, R ma,
+                    const R *n, const R *vij, R depth, double step, R *state, R *f)
 {
-  const double en = damper * 2.0 * sqrt(kn*ma);
-  const double vn = dot(vij, n);
-  const double fn = kn*depth + en*vn;
+  const R en = like(ma, damper) * 2.0 * like(ma, sqrt(kn*ma));
+  const R vn = dot(vij, n);
+  const R fn = kn*depth + en*vn;
   f[0] = fn*n[0];
   f[1] = fn*n[1];
   f[2] = fn*n[2];
-  const double kt = kn * kskn;
-  const double et = en * kskn;
-  double vt[3], ft[3];
+  const R kt = like(ma, kn) * kskn;
+  const R et = en * kskn;
+  R vt[3], ft[3];
   vt[0] = vij[0] - vn*n[0];
   vt[1] = vij[1] - vn*n[1];
   vt[2] = vij[2] - vn*n[2];
@@ -416,8 +417,8 @@ PG_TT void granular(double kn, double damper, double kskn, double mus, double mu
   ft[0] = kt*state[0] + et*vt[0];
   ft[1] = kt*state[1] + et*vt[1];
   ft[2] = kt*state[2] + et*vt[2];
-  const double len = sqrt(dot(ft, ft));
-  double lim = mus*fn;
+  const R len = like(ma, sqrt(dot(ft, ft)));
+  R lim = mus*fn;
   if (len > lim)
   {
     lim = mud*fn/len;
