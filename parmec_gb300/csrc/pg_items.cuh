@@ -1261,11 +1261,9 @@ __device__ __forceinline__ bool obstacles_item(const PgDev &d, int t, double ste
 
 // obstacle points (after every triangle used the old point), obstacle
 // velocity state, and the step counters (one thread)
-__device__ __forceinline__ void tail_item(const PgDev &d, double step, int use_row)
+__device__ __forceinline__ void obstacle_points(const PgDev &d, double step, int use_row, int row, int first, int by)
 {
-  const int row = use_row ? *d.stepno : 0;
-  const long long gs = use_row ? *d.gstep : 0;
-  for (int o = 0; o < d.obsnum; o ++)
+  for (int o = first; o < d.obsnum; o += by)
   {
     // the obstacle's loads first, then its scene test (one memory latency)
     const int sc = d.oscene[o];
@@ -1285,6 +1283,14 @@ __device__ __forceinline__ void tail_item(const PgDev &d, double step, int use_r
       for (int k = 0; k < 3; k ++) { d.obsang[3*o+k] = a[k]; d.obslin[3*o+k] = v[k]; }
     x[0] = p[0] + step*v[0]; x[1] = p[1] + step*v[1]; x[2] = p[2] + step*v[2];
   }
+}
+
+// by one thread
+__device__ __forceinline__ void tail_item(const PgDev &d, double step, int use_row)
+{
+  const int row = use_row ? *d.stepno : 0;
+  const long long gs = use_row ? *d.gstep : 0;
+  obstacle_points(d, step, use_row, row, 0, 1);
   if (use_row)
   {
     *d.stepno = row + 1;
@@ -1306,33 +1312,47 @@ static __device__ __noinline__ bool obstacles_front(const PgDev &d, int t, doubl
   return obstacles_item(d, t, step, 1);
 }
 
-static __device__ __noinline__ void step_end(const PgDev &d, double step)
+// by one block, row and gs the step counters: adaptive, the obstacles move by
+// (step0 + step1)/2, and step1 is recorded for the host and becomes the next
+// step's step0
+static __device__ __noinline__ void step_end(const PgDev &d, double step, int row, long long gs)
 {
+  const double h1 = d.hs ? d.hs[1] : 0.0;
+  obstacle_points(d, d.hs ? 0.5*(d.hs[0] + h1) : step, 1, row, threadIdx.x, blockDim.x);
+  __syncthreads();                             // every thread has read the steps
+  if (threadIdx.x != 0) return;
   *d.obs_done = 0;
   if (d.cwork_n) *d.cwork_n = 0;
   if (d.hs)
   {
-    // adaptive: the obstacles move by (step0 + step1)/2; step1 is recorded
-    // for the host and becomes the next step's step0
-    const double h1 = d.hs[1];
-    const double st = 0.5*(d.hs[0] + h1);
-    d.hrec[*d.stepno] = h1;
-    tail_item(d, st, 1);
+    d.hrec[row] = h1;
     d.hs[0] = h1;
-    return;
   }
-  tail_item(d, step, 1);
+  *d.stepno = row + 1;
+  *d.gstep = gs + 1;
 }
 
+// The counters are asked for before the block is counted: the last block's
+// way to the end is one atomic and one store.  Its release orders the block's
+// reads (and __syncthreads those of its threads) before the last block's
+// writes, its acquire the last block's after them; two full fences around it
+// took 2 us more of a step.
 __device__ __forceinline__ void step_done(const PgDev &d, double step, int last)
 {
   if (!last) return;
+  __shared__ int ends, row;
+  __shared__ long long gs;
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  __threadfence();
-  if (atomicAdd(d.obs_done, 1) != (int)gridDim.x - 1) return;
-  __threadfence();
-  step_end(d, step);
+  if (threadIdx.x == 0)
+  {
+    row = *d.stepno;
+    gs = *d.gstep;
+    int n;
+    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(n) : "l"(d.obs_done) : "memory");
+    ends = n == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (ends) step_end(d, step, row, gs);
 }
 
 // The scene gravities of a step, taken by the first blocks of its first

@@ -253,7 +253,7 @@ __global__ void k_obstacles_tail(PgDev d, double step)
 // the end of a step in a launch of its own
 __global__ void k_step_end(PgDev d, double step)
 {
-  if (threadIdx.x == 0) pgk::step_end(d, step);
+  pgk::step_end(d, step, *d.stepno, *d.gstep);
 }
 
 using pgk::pairing;
@@ -1575,19 +1575,15 @@ __device__ __forceinline__ R add_times_zero(R F, double m, double g)
 
 // half = step/2 and hstep = (step + step1)/2 come from the host (the same
 // IEEE operations), except where the step is chosen on the device
-// WIDE: contact entries whose loads are in flight together, and the blocks
-// asked for per SM.  A scene whose particles fill less than two blocks an SM
-// waits for its chain of loads (flag, then force and point, of one entry
-// after another): it takes four entries at a time in 2 x 24 more registers.
-// Larger ones hide one warp's loads behind the others' FP64 work and need the
-// warps: one entry at a time in 96 registers.
-template <int MODE, int WIDE>
-__global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integrate(PgDev d, double step, double half, double hstep, int oblocks, int last)
+// One thread per particle, one contact entry at a time in 96 registers: a
+// warp's loads wait behind the other warps' FP64 work.  Scenes that leave
+// schedulers idle take k_integrate_quad.
+template <int MODE>
+__global__ void __launch_bounds__(TPB, PG_INTEGRATE_MINB) k_integrate(PgDev d, double step, double half, double hstep, int oblocks, int last)
 {
   // fused modes: the first blocks move the obstacle triangles; `last`: the last
   // block to finish ends the step
-  // one warp an SM gains nothing from f64
-  typedef typename std::conditional<(WIDE > 1), double, f64>::type R;
+  typedef f64 R;
   const Num<R> N;
   const int i = ((int)blockIdx.x - oblocks) * (int)blockDim.x + (int)threadIdx.x;
   bool need = false;
@@ -1646,29 +1642,17 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
       // as k_contacts_sum sums them into fm and tm in the adaptive mode
       R fs[3] = {N(0.0), N(0.0), N(0.0)}, ts[3] = {N(0.0), N(0.0), N(0.0)};
       const int cnt = d.ncnt[e];
-      for (int k0 = 0; k0 < cnt; k0 += WIDE)
+      for (int k = 0; k < cnt; k ++)
       {
-        bool on[WIDE];
-        double f[WIDE][3], p[WIDE][3];
-        #pragma unroll
-        for (int j = 0; j < WIDE; j ++) on[j] = k0 + j < cnt && d.nflag[(size_t)(k0 + j) * d.estride + e] != 0;
-        #pragma unroll
-        for (int j = 0; j < WIDE; j ++)
-          if (on[j])
-          {
-            const size_t idx = (size_t)(k0 + j) * d.estride + e;
-            for (int c = 0; c < 3; c ++) { f[j][c] = d.nfrc[c][idx]; p[j][c] = d.npnt[c][idx]; }
-          }
-        #pragma unroll
-        for (int j = 0; j < WIDE; j ++)
-          if (on[j])
-          {
-            const R a[3] = {p[j][0]-po[0], p[j][1]-po[1], p[j][2]-po[2]};
-            fs[0] += f[j][0]; fs[1] += f[j][1]; fs[2] += f[j][2];
-            ts[0] += a[1]*f[j][2] - a[2]*f[j][1];
-            ts[1] += a[2]*f[j][0] - a[0]*f[j][2];
-            ts[2] += a[0]*f[j][1] - a[1]*f[j][0];
-          }
+        const size_t idx = (size_t)k * d.estride + e;
+        if (d.nflag[idx] == 0) continue;
+        double f[3], p[3];
+        for (int c = 0; c < 3; c ++) { f[c] = d.nfrc[c][idx]; p[c] = d.npnt[c][idx]; }
+        const R a[3] = {p[0]-po[0], p[1]-po[1], p[2]-po[2]};
+        fs[0] += f[0]; fs[1] += f[1]; fs[2] += f[2];
+        ts[0] += a[1]*f[2] - a[2]*f[1];
+        ts[1] += a[2]*f[0] - a[0]*f[2];
+        ts[2] += a[0]*f[1] - a[1]*f[0];
       }
       F[0] = fs[0]; F[1] = fs[1]; F[2] = fs[2];
       T[0] = ts[0]; T[1] = ts[1]; T[2] = ts[2];
@@ -1683,25 +1667,14 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
     if (E)
     {
       const int rb = d.soff[i], re = d.soff[i+1];
-      for (int r0 = rb; r0 < re; r0 += WIDE)
+      for (int r = rb; r < re; r ++)
       {
-      int refs[WIDE];
-      bool on[WIDE];
-      double fr[WIDE][3], pr[WIDE][3];
-      #pragma unroll
-      for (int j = 0; j < WIDE; j ++) refs[j] = r0 + j < re ? d.rref[r0 + j] : -1;
-      #pragma unroll
-      for (int j = 0; j < WIDE; j ++) on[j] = refs[j] >= 0 && d.nflag[refs[j]] != 0;
-      #pragma unroll
-      for (int j = 0; j < WIDE; j ++)
-        if (on[j]) for (int c = 0; c < 3; c ++) { fr[j][c] = d.nfrc[c][refs[j]]; pr[j][c] = d.npnt[c][refs[j]]; }
-      #pragma unroll
-      for (int j = 0; j < WIDE; j ++)
-      {
-        if (!on[j]) continue;
-        const int ref = refs[j];
-        const double f[3] = {-fr[j][0], -fr[j][1], -fr[j][2]};
-        const R a[3] = {pr[j][0]-po[0], pr[j][1]-po[1], pr[j][2]-po[2]};
+        const int ref = d.rref[r];
+        if (d.nflag[ref] == 0) continue;
+        double fr[3], pr[3];
+        for (int c = 0; c < 3; c ++) { fr[c] = d.nfrc[c][ref]; pr[c] = d.npnt[c][ref]; }
+        const double f[3] = {-fr[0], -fr[1], -fr[2]};
+        const R a[3] = {pr[0]-po[0], pr[1]-po[1], pr[2]-po[2]};
         F[0] += f[0]; F[1] += f[1]; F[2] += f[2];
         T[0] += a[1]*f[2] - a[2]*f[1];
         T[1] += a[2]*f[0] - a[0]*f[2];
@@ -1735,7 +1708,6 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
           nvmul(Li, arm, A);
           krot_add(krot, A);
         }
-      }
       }
     }
     F[0] = add_times_zero(F[0], ma, grav[0]);
@@ -2067,6 +2039,8 @@ __global__ void __launch_bounds__(TPB, WIDE > 1 ? 1 : PG_INTEGRATE_MINB) k_integ
   if (FUSED && d.ellnum) flag_rebuild(d, need);
   if (FUSED) pgk::step_done(d, step0, last);
 }
+
+#include "pg_quad.cuh"
 
 // ---------------------------------------------------------------- torsion springs
 // trqspr_task (forces.ispc:1415-2057), one thread per torsion spring: the
@@ -2730,8 +2704,12 @@ void pg_launch_spring_runs(const PgDev &d, cudaStream_t s)
 
 void pg_launch_step_end(const PgDev &d, cudaStream_t s, double step) { k_step_end<<<1, 32, 0, s>>>(d, step); }
 
-// a scene of few particles takes the latency-bound form in blocks of one
-// warp, so that its warps spread over the SMs
+// Scenes of up to 19,456 particles take four lanes a particle in blocks of one
+// warp, so that the warps spread over the SMs.  The line is where the four
+// lanes fill every scheduler four warps deep: a step of 17,576 falling spheres
+// measures the same on both sides of it (the update 30 us against 29 for one
+// thread a particle with four entries' loads in flight), of 9,261 24 against
+// 28, of 2,197 21 against 28.
 template <int MODE>
 static void launch_integrate(const PgDev &d, cudaStream_t s, double step, double half, double hstep)
 {
@@ -2741,12 +2719,12 @@ static void launch_integrate(const PgDev &d, cudaStream_t s, double step, double
     if (fused) pg_launch_obstacles_tail(d, s, step);
     return;
   }
-  const bool few = d.parnum <= PG_SMALL_SCENE;
-  const int B = few ? 32 : TPB;
-  const int ob = fused && d.obsnum ? (d.trinum + B - 1) / B : 0, nb = (d.parnum + B - 1) / B;
-  const int last = pg_ends_step(ob + nb, few ? 16 : PG_INTEGRATE_MINB);
-  if (few) k_integrate<MODE, 4><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
-  else k_integrate<MODE, 1><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
+  const bool quad = d.parnum <= PG_SMALL_SCENE;
+  const int B = quad ? 32 : TPB, P = quad ? 8 : B;
+  const int ob = fused && d.obsnum ? (d.trinum + B - 1) / B : 0, nb = (d.parnum + P - 1) / P;
+  const int last = pg_ends_step(ob + nb, quad ? 16 : PG_INTEGRATE_MINB);
+  if (quad) k_integrate_quad<MODE><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
+  else k_integrate<MODE><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
   if (fused && !last) pg_launch_step_end(d, s, step);
 }
 
