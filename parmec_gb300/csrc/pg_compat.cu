@@ -183,8 +183,7 @@ bool ready()
   d.kn = 32;
   d.kr = 32;
   d.record_geometry = 1;
-  d.tab_prs_stride = 3;
-  d.tab_obs_stride = 3;
+  d.tab_row = 0;                               // one step a call
   const int one = 1;
   bool ok = grow(d.sactive, 1) && up(d.sactive, &one, 1) && grow(d.stbeg, 1) && grow(d.stend, 1) &&
             grow(d.sexc_on, 1) && grow(d.sexc, PG_EXC_LEN) && grow(d.sgrav, 3) && grow(d.sstart, 1) &&

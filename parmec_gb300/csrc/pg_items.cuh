@@ -1158,11 +1158,11 @@ __device__ __forceinline__ double excite_term(const PgDev &d, const double *e, i
 
 __device__ __forceinline__ void excite_store(const PgDev &d, int sc, double sum)
 {
-  const double *tab = d.t_gravity + 3*(size_t)(*d.stepno), *e = d.sexc + (size_t)PG_EXC_LEN * sc;
+  const double *tab = d.t_gravity + (size_t)d.tab_row * (*d.stepno), *e = d.sexc + (size_t)PG_EXC_LEN * sc;
   const bool on = d.sexc_on[sc] != 0;
   if (sc == 0 && d.damp_f)
   {
-    const double *damp = d.t_damping + 6*(size_t)(*d.stepno);
+    const double *damp = d.t_damping + (size_t)d.tab_row * (*d.stepno);
     for (int k = 0; k < 6; k ++) d.damp_f[k] = (float)damp[k];
   }
   for (int k = 0; k < 3; k ++)
@@ -1222,8 +1222,8 @@ __device__ __forceinline__ bool obstacles_item(const PgDev &d, int t, double ste
   if (use_row)
   {
     const int row = *d.stepno;
-    ang = d.t_obs_ang + (size_t)row * d.tab_obs_stride + 3*o;
-    lin = d.t_obs_lin + (size_t)row * d.tab_obs_stride + 3*o;
+    ang = d.t_obs_ang + (size_t)row * d.tab_row + 3*o;
+    lin = d.t_obs_lin + (size_t)row * d.tab_row + 3*o;
   }
   else
   {
@@ -1273,8 +1273,8 @@ __device__ __forceinline__ void obstacle_points(const PgDev &d, double step, int
     if (use_row)
       for (int k = 0; k < 3; k ++)
       {
-        a[k] = d.t_obs_ang[(size_t)row * d.tab_obs_stride + 3*o + k];
-        v[k] = d.t_obs_lin[(size_t)row * d.tab_obs_stride + 3*o + k];
+        a[k] = d.t_obs_ang[(size_t)row * d.tab_row + 3*o + k];
+        v[k] = d.t_obs_lin[(size_t)row * d.tab_row + 3*o + k];
       }
     else
       for (int k = 0; k < 3; k ++) v[k] = d.obslin[3*o+k];

@@ -513,8 +513,8 @@ __device__ __forceinline__ bool mx_integrate_item(const PgDev &d, int i, double 
     for (int pp = pb; pp < pe; pp ++)
     {
       const int q = d.prs_list[pp];
-      const double *lin = d.t_prs_lin + (size_t)row * d.tab_prs_stride + 3*q;
-      const double *ang = d.t_prs_ang + (size_t)row * d.tab_prs_stride + 3*q;
+      const double *lin = d.t_prs_lin + (size_t)row * d.tab_row + 3*q;
+      const double *ang = d.t_prs_ang + (size_t)row * d.tab_row + 3*q;
       if (d.prslin[q] && d.linkind[q] == 1) for (int c = 0; c < 3; c ++) F[c] = ma * (float)lin[c];
       else if (d.prslin[q] && d.linkind[q] == 0) F[0] = F[1] = F[2] = 0.0f;
       if (d.prsang[q] && d.angkind[q] == 1)
@@ -612,8 +612,8 @@ __device__ __forceinline__ bool mx_integrate_item(const PgDev &d, int i, double 
       for (int pp = pb; pp < pe; pp ++)
       {
         const int q = d.prs_list[pp];
-        const double *lin = d.t_prs_lin + (size_t)row * d.tab_prs_stride + 3*q;
-        const double *ang = d.t_prs_ang + (size_t)row * d.tab_prs_stride + 3*q;
+        const double *lin = d.t_prs_lin + (size_t)row * d.tab_row + 3*q;
+        const double *ang = d.t_prs_ang + (size_t)row * d.tab_row + 3*q;
         if (d.prslin[q] && d.linkind[q] == 0) for (int c = 0; c < 3; c ++) v[c] = df_from(lin[c]);
         if (d.prsang[q] && d.angkind[q] == 0)
         {

@@ -167,6 +167,8 @@ __device__ __forceinline__ bool quad_settled(const Quad &q, double O, double Tb,
   return q.every(ok && (torque || spin));
 }
 
+// `last` in the adaptive force sums: the master sides are summed here, as
+// k_contacts_sum would
 template <int MODE>
 __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, double half, double hstep, int oblocks, int last)
 {
@@ -194,7 +196,7 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
     // what the update reads of the particle, asked for before anything waits
     const int sc = d.pscene[i], e = d.pell ? d.pell[i] : -1, E = d.ellnum, row = *d.stepno;
     const int rb = SUMS && E ? d.soff[i] : 0, re = SUMS && E ? d.soff[i+1] : 0;
-    const bool masters = SUMS && e >= 0 && !ADAPT && d.cwork;
+    const bool masters = SUMS && e >= 0 && d.cwork && (!ADAPT || last);
     const double po = d.position[c][i], ma = d.mass[i];
     double Lr[3], Lc[3], O = 0.0, o = 0.0, v = 0.0, Jr[3], Ir[3], im = 0.0, X = 0.0, C = 0.0, C0 = 0.0;
     bool iso = false, skip = false;
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
     }
     const bool runs = sc >= 0 && d.sactive[sc];
     const double grav = SUMS && sc >= 0 ? d.sgrav[3*sc + c] : 0.0;
-    const double damp = MOVES ? d.t_damping[6*(size_t)row + c] : 0.0, spin_damp = MOVES ? d.t_damping[6*(size_t)row + 3 + c] : 0.0;
+    const double damp = MOVES ? d.t_damping[(size_t)row * d.tab_row + c] : 0.0, spin_damp = MOVES ? d.t_damping[(size_t)row * d.tab_row + 3 + c] : 0.0;
     const int own = masters ? d.ncnt[e] : 0;
     if (MODE == INT_FORCES_ADAPT || MODE == INT_DYN_FUSED)
     {
@@ -244,7 +246,7 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
       krd += dt - A*A;
       kro += -(c == 2 ? a[1] : a[0]) * (c == 0 ? a[1] : a[2]);
     };
-    if (ADAPT && e >= 0)
+    if (ADAPT && e >= 0 && !masters)
     {
       kact = d.akact[c][i];
       krd = d.akrot[c][i];
@@ -260,8 +262,8 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
     else
     {
     // the contacts the particle's sphere is master of, in slot order (summed
-    // before, into fm and tm, in the adaptive mode), then those it is slave
-    // of, in master order (forces.ispc:539-569)
+    // before, into fm and tm, where another pass needs them), then those it is
+    // slave of, in master order (forces.ispc:539-569)
     constexpr int W = PG_QUAD_WIDE;
     if (e >= 0 && !masters) { F = d.fm[c][i]; T = d.tm[c][i]; }
     const int n = own + re - rb;
@@ -300,23 +302,34 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
         T += a1*g2 - a2*g1;
         if (ADAPT)
         {
-          // slave side (forces.ispc:539-567; its only entries): the force direction, and the
-          // contact's own stiffness and damping (the reference reads slave
-          // records whose kcur/ecur nothing sets)
-          double u = g, len = sqrt(q.dot(g, g));
-          if (len != 0.0)
-          {
-            len = 1.0/len;
-            u *= len;
-          }
-          else u = 0.0;
-          kact += fabs(u);
+          // master side (forces.ispc:505-522): the normal; slave side
+          // (forces.ispc:539-567): the force direction, and the contact's own
+          // stiffness and damping (the reference reads slave records whose
+          // kcur/ecur nothing sets)
           const int ms = r % d.estride, code = d.ncode[r];
+          double u;
+          if (slave)
+          {
+            u = g;
+            double len = sqrt(q.dot(g, g));
+            if (len != 0.0)
+            {
+              len = 1.0/len;
+              u *= len;
+            }
+            else u = 0.0;
+          }
+          else u = d.nnrm[c][r];
+          kact += fabs(u);
           const int ij = pairing(d, d.ellcol[ms], code >= 0 ? d.ellcol[code] : d.tricol[-code-1]);
           const double kc = d.iparam[0][ij];
           double ec;
           if (d.nen) ec = d.nen[r];
-          else ec = d.iparam[1][ij] * 2.0 * sqrt(kc*(1.0 / (d.invm[d.part[ms]] + d.invm[i])));
+          else
+          {
+            const int pj = slave ? i : code >= 0 ? d.part[code] : d.triobs[-code-1];
+            ec = d.iparam[1][ij] * 2.0 * sqrt(kc*(pj >= 0 ? 1.0 / (d.invm[d.part[ms]] + d.invm[pj]) : ma));
+          }
           kmax = kc > kmax ? kc : kmax;
           emax = ec > emax ? ec : emax;
           arm_stiffness(q.mul(Lr, q.of(a2, q.c1)));
@@ -470,8 +483,8 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
     for (int pp = pb; pp < pe; pp ++)
     {
       const int s = d.prs_list[pp];
-      const double lin = d.t_prs_lin[(size_t)row * d.tab_prs_stride + 3*s + c];
-      const double ang = d.t_prs_ang[(size_t)row * d.tab_prs_stride + 3*s + c];
+      const double lin = d.t_prs_lin[(size_t)row * d.tab_row + 3*s + c];
+      const double ang = d.t_prs_ang[(size_t)row * d.tab_row + 3*s + c];
       if (d.prslin[s] && d.linkind[s] == 1) F = ma * lin;
       else if (d.prslin[s] && d.linkind[s] == 0) F = 0.0;
       if (d.prsang[s] && d.angkind[s] == 1) T = q.mul(Jr, ang);
@@ -539,10 +552,10 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
       for (int pp = pb; pp < pe; pp ++)
       {
         const int s = d.prs_list[pp];
-        if (d.prslin[s] && d.linkind[s] == 0) v = d.t_prs_lin[(size_t)row * d.tab_prs_stride + 3*s + c];
+        if (d.prslin[s] && d.linkind[s] == 0) v = d.t_prs_lin[(size_t)row * d.tab_row + 3*s + c];
         if (d.prsang[s] && d.angkind[s] == 0)
         {
-          o = d.t_prs_ang[(size_t)row * d.tab_prs_stride + 3*s + c];
+          o = d.t_prs_ang[(size_t)row * d.tab_row + 3*s + c];
           double col[3];
           for (int k = 0; k < 3; k ++) col[k] = q.own(q.of(L2[0], k), q.of(L2[1], k), q.of(L2[2], k));
           O = q.mul(col, o);
@@ -565,10 +578,10 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
       for (int pp = pb; pp < pe; pp ++)
       {
         const int s = d.prs_list[pp];
-        if (d.prslin[s] && d.linkind[s] == 0 && writes) d.linear[c][i] = d.t_prs_lin[(size_t)row * d.tab_prs_stride + 3*s + c];
+        if (d.prslin[s] && d.linkind[s] == 0 && writes) d.linear[c][i] = d.t_prs_lin[(size_t)row * d.tab_row + 3*s + c];
         if (d.prsang[s] && d.angkind[s] == 0)
         {
-          const double oo = d.t_prs_ang[(size_t)row * d.tab_prs_stride + 3*s + c];
+          const double oo = d.t_prs_ang[(size_t)row * d.tab_row + 3*s + c];
           const double Oc = q.mul(Lc, oo);
           if (writes) { d.angular[c][i] = Oc; d.angular[3+c][i] = oo; }
         }

@@ -30,6 +30,7 @@ struct pg_session
   std::vector<int> stbeg_h, stend_h;
   size_t ncells = 0;
   int prs_stride = 3, obs_stride = 3;
+  std::vector<double> tab_rows;   // the tables of a call as its one copy takes them
   std::vector<int> h_pell;
   std::vector<int> h_part;                 // sphere -> particle map the device's eorder was built from
   // per kernel group timing with CUDA events on the session stream
@@ -687,26 +688,33 @@ int download_ranges(pg_session *s, pg_scene *sc, Ranges r)
   return PG_OK;
 }
 
+// the values of a step in the tables, in the order of their pointers
+void table_widths(const pg_session *s, size_t w[7])
+{
+  const size_t widths[7] = {1, 3, 6, (size_t)s->prs_stride, (size_t)s->prs_stride, (size_t)s->obs_stride, (size_t)s->obs_stride};
+  for (int k = 0; k < 7; k ++) w[k] = widths[k];
+}
+
 int ensure_tables(pg_session *s, int n)
 {
   PgDev &d = s->d;
   if (n <= s->tab_cap) return PG_OK;
   int cap = std::max(n, 2 * s->tab_cap);
   drop_graph(s);
-  double **arrs[7] = {&d.t_curtime, &d.t_gravity, &d.t_damping, &d.t_prs_lin, &d.t_prs_ang, &d.t_obs_ang, &d.t_obs_lin};
-  size_t widths[7] = {1, 3, 6, (size_t)s->prs_stride, (size_t)s->prs_stride, (size_t)s->obs_stride, (size_t)s->obs_stride};
-  for (int k = 0; k < 7; k ++)
+  if (d.t_curtime)
   {
-    if (*arrs[k])
-    {
-      CK(cudaStreamSynchronize(s->stream));
-      auto it = std::find(s->allocs.begin(), s->allocs.end(), (void *)*arrs[k]);
-      if (it != s->allocs.end()) s->allocs.erase(it);
-      CK(cudaFree(*arrs[k]));
-      *arrs[k] = nullptr;
-    }
-    TRY(dalloc(s, arrs[k], (size_t)cap * widths[k]));
+    CK(cudaStreamSynchronize(s->stream));
+    auto it = std::find(s->allocs.begin(), s->allocs.end(), (void *)d.t_curtime);
+    if (it != s->allocs.end()) s->allocs.erase(it);
+    CK(cudaFree(d.t_curtime));
+    d.t_curtime = nullptr;
+    s->tab_cap = 0;
   }
+  TRY(dalloc(s, &d.t_curtime, (size_t)cap * d.tab_row));
+  double **arrs[7] = {&d.t_curtime, &d.t_gravity, &d.t_damping, &d.t_prs_lin, &d.t_prs_ang, &d.t_obs_ang, &d.t_obs_lin};
+  size_t widths[7];
+  table_widths(s, widths);
+  for (int k = 1; k < 7; k ++) *arrs[k] = *arrs[k-1] + widths[k-1];
   s->tab_cap = cap;
   return PG_OK;
 }
@@ -1292,7 +1300,7 @@ void enqueue_step_adaptive(pg_session *s)
   pg_launch_spring_runs(d, s->stream);
   pg_launch_torsion(d, s->stream, 0.0);
   pg_launch_unspring(d, s->stream);
-  pg_launch_force_sums_adapt(d, s->stream);
+  pg_launch_force_sums_adapt(d, s->stream, true);
   pg_launch_adapt_step(d, s->stream);
   pg_launch_dynamics_fused(d, s->stream);
   pg_launch_mesh(d, s->stream);
@@ -1300,11 +1308,11 @@ void enqueue_step_adaptive(pg_session *s)
 
 int adaptive_kernel_count(const PgDev &d)
 {
-  int n = pg_rebuild_kernel_count(d) + 1 + pg_contacts_kernel_count(d);   // the step's selection
+  int n = pg_rebuild_kernel_count(d) + pg_contacts_kernel_count(d);
   if (!d.ellnum && !d.sprnum) n += 1;             // excite
   if (d.sprnum) n += 1 + (d.nbig > 0 ? 4 : 0) + (d.unsprnum ? 1 : 0);
   if (d.trqsprnum) n += 1;
-  n += d.parnum ? 3 : 1;                          // force sums, minimum, dynamics with obstacles and tail
+  n += d.parnum ? 3 : 2;                          // force sums, minimum with the selection, dynamics with obstacles and tail; or the selection and the tail
   if (d.nodnum) n += 1;
   if (d.facnum) n += 1;
   return n;
@@ -1314,21 +1322,18 @@ int adaptive_kernel_count(const PgDev &d)
 int upload_tables(pg_session *s, const pg_steptab *tab, int n)
 {
   PgDev &d = s->d;
-  std::vector<double> zeros;
-  auto put = [&](double *dst, const double *src, size_t width) -> int {
-    if (src) return h2d(s, dst, src, (size_t)n * width);
-    zeros.assign((size_t)n * width, 0.0);
-    int r = h2d(s, dst, zeros.data(), (size_t)n * width);
-    if (r == PG_OK && cudaStreamSynchronize(s->stream) != cudaSuccess) return PG_ERR_CUDA;
-    return r;
-  };
-  TRY(put(d.t_curtime, tab->curtime, 1));
-  TRY(put(d.t_gravity, tab->gravity, 3));
-  TRY(put(d.t_damping, tab->damping, 6));
-  TRY(put(d.t_prs_lin, tab->prs_lin, s->prs_stride));
-  TRY(put(d.t_prs_ang, tab->prs_ang, s->prs_stride));
-  TRY(put(d.t_obs_ang, tab->obs_ang, s->obs_stride));
-  TRY(put(d.t_obs_lin, tab->obs_lin, s->obs_stride));
+  const double *src[7] = {tab->curtime, tab->gravity, tab->damping, tab->prs_lin, tab->prs_ang, tab->obs_ang, tab->obs_lin};
+  size_t w[7];
+  table_widths(s, w);
+  // one row a step, so that one copy takes them all: the adaptive loop makes a
+  // call a step, and seven copies took 20 us of it
+  std::vector<double> &rows = s->tab_rows;
+  rows.assign((size_t)n * d.tab_row, 0.0);
+  size_t at = 0;
+  for (int k = 0; k < 7; at += w[k ++])
+    if (src[k])
+      for (int r = 0; r < n; r ++) std::copy(src[k] + r * w[k], src[k] + (r + 1) * w[k], &rows[(size_t)r * d.tab_row + at]);
+  TRY(h2d(s, d.t_curtime, rows.data(), rows.size()));
   CK(cudaMemsetAsync(d.stepno, 0, sizeof(int), s->stream));
   if (d.ustep) TRY(h2d(s, d.ustep, &tab->stepnum, 1));
   return PG_OK;
@@ -1379,8 +1384,12 @@ int pg_session_create(const pg_scene *sc, int form, pg_session **out)
   d.kn = 32; d.kr = 32;
   s->prs_stride = 3 * std::max(1, sc->prsnum);
   s->obs_stride = 3 * std::max(1, sc->obsnum);
-  d.tab_prs_stride = s->prs_stride;
-  d.tab_obs_stride = s->obs_stride;
+  {
+    size_t w[7];
+    table_widths(s, w);
+    d.tab_row = 0;
+    for (size_t k : w) d.tab_row += (int)k;
+  }
   if ((r = allocate(s, sc)) != PG_OK) goto fail;
   if ((r = dalloc(s, &d.stepno, 1)) != PG_OK) goto fail;
   if ((r = dalloc(s, &d.rebuild, 1)) != PG_OK) goto fail;

@@ -106,9 +106,10 @@ struct PgDev
   int *prs_list;            // prescription indices in input order
   int *prslin, *prsang, *linkind, *angkind;
 
-  // ---- per-step host tables on the device
+  // ---- per-step host tables on the device: row r of each starts at
+  // r * tab_row (a session keeps them in one allocation, a step a row)
   double *t_curtime, *t_gravity, *t_damping, *t_prs_lin, *t_prs_ang, *t_obs_ang, *t_obs_lin;
-  int tab_prs_stride, tab_obs_stride;   // rows: prsnum*3, obsnum*3 (at least 3)
+  int tab_row;
   int *stepno;              // device step counter (row of the tables)
 
   // ---- contact candidates (Verlet lists), master side, slot-major

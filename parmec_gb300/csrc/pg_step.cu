@@ -68,7 +68,7 @@ __device__ __forceinline__ void flag_rebuild(const PgDev &d, bool need)
 
 
 // gravity of a particle's scene for this step (written by k_excite)
-__device__ __forceinline__ void scene_gravity(const PgDev &d, int sc, double, const double *, double g[3])
+__device__ __forceinline__ void scene_gravity(const PgDev &d, int sc, double g[3])
 {
   g[0] = d.sgrav[3*sc]; g[1] = d.sgrav[3*sc+1]; g[2] = d.sgrav[3*sc+2];
 }
@@ -870,7 +870,6 @@ __global__ void __launch_bounds__(32) k_contacts_few(PgDev d, double step, int S
   }
 }
 
-template <bool ADAPT>
 __global__ void __launch_bounds__(TPB) k_contacts_sum(PgDev d)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -883,7 +882,7 @@ __global__ void __launch_bounds__(TPB) k_contacts_sum(PgDev d)
   {
     const double x[3] = {d.position[0][pi], d.position[1][pi], d.position[2][pi]};
     double L[9];
-    if (ADAPT) for (int k = 0; k < 9; k ++) L[k] = d.rotation[k][pi];
+    for (int k = 0; k < 9; k ++) L[k] = d.rotation[k][pi];
     for (int k = 0; k < cnt; k ++)
     {
       const size_t idx = (size_t)k * d.estride + i;
@@ -894,39 +893,33 @@ __global__ void __launch_bounds__(TPB) k_contacts_sum(PgDev d)
       ts[0] += a[1]*f[2] - a[2]*f[1];
       ts[1] += a[2]*f[0] - a[0]*f[2];
       ts[2] += a[0]*f[1] - a[1]*f[0];
-      if (ADAPT)
+      const int code = d.ncode[idx];
+      const int pj = code >= 0 ? d.part[code] : d.triobs[-code-1];
+      const int ij = pairing(d, d.ellcol[i], code >= 0 ? d.ellcol[code] : d.tricol[-code-1]);
+      const double kn = d.iparam[0][ij];
+      double en;
+      if (d.nen) en = d.nen[idx];
+      else
       {
-        const int code = d.ncode[idx];
-        const int pj = code >= 0 ? d.part[code] : d.triobs[-code-1];
-        const int ij = pairing(d, d.ellcol[i], code >= 0 ? d.ellcol[code] : d.tricol[-code-1]);
-        const double kn = d.iparam[0][ij];
-        double en;
-        if (d.nen) en = d.nen[idx];
-        else
-        {
-          double ma = pj >= 0 ? 1.0 / (d.invm[pi] + d.invm[pj]) : d.mass[pi];
-          en = d.iparam[1][ij] * 2.0 * sqrt(kn*ma);
-        }
-        kact0[0] += fabs(d.nnrm[0][idx]);
-        kact0[1] += fabs(d.nnrm[1][idx]);
-        kact0[2] += fabs(d.nnrm[2][idx]);
-        kmax0 = kn > kmax0 ? kn : kmax0;
-        emax0 = en > emax0 ? en : emax0;
-        double A[3];
-        nvmul(L, a, A);
-        krot_add(krot0, A);
+        double ma = pj >= 0 ? 1.0 / (d.invm[pi] + d.invm[pj]) : d.mass[pi];
+        en = d.iparam[1][ij] * 2.0 * sqrt(kn*ma);
       }
+      kact0[0] += fabs(d.nnrm[0][idx]);
+      kact0[1] += fabs(d.nnrm[1][idx]);
+      kact0[2] += fabs(d.nnrm[2][idx]);
+      kmax0 = kn > kmax0 ? kn : kmax0;
+      emax0 = en > emax0 ? en : emax0;
+      double A[3];
+      nvmul(L, a, A);
+      krot_add(krot0, A);
     }
   }
   d.fm[0][pi] = fs[0]; d.fm[1][pi] = fs[1]; d.fm[2][pi] = fs[2];
   d.tm[0][pi] = ts[0]; d.tm[1][pi] = ts[1]; d.tm[2][pi] = ts[2];
-  if (ADAPT)
-  {
-    for (int k = 0; k < 3; k ++) d.akact[k][pi] = kact0[k];
-    for (int k = 0; k < 6; k ++) d.akrot[k][pi] = krot0[k];
-    d.akmax[pi] = kmax0;
-    d.aemax[pi] = emax0;
-  }
+  for (int k = 0; k < 3; k ++) d.akact[k][pi] = kact0[k];
+  for (int k = 0; k < 6; k ++) d.akrot[k][pi] = krot0[k];
+  d.akmax[pi] = kmax0;
+  d.aemax[pi] = emax0;
 }
 
 // ---------------------------------------------------------------- springs (forces.ispc:641-1412)
@@ -1008,7 +1001,7 @@ __global__ void __launch_bounds__(TPB) k_springs(PgDev d, double step, int xbloc
   int i = (blockIdx.x - xblocks) * blockDim.x + threadIdx.x;
   if (i >= d.sprnum) return;
   if (ADAPT) step = d.hs[0];
-  const double time = d.t_curtime[*d.stepno];
+  const double time = d.t_curtime[(size_t)d.tab_row * (*d.stepno)];
   const int j = d.sprpart[0][i], k = d.sprpart[1][i];
   double len = 0.0, inv, velocity, spring_force = 0.0, dashpot_force, total_force;
   double Yj[3], Yk[3] = {0.0, 0.0, 0.0}, p[3], q[3], z[3] = {0.0, 0.0, 0.0}, w[3], frc[3], u[3], a[3], b[3] = {0.0, 0.0, 0.0};
@@ -1608,7 +1601,7 @@ __global__ void __launch_bounds__(TPB, PG_INTEGRATE_MINB) k_integrate(PgDev d, d
   if (i < d.parnum && d.pscene[i] >= 0 && d.sactive[d.pscene[i]])
   {
     const int row = *d.stepno;
-    const double *damping = d.t_damping + 6*(size_t)row;
+    const double *damping = d.t_damping + (size_t)row * d.tab_row;
     const bool typo = (d.compat & PG_COMPAT_EXPMAP) != 0;
     const int E = d.ellnum;
     const R po[3] = {N(d.position[0][i]), N(d.position[1][i]), N(d.position[2][i])};
@@ -1635,7 +1628,7 @@ __global__ void __launch_bounds__(TPB, PG_INTEGRATE_MINB) k_integrate(PgDev d, d
     else
     {
     double grav[3];
-    scene_gravity(d, d.pscene[i], step, d.t_gravity + 3*(size_t)row, grav);
+    scene_gravity(d, d.pscene[i], grav);
     if (e >= 0 && !ADAPT && d.cwork)
     {
       // the master side of the sphere's contacts, summed here in slot order
@@ -1867,8 +1860,8 @@ __global__ void __launch_bounds__(TPB, PG_INTEGRATE_MINB) k_integrate(PgDev d, d
     for (int pp = pb; pp < pe; pp ++)
     {
       const int q = d.prs_list[pp];
-      const double *lin = d.t_prs_lin + (size_t)row * d.tab_prs_stride + 3*q;
-      const double *ang = d.t_prs_ang + (size_t)row * d.tab_prs_stride + 3*q;
+      const double *lin = d.t_prs_lin + (size_t)row * d.tab_row + 3*q;
+      const double *ang = d.t_prs_ang + (size_t)row * d.tab_row + 3*q;
       if (d.prslin[q] && d.linkind[q] == 1)
       {
         for (int k = 0; k < 3; k ++) F[k] = N(ma * lin[k]);
@@ -1978,8 +1971,8 @@ __global__ void __launch_bounds__(TPB, PG_INTEGRATE_MINB) k_integrate(PgDev d, d
       for (int pp = pb; pp < pe; pp ++)
       {
         const int q = d.prs_list[pp];
-        const double *lin = d.t_prs_lin + (size_t)row * d.tab_prs_stride + 3*q;
-        const double *ang = d.t_prs_ang + (size_t)row * d.tab_prs_stride + 3*q;
+        const double *lin = d.t_prs_lin + (size_t)row * d.tab_row + 3*q;
+        const double *ang = d.t_prs_ang + (size_t)row * d.tab_row + 3*q;
         if (d.prslin[q] && d.linkind[q] == 0) for (int k = 0; k < 3; k ++) v[k] = N(lin[k]);
         if (d.prsang[q] && d.angkind[q] == 0)
         {
@@ -2004,8 +1997,8 @@ __global__ void __launch_bounds__(TPB, PG_INTEGRATE_MINB) k_integrate(PgDev d, d
       for (int pp = pb; pp < pe; pp ++)
       {
         const int q = d.prs_list[pp];
-        const double *lin = d.t_prs_lin + (size_t)row * d.tab_prs_stride + 3*q;
-        const double *ang = d.t_prs_ang + (size_t)row * d.tab_prs_stride + 3*q;
+        const double *lin = d.t_prs_lin + (size_t)row * d.tab_row + 3*q;
+        const double *ang = d.t_prs_ang + (size_t)row * d.tab_row + 3*q;
         if (d.prslin[q] && d.linkind[q] == 0)
           for (int k = 0; k < 3; k ++) d.linear[k][i] = lin[k];
         if (d.prsang[q] && d.angkind[q] == 0)
@@ -2288,7 +2281,18 @@ __global__ void k_unspring(PgDev d)
 // order as their bit patterns, so the minimum is an integer atomicMin (NaN
 // patterns sort above every finite step and never win, as NaN is dropped by
 // the reference's min).
-__global__ void __launch_bounds__(TPB) k_adapt_min(PgDev d)
+// step1 = factor * the smallest critical step, or step0 when nothing is
+// restrained; re-arms the minimum for the next step
+__device__ __forceinline__ void adapt_select(const PgDev &d)
+{
+  const double hmin = __longlong_as_double((long long)atomicExch(d.hmin, 0x7fefffffffffffffull));
+  d.hs[1] = hmin < 1.7976931348623157e308 ? d.hs[2]*hmin : d.hs[0];
+}
+
+// One warp a block: a particle's critical step is one chain of roots and
+// quotients, and the warps spread over the SMs.  With a counter (a session's
+// step) the last block selects the step.
+__global__ void __launch_bounds__(32) k_adapt_min(PgDev d)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long bits = 0x7fefffffffffffffull;          // DBL_MAX
@@ -2305,7 +2309,14 @@ __global__ void __launch_bounds__(TPB) k_adapt_min(PgDev d)
     const unsigned long long other = __shfl_down_sync(0xffffffffu, bits, o);
     bits = other < bits ? other : bits;
   }
-  if ((threadIdx.x & 31) == 0) atomicMin(d.hmin, bits);
+  if (threadIdx.x != 0) return;
+  atomicMin(d.hmin, bits);
+  if (!d.obs_done) return;
+  int n;
+  asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(n) : "l"(d.obs_done) : "memory");
+  if (n != (int)gridDim.x - 1) return;
+  *d.obs_done = 0;
+  adapt_select(d);
 }
 
 // ---------------------------------------------------------------- CRITICAL (parmec.ispc:485-888)
@@ -2532,14 +2543,11 @@ __global__ void k_eqm_one(PgDev d, int part2, const double *pts, double *out)
   out[0] = eqm(d, 0, pts, part2 >= 0 ? 1 : -1, pts + 3, dot3(dir, dir) > 0.0 ? dir : nullptr);
 }
 
-// step1 = factor * the smallest critical step, or step0 when nothing is
-// restrained; re-arms the minimum for the next step
+// the selection in a launch of its own, for the drop-in export and a step
+// without particles
 __global__ void k_adapt_select(PgDev d)
 {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double hmin = __longlong_as_double((long long)*d.hmin);
-  d.hs[1] = hmin < 1.7976931348623157e308 ? d.hs[2]*hmin : d.hs[0];
-  *d.hmin = 0x7fefffffffffffffull;
+  if (threadIdx.x == 0 && blockIdx.x == 0) adapt_select(d);
 }
 
 } // namespace
@@ -2600,6 +2608,14 @@ static int eval_blocks()
   return nb;
 }
 
+// whether the update of an adaptive step sums the master sides of its contacts
+// itself (k_integrate_quad; a pass of its own takes 21 us of a step of 2,197
+// spheres, in the update 5)
+static bool sums_in_update(const PgDev &d)
+{
+  return d.cwork && d.cwork_n && d.ellnum <= PG_SMALL_SCENE && d.parnum <= PG_SMALL_SCENE;
+}
+
 // in_step: a session's step, whose end empties the work queue and whose scene
 // gravities (nothing else having taken them) the probe's first blocks take
 void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_step)
@@ -2617,7 +2633,7 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
       else if (d.hs) k_contacts_few<false, true><<<nb, 32, 0, s>>>(d, step, S, xb);
       else if (d.record_geometry) k_contacts_few<true, false><<<nb, 32, 0, s>>>(d, step, S, xb);
       else k_contacts_few<false, false><<<nb, 32, 0, s>>>(d, step, S, xb);
-      if (d.hs) k_contacts_sum<true><<<nblk(d.ellnum), TPB, 0, s>>>(d);
+      if (d.hs && !(in_step && sums_in_update(d))) k_contacts_sum<<<nblk(d.ellnum), TPB, 0, s>>>(d);
       return;
     }
     if (!in_step) cudaMemsetAsync(d.cwork_n, 0, sizeof(int), s);
@@ -2628,7 +2644,7 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
     {
       if (d.record_geometry) k_contacts_eval<true, true><<<nb, TPB, 0, s>>>(d, step);
       else k_contacts_eval<false, true><<<nb, TPB, 0, s>>>(d, step);
-      k_contacts_sum<true><<<nblk(d.ellnum), TPB, 0, s>>>(d);
+      k_contacts_sum<<<nblk(d.ellnum), TPB, 0, s>>>(d);
     }
     else
     {
@@ -2711,7 +2727,7 @@ void pg_launch_step_end(const PgDev &d, cudaStream_t s, double step) { k_step_en
 // thread a particle with four entries' loads in flight), of 9,261 24 against
 // 28, of 2,197 21 against 28.
 template <int MODE>
-static void launch_integrate(const PgDev &d, cudaStream_t s, double step, double half, double hstep)
+static void launch_integrate(const PgDev &d, cudaStream_t s, double step, double half, double hstep, bool masters = false)
 {
   constexpr bool fused = MODE == INT_FUSED || MODE == INT_DYN_FUSED;
   if (!d.parnum)
@@ -2722,7 +2738,7 @@ static void launch_integrate(const PgDev &d, cudaStream_t s, double step, double
   const bool quad = d.parnum <= PG_SMALL_SCENE;
   const int B = quad ? 32 : TPB, P = quad ? 8 : B;
   const int ob = fused && d.obsnum ? (d.trinum + B - 1) / B : 0, nb = (d.parnum + P - 1) / P;
-  const int last = pg_ends_step(ob + nb, quad ? 16 : PG_INTEGRATE_MINB);
+  const int last = fused ? pg_ends_step(ob + nb, quad ? 16 : PG_INTEGRATE_MINB) : masters;
   if (quad) k_integrate_quad<MODE><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
   else k_integrate<MODE><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
   if (fused && !last) pg_launch_step_end(d, s, step);
@@ -2743,15 +2759,16 @@ void pg_launch_dynamics(const PgDev &d, cudaStream_t s, double step0, double ste
   launch_integrate<INT_DYNAMICS>(d, s, step0, 0.5*step0, 0.5*(step0+step1));
 }
 
-void pg_launch_force_sums_adapt(const PgDev &d, cudaStream_t s)
+// in_step: after pg_launch_contacts with in_step
+void pg_launch_force_sums_adapt(const PgDev &d, cudaStream_t s, bool in_step)
 {
-  launch_integrate<INT_FORCES_ADAPT>(d, s, 0.0, 0.0, 0.0);
+  launch_integrate<INT_FORCES_ADAPT>(d, s, 0.0, 0.0, 0.0, in_step && sums_in_update(d));
 }
 
 void pg_launch_adapt_step(const PgDev &d, cudaStream_t s)
 {
-  if (d.parnum) k_adapt_min<<<nblk(d.parnum), TPB, 0, s>>>(d);
-  k_adapt_select<<<1, 32, 0, s>>>(d);
+  if (d.parnum) k_adapt_min<<<(d.parnum + 31) / 32, 32, 0, s>>>(d);
+  if (!d.parnum || !d.obs_done) k_adapt_select<<<1, 32, 0, s>>>(d);
 }
 
 void pg_launch_critical_perspring(const PgDev &d, cudaStream_t s, double *h, double *om, double *ra)
