@@ -385,12 +385,12 @@ __global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g)
 }
 
 // 5b. the vertex-triangle and the edge-edge distances asked for, one thread
-// each, so that a warp runs one kind on all its lanes
-__global__ void __launch_bounds__(TPB) k_tt_vertex_face(PgTT g)
+// each, so that a warp runs one kind on all its lanes: the first vb blocks
+// take the one kind, the others the other
+__device__ __forceinline__ void tt_vertex_face(const PgTT &g, const pg::Num<pg::f64> &N, int first, int by)
 {
-  const pg::Num<pg::f64> N;
   const int n = min(g.qn[2], g.vcap);
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
+  for (int w = first; w < n; w += by)
   {
     const unsigned it = g.vit[w];
     if (it == ~0u) continue;
@@ -413,11 +413,10 @@ __global__ void __launch_bounds__(TPB) k_tt_vertex_face(PgTT g)
   }
 }
 
-__global__ void __launch_bounds__(TPB) k_tt_edge_edge(PgTT g)
+__device__ __forceinline__ void tt_edge_edge(const PgTT &g, const pg::Num<pg::f64> &N, int first, int by)
 {
-  const pg::Num<pg::f64> N;
   const int n = min(g.qn[3], g.ecap);
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
+  for (int w = first; w < n; w += by)
   {
     const unsigned it = g.eit[w];
     if (it == ~0u) continue;
@@ -438,6 +437,16 @@ __global__ void __launch_bounds__(TPB) k_tt_edge_edge(PgTT g)
     o[1] = s;
     o[2] = t;
   }
+}
+
+// One launch: the second kind fills the SMs as the first runs out (16x16
+// lattice: 23 + 21 us in two launches, 33 in one).
+__global__ void __launch_bounds__(TPB) k_tt_distances(PgTT g, int vb)
+{
+  const pg::Num<pg::f64> N;
+  const int b = blockIdx.x;
+  if (b < vb) tt_vertex_face(g, N, b * TPB + threadIdx.x, vb * TPB);
+  else tt_edge_edge(g, N, (b - vb) * TPB + threadIdx.x, (gridDim.x - vb) * TPB);
 }
 
 // granular force of pair k with the contact found (depth > 0: active)
@@ -547,19 +556,16 @@ __global__ void __launch_bounds__(TPB, 4) k_tt_near(PgDev d, PgTT g, double step
     }
     tt_force(d, g, N, k, f, u, depth, point, normal, step);
   }
-}
-
-// 5d. the pairs that need every test: triangles that may intersect,
-// degenerate ones, and those whose distances found no room
-__global__ void __launch_bounds__(TPB) k_tt_full(PgDev d, PgTT g, double step)
-{
-  const int n = g.qn[1];
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
+  // 5d. the pairs that need every test: triangles that may intersect,
+  // degenerate ones, and those whose distances found no room
+  const int nf = g.qn[1];
+  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nf; w += gridDim.x * blockDim.x)
   {
     const int k = g.full[w], f = g.pf[k], u = g.pu[k];
-    double point[3], normal[3];
-    const double depth = tt_contact(d, g, f, u, point, normal);
-    tt_force(d, g, pg::Num<double>(), k, f, u, depth, point, normal, step);
+    double po[3], no[3];
+    const pg::f64 depth = N(tt_contact(d, g, f, u, po, no));
+    const pg::f64 point[3] = {N(po[0]), N(po[1]), N(po[2])}, normal[3] = {N(no[0]), N(no[1]), N(no[2])};
+    tt_force(d, g, N, k, f, u, depth, point, normal, step);
   }
 }
 
@@ -639,15 +645,19 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tt_active(PgTT g)
   if (threadIdx.x == 0) g.etile[blockIdx.x] = sum;
 }
 
-__global__ void __launch_bounds__(1024) k_tt_tiles(PgTT g, int tiles)
-{
-  __shared__ int part[1024];
-  pgk::block_scan_seq(g.etile, tiles, part);
-}
-
+// Each block counts the tiles before its own again instead of waiting for a
+// scan in a launch of its own (tiles of 4 bytes, in L2).
 __global__ void __launch_bounds__(TILE_THREADS) k_tt_select(PgTT g)
 {
+  __shared__ int tiles[TILE_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = 2 * g.np;
+  int tile = 0;
+  for (int t = threadIdx.x; t < (int)blockIdx.x; t += TILE_THREADS) tile += g.etile[t];
+  tile = __reduce_add_sync(0xffffffffu, tile);
+  if (lane == 0) tiles[warp] = tile;
+  __syncthreads();
+  tile = 0;
+  for (int t = 0; t < TILE_THREADS / 32; t ++) tile += tiles[t];
   // the tile's 32 words, one a lane: active entries before each
   const unsigned word = g.ebits[blockIdx.x * (PG_TT_TILE / 32) + lane];
   int before = __popc(word);
@@ -656,7 +666,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tt_select(PgTT g)
     const int v = __shfl_up_sync(0xffffffffu, before, o);
     if (lane >= o) before += v;
   }
-  before += g.etile[blockIdx.x] - __popc(word);
+  before += tile - __popc(word);
   for (int it = 0; it < PG_TT_TILE / TILE_THREADS; it ++)
   {
     const int wd = it * (TILE_THREADS / 32) + warp;
@@ -675,19 +685,10 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tt_select(PgTT g)
 // 6c. sums of entries [b, e) of elist, e - b <= PG_TT_CHUNK: lane sums over
 // entries lane, lane+32, ..., then the lane sums in lane order, one lane per
 // component.  Four entries' loads are issued before the first is added.
-// One warp sums all six components (18 FP64 instructions an entry, 64 clocks
-// each); with SPLIT four warps of a block share them, the force by warp 0 and
-// a component of the torque by each other (a chain of 6 an entry, but four
-// times the lane sums): for the long sums of few particles, where the chip
-// waits for the chain (a chunk 57 -> 34 us), not for thousands of short ones
-// (4,097 particles 35 -> 73 us).  Returns component `lane` (warp 0: force;
-// without SPLIT all six) or, in lane 0, torque component warp - 1.
-template <bool SPLIT>
+// Returns component `lane`, force then torque.
 __device__ __forceinline__ double chunk_sum(const PgTT &g, const double *x, int b, int e, double (*part)[6])
 {
-  const int lane = threadIdx.x & 31, warp = SPLIT ? threadIdx.x >> 5 : 0;
-  const int c1 = warp % 3, c2 = (warp + 1) % 3;          // torque component warp-1: a[c1] f[c2] - a[c2] f[c1]
-  const bool force = !SPLIT || warp == 0;
+  const int lane = threadIdx.x & 31;
   double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   for (int q0 = b + lane; q0 < e; q0 += 128)
   {
@@ -699,39 +700,95 @@ __device__ __forceinline__ double chunk_sum(const PgTT &g, const double *x, int 
     for (int j = 0; j < 4; j ++)
     {
       const int k = v[j] >= 0 ? v[j] >> 1 : 0;
-      if (force) for (int c = 0; c < 3; c ++) f[j][c] = g.f[c][k];
-      if (!SPLIT) for (int c = 0; c < 3; c ++) p[j][c] = g.p[c][k];
-      else if (!force) { f[j][0] = g.f[c1][k]; f[j][1] = g.f[c2][k]; f[j][2] = 0.0; p[j][0] = g.p[c1][k]; p[j][1] = g.p[c2][k]; }
+      for (int c = 0; c < 3; c ++) { f[j][c] = g.f[c][k]; p[j][c] = g.p[c][k]; }
     }
     #pragma unroll
     for (int j = 0; j < 4; j ++)
     {
       if (v[j] < 0) break;
       if (v[j] & 1) { f[j][0] = -f[j][0]; f[j][1] = -f[j][1]; f[j][2] = -f[j][2]; }
-      if (force) { s[0] += f[j][0]; s[1] += f[j][1]; s[2] += f[j][2]; }
-      if (!SPLIT)
-      {
-        const double a[3] = {p[j][0]-x[0], p[j][1]-x[1], p[j][2]-x[2]};
-        s[3] += a[1]*f[j][2] - a[2]*f[j][1];
-        s[4] += a[2]*f[j][0] - a[0]*f[j][2];
-        s[5] += a[0]*f[j][1] - a[1]*f[j][0];
-      }
-      else if (!force) s[0] += (p[j][0]-x[c1])*f[j][1] - (p[j][1]-x[c2])*f[j][0];
+      s[0] += f[j][0]; s[1] += f[j][1]; s[2] += f[j][2];
+      const double a[3] = {p[j][0]-x[0], p[j][1]-x[1], p[j][2]-x[2]};
+      s[3] += a[1]*f[j][2] - a[2]*f[j][1];
+      s[4] += a[2]*f[j][0] - a[0]*f[j][2];
+      s[5] += a[0]*f[j][1] - a[1]*f[j][0];
     }
   }
   for (int c = 0; c < 6; c ++) part[lane][c] = s[c];
   __syncwarp();
   double acc = 0.0;
-  if (lane < (!SPLIT ? 6 : force ? 3 : 1)) for (int L = 0; L < 32; L ++) acc += part[L][lane];
+  if (lane < 6) for (int L = 0; L < 32; L ++) acc += part[L][lane];
   return acc;
 }
 
-// particles of at most one chunk of active entries, one warp each
-__global__ void __launch_bounds__(TPB) k_tt_sums(PgDev d, PgTT g)
+// Component q of the same sum by a block: the warps take the entries' terms
+// side by side, the first adds them up.  A chain of 40 + 64 FP64 instructions
+// of 64 clocks where the sum of all six by one warp has 600; for the long sums
+// of few particles, where the chip waits for the chain (a full chunk 57 us by
+// one warp, 13 by six blocks), not for thousands of short ones (4,097
+// particles: 35 us by a warp each, 73 by blocks).
+__device__ __forceinline__ double chunk_component(const PgTT &g, int w, int q, int b, int e, const PgDev &d, double (*term)[32])
 {
-  __shared__ double part[TPB / 32][32][6];
-  const int lane = threadIdx.x & 31;
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  constexpr int EACH = PG_TT_CHUNK / TPB;                // entries a lane
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c1 = q < 3 ? q : (q + 1) % 3, c2 = (q + 2) % 3;   // torque q-3: a[c1] f[c2] - a[c2] f[c1]
+  const double x1 = d.position[c1][w], x2 = d.position[c2][w];
+  int v[EACH];
+  #pragma unroll
+  for (int j = 0; j < EACH; j ++)
+  {
+    const int k = b + lane + 32 * (warp * EACH + j);
+    v[j] = k < e ? g.elist[k] : -1;
+  }
+  double f1[EACH], f2[EACH], p1[EACH], p2[EACH];
+  #pragma unroll
+  for (int j = 0; j < EACH; j ++)
+  {
+    const int k = v[j] >= 0 ? v[j] >> 1 : 0;
+    f1[j] = g.f[c1][k];
+    if (q >= 3) { f2[j] = g.f[c2][k]; p1[j] = g.p[c1][k]; p2[j] = g.p[c2][k]; }
+  }
+  #pragma unroll
+  for (int j = 0; j < EACH; j ++)
+  {
+    if (v[j] < 0) break;
+    const double s1 = v[j] & 1 ? -f1[j] : f1[j];
+    if (q < 3) term[warp * EACH + j][lane] = s1;
+    else
+    {
+      const double s2 = v[j] & 1 ? -f2[j] : f2[j];
+      term[warp * EACH + j][lane] = (p1[j]-x1)*s2 - (p2[j]-x2)*s1;
+    }
+  }
+  __syncthreads();
+  if (warp != 0) return 0.0;
+  double s = 0.0;
+  for (int j = 0; b + lane + 32*j < e; j ++) s += term[j][lane];
+  __syncwarp();
+  term[0][lane] = s;
+  __syncwarp();
+  double acc = 0.0;
+  if (lane == 0) for (int L = 0; L < 32; L ++) acc += term[0][L];
+  return acc;
+}
+
+// The first 6 nchunks blocks take a component of a chunk each, of the
+// particles that may have more than one chunk (k_tt_totals adds theirs up),
+// the others a warp a particle of at most one.
+__global__ void __launch_bounds__(TPB, 4) k_tt_sums(PgDev d, PgTT g, int nchunks)
+{
+  __shared__ union { double part[TPB / 32][32][6]; double term[PG_TT_CHUNK / 32][32]; } sh;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if ((int)blockIdx.x < 6 * nchunks)
+  {
+    const int c = blockIdx.x / 6, k = blockIdx.x % 6, q = g.chmap[c], w = g.bigp[q], n = g.plast[w] - g.pfirst[w];
+    const int b = g.pfirst[w] + (c - g.bigoff[q]) * PG_TT_CHUNK, e = min(b + PG_TT_CHUNK, g.plast[w]);
+    if (b >= e || n <= PG_TT_CHUNK) return;
+    const double acc = chunk_component(g, w, k, b, e, d, sh.term);
+    if (threadIdx.x == 0) g.csum[k][c] = acc;
+    return;
+  }
+  const int w = (blockIdx.x - 6 * nchunks) * (TPB / 32) + warp;
   if (w >= d.parnum) return;
   const int b = g.pfirst[w], e = g.plast[w];
   if (e - b > PG_TT_CHUNK) return;
@@ -739,25 +796,10 @@ __global__ void __launch_bounds__(TPB) k_tt_sums(PgDev d, PgTT g)
   if (e > b)
   {
     const double x[3] = {d.position[0][w], d.position[1][w], d.position[2][w]};
-    acc += chunk_sum<false>(g, x, b, e, part[threadIdx.x >> 5]);
+    acc += chunk_sum(g, x, b, e, sh.part[warp]);
   }
   if (lane < 3) d.ttF[lane][w] = acc;
   else if (lane < 6) d.ttT[lane - 3][w] = acc;
-}
-
-// the others: one block per chunk, then one thread per component, the chunk
-// sums in chunk order
-__global__ void __launch_bounds__(TPB) k_tt_chunk_sums(PgDev d, PgTT g)
-{
-  __shared__ double part[TPB / 32][32][6];
-  const int c = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int q = g.chmap[c], w = g.bigp[q];
-  const int b = g.pfirst[w] + (c - g.bigoff[q]) * PG_TT_CHUNK, e = min(b + PG_TT_CHUNK, g.plast[w]);
-  if (b >= e) return;
-  const double x[3] = {d.position[0][w], d.position[1][w], d.position[2][w]};
-  const double acc = chunk_sum<true>(g, x, b, e, part[warp]);
-  if (warp == 0) { if (lane < 3) g.csum[lane][c] = acc; }
-  else if (lane == 0) g.csum[2 + warp][c] = acc;
 }
 
 __global__ void __launch_bounds__(TPB) k_tt_totals(PgDev d, PgTT g)
@@ -825,24 +867,21 @@ void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, double step)
 {
   if (g.np > 0)
   {
-    static const int bv = resident_blocks(k_tt_vertex_face), be = resident_blocks(k_tt_edge_edge),
-                     bn = resident_blocks(k_tt_near), bf = resident_blocks(k_tt_full);
+    static const int bd = resident_blocks(k_tt_distances), bn = resident_blocks(k_tt_near);
     auto upto = [](int most, long long n) { const int b = nblk(n); return b < most ? b : most; };
+    const int bv = upto(bd, 6LL * g.np), be = upto(bd, 9LL * g.np);
     const int tiles = (2 * g.np + PG_TT_TILE - 1) / PG_TT_TILE;
     cudaMemsetAsync(g.qn, 0, 4 * sizeof(int), s);
     k_tt_judge<<<nblk(g.np), TPB, 0, s>>>(d, g);
-    k_tt_vertex_face<<<upto(bv, 6LL * g.np), TPB, 0, s>>>(g);
-    k_tt_edge_edge<<<upto(be, 9LL * g.np), TPB, 0, s>>>(g);
+    k_tt_distances<<<bv + be, TPB, 0, s>>>(g, bv);
     k_tt_near<<<upto(bn, g.np), TPB, 0, s>>>(d, g, step);
-    k_tt_full<<<upto(bf, g.np), TPB, 0, s>>>(d, g, step);
     k_tt_active<<<tiles, TILE_THREADS, 0, s>>>(g);
-    k_tt_tiles<<<1, 1024, 0, s>>>(g, tiles);
     k_tt_select<<<tiles, TILE_THREADS, 0, s>>>(g);
   }
-  if (d.parnum > 0) k_tt_sums<<<nblk(32LL * d.parnum), TPB, 0, s>>>(d, g);
+  const int nchunks = g.nbig > 0 ? g.nchunks : 0;
+  if (d.parnum > 0) k_tt_sums<<<6 * nchunks + nblk(32LL * d.parnum), TPB, 0, s>>>(d, g, nchunks);
   if (g.nbig > 0)
   {
-    k_tt_chunk_sums<<<g.nchunks, TPB, 0, s>>>(d, g);
     k_tt_totals<<<nblk(6LL * g.nbig), TPB, 0, s>>>(d, g);
   }
 }
@@ -860,4 +899,4 @@ int pg_tt_search_kernels(const PgTT &g, int trinum)
          (g.np > 0 ? 4 + pg_sort_kernel_count(2 * g.np, g.epasses) + (g.nbig > 0 ? 1 : 0) : 0);
 }
 
-int pg_tt_step_kernels(const PgTT &g) { return 2 + (g.np > 0 ? 8 : 0) + (g.nbig > 0 ? 2 : 0); }
+int pg_tt_step_kernels(const PgTT &g) { return 2 + (g.np > 0 ? 5 : 0) + (g.nbig > 0 ? 1 : 0); }
