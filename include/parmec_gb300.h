@@ -449,8 +449,8 @@ int pg_session_global_step(pg_session *s, long long *step);
 
 /* Time kernel groups with CUDA events on the session stream during
  * pg_session_run (on != 0) and reset the accumulators.  Groups: 0 rebuild of
- * candidate lists, 1 contacts, 2 springs, 3 integrate, 4 mesh nodes/faces,
- * 5 obstacles and step tail. */
+ * candidate lists, 1 contacts, 2 springs, 3 integrate (with the obstacles and
+ * the end of the step), 4 mesh nodes/faces, 5 nothing (kept for the layout). */
 int pg_session_profile(pg_session *s, int on);
 
 /* Accumulated milliseconds and kernel launches per group (8 entries each). */

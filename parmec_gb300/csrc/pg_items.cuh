@@ -1136,13 +1136,13 @@ __device__ bool rebuild_all(const PgDev &d, int passes, int epasses, RebuildSmem
 
 
 // ================================================================ per-step scene state
-// gravity of scene sc for this step: the step table's row, or the scene's
+// Gravity of scene sc for this step: the step table's row, or the scene's
 // base excitation g0 + dir * sum_k amp_k sin(2 pi freq_k t + phase_k) at its
 // local time t = (global step - start step) * step.  Written with explicit
 // round-to-nearest operations: the same bits whether or not the compiler
-// contracts multiply-adds.
-// One term of the sum, and what the scene's gravity (and in FP32 with it, the
-// damping row) becomes with the sum.
+// contracts multiply-adds.  The number of terms, one term of the sum, and what
+// the scene's gravity (and in FP32 with it, the damping row) becomes with the
+// sum:
 __device__ __forceinline__ int excite_terms(const double *e)
 {
   const int nk = (int)e[6];

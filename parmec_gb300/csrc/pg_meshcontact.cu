@@ -1,42 +1,46 @@
 // pg_meshcontact.cu -- mesh-mesh contact between triangles of different
 // particles (an extension; off unless pg_session_mesh_contact turns it on).
 //
-// Every step, before the force sums:
-//   1. each mesh triangle's box (its vertices' bounds widened by the swept
-//      radius r) and its grid cell, or the "big" range for triangles larger
-//      than a cell;
-//   2. a stable radix sort of the triangles by cell, and the cell ranges;
+// Every step, before the force sums, box and difference arrays of each mesh
+// triangle (1); when a vertex has moved by half the skin since the last
+// search, the pair list anew (2-4); then the narrow phase of the list (5) and
+// the sums (6):
+//   1. each triangle's edges, squared edge lengths and plane normal, a float
+//      copy of its vertices for the filter, and whether a vertex moved by half
+//      the skin;
+//   2. each triangle's box (its vertices' bounds widened by the swept radius r
+//      and the skin) and its grid cell, or the "big" range for triangles
+//      larger than a cell; a stable radix sort of the triangles by cell, and
+//      the cell ranges;
 //   3. each triangle finds its partners among the triangles of the 27 cells
 //      around its own (and among the big ones), keeps those whose boxes
-//      overlap with positive measure (two triangles closer than 2r have such
-//      boxes; boxes that only touch hold no contact), and sorts them by index.  A pair is found by one triangle
+//      overlap, and sorts them by index.  A pair is found by one triangle
 //      only: between two small triangles (or two big ones) by the lower
 //      index, between a small and a big one by the small one;
 //   4. the pairs, in the order of the finding triangles and their sorted
 //      partners (an exclusive scan of the counts gives each triangle's
-//      offset);
-//   5. which of a pair's fifteen feature distances can decide its contact, in
-//      FP32 with certain bounds (pg_ttfilter.cuh): most pairs are apart, the
-//      others ask for 7 distances on average (parallel faces tie).  Those
-//      are taken in FP64 by one thread each, vertex-triangle and edge-edge
-//      distances in launches of their own, so that every warp runs one kind
-//      on all its lanes; then one thread per near pair takes the first of
-//      the smallest, the contact it gives (pg_tritri.cuh) and the granular
-//      law with the pair's tangential state, carried over from the previous
-//      step's pair list by (finder, partner).  Pairs that may intersect and
+//      offset), with the tangential state of the pairs of the last list, by
+//      (finder, partner); two entries a pair, sorted by particle;
+//   5. whether a pair's boxes without the skin overlap with positive measure
+//      (triangles closer than 2r have such boxes), and which of its fifteen
+//      feature distances can decide its contact, in FP32 with certain bounds
+//      (pg_ttfilter.cuh): most pairs are apart, the others ask for 7 distances
+//      on average (parallel faces tie).  Those are taken in FP64 by one thread
+//      each, every warp one kind on all its lanes; then one thread per near
+//      pair takes the first of the smallest, the contact it gives
+//      (pg_tritri.cuh) and the granular law.  Pairs that may intersect and
 //      degenerate triangles take the whole narrow phase.  Bound by the FP64
 //      pipe; evaluating all fifteen distances and six crossing tests of
 //      every pair that a plane test left took 3.2 ms a step on the 64x64
-//      lattice (658,000 pairs), this takes 0.95 ms;
+//      lattice (658,000 pairs), the whole stage now takes 0.8 ms;
 //   6. the force of each active pair goes to its two particles (+f to the
-//      finder's, -f to the partner's): the entries are sorted by particle
-//      (stably, so in pair order) and summed per particle in chunks of
-//      PG_TT_CHUNK entries: one warp per chunk, lane L taking entries L,
-//      L+32, ... of the chunk from zero and the 32 lane sums added in lane
-//      order; then the chunk sums in chunk order from zero, one thread per
-//      particle.  A particle with many contacts (a base plate under a whole
-//      lattice) spreads over many warps.  k_integrate adds these sums after
-//      gravity.
+//      finder's, -f to the partner's): the entries of active pairs, selected
+//      in the list's order, are summed per particle in chunks of PG_TT_CHUNK:
+//      lane L of 32 takes entries L, L+32, ... of the chunk from zero and the
+//      32 lane sums are added in lane order; then the chunk sums in chunk
+//      order from zero, one thread per particle and component.  A particle
+//      with many contacts (a base plate under a whole lattice) spreads over
+//      many blocks.  k_integrate adds these sums after gravity.
 // The CPU oracle restates the same definitions with a brute-force search.
 #include <cuda_runtime.h>
 #include <cstdio>

@@ -2,13 +2,19 @@
 //
 // One step of the reference loop (parmec.cpp:2418-2517) runs as
 //   [rebuild of candidate lists, only when some sphere moved > skin/2]
-//   k_contacts   per sphere: narrow phase of its candidates, granular force,
-//                contact state, master-side partial sums  (condet + contacts_task)
-//   k_springs    per spring: nonlinear spring/dashpot/friction force (springs_task)
-//   k_integrate  per particle: slave-side sums + gravity + spring flushes,
-//                prescribed motion, Lie-group integration, sphere centres
-//                (contacts_acc_task + prescribe_* + dynamics_task + ellipsoids_task)
-//   k_nodes/k_faces, k_obstacles, k_tail
+//   contacts     narrow phase of the spheres' candidates, granular force,
+//                contact state (condet + contacts_task): k_contacts_few in one
+//                launch for a small scene, else k_contacts_probe and
+//                k_contacts_eval; the scene gravities beside the first of them
+//   k_springs    per spring: nonlinear spring/dashpot/friction force
+//                (springs_task); long flush runs in k_spring_run_*
+//   k_integrate  per particle (k_integrate_quad, pg_quad.cuh, for a small
+//                scene): master- and slave-side contact sums + gravity + spring
+//                flushes, prescribed motion, Lie-group integration, sphere
+//                centres (contacts_acc_task + prescribe_* + dynamics_task +
+//                ellipsoids_task); its first blocks move the obstacles, its
+//                last block ends the step
+//   k_nodes/k_faces
 // All sums run in a fixed order (master list in partner order, then slave
 // list in master order), so results repeat bit for bit from run to run.
 #include <cuda_runtime.h>
@@ -28,8 +34,8 @@ constexpr int TPB = 128;
 
 // minimum resident blocks per SM asked of the FP64 particle update and of
 // the contact evaluation (register budget against warps in flight).  The
-// particle update at 1, 4 and 5 blocks (144, 128, 96 registers): 571, 552,
-// 547 us on the 1,048,576-sphere drum and 56, 52, 48 us on 230,000 shaken
+// particle update at 3, 4 and 5 blocks (168, 128, 96 registers): 519, 492,
+// 480 us on the 1,048,576-sphere drum and 59, 53, 51 us on 43,000 shaken
 // spheres; a warp waits for its loads while others hold the FP64 pipe.
 #ifndef PG_INTEGRATE_MINB
 #define PG_INTEGRATE_MINB 5
