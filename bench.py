@@ -609,8 +609,8 @@ def main():
     # launch divided by the spheres), scaled to the full drum; the contact
     # group is its probe and evaluation passes, the integration takes the
     # master-side contact sums
-    traffic_per_unit = {"integrate": 404.0, "contacts": 251.0}
-    fp64_per_unit = {"integrate": 298.0, "contacts": 155.0}
+    traffic_per_unit = {"integrate": 410.0, "contacts": 247.0}
+    fp64_per_unit = {"integrate": 183.0, "contacts": 155.0}
     traffic = traffic_per_unit[dom] * P if dom in traffic_per_unit else None
     fp64 = None
     if dom in fp64_per_unit:

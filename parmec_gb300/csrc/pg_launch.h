@@ -23,7 +23,8 @@ void pg_launch_dynamics(const PgDev &d, cudaStream_t s, double step0, double ste
 // adaptive stepping (d.hs set): force sums with the stiffness terms, the step
 // choice on the device (adaptive_timestep), and the rest of the step
 void pg_launch_force_sums_adapt(const PgDev &d, cudaStream_t s, bool in_step = false);
-void pg_launch_adapt_step(const PgDev &d, cudaStream_t s);
+bool pg_adapt_in_sums(const PgDev &d);
+void pg_launch_adapt_step(const PgDev &d, cudaStream_t s, bool in_step = false);
 void pg_launch_dynamics_fused(const PgDev &d, cudaStream_t s);
 void pg_launch_critical_perspring(const PgDev &d, cudaStream_t s, double *h, double *om, double *ra);
 void pg_launch_critical_perparticle(const PgDev &d, cudaStream_t s, double *ke, int use_contacts, double *h,

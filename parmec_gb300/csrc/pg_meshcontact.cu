@@ -43,6 +43,7 @@
 //      many blocks.  k_integrate adds these sums after gravity.
 // The CPU oracle restates the same definitions with a brute-force search.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdio>
 #include "pg_items.cuh"
 #include "pg_launch.h"
@@ -502,10 +503,12 @@ __device__ __noinline__ double tt_contact(const PgDev &d, const PgTT &g, int f, 
 // as the full search keeps it; then the granular force.  The plane test,
 // which calls a pair apart that the distances would call touching only
 // within its rounding, is taken for depths below 1e-9 of the pair's size.
-// Bound by FP64 issue and by the gathers before it: four blocks an SM hide
-// more of them than three or five (a step of a 48x48 lattice pressed together
-// 898 us against 910 and 904; 926 with constants as operands and three).
-__global__ void __launch_bounds__(TPB, 4) k_tt_near(PgDev d, PgTT g, double step)
+// Bound by FP64 issue and by the gathers before it: 16 warps an SM hide more of
+// them than 12 or 20 (a step of the 64x64 lattice 898 us against 910 and 904;
+// 926 with constants as operands and 12).  In blocks of one warp the last wave
+// of a small scene is spread over more SMs (a step of the 16x16 lattice 176 ->
+// 173 us).
+__global__ void __launch_bounds__(32, 16) k_tt_near(PgDev d, PgTT g, double step)
 {
   const pg::Num<pg::f64> N;
   const int n = g.qn[0];
@@ -575,12 +578,12 @@ __global__ void __launch_bounds__(TPB, 4) k_tt_near(PgDev d, PgTT g, double step
 
 // resident blocks over every SM, for the loops over device-side counts
 template <class K>
-int resident_blocks(K k)
+int resident_blocks(K k, int tpb = TPB)
 {
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, tpb, 0);
   return (sms > 0 ? sms : 152) * (per > 0 ? per : 4);
 }
 
@@ -871,14 +874,14 @@ void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, double step)
 {
   if (g.np > 0)
   {
-    static const int bd = resident_blocks(k_tt_distances), bn = resident_blocks(k_tt_near);
+    static const int bd = resident_blocks(k_tt_distances), bn = resident_blocks(k_tt_near, 32);
     auto upto = [](int most, long long n) { const int b = nblk(n); return b < most ? b : most; };
     const int bv = upto(bd, 6LL * g.np), be = upto(bd, 9LL * g.np);
     const int tiles = (2 * g.np + PG_TT_TILE - 1) / PG_TT_TILE;
     cudaMemsetAsync(g.qn, 0, 4 * sizeof(int), s);
     k_tt_judge<<<nblk(g.np), TPB, 0, s>>>(d, g);
     k_tt_distances<<<bv + be, TPB, 0, s>>>(g, bv);
-    k_tt_near<<<upto(bn, g.np), TPB, 0, s>>>(d, g, step);
+    k_tt_near<<<std::min((g.np + 31) / 32, bn), 32, 0, s>>>(d, g, step);
     k_tt_active<<<tiles, TILE_THREADS, 0, s>>>(g);
     k_tt_select<<<tiles, TILE_THREADS, 0, s>>>(g);
   }

@@ -168,7 +168,7 @@ __device__ __forceinline__ bool quad_settled(const Quad &q, double O, double Tb,
 }
 
 // `last` in the adaptive force sums: the master sides are summed here, as
-// k_contacts_sum would
+// k_contacts_sum would, and the step chosen, as by k_adapt_min
 template <int MODE>
 __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, double half, double hstep, int oblocks, int last)
 {
@@ -177,6 +177,7 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
   constexpr bool SUMS = MODE != INT_DYNAMICS && MODE != INT_DYN_FUSED;
   constexpr bool MOVES = MODE != INT_FORCES && MODE != INT_FORCES_ADAPT;
   bool need = false;
+  unsigned long long chosen = 0x7fefffffffffffffull;        // DBL_MAX
   const double step0 = step;
   if (FUSED && (int)blockIdx.x < oblocks)
   {
@@ -464,9 +465,20 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
     if (!MOVES)
     {
       if (writes) { d.force[c][i] = F; d.torque[c][i] = T; }
-      return;
+      if (ADAPT && last)
+      {
+        double J[9];
+        for (int k = 0; k < 9; k ++) J[k] = d.inertia[k][i];
+        double ka[3], kr[6], om, ra;
+        q.all(kact, ka);
+        q.all(krd, kr);
+        q.all(kro, kr + 3);
+        const double h = critical_step(ka, kmax, emax, kr, ma, J, &om, &ra);
+        chosen = (unsigned long long)__double_as_longlong(h);
+      }
     }
-
+    if (MOVES)
+    {
     // restrain_forces (restrain.ispc:93-133), in input order; the drop-in
     // entry points run it as its own export
     if (FUSED && d.rstnum)
@@ -603,7 +615,9 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
       need = r0 + r1 + r2 > d.half_skin_sq_f;
     }
     }
+    }
   }
+  if (ADAPT && last) adapt_min(d, chosen);
   if (FUSED && d.ellnum) flag_rebuild(d, need);
   if (FUSED) pgk::step_done(d, step0, last);
 }

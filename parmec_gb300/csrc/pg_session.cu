@@ -1301,7 +1301,7 @@ void enqueue_step_adaptive(pg_session *s)
   pg_launch_torsion(d, s->stream, 0.0);
   pg_launch_unspring(d, s->stream);
   pg_launch_force_sums_adapt(d, s->stream, true);
-  pg_launch_adapt_step(d, s->stream);
+  pg_launch_adapt_step(d, s->stream, true);
   pg_launch_dynamics_fused(d, s->stream);
   pg_launch_mesh(d, s->stream);
 }
@@ -1312,7 +1312,9 @@ int adaptive_kernel_count(const PgDev &d)
   if (!d.ellnum && !d.sprnum) n += 1;             // excite
   if (d.sprnum) n += 1 + (d.nbig > 0 ? 4 : 0) + (d.unsprnum ? 1 : 0);
   if (d.trqsprnum) n += 1;
-  n += d.parnum ? 3 : 2;                          // force sums, minimum with the selection, dynamics with obstacles and tail; or the selection and the tail
+  // force sums, the minimum with the selection unless they take it, dynamics
+  // with obstacles and tail; without particles the selection and the tail
+  n += d.parnum && !pg_adapt_in_sums(d) ? 3 : 2;
   if (d.nodnum) n += 1;
   if (d.facnum) n += 1;
   return n;

@@ -2039,6 +2039,33 @@ __global__ void __launch_bounds__(TPB, PG_INTEGRATE_MINB) k_integrate(PgDev d, d
   if (FUSED) pgk::step_done(d, step0, last);
 }
 
+// step1 = factor * the smallest critical step, or step0 when nothing is
+// restrained; re-arms the minimum for the next step
+__device__ __forceinline__ void adapt_select(const PgDev &d)
+{
+  const double hmin = __longlong_as_double((long long)atomicExch(d.hmin, 0x7fefffffffffffffull));
+  d.hs[1] = hmin < 1.7976931348623157e308 ? d.hs[2]*hmin : d.hs[0];
+}
+
+// The smallest of the bits of the lanes' critical steps, of a block of one warp,
+// into d.hmin; with a counter (a session's step) the last block selects the step
+__device__ __forceinline__ void adapt_min(const PgDev &d, unsigned long long bits)
+{
+  for (int o = 16; o > 0; o >>= 1)
+  {
+    const unsigned long long other = __shfl_down_sync(0xffffffffu, bits, o);
+    bits = other < bits ? other : bits;
+  }
+  if (threadIdx.x != 0) return;
+  atomicMin(d.hmin, bits);
+  if (!d.obs_done) return;
+  int n;
+  asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(n) : "l"(d.obs_done) : "memory");
+  if (n != (int)gridDim.x - 1) return;
+  *d.obs_done = 0;
+  adapt_select(d);
+}
+
 #include "pg_quad.cuh"
 
 // ---------------------------------------------------------------- torsion springs
@@ -2287,17 +2314,8 @@ __global__ void k_unspring(PgDev d)
 // order as their bit patterns, so the minimum is an integer atomicMin (NaN
 // patterns sort above every finite step and never win, as NaN is dropped by
 // the reference's min).
-// step1 = factor * the smallest critical step, or step0 when nothing is
-// restrained; re-arms the minimum for the next step
-__device__ __forceinline__ void adapt_select(const PgDev &d)
-{
-  const double hmin = __longlong_as_double((long long)atomicExch(d.hmin, 0x7fefffffffffffffull));
-  d.hs[1] = hmin < 1.7976931348623157e308 ? d.hs[2]*hmin : d.hs[0];
-}
-
 // One warp a block: a particle's critical step is one chain of roots and
-// quotients, and the warps spread over the SMs.  With a counter (a session's
-// step) the last block selects the step.
+// quotients, and the warps spread over the SMs.
 __global__ void __launch_bounds__(32) k_adapt_min(PgDev d)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2310,19 +2328,7 @@ __global__ void __launch_bounds__(32) k_adapt_min(PgDev d)
     const double h = critical_step(kact, d.akmax[i], d.aemax[i], krot, d.mass[i], J, &om, &ra);
     bits = (unsigned long long)__double_as_longlong(h);
   }
-  for (int o = 16; o > 0; o >>= 1)
-  {
-    const unsigned long long other = __shfl_down_sync(0xffffffffu, bits, o);
-    bits = other < bits ? other : bits;
-  }
-  if (threadIdx.x != 0) return;
-  atomicMin(d.hmin, bits);
-  if (!d.obs_done) return;
-  int n;
-  asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(n) : "l"(d.obs_done) : "memory");
-  if (n != (int)gridDim.x - 1) return;
-  *d.obs_done = 0;
-  adapt_select(d);
+  adapt_min(d, bits);
 }
 
 // ---------------------------------------------------------------- CRITICAL (parmec.ispc:485-888)
@@ -2614,12 +2620,12 @@ static int eval_blocks()
   return nb;
 }
 
-// whether the update of an adaptive step sums the master sides of its contacts
-// itself (k_integrate_quad; a pass of its own takes 21 us of a step of 2,197
-// spheres, in the update 5)
-static bool sums_in_update(const PgDev &d)
+// whether the force sums of a session's adaptive step also sum the master sides
+// of the contacts and choose the step (k_integrate_quad; the passes of their
+// own take 21 and 40 us of a step of 2,197 spheres)
+bool pg_adapt_in_sums(const PgDev &d)
 {
-  return d.cwork && d.cwork_n && d.ellnum <= PG_SMALL_SCENE && d.parnum <= PG_SMALL_SCENE;
+  return d.obs_done && (!d.ellnum || (d.cwork && d.cwork_n)) && d.ellnum <= PG_SMALL_SCENE && d.parnum <= PG_SMALL_SCENE;
 }
 
 // in_step: a session's step, whose end empties the work queue and whose scene
@@ -2639,7 +2645,7 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
       else if (d.hs) k_contacts_few<false, true><<<nb, 32, 0, s>>>(d, step, S, xb);
       else if (d.record_geometry) k_contacts_few<true, false><<<nb, 32, 0, s>>>(d, step, S, xb);
       else k_contacts_few<false, false><<<nb, 32, 0, s>>>(d, step, S, xb);
-      if (d.hs && !(in_step && sums_in_update(d))) k_contacts_sum<<<nblk(d.ellnum), TPB, 0, s>>>(d);
+      if (d.hs && !(in_step && pg_adapt_in_sums(d))) k_contacts_sum<<<nblk(d.ellnum), TPB, 0, s>>>(d);
       return;
     }
     if (!in_step) cudaMemsetAsync(d.cwork_n, 0, sizeof(int), s);
@@ -2768,11 +2774,12 @@ void pg_launch_dynamics(const PgDev &d, cudaStream_t s, double step0, double ste
 // in_step: after pg_launch_contacts with in_step
 void pg_launch_force_sums_adapt(const PgDev &d, cudaStream_t s, bool in_step)
 {
-  launch_integrate<INT_FORCES_ADAPT>(d, s, 0.0, 0.0, 0.0, in_step && sums_in_update(d));
+  launch_integrate<INT_FORCES_ADAPT>(d, s, 0.0, 0.0, 0.0, in_step && pg_adapt_in_sums(d));
 }
 
-void pg_launch_adapt_step(const PgDev &d, cudaStream_t s)
+void pg_launch_adapt_step(const PgDev &d, cudaStream_t s, bool in_step)
 {
+  if (d.parnum && in_step && pg_adapt_in_sums(d)) return;     // the force sums chose it
   if (d.parnum) k_adapt_min<<<(d.parnum + 31) / 32, 32, 0, s>>>(d);
   if (!d.parnum || !d.obs_done) k_adapt_select<<<1, 32, 0, s>>>(d);
 }
