@@ -325,7 +325,7 @@ PG_DEV void spin_iso(R *O, R *Tb, double js, double is, double step, double half
 // settled, of the hopper fill 82 to 93.  With exp_terms and the unturned
 // rotations k_integrate takes 207 FP64 instructions a warp instead of 298:
 // 697 -> 547 us on the 1,048,576-sphere drum (480 with register operands),
-// 121 -> 48 us on 230,000 spheres of shaken boxes (most of them not turning
+// 121 -> 48 us on 207,000 spheres of shaken boxes (most of them not turning
 // yet).
 template <class R>
 PG_DEV bool gyro_settled(const R *O, const R *Tb, double js, double is, double step,

@@ -35,7 +35,7 @@ constexpr int TPB = 128;
 // minimum resident blocks per SM asked of the FP64 particle update and of
 // the contact evaluation (register budget against warps in flight).  The
 // particle update at 3, 4 and 5 blocks (168, 128, 96 registers): 519, 492,
-// 480 us on the 1,048,576-sphere drum and 59, 53, 51 us on 43,000 shaken
+// 480 us on the 1,048,576-sphere drum and 59, 53, 51 us on 207,000 shaken
 // spheres; a warp waits for its loads while others hold the FP64 pipe.
 #ifndef PG_INTEGRATE_MINB
 #define PG_INTEGRATE_MINB 5
