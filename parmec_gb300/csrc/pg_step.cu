@@ -190,13 +190,15 @@ __global__ void k_spheres(PgDev d)
 
 __global__ void k_nodes(PgDev d, int skip_analytical)
 {
+  const Num<f64> N;
   int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= d.nodnum) return;
   int j = d.nodpart[n];
   if (skip_analytical && (d.flags[j] & PG_FLAG_ANALYTICAL)) return;
-  double L[9], X[3], x[3], C[3], c[3];
-  for (int k = 0; k < 9; k ++) L[k] = d.rotation[k][j];
-  for (int k = 0; k < 3; k ++) { X[k] = d.position[3+k][j]; x[k] = d.position[k][j]; C[k] = d.nodes[3+k][n]; }
+  double X[3], C[3];
+  f64 L[9], x[3], c[3];
+  for (int k = 0; k < 9; k ++) L[k] = N(d.rotation[k][j]);
+  for (int k = 0; k < 3; k ++) { X[k] = d.position[3+k][j]; x[k] = N(d.position[k][j]); C[k] = d.nodes[3+k][n]; }
   body_point(x, L, X, C, c);
   for (int k = 0; k < 3; k ++) d.nodes[k][n] = c[k];
 }
@@ -1000,29 +1002,34 @@ __device__ double eqm(const PgDev &d, int part1, const double *point1, int part2
 // its stiffness terms (forces.ispc:1248-1345) in sad, zeros when its total
 // force is zero.  The k arm is taken in the k particle's frame (the reference
 // rotates it with the j particle's rotation, forces.ispc:1341).
+// Bound by FP64 issue, about 150 instructions a spring, half of them the ends'
+// points and velocities with register operands (196,096 springs: a step 186 ->
+// 180 us, of 27,456 53.4 -> 52.7, with the nodes likewise 177 and 52.2).
 template <bool ADAPT>
 __global__ void __launch_bounds__(TPB) k_springs(PgDev d, double step, int xblocks)
 {
   if (pgk::excite_front(d, xblocks, step)) return;
+  typedef f64 R;
+  const Num<R> N;
   int i = (blockIdx.x - xblocks) * blockDim.x + threadIdx.x;
   if (i >= d.sprnum) return;
   if (ADAPT) step = d.hs[0];
   const double time = d.t_curtime[(size_t)d.tab_row * (*d.stepno)];
   const int j = d.sprpart[0][i], k = d.sprpart[1][i];
   double len = 0.0, inv, velocity, spring_force = 0.0, dashpot_force, total_force;
-  double Yj[3], Yk[3] = {0.0, 0.0, 0.0}, p[3], q[3], z[3] = {0.0, 0.0, 0.0}, w[3], frc[3], u[3], a[3], b[3] = {0.0, 0.0, 0.0};
+  const R zero = N(0.0);
+  R Yj[3], Yk[3] = {zero, zero, zero}, p[3], q[3], z[3] = {zero, zero, zero}, w[3], frc[3], u[3], a[3], b[3] = {zero, zero, zero};
   double stiffness = 0.0, damping = 0.0;
-  double oj[3], vj[3], xj[3], Xj[3], Lj[9];
+  R oj[3], vj[3], xj[3], Xj[3], Lj[9];
   for (int m = 0; m < 3; m ++)
   {
-    oj[m] = d.angular[3+m][j]; vj[m] = d.linear[m][j]; xj[m] = d.position[m][j]; Xj[m] = d.position[3+m][j];
+    oj[m] = N(d.angular[3+m][j]); vj[m] = N(d.linear[m][j]); xj[m] = N(d.position[m][j]); Xj[m] = N(d.position[3+m][j]);
   }
-  for (int m = 0; m < 9; m ++) Lj[m] = d.rotation[m][j];
+  for (int m = 0; m < 9; m ++) Lj[m] = N(d.rotation[m][j]);
   const int flg0 = d.sprflg[i];
   int flg = flg0;
 
-  Yj[0] = d.sprpnt[3][i]; Yj[1] = d.sprpnt[4][i]; Yj[2] = d.sprpnt[5][i];
-  Yj[0] = Yj[0] - Xj[0]; Yj[1] = Yj[1] - Xj[1]; Yj[2] = Yj[2] - Xj[2];
+  Yj[0] = d.sprpnt[3][i] - Xj[0]; Yj[1] = d.sprpnt[4][i] - Xj[1]; Yj[2] = d.sprpnt[5][i] - Xj[2];
   nvaddmul(xj, Lj, Yj, p);
   d.sprpnt[0][i] = p[0]; d.sprpnt[1][i] = p[1]; d.sprpnt[2][i] = p[2];
   u[0] = vj[0]; u[1] = vj[1]; u[2] = vj[2];
@@ -1034,20 +1041,19 @@ __global__ void __launch_bounds__(TPB) k_springs(PgDev d, double step, int xbloc
 
   if (k >= 0)
   {
-    double ok[3], vk[3], xk[3], Xk[3], Lk[9];
+    R ok[3], vk[3], xk[3], Xk[3], Lk[9];
     for (int m = 0; m < 3; m ++)
     {
-      ok[m] = d.angular[3+m][k]; vk[m] = d.linear[m][k]; xk[m] = d.position[m][k]; Xk[m] = d.position[3+m][k];
+      ok[m] = N(d.angular[3+m][k]); vk[m] = N(d.linear[m][k]); xk[m] = N(d.position[m][k]); Xk[m] = N(d.position[3+m][k]);
     }
-    for (int m = 0; m < 9; m ++) Lk[m] = d.rotation[m][k];
+    for (int m = 0; m < 9; m ++) Lk[m] = N(d.rotation[m][k]);
     if (flg & PG_SPRDIR_PROJECT)
     {
-      w[0] = d.sprdir[3][i]; w[1] = d.sprdir[4][i]; w[2] = d.sprdir[5][i];
+      w[0] = N(d.sprdir[3][i]); w[1] = N(d.sprdir[4][i]); w[2] = N(d.sprdir[5][i]);
       nvmul(Lk, w, z);
       d.sprdir[0][i] = z[0]; d.sprdir[1][i] = z[1]; d.sprdir[2][i] = z[2];
     }
-    Yk[0] = d.sprpnt[9][i]; Yk[1] = d.sprpnt[10][i]; Yk[2] = d.sprpnt[11][i];
-    Yk[0] = Yk[0] - Xk[0]; Yk[1] = Yk[1] - Xk[1]; Yk[2] = Yk[2] - Xk[2];
+    Yk[0] = d.sprpnt[9][i] - Xk[0]; Yk[1] = d.sprpnt[10][i] - Xk[1]; Yk[2] = d.sprpnt[11][i] - Xk[2];
     nvaddmul(xk, Lk, Yk, q);
     d.sprpnt[6][i] = q[0]; d.sprpnt[7][i] = q[1]; d.sprpnt[8][i] = q[2];
     u[0] += vk[0]; u[1] += vk[1]; u[2] += vk[2];
@@ -1058,22 +1064,22 @@ __global__ void __launch_bounds__(TPB) k_springs(PgDev d, double step, int xbloc
   }
   else
   {
-    q[0] = d.sprpnt[6][i]; q[1] = d.sprpnt[7][i]; q[2] = d.sprpnt[8][i];
-    if (flg & PG_SPRDIR_PROJECT) { z[0] = d.sprdir[0][i]; z[1] = d.sprdir[1][i]; z[2] = d.sprdir[2][i]; }
+    q[0] = N(d.sprpnt[6][i]); q[1] = N(d.sprpnt[7][i]); q[2] = N(d.sprpnt[8][i]);
+    if (flg & PG_SPRDIR_PROJECT) { z[0] = N(d.sprdir[0][i]); z[1] = N(d.sprdir[1][i]); z[2] = N(d.sprdir[2][i]); }
   }
 
   switch (flg & (PG_SPRDIR_FOLLOWER|PG_SPRDIR_CONSTANT|PG_SPRDIR_PLANAR|PG_SPRDIR_PROJECT))
   {
     case PG_SPRDIR_FOLLOWER:
       w[0] = q[0] - p[0]; w[1] = q[1] - p[1]; w[2] = q[2] - p[2];
-      len = sqrt(dot3(w, w));
+      len = sqrt((double)dot3(w, w));
       inv = len > 0.0 ? 1.0/len : 0.0;
       z[0] = inv*w[0]; z[1] = inv*w[1]; z[2] = inv*w[2];
       d.sprdir[0][i] = z[0]; d.sprdir[1][i] = z[1]; d.sprdir[2][i] = z[2];
       break;
     case PG_SPRDIR_CONSTANT:
       w[0] = q[0] - p[0]; w[1] = q[1] - p[1]; w[2] = q[2] - p[2];
-      z[0] = d.sprdir[0][i]; z[1] = d.sprdir[1][i]; z[2] = d.sprdir[2][i];
+      z[0] = N(d.sprdir[0][i]); z[1] = N(d.sprdir[1][i]); z[2] = N(d.sprdir[2][i]);
       len = dot3(w, z);
       break;
     case PG_SPRDIR_PLANAR:
@@ -1082,7 +1088,7 @@ __global__ void __launch_bounds__(TPB) k_springs(PgDev d, double step, int xbloc
       w[0] -= inv*d.sprdir[3][i];
       w[1] -= inv*d.sprdir[4][i];
       w[2] -= inv*d.sprdir[5][i];
-      len = sqrt(dot3(w, w));
+      len = sqrt((double)dot3(w, w));
       inv = len > 0.0 ? 1.0/len : 0.0;
       z[0] = inv*w[0]; z[1] = inv*w[1]; z[2] = inv*w[2];
       d.sprdir[0][i] = z[0]; d.sprdir[1][i] = z[1]; d.sprdir[2][i] = z[2];
@@ -1180,7 +1186,8 @@ __global__ void __launch_bounds__(TPB) k_springs(PgDev d, double step, int xbloc
     velocity = dot3(z, u);
     if (d.dashidx[i]+1 == d.dashidx[i+1])
     {
-      double mass = eqm(d, j, Yj, k, Yk, z);
+      const double yj[3] = {Yj[0], Yj[1], Yj[2]}, yk[3] = {Yk[0], Yk[1], Yk[2]}, zd[3] = {z[0], z[1], z[2]};
+      double mass = eqm(d, j, yj, k, yk, zd);
       double ratio = d.dashpot[0][d.dashidx[i]];
       damping = ratio * 2.0 * sqrt(fabs(stiffness) * mass);
       dashpot_force = velocity * damping;
@@ -2696,9 +2703,12 @@ void pg_launch_springs(const PgDev &d, cudaStream_t s, double step, bool in_step
     if (excite) pg_launch_excite(d, s, step);
     return;
   }
-  const int xb = excite ? nblk(pgk::EXCITE_LANES * d.nscene) : 0;
-  if (d.hs) k_springs<true><<<xb + nblk(d.sprnum), TPB, 0, s>>>(d, step, xb);
-  else k_springs<false><<<xb + nblk(d.sprnum), TPB, 0, s>>>(d, step, xb);
+  // blocks of one warp spread the last wave over more SMs (the 27,456 springs of
+  // the 96x96 lattice: a step 56.2 us in blocks of 128, 53.4 of 32)
+  constexpr int B = 32;
+  const int xb = excite ? (pgk::EXCITE_LANES * d.nscene + B - 1) / B : 0, nb = xb + (d.sprnum + B - 1) / B;
+  if (d.hs) k_springs<true><<<nb, B, 0, s>>>(d, step, xb);
+  else k_springs<false><<<nb, B, 0, s>>>(d, step, xb);
 }
 
 void pg_launch_torsion(const PgDev &d, cudaStream_t s, double step)
