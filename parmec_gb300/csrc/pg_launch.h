@@ -24,6 +24,7 @@ void pg_launch_dynamics(const PgDev &d, cudaStream_t s, double step0, double ste
 // choice on the device (adaptive_timestep), and the rest of the step
 void pg_launch_force_sums_adapt(const PgDev &d, cudaStream_t s, bool in_step = false);
 bool pg_adapt_in_sums(const PgDev &d);
+int pg_spring_run_kernel_count(const PgDev &d, bool adaptive);
 void pg_launch_adapt_step(const PgDev &d, cudaStream_t s, bool in_step = false);
 void pg_launch_dynamics_fused(const PgDev &d, cudaStream_t s);
 void pg_launch_critical_perspring(const PgDev &d, cudaStream_t s, double *h, double *om, double *ra);

@@ -358,9 +358,8 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
         bool started = false;
         if (run >= 0)
         {
-          // a long run, summed in the same order by k_spring_run_groups
-          af = d.sbig_sum[6*run + c];
-          at = d.sbig_sum[6*run + 3 + c];
+          // a long run, its groups summed in the same order by k_spring_run_groups
+          run_total(d, run, w, c, af, at);
         }
         else
         for (int s = w.y; s < w.z; s ++)

@@ -399,7 +399,7 @@ int upload_static(pg_session *s, const pg_scene *sc)
     d.nbig_groups = pg_spring_run_groups(big);
     TRY(dalloc(s, &d.sbig, std::max<size_t>(1, big.size())));
     TRY(dalloc(s, &d.sbig_sum, 6 * std::max<size_t>(1, big.size())));
-    TRY(dalloc(s, &d.sbig_grp, 32 * 12 * std::max<size_t>(1, big.size())));
+    TRY(dalloc(s, &d.sbig_grp, 2 * 32 * 12 * std::max<size_t>(1, big.size())));
     TRY(h2d(s, d.sbig, big.data(), big.size()));
     CK(cudaStreamSynchronize(s->stream));
   }
@@ -1310,7 +1310,7 @@ int adaptive_kernel_count(const PgDev &d)
 {
   int n = pg_rebuild_kernel_count(d) + pg_contacts_kernel_count(d);
   if (!d.ellnum && !d.sprnum) n += 1;             // excite
-  if (d.sprnum) n += 1 + (d.nbig > 0 ? 4 : 0) + (d.unsprnum ? 1 : 0);
+  if (d.sprnum) n += 1 + pg_spring_run_kernel_count(d, true) + (d.unsprnum ? 1 : 0);
   if (d.trqsprnum) n += 1;
   // force sums, the minimum with the selection unless they take it, dynamics
   // with obstacles and tail; without particles the selection and the tail
