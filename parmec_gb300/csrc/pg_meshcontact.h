@@ -55,7 +55,8 @@ struct PgTT
   int *qn = nullptr;              // [4] near pairs, full pairs, vertex-face and edge-edge distances
   unsigned char *act = nullptr;   // [cap] in contact
   double *st[3] = {}, *f[3] = {}, *p[3] = {};   // tangential state, force on the finder's particle, point
-  // the previous list (state carried by (finder, partner) at a search)
+  // the previous list, pnp pairs (state carried by (finder, partner) at a search)
+  int pnp = 0;
   int *poff = nullptr, *ppu = nullptr;
   unsigned char *pact = nullptr;
   double *pst[3] = {};

@@ -14,6 +14,7 @@
 #include "pg_state.h"
 #include "pg_launch.h"
 #include "pg_meshcontact.h"
+#include "pg_ttbuffers.h"
 #include "../../include/parmec_gb300.h"
 
 #define PG_GRAPH_STEPS 8          // steps per replay of the multi-step graph
@@ -1093,54 +1094,19 @@ void enqueue_step(pg_session *s, double step)
   pg_launch_mesh(d, s->stream);
 }
 
-// room for np pairs: the list arrays and the narrow phase's work are made
-// anew, the previous list (pnp pairs), whose state the new one takes, moved
-int tt_pair_buffers(pg_session *s, int np, int pnp)
+// device memory of the session for the lists of the mesh contact
+struct SessionMem
 {
-  PgTT &g = s->tt;
-  const int cap = np + np / 2 + 1024;
-  int *ppu = nullptr; unsigned char *pact = nullptr; double *pst[3] = {};
-  TRY(dalloc(s, &ppu, cap)); TRY(dalloc(s, &pact, cap));
-  for (int c = 0; c < 3; c ++) TRY(dalloc(s, &pst[c], cap));
-  if (pnp > 0)
+  pg_session *s;
+  template <class T> int make(T **p, size_t n) { return dalloc(s, p, n); }
+  template <class T> void drop(T **p) { release(s, (void *)*p); *p = nullptr; }
+  template <class T> int copy(T *to, const T *from, size_t n)
   {
-    CK(cudaMemcpyAsync(ppu, g.ppu, (size_t)pnp * sizeof(int), cudaMemcpyDeviceToDevice, s->stream));
-    CK(cudaMemcpyAsync(pact, g.pact, (size_t)pnp, cudaMemcpyDeviceToDevice, s->stream));
-    for (int c = 0; c < 3; c ++)
-      CK(cudaMemcpyAsync(pst[c], g.pst[c], (size_t)pnp * sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
+    CK(cudaMemcpyAsync(to, from, n * sizeof(T), cudaMemcpyDeviceToDevice, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    return PG_OK;
   }
-  CK(cudaStreamSynchronize(s->stream));
-  for (void *q : {(void *)g.pf, (void *)g.pu, (void *)g.act, (void *)g.ppu, (void *)g.pact, (void *)g.near,
-                  (void *)g.full, (void *)g.vit, (void *)g.eit, (void *)g.vres, (void *)g.eres, (void *)g.ekeys[0],
-                  (void *)g.ekeys[1], (void *)g.evals[0], (void *)g.evals[1], (void *)g.ehist, (void *)g.ebits,
-                  (void *)g.etile, (void *)g.elist, (void *)g.bigp, (void *)g.bigoff})
-    release(s, q);
-  for (int c = 0; c < 3; c ++) for (void *q : {(void *)g.st[c], (void *)g.f[c], (void *)g.p[c], (void *)g.pst[c]}) release(s, q);
-  g.ppu = ppu; g.pact = pact;
-  TRY(dalloc(s, &g.pf, cap)); TRY(dalloc(s, &g.pu, cap)); TRY(dalloc(s, &g.act, cap));
-  for (int c = 0; c < 3; c ++)
-  {
-    g.pst[c] = pst[c];
-    TRY(dalloc(s, &g.st[c], cap)); TRY(dalloc(s, &g.f[c], cap)); TRY(dalloc(s, &g.p[c], cap));
-  }
-  // room for 2 vertex-triangle and 3 edge-edge distances a pair (the spring
-  // lattice, whose faces lie parallel, asks for 1.3 and 2.4); pairs beyond
-  // it take the whole narrow phase
-  g.vcap = (int)std::min(2LL * cap, 0x7fff0000LL);
-  g.ecap = (int)std::min(3LL * cap, 0x7fff0000LL);
-  TRY(dalloc(s, &g.near, cap)); TRY(dalloc(s, &g.full, cap));
-  TRY(dalloc(s, &g.vit, g.vcap)); TRY(dalloc(s, &g.eit, g.ecap));
-  TRY(dalloc(s, &g.vres, 3 * (size_t)g.vcap)); TRY(dalloc(s, &g.eres, 3 * (size_t)g.ecap));
-  const size_t E = 2 * (size_t)cap, tiles = (E + PG_TT_TILE - 1) / PG_TT_TILE;
-  for (int k = 0; k < 2; k ++) { TRY(dalloc(s, &g.ekeys[k], E)); TRY(dalloc(s, &g.evals[k], E)); }
-  TRY(dalloc(s, &g.ehist, pg_sort_hist_len((int)E)));
-  TRY(dalloc(s, &g.ebits, tiles * (PG_TT_TILE / 32)));
-  TRY(dalloc(s, &g.etile, tiles));
-  TRY(dalloc(s, &g.elist, E));
-  TRY(dalloc(s, &g.bigp, E / PG_TT_CHUNK + 1)); TRY(dalloc(s, &g.bigoff, E / PG_TT_CHUNK + 1));
-  g.cap = cap;
-  return PG_OK;
-}
+};
 
 // a new pair list: its pairs, the state of the previous list's, the entry
 // order of the sums.  The host waits twice, for the pair count and for the
@@ -1149,39 +1115,32 @@ int tt_search(pg_session *s)
 {
   PgDev &d = s->d;
   PgTT &g = s->tt;
-  const int pnp = g.valid ? g.np : 0;
-  std::swap(g.off, g.poff);
-  std::swap(g.pu, g.ppu);
-  std::swap(g.act, g.pact);
-  for (int c = 0; c < 3; c ++) std::swap(g.st[c], g.pst[c]);
-  g.valid = 0;
-  if (!pnp) CK(cudaMemsetAsync(g.poff, 0, ((size_t)d.trinum + 1) * sizeof(int), s->stream));
+  SessionMem mem{s};
+  if (g.valid)
+  {
+    // this list becomes the previous one; after a search that failed the
+    // previous one still stands
+    g.pnp = g.np;
+    std::swap(g.off, g.poff);
+    std::swap(g.pu, g.ppu);
+    std::swap(g.act, g.pact);
+    for (int c = 0; c < 3; c ++) std::swap(g.st[c], g.pst[c]);
+    g.valid = 0;
+  }
+  if (!g.pnp) CK(cudaMemsetAsync(g.poff, 0, ((size_t)d.trinum + 1) * sizeof(int), s->stream));
   pg_tt_search(d, g, s->stream);
   CK(cudaMemcpyAsync(s->tt_host, g.moved, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   const int np = s->tt_host[1];
   if (np > 0x3fffffff) return PG_ERR_CAPACITY;
-  if (np > g.cap || !g.pf) TRY(tt_pair_buffers(s, np, pnp));
+  if (np > g.cap || !g.cap) TRY(pg_tt_pair_room(g, np, mem));
   g.np = np;
   pg_tt_list(d, g, s->stream);
   CK(cudaMemcpyAsync(s->tt_host, g.moved, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   g.nbig = s->tt_host[2];
   g.nchunks = s->tt_host[3];
-  if (g.nchunks > g.ccap)
-  {
-    const int cap = g.nchunks + g.nchunks / 2;
-    release(s, g.chmap);
-    g.chmap = nullptr;
-    TRY(dalloc(s, &g.chmap, (size_t)cap));
-    for (int c = 0; c < 6; c ++)
-    {
-      release(s, g.csum[c]);
-      g.csum[c] = nullptr;
-      TRY(dalloc(s, &g.csum[c], (size_t)cap));
-    }
-    g.ccap = cap;
-  }
+  if (g.nchunks > g.ccap) TRY(pg_tt_chunk_room(g, g.nchunks, mem));
   pg_tt_chunk_map(g, s->stream);
   s->launches += pg_tt_search_kernels(g, d.trinum);
   g.valid = 1;
@@ -1729,9 +1688,10 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
   int pb = 1;
   while ((1u << pb) <= (unsigned)P) pb ++;
   g.epasses = pg_sort_passes_bits(pb);
+  SessionMem mem{s};
+  d.tt_on = 0;                                 // until everything is there
   if (!g.big)
   {
-    TRY(dalloc(s, &g.big, T));
     for (int c = 0; c < 6; c ++) TRY(dalloc(s, &g.box[c], T));
     TRY(dalloc(s, &g.cell, T));
     for (int k = 0; k < 2; k ++) { TRY(dalloc(s, &g.keys[k], T)); TRY(dalloc(s, &g.vals[k], T)); }
@@ -1748,14 +1708,16 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
     TRY(dalloc(s, &g.fv, 3 * (size_t)T));
     TRY(dalloc(s, &g.geo, (size_t)PG_TT_GEO * T));
     for (int c = 0; c < 3; c ++) { TRY(dalloc(s, &d.ttF[c], P)); TRY(dalloc(s, &d.ttT[c], P)); }
+    TRY(dalloc(s, &g.big, T));                 // the last: says that the others are there
   }
-  release(s, g.cstart);
-  release(s, g.cend);
+  mem.drop(&g.cstart);
+  mem.drop(&g.cend);
   TRY(dalloc(s, &g.cstart, (size_t)g.ncells + 1));
   TRY(dalloc(s, &g.cend, (size_t)g.ncells + 1));
   TRY(h2d(s, g.big, big, T));
   // no pairs carried into the first step
   g.valid = 0;
+  g.pnp = 0;
   CK(cudaStreamSynchronize(s->stream));
   d.tt_on = 1;
   return PG_OK;
