@@ -11,6 +11,7 @@
 // pgtf::judge), where their results start, a bound on the smallest
 struct PgTTNear { int pair; unsigned mask; int vbase, ebase; float upper, size; };
 #define PG_TT_GEO 28
+#define PG_TT_MOST 0x3fffffff     // pairs a list may hold
 
 // a triangle's box at a search, widened by r and half the skin (rounded
 // outwards), its particle (-1: not of a mesh) and whether it is big
@@ -41,6 +42,7 @@ struct PgTT
   int *cstart = nullptr, *cend = nullptr;   // [ncells + 1]: the last range holds the big triangles
   int *cnt = nullptr, *off = nullptr;       // [trinum], [trinum + 1]
   int cap = 0, np = 0;            // pair capacity and pairs
+  int most = PG_TT_MOST;          // more pairs than these are refused
   int *pf = nullptr, *pu = nullptr;         // [cap] finder and partner of each pair
   // the narrow phase's work (pg_ttfilter.cuh): float copies of the triangles
   // and their FP64 differences, the pairs that may touch with what decides

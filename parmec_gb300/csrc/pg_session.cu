@@ -1072,7 +1072,7 @@ PgDev live_view(const pg_session *s)
   return v;
 }
 
-void enqueue_step(pg_session *s, double step)
+int enqueue_step(pg_session *s, double step)
 {
   const PgDev d = live_view(s);
   // the scene gravities are taken beside the first of these that runs, the
@@ -1082,16 +1082,17 @@ void enqueue_step(pg_session *s, double step)
   {
     pg_launch_contacts_mx(d, s->stream, step);
     pg_launch_integrate_mx(d, s->stream, step);
-    return;
+    return PG_OK;
   }
   pg_launch_contacts(d, s->stream, step, true);
   pg_launch_springs(d, s->stream, step, true);
   pg_launch_spring_runs(d, s->stream);
   pg_launch_torsion(d, s->stream, step);
   pg_launch_unspring(d, s->stream);
-  if (d.tt_on) tt_stage(s, step);
+  if (d.tt_on) TRY(tt_stage(s, step));
   pg_launch_integrate(d, s->stream, step);
   pg_launch_mesh(d, s->stream);
+  return PG_OK;
 }
 
 // device memory of the session for the lists of the mesh contact
@@ -1132,7 +1133,7 @@ int tt_search(pg_session *s)
   CK(cudaMemcpyAsync(s->tt_host, g.moved, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   const int np = s->tt_host[1];
-  if (np > 0x3fffffff) return PG_ERR_CAPACITY;
+  if (np > g.most) return PG_ERR_CAPACITY;
   if (np > g.cap || !g.cap) TRY(pg_tt_pair_room(g, np, mem));
   g.np = np;
   pg_tt_list(d, g, s->stream);
@@ -1147,11 +1148,7 @@ int tt_search(pg_session *s)
   return PG_OK;
 }
 
-// the mesh-contact stage of one step: boxes, a new pair list when a triangle
-// left its neighbourhood, contacts and per-particle sums.  It reads back
-// whether a list is due (one host wait per step), so steps with mesh contact
-// are not captured in graphs.
-int tt_stage(pg_session *s, double step)
+int tt_contacts(pg_session *s, double step)
 {
   PgDev &d = s->d;
   PgTT &g = s->tt;
@@ -1166,6 +1163,18 @@ int tt_stage(pg_session *s, double step)
   return PG_OK;
 }
 
+// the mesh-contact stage of one step: boxes, a new pair list when a triangle
+// left its neighbourhood, contacts and per-particle sums.  It reads back
+// whether a list is due (one host wait per step), so steps with mesh contact
+// are not captured in graphs.  Where it fails the step ends here, and with it
+// the run: the contacts' work queue, which the step's end empties, is emptied.
+int tt_stage(pg_session *s, double step)
+{
+  const int rc = tt_contacts(s, step);
+  if (rc != PG_OK && s->d.cwork_n) cudaMemsetAsync(s->d.cwork_n, 0, sizeof(int), s->stream);
+  return rc;
+}
+
 // capture one step into a CUDA graph (kernel arguments are baked in: the
 // graph is re-captured when a buffer is reallocated or the step changes)
 int capture_step(pg_session *s, double step)
@@ -1173,8 +1182,9 @@ int capture_step(pg_session *s, double step)
   if (s->graph_exec && !s->graph_adapt && s->graph_step == step) return PG_OK;
   drop_graph(s);
   CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-  enqueue_step(s, step);
+  const int rc = enqueue_step(s, step);
   CK(cudaStreamEndCapture(s->stream, &s->graph));
+  TRY(rc);
   CK(cudaGraphInstantiate(&s->graph_exec, s->graph, 0));
   s->graph_step = step;
   s->graph_adapt = 0;
@@ -1187,8 +1197,10 @@ int capture_steps(pg_session *s, double step)
   TRY(capture_step(s, step));
   if (s->graphn_exec) return PG_OK;
   CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-  for (int k = 0; k < PG_GRAPH_STEPS; k ++) enqueue_step(s, step);
+  int rc = PG_OK;
+  for (int k = 0; k < PG_GRAPH_STEPS && rc == PG_OK; k ++) rc = enqueue_step(s, step);
   CK(cudaStreamEndCapture(s->stream, &s->graphn));
+  TRY(rc);
   CK(cudaGraphInstantiate(&s->graphn_exec, s->graphn, 0));
   return PG_OK;
 }
@@ -1473,6 +1485,7 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
     return PG_OK;
   }
   const int per_step = pg_rebuild_kernel_count(d) + pg_step_kernel_count(d);
+  bool counted = false;
   if (!s->profile && s->use_graph && !d.tt_on)
   {
     TRY(capture_step(s, step));
@@ -1486,7 +1499,12 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
   }
   else if (!s->profile)
   {
-    for (int k = 0; k < n; k ++) enqueue_step(s, step);
+    for (int k = 0; k < n; k ++)
+    {
+      TRY(enqueue_step(s, step));
+      s->launches += per_step;
+    }
+    counted = true;
   }
   else
   {
@@ -1536,7 +1554,7 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
       }
     }
   }
-  s->launches += (long long)per_step * n;
+  if (!counted) s->launches += (long long)per_step * n;
   CK(cudaGetLastError());
   if (wait) CK(cudaStreamSynchronize(s->stream));
   return PG_OK;
@@ -1720,6 +1738,13 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
   g.pnp = 0;
   CK(cudaStreamSynchronize(s->stream));
   d.tt_on = 1;
+  return PG_OK;
+}
+
+int pg_session_mesh_contact_room(pg_session *s, int pairs)
+{
+  if (!s || pairs < 0) return PG_ERR_ARGUMENT;
+  s->tt.most = pairs > 0 ? std::min(pairs, PG_TT_MOST) : PG_TT_MOST;
   return PG_OK;
 }
 

@@ -1,0 +1,78 @@
+"""The mesh contact's pair list where it changes: room, searches, far places.
+
+Every comparison is with the oracle's brute-force search, bit for bit.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+from helpers import assert_bitwise
+
+pytestmark = pytest.mark.gpu
+
+DT = 1e-5
+
+
+def pile(origin=(0.0, 0.0, 0.0), layers=2, side=3, seed=3, radius=1e-3):
+    """Layers of 10 mm cubes on a fixed plate, 0.1 mm outside the reach of one
+    another, the upper ones turning; an upper layer falls at 1 m/s."""
+    from parmec_gb300 import mesh
+    from parmec_gb300.model import Model
+    rng = np.random.default_rng(seed)
+    m = Model()
+    mat = m.material(2500.0, 1e9, 0.25)
+    o = np.asarray(origin, dtype=np.float64)
+    lo, hi = o - (0.01, 0.01, 0.005), o + (0.014 * side, 0.014 * side, 0.0)
+    c = [(x, y, z) for z in (lo[2], hi[2]) for x, y in ((lo[0], lo[1]), (hi[0], lo[1]), (hi[0], hi[1]), (lo[0], hi[1]))]
+    plate = m.mesh([v for p in c for v in p], [8, 0, 1, 2, 3, 4, 5, 6, 7, mat], mat, 2)
+    m.prescribe_motion(plate, linear=lambda t: (0.0, 0.0, 0.0), angular=lambda t: (0.0, 0.0, 0.0), kind="vv")
+    org = [(0.014 * i + 1e-3 * rng.uniform(-1, 1), 0.014 * j, 0.0021 + 0.0121 * k)
+           for k in range(layers) for i in range(side) for j in range(side)]
+    parts = mesh.hex_grid(m, o + np.array(org), 0.01, mat, 1)
+    for p in parts[side * side:]:
+        m.velocity(int(p), linear=(0.0, 0.0, -1.0), angular=tuple(float(x) for x in rng.normal(0.0, 2.0, size=3)))
+    m.granular(0, 0, 1e5, 0.3, 0.4)
+    m.set_gravity(0.0, 0.0, -9.81)
+    m.mesh_contact(radius)
+    return m
+
+
+def pair(make):
+    from oracle.pyoracle import OracleEngine
+    from parmec_gb300.engine import GpuEngine
+    return (make(), GpuEngine()), (make(), OracleEngine())
+
+
+def dem(both, steps, first=False):
+    for m, eng in both:
+        m.dem((steps - (0.5 if first else 0.0)) * DT, DT, interval=1e9, engine=eng)
+    assert_bitwise(both[0][0], both[1][0])
+    assert both[0][1].mesh_contact_stats() == both[1][1].mesh_contact_stats()
+    return both[1][1].mesh_contact_stats()
+
+
+def test_refused_list_ends_the_run_and_the_session_goes_on(gpu_lib, oracle_lib):
+    """A search that finds more pairs than there is room for ends the run with
+    an error, at the step it belongs to; with room again the session goes on
+    from there, its contacts' state unbroken."""
+    from parmec_gb300 import abi, driver
+    both = (mg, eg), _ = pair(pile)
+    assert dem(both, 300, first=True)[1] > 0
+    tabs = driver.StepTables(mg, [mg.curtime + k * DT for k in range(400)], DT, [1e9, 1e9], [None, None], [-1, -1])
+    done0 = eg.global_step()
+    assert eg.lib.pg_session_mesh_contact_room(eg.sess, 1) == abi.PG_OK
+    tab = tabs.ctab(0, 400)
+    assert eg.lib.pg_session_run(eg.sess, ctypes.byref(tab), DT) == abi.PG_ERR_CAPACITY
+    done = eg.global_step() - done0
+    assert 0 < done < 400
+    assert eg.lib.pg_session_run(eg.sess, ctypes.byref(tab), DT) == abi.PG_ERR_CAPACITY
+    assert eg.global_step() == done0 + done
+    assert eg.lib.pg_session_mesh_contact_room(eg.sess, 0) == abi.PG_OK
+    tab = tabs.ctab(done, 400)
+    assert eg.lib.pg_session_run(eg.sess, ctypes.byref(tab), DT) == abi.PG_OK
+    eg.download()
+    mo, eo = both[1]
+    mo.dem(400 * DT, DT, interval=1e9, engine=eo)
+    assert_bitwise(mg, mo)
+    assert eg.mesh_contact_stats() == eo.mesh_contact_stats()
