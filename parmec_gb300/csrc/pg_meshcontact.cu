@@ -267,27 +267,28 @@ __global__ void __launch_bounds__(TPB) k_tt_find(PgDev d, PgTT g)
   }
 }
 
-// 4. exclusive scan of the counts in one block (off[n] = total)
+// 4. exclusive scan of the counts in one block (off[n] = total); a total
+// beyond 31 bits is given as the largest int, which no list may hold
 __global__ void __launch_bounds__(1024) k_tt_scan(const int *in, int *out, int n, int *total)
 {
-  __shared__ int part[1024];
+  __shared__ long long part[1024];
   const int tid = threadIdx.x;
   const int per = (n + 1023) / 1024;
   const int b = tid * per, e = b + per < n ? b + per : n;
-  int s = 0;
+  long long s = 0;
   for (int i = b; i < e; i ++) s += in[i];
   part[tid] = s;
   __syncthreads();
   for (int o = 1; o < 1024; o <<= 1)
   {
-    const int v = tid >= o ? part[tid - o] : 0;
+    const long long v = tid >= o ? part[tid - o] : 0;
     __syncthreads();
     part[tid] += v;
     __syncthreads();
   }
-  int acc = tid ? part[tid - 1] : 0;
-  for (int i = b; i < e; i ++) { const int v = in[i]; out[i] = acc; acc += v; }
-  if (tid == 1023) { out[n] = part[1023]; *total = part[1023]; }
+  long long acc = tid ? part[tid - 1] : 0;
+  for (int i = b; i < e; i ++) { const int v = in[i]; out[i] = (int)acc; acc += v; }
+  if (tid == 1023) out[n] = *total = (int)min(part[1023], 0x7fffffffLL);
 }
 
 // the boxes of pair k overlap with positive measure this step
@@ -311,8 +312,9 @@ __global__ void __launch_bounds__(TPB) k_tt_counts(PgTT g, int *out2)
 // than 2r get their result (inactive), the others a place in the list of
 // near pairs with the distances that can decide them, or in the list of
 // pairs that need every test.  One thread per pair; list places and item
-// ranges by one atomic per list and warp.
-__device__ __forceinline__ int warp_take(int *count, int n)
+// ranges by one atomic per list and warp, counted in 64 bits: a pair asks for
+// up to nine distances of a kind.
+__device__ __forceinline__ long long warp_take(unsigned long long *count, int n)
 {
   const unsigned all = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -322,8 +324,8 @@ __device__ __forceinline__ int warp_take(int *count, int n)
     const int v = __shfl_up_sync(all, s, o);
     if (lane >= o) s += v;
   }
-  int base = 0;
-  if (lane == 31 && s) base = atomicAdd(count, s);
+  long long base = 0;
+  if (lane == 31 && s) base = (long long)atomicAdd(count, (unsigned long long)s);
   base = __shfl_sync(all, base, 31);
   return base + s - n;
 }
@@ -371,21 +373,23 @@ __global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g)
     if (verdict == pgtf::APART) g.act[k] = 0;
   }
   int nv = verdict == pgtf::NEAR ? __popc(mask & 63u) : 0, ne = verdict == pgtf::NEAR ? __popc(mask >> 6) : 0;
-  const int vb = warp_take(g.qn + 2, nv), eb = warp_take(g.qn + 3, ne);
+  const long long vb = warp_take(g.qn + 2, nv), eb = warp_take(g.qn + 3, ne);
   if (verdict == pgtf::NEAR && (vb + nv > g.vcap || eb + ne > g.ecap)) verdict = pgtf::FULL;   // no room for its items
-  const int np = warp_take(g.qn, verdict == pgtf::NEAR), z = warp_take(g.qn + 1, verdict == pgtf::FULL);
+  const long long np = warp_take(g.qn, verdict == pgtf::NEAR);
+  if (verdict == pgtf::NEAR && np >= PG_TT_NEAR) verdict = pgtf::FULL;                         // nor for their number
+  const long long z = warp_take(g.qn + 1, verdict == pgtf::FULL);
   // (items of a pair that found no room in the other list name no pair)
   if (nv + ne && verdict == pgtf::FULL)
   {
-    for (int j = vb; j < vb + nv && j < g.vcap; j ++) g.vit[j] = ~0u;
-    for (int j = eb; j < eb + ne && j < g.ecap; j ++) g.eit[j] = ~0u;
+    for (long long j = vb; j < vb + nv && j < g.vcap; j ++) g.vit[j] = ~0u;
+    for (long long j = eb; j < eb + ne && j < g.ecap; j ++) g.eit[j] = ~0u;
   }
   if (verdict == pgtf::FULL) g.full[z] = k;
   if (verdict != pgtf::NEAR) return;
-  g.near[np] = {k, mask, vb, eb, upper, size};
-  int j = vb;
+  g.near[np] = {k, mask, (int)vb, (int)eb, upper, size};
+  int j = (int)vb;
   for (unsigned m = mask & 63u; m; m &= m - 1) g.vit[j ++] = (unsigned)np << 4 | (unsigned)(__ffs(m) - 1);
-  j = eb;
+  j = (int)eb;
   for (unsigned m = mask >> 6; m; m &= m - 1) g.eit[j ++] = (unsigned)np << 4 | (unsigned)(__ffs(m) - 1);
 }
 
@@ -394,7 +398,7 @@ __global__ void __launch_bounds__(TPB) k_tt_judge(PgDev d, PgTT g)
 // take the one kind, the others the other
 __device__ __forceinline__ void tt_vertex_face(const PgTT &g, const pg::Num<pg::f64> &N, int first, int by)
 {
-  const int n = min(g.qn[2], g.vcap);
+  const int n = (int)min(g.qn[2], (unsigned long long)g.vcap);
   for (int w = first; w < n; w += by)
   {
     const unsigned it = g.vit[w];
@@ -420,7 +424,7 @@ __device__ __forceinline__ void tt_vertex_face(const PgTT &g, const pg::Num<pg::
 
 __device__ __forceinline__ void tt_edge_edge(const PgTT &g, const pg::Num<pg::f64> &N, int first, int by)
 {
-  const int n = min(g.qn[3], g.ecap);
+  const int n = (int)min(g.qn[3], (unsigned long long)g.ecap);
   for (int w = first; w < n; w += by)
   {
     const unsigned it = g.eit[w];
@@ -511,7 +515,7 @@ __device__ __noinline__ double tt_contact(const PgDev &d, const PgTT &g, int f, 
 __global__ void __launch_bounds__(32, 16) k_tt_near(PgDev d, PgTT g, double step)
 {
   const pg::Num<pg::f64> N;
-  const int n = g.qn[0];
+  const int n = (int)min(g.qn[0], (unsigned long long)PG_TT_NEAR);
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
   {
     const PgTTNear e = g.near[w];
@@ -565,7 +569,7 @@ __global__ void __launch_bounds__(32, 16) k_tt_near(PgDev d, PgTT g, double step
   }
   // 5d. the pairs that need every test: triangles that may intersect,
   // degenerate ones, and those whose distances found no room
-  const int nf = g.qn[1];
+  const int nf = (int)g.qn[1];
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nf; w += gridDim.x * blockDim.x)
   {
     const int k = g.full[w], f = g.pf[k], u = g.pu[k];
@@ -878,7 +882,7 @@ void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, double step)
     auto upto = [](int most, long long n) { const int b = nblk(n); return b < most ? b : most; };
     const int bv = upto(bd, 6LL * g.np), be = upto(bd, 9LL * g.np);
     const int tiles = (2 * g.np + PG_TT_TILE - 1) / PG_TT_TILE;
-    cudaMemsetAsync(g.qn, 0, 4 * sizeof(int), s);
+    cudaMemsetAsync(g.qn, 0, 4 * sizeof(*g.qn), s);
     k_tt_judge<<<nblk(g.np), TPB, 0, s>>>(d, g);
     k_tt_distances<<<bv + be, TPB, 0, s>>>(g, bv);
     k_tt_near<<<std::min((g.np + 31) / 32, bn), 32, 0, s>>>(d, g, step);

@@ -11,7 +11,12 @@
 // pgtf::judge), where their results start, a bound on the smallest
 struct PgTTNear { int pair; unsigned mask; int vbase, ebase; float upper, size; };
 #define PG_TT_GEO 28
-#define PG_TT_MOST 0x3fffffff     // pairs a list may hold
+// pairs a list may hold: its entries, three a pair with the room to grow, are
+// numbered by 31 bits.  Distances are numbered by 31 bits with room for a
+// grid's stride above, near pairs by 28 (four name the distance).
+#define PG_TT_MOST 0x2a000000
+#define PG_TT_DISTANCES 0x7f000000
+#define PG_TT_NEAR 0x10000000
 
 // a triangle's box at a search, widened by r and half the skin (rounded
 // outwards), its particle (-1: not of a mesh) and whether it is big
@@ -54,7 +59,7 @@ struct PgTT
   unsigned *vit = nullptr, *eit = nullptr;  // [vcap], [ecap] near pair << 4 | candidate; vit then holds the region
   double *vres = nullptr, *eres = nullptr;  // [.cap][3] squared distance and the closest points' parameters
   int vcap = 0, ecap = 0;
-  int *qn = nullptr;              // [4] near pairs, full pairs, vertex-face and edge-edge distances
+  unsigned long long *qn = nullptr;   // [4] near pairs, full pairs, vertex-face and edge-edge distances
   unsigned char *act = nullptr;   // [cap] in contact
   double *st[3] = {}, *f[3] = {}, *p[3] = {};   // tangential state, force on the finder's particle, point
   // the previous list, pnp pairs (state carried by (finder, partner) at a search)

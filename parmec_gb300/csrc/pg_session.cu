@@ -1784,8 +1784,8 @@ int pg_session_mesh_contact_stats(pg_session *s, int *pairs, int *active)
   *pairs = *active = 0;
   if (!s->d.tt_on || !s->tt.valid) return PG_OK;
   int n[2] = {0, 0};
-  pg_tt_count(s->d, s->tt, s->tt.qn, s->stream);         // (the step's counters are free between steps)
-  TRY(d2h(s, n, s->tt.qn, 2));
+  pg_tt_count(s->d, s->tt, s->tt.moved, s->stream);      // (its flags are free between steps)
+  TRY(d2h(s, n, s->tt.moved, 2));
   CK(cudaStreamSynchronize(s->stream));
   *pairs = n[0];
   *active = n[1];

@@ -52,8 +52,8 @@ int pg_tt_pair_room(PgTT &g, int np, Mem &mem)
   // room for 2 vertex-triangle and 3 edge-edge distances a pair (the spring
   // lattice, whose faces lie parallel, asks for 1.3 and 2.4); pairs beyond
   // it take the whole narrow phase
-  g.vcap = (int)std::min(2LL * cap, 0x7fff0000LL);
-  g.ecap = (int)std::min(3LL * cap, 0x7fff0000LL);
+  g.vcap = (int)std::min(2LL * cap, (long long)PG_TT_DISTANCES);
+  g.ecap = (int)std::min(3LL * cap, (long long)PG_TT_DISTANCES);
   make(g.near, cap); make(g.full, cap);
   make(g.vit, g.vcap); make(g.eit, g.ecap);
   make(g.vres, 3 * (size_t)g.vcap); make(g.eres, 3 * (size_t)g.ecap);

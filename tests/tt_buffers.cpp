@@ -3,7 +3,8 @@
 // that grow with and without a previous list.  No pointer may be left to
 // memory that was given back, no memory given back twice or lost, the room
 // said to be there must be there, the previous list must be whole, and the
-// same call must succeed afterwards.
+// same call must succeed afterwards.  Then the largest list there may be: its
+// arrays must have room for what the kernels number in it, in their types.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -18,11 +19,15 @@ struct FakeMem
 {
   std::map<void *, size_t> live;
   int fail_at = -1, calls = 0;
+  bool pretend = false;                                  // sizes alone
+  size_t total = 0;
   bool fails() { return calls ++ == fail_at; }
   template <class T> int make(T **p, size_t n)
   {
     if (fails()) return -3;
-    void *q = calloc(n ? n : 1, sizeof(T));
+    if (n > ((size_t)1 << 34)) bad ++;                   // a length that went below zero
+    total += n * sizeof(T);
+    void *q = pretend ? (void *)(live.size() * 64 + 64) : calloc(n ? n : 1, sizeof(T));
     live[q] = n * sizeof(T);
     *p = (T *)q;
     return 0;
@@ -118,6 +123,18 @@ int main()
         tried ++;
         if (!failed) break;
       }
+  for (const int np : {0x10000000, 0x10000001, PG_TT_MOST})
+  {
+    FakeMem mem;
+    mem.pretend = true;
+    PgTT g;
+    if (pg_tt_pair_room(g, np, mem)) bad ++;
+    check(g, mem);
+    const long long cap = g.cap, stride = 1 << 22;       // stride: threads of the largest grid
+    bad += cap < np || 2 * cap > 0x7fffffff;             // two entries a pair, in an int
+    bad += g.vcap <= 0 || g.ecap <= 0 || g.vcap + stride > 0x7fffffff || g.ecap + stride > 0x7fffffff;
+    bad += ((PG_TT_NEAR - 1LL) << 4 | 15) > 0xffffffffLL; // a near pair's place and the distance, in 32 bits
+  }
   printf("%ld %ld\n", bad, tried);
   return 0;
 }
