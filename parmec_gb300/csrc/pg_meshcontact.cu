@@ -114,7 +114,10 @@ __global__ void __launch_bounds__(TPB) k_tt_boxes(PgDev d, PgTT g)
   if (__syncthreads_or(moved) && threadIdx.x == 0) g.moved[0] = 1;
 }
 
-// 2. a search: reference vertices, search boxes and cell keys
+// 2. a search: reference vertices, search boxes and cell keys.  The boxes are
+// FP64, as the ones they stand for: single precision would widen them by the
+// distance from the origin (10 mm cubes 1 mm apart had no pair near it, 8,124
+// at 10 km, and too many for a triangle's list at 300 km).
 __global__ void __launch_bounds__(TPB) k_tt_keys(PgDev d, PgTT g)
 {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -123,7 +126,7 @@ __global__ void __launch_bounds__(TPB) k_tt_keys(PgDev d, PgTT g)
   PgTTBox bx;
   bx.owner = -1;
   bx.big = 0;
-  for (int c = 0; c < 3; c ++) bx.lo[c] = bx.hi[c] = 0.0f;
+  for (int c = 0; c < 3; c ++) bx.lo[c] = bx.hi[c] = 0;
   if (mesh_tri(d, t))
   {
     double v[3][3], mid[3];
@@ -137,8 +140,8 @@ __global__ void __launch_bounds__(TPB) k_tt_keys(PgDev d, PgTT g)
       l = l < e ? l : e;
       h = h > e ? h : e;
       mid[c] = 0.5*((l - g.r) + (h + g.r));
-      bx.lo[c] = __double2float_rd(l - w);
-      bx.hi[c] = __double2float_ru(h + w);
+      bx.lo[c] = lo_key(l - w);
+      bx.hi[c] = hi_key(h + w);
     }
     bx.owner = d.triobs[t];
     bx.big = g.big[t];

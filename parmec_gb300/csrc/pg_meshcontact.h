@@ -18,9 +18,9 @@ struct PgTTNear { int pair; unsigned mask; int vbase, ebase; float upper, size; 
 #define PG_TT_DISTANCES 0x7f000000
 #define PG_TT_NEAR 0x10000000
 
-// a triangle's box at a search, widened by r and half the skin (rounded
-// outwards), its particle (-1: not of a mesh) and whether it is big
-struct PgTTBox { float lo[3], hi[3]; int owner, big; };
+// a triangle's box at a search, widened by r and half the skin, in the keys of
+// PgTT.box, its particle (-1: not of a mesh) and whether it is big
+struct PgTTBox { unsigned long long lo[3], hi[3]; int owner, big; };
 
 struct PgTT
 {

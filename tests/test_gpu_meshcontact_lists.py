@@ -76,3 +76,31 @@ def test_refused_list_ends_the_run_and_the_session_goes_on(gpu_lib, oracle_lib):
     mo.dem(400 * DT, DT, interval=1e9, engine=eo)
     assert_bitwise(mg, mo)
     assert eg.mesh_contact_stats() == eo.mesh_contact_stats()
+
+
+@pytest.mark.parametrize("origin", [(0.0, 0.0, 0.0), (3e5, -3e5, 1e4)])
+def test_pile_far_from_the_origin_bitwise(origin, gpu_lib, oracle_lib):
+    """Searches while the upper layer falls, near the origin and where a
+    georeferenced scene lies."""
+    both = pair(lambda: pile(origin))
+    dem(both, 100, first=True)
+    assert dem(both, 300)[1] > 20
+
+
+def test_boxes_far_from_the_origin_find_no_more_pairs(gpu_lib):
+    """A 5 x 5 x 5 stack of 10 mm cubes 1 mm apart, reach 0.2 mm: no pair,
+    wherever it stands."""
+    from parmec_gb300 import mesh
+    from parmec_gb300.engine import GpuEngine
+    from parmec_gb300.model import Model
+    for x in (0.0, 1e4, 3e5):
+        m = Model()
+        mat = m.material(2500.0, 1e9, 0.25)
+        g = np.stack(np.meshgrid(*(np.arange(5),) * 3, indexing="ij"), -1).reshape(-1, 3)
+        mesh.hex_grid(m, x + 0.011 * g, 0.01, mat, 1)
+        m.granular(0, 0, 1e5, 0.3, 0.4)
+        m.mesh_contact(1e-4)
+        eng = GpuEngine()
+        m.dem(2 * DT, DT, interval=1e9, engine=eng)
+        assert eng.mesh_contact_stats() == (0, 0)
+        eng.close()
