@@ -238,7 +238,9 @@ __global__ void __launch_bounds__(TPB) k_tt_find(PgDev d, PgTT g)
     }
     if (cnt > PG_TT_KMAX)
     {
-      if (lane == 0) pgk::set_err(d, PG_ERR_CAPACITY, 40, t, cnt);
+      // partners in the skin alone never end a run: the host searches without
+      if (lane == 0 && g.skin > 0.0) g.moved[0] = 2;
+      else if (lane == 0) pgk::set_err(d, PG_ERR_CAPACITY, 40, t, cnt);
       cnt = PG_TT_KMAX;
     }
   }

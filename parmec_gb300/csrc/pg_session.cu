@@ -1111,7 +1111,7 @@ struct SessionMem
 
 // a new pair list: its pairs, the state of the previous list's, the entry
 // order of the sums.  The host waits twice, for the pair count and for the
-// number of particles with long sums.
+// number of particles with long sums (once more where it drops the skin).
 int tt_search(pg_session *s)
 {
   PgDev &d = s->d;
@@ -1129,9 +1129,19 @@ int tt_search(pg_session *s)
     g.valid = 0;
   }
   if (!g.pnp) CK(cudaMemsetAsync(g.poff, 0, ((size_t)d.trinum + 1) * sizeof(int), s->stream));
-  pg_tt_search(d, g, s->stream);
-  CK(cudaMemcpyAsync(s->tt_host, g.moved, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-  CK(cudaStreamSynchronize(s->stream));
+  for (;;)
+  {
+    pg_tt_search(d, g, s->stream);
+    CK(cudaMemcpyAsync(s->tt_host, g.moved, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    if (s->tt_host[0] != 2) break;
+    // a triangle has more partners than its list holds with those the skin
+    // adds (it is small against the cells, whose size sets the skin where the
+    // radius is smaller still): the boxes alone from here on, found anew when
+    // anything moves
+    g.skin = 0.0;
+    CK(cudaMemsetAsync(g.moved, 0, sizeof(int), s->stream));
+  }
   const int np = s->tt_host[1];
   if (np > g.most) return PG_ERR_CAPACITY;
   if (np > g.cap || !g.cap) TRY(pg_tt_pair_room(g, np, mem));

@@ -104,3 +104,18 @@ def test_boxes_far_from_the_origin_find_no_more_pairs(gpu_lib):
         m.dem(2 * DT, DT, interval=1e9, engine=eng)
         assert eng.mesh_contact_stats() == (0, 0)
         eng.close()
+
+
+def test_more_partners_in_the_skin_than_a_list_holds(gpu_lib, oracle_lib):
+    """Cubes in a grid of cells a hundred times their size: the skin, a part of
+    the cell, reaches more triangles than a list holds, the swept boxes do not."""
+    from parmec_gb300 import abi
+    from parmec_gb300.mesh import mesh_contact_grid
+    both = (mg, eg), _ = pair(lambda: pile(layers=3))
+    eg.attach(mg)
+    mg.engine, mg._dirty = eg, False
+    cell, big = mesh_contact_grid(mg)
+    assert 27 * 12 - 12 > 256 and 0.5 * cell > 0.0021
+    assert eg.lib.pg_session_mesh_contact(eg.sess, 1e-3, 100.0 * cell, big.ctypes.data) == abi.PG_OK
+    dem(both, 30, first=True)
+    assert dem(both, 100)[1] > 20
