@@ -149,11 +149,7 @@ __global__ void __launch_bounds__(TPB) k_tt_keys(PgDev d, PgTT g)
     else
     {
       int ix[3];
-      for (int c = 0; c < 3; c ++)
-      {
-        const double q = floor((mid[c] - g.org[c]) / g.h);
-        ix[c] = q < 0.0 ? 0 : (q > (double)(g.dim[c]-1) ? g.dim[c]-1 : (int)q);
-      }
+      for (int c = 0; c < 3; c ++) ix[c] = pgtf::grid_cell(mid[c], g.org[c], g.h, g.dim[c]);
       key = (unsigned)((ix[2]*g.dim[1] + ix[1])*g.dim[0] + ix[0]);
     }
     g.cell[t] = (int)key;

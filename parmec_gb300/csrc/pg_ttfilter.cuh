@@ -168,6 +168,15 @@ PG_TF int judge(const float a[3][3], const float b[3][3], float ea, float eb, fl
   return m ? NEAR : FULL;
 }
 
+// grid cell of coordinate x along an axis of `dim` cells; beyond them, the
+// nearest.  A NaN (a scene that has blown up) takes cell 0: converted to an
+// integer it would name a cell outside of the table.
+PG_TF int grid_cell(double x, double org, double h, int dim)
+{
+  const double q = (x - org) / h;
+  return q >= (double)dim ? dim - 1 : q >= 1.0 ? (int)q : 0;
+}
+
 // Float copies of a triangle's vertices relative to org, and the bound on
 // their error: infinite when the triangle is degenerate (a height below 1e-4
 // of its longest edge, tested in FP64) or not finite

@@ -14,27 +14,33 @@ pytestmark = pytest.mark.gpu
 DT = 1e-5
 
 
-def pile(origin=(0.0, 0.0, 0.0), layers=2, side=3, seed=3, radius=1e-3):
-    """Layers of 10 mm cubes on a fixed plate, 0.1 mm outside the reach of one
-    another, the upper ones turning; an upper layer falls at 1 m/s."""
+def pile(origin=(0.0, 0.0, 0.0), layers=2, side=3, seed=3, radius=1e-3, first=0.0021, gap=0.0021):
+    """Layers of 10 mm cubes over a fixed plate (`first` and `gap` above what
+    lies below, 0.1 mm outside the reach), the upper ones turning and falling
+    at 1 m/s.  The pile
+    is made near zero and moved to its origin (the volume integrals of a MESH
+    lose a small body's inertia far away)."""
     from parmec_gb300 import mesh
     from parmec_gb300.model import Model
     rng = np.random.default_rng(seed)
     m = Model()
     mat = m.material(2500.0, 1e9, 0.25)
-    o = np.asarray(origin, dtype=np.float64)
-    lo, hi = o - (0.01, 0.01, 0.005), o + (0.014 * side, 0.014 * side, 0.0)
+    lo, hi = (-0.01, -0.01, -0.005), (0.014 * side, 0.014 * side, 0.0)
     c = [(x, y, z) for z in (lo[2], hi[2]) for x, y in ((lo[0], lo[1]), (hi[0], lo[1]), (hi[0], hi[1]), (lo[0], hi[1]))]
     plate = m.mesh([v for p in c for v in p], [8, 0, 1, 2, 3, 4, 5, 6, 7, mat], mat, 2)
     m.prescribe_motion(plate, linear=lambda t: (0.0, 0.0, 0.0), angular=lambda t: (0.0, 0.0, 0.0), kind="vv")
-    org = [(0.014 * i + 1e-3 * rng.uniform(-1, 1), 0.014 * j, 0.0021 + 0.0121 * k)
+    org = [(0.014 * i + 1e-3 * rng.uniform(-1, 1), 0.014 * j, first + (0.01 + gap) * k)
            for k in range(layers) for i in range(side) for j in range(side)]
-    parts = mesh.hex_grid(m, o + np.array(org), 0.01, mat, 1)
+    parts = mesh.hex_grid(m, np.array(org), 0.01, mat, 1)
     for p in parts[side * side:]:
         m.velocity(int(p), linear=(0.0, 0.0, -1.0), angular=tuple(float(x) for x in rng.normal(0.0, 2.0, size=3)))
-    m.granular(0, 0, 1e5, 0.3, 0.4)
+    m.granular(0, 0, 1e4, 0.3, 0.4)
     m.set_gravity(0.0, 0.0, -9.81)
     m.mesh_contact(radius)
+    for c in range(3):
+        m.P.position[[c, 3 + c], :m.parnum] += origin[c]
+        m.N.nodes[[c, 3 + c], :m.nodnum] += origin[c]
+        m.Tr.tri[[c, 3 + c, 6 + c], :m.trinum] += origin[c]
     return m
 
 
