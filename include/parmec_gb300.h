@@ -317,11 +317,13 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
  * restore the whole arrays.  The next step rebuilds the candidate lists. */
 int pg_session_set_live(pg_session *s, int particles, int spheres, int triangles);
 
-/* Self-test of the mesh contact's limit: pair lists of more than 'pairs' pairs
- * end a run with PG_ERR_CAPACITY (0: the limit of the list itself).  The steps
- * before the one that ended the run are done, that one is not, and the contacts
- * keep their state: with more room, or memory, the session runs on from there. */
-int pg_session_mesh_contact_room(pg_session *s, int pairs);
+/* Self-test of the mesh contact's limits (0: the list's own).  Lists of more
+ * than 'pairs' pairs end a run with PG_ERR_CAPACITY: the steps before the one
+ * that ended it are done, that one is not, and the contacts keep their state;
+ * with more room, or memory, the session runs on from there.  'vertex' and
+ * 'edge' bound the vertex-face and edge-edge distances of a step's filter;
+ * pairs beyond them take the whole narrow phase, with the same results. */
+int pg_session_mesh_contact_room(pg_session *s, int pairs, int vertex, int edge);
 
 /* Triangle pairs whose boxes overlapped in the last step, and those in contact. */
 int pg_session_mesh_contact_stats(pg_session *s, int *pairs, int *active);

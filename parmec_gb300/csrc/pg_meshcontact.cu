@@ -875,8 +875,11 @@ void pg_tt_chunk_map(PgTT &g, cudaStream_t s)
   if (g.nbig > 0) k_tt_chmap<<<g.nbig, TPB, 0, s>>>(g);
 }
 
-void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, double step)
+void pg_tt_forces(const PgDev &d, const PgTT &list, cudaStream_t s, double step)
 {
+  PgTT g = list;
+  g.vcap = std::min(g.vcap, g.vmost);
+  g.ecap = std::min(g.ecap, g.emost);
   if (g.np > 0)
   {
     static const int bd = resident_blocks(k_tt_distances), bn = resident_blocks(k_tt_near, 32);

@@ -59,6 +59,7 @@ struct PgTT
   unsigned *vit = nullptr, *eit = nullptr;  // [vcap], [ecap] near pair << 4 | candidate; vit then holds the region
   double *vres = nullptr, *eres = nullptr;  // [.cap][3] squared distance and the closest points' parameters
   int vcap = 0, ecap = 0;
+  int vmost = PG_TT_DISTANCES, emost = PG_TT_DISTANCES;   // not all of the room is taken (a self-test)
   unsigned long long *qn = nullptr;   // [4] near pairs, full pairs, vertex-face and edge-edge distances
   unsigned char *act = nullptr;   // [cap] in contact
   double *st[3] = {}, *f[3] = {}, *p[3] = {};   // tangential state, force on the finder's particle, point
@@ -91,7 +92,7 @@ void pg_tt_prepare(const PgDev &d, PgTT &g, cudaStream_t s);              // box
 void pg_tt_search(const PgDev &d, PgTT &g, cudaStream_t s);               // pairs of each triangle; total in moved[1]
 void pg_tt_list(const PgDev &d, PgTT &g, cudaStream_t s);                 // the list of g.np pairs and its entry order
 void pg_tt_chunk_map(PgTT &g, cudaStream_t s);                            // chunks of the big particles
-void pg_tt_forces(const PgDev &d, PgTT &g, cudaStream_t s, double step);  // contacts and per-particle sums
+void pg_tt_forces(const PgDev &d, const PgTT &g, cudaStream_t s, double step);  // contacts and per-particle sums
 void pg_tt_count(const PgDev &d, const PgTT &g, int *out2, cudaStream_t s);   // overlapping and active pairs
 int pg_tt_search_kernels(const PgTT &g, int trinum);
 int pg_tt_step_kernels(const PgTT &g);

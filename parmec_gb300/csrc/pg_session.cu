@@ -1751,10 +1751,13 @@ int pg_session_mesh_contact(pg_session *s, double radius, double cell, const uns
   return PG_OK;
 }
 
-int pg_session_mesh_contact_room(pg_session *s, int pairs)
+int pg_session_mesh_contact_room(pg_session *s, int pairs, int vertex, int edge)
 {
-  if (!s || pairs < 0) return PG_ERR_ARGUMENT;
-  s->tt.most = pairs > 0 ? std::min(pairs, PG_TT_MOST) : PG_TT_MOST;
+  if (!s || pairs < 0 || vertex < 0 || edge < 0) return PG_ERR_ARGUMENT;
+  auto most = [](int asked, int limit) { return asked > 0 ? std::min(asked, limit) : limit; };
+  s->tt.most = most(pairs, PG_TT_MOST);
+  s->tt.vmost = most(vertex, PG_TT_DISTANCES);
+  s->tt.emost = most(edge, PG_TT_DISTANCES);
   return PG_OK;
 }
 

@@ -67,14 +67,14 @@ def test_refused_list_ends_the_run_and_the_session_goes_on(gpu_lib, oracle_lib):
     assert dem(both, 300, first=True)[1] > 0
     tabs = driver.StepTables(mg, [mg.curtime + k * DT for k in range(400)], DT, [1e9, 1e9], [None, None], [-1, -1])
     done0 = eg.global_step()
-    assert eg.lib.pg_session_mesh_contact_room(eg.sess, 1) == abi.PG_OK
+    assert eg.lib.pg_session_mesh_contact_room(eg.sess, 1, 0, 0) == abi.PG_OK
     tab = tabs.ctab(0, 400)
     assert eg.lib.pg_session_run(eg.sess, ctypes.byref(tab), DT) == abi.PG_ERR_CAPACITY
     done = eg.global_step() - done0
     assert 0 < done < 400
     assert eg.lib.pg_session_run(eg.sess, ctypes.byref(tab), DT) == abi.PG_ERR_CAPACITY
     assert eg.global_step() == done0 + done
-    assert eg.lib.pg_session_mesh_contact_room(eg.sess, 0) == abi.PG_OK
+    assert eg.lib.pg_session_mesh_contact_room(eg.sess, 0, 0, 0) == abi.PG_OK
     tab = tabs.ctab(done, 400)
     assert eg.lib.pg_session_run(eg.sess, ctypes.byref(tab), DT) == abi.PG_OK
     eg.download()
@@ -125,3 +125,25 @@ def test_more_partners_in_the_skin_than_a_list_holds(gpu_lib, oracle_lib):
     assert eg.lib.pg_session_mesh_contact(eg.sess, 1e-3, 100.0 * cell, big.ctypes.data) == abi.PG_OK
     dem(both, 30, first=True)
     assert dem(both, 100)[1] > 20
+
+
+def test_pair_arrays_grow_with_contacts_carried(gpu_lib, oracle_lib):
+    """36 cubes resting on the plate when as many fall on them: the list
+    outgrows its arrays while contacts hold tangential state."""
+    both = pair(lambda: pile(side=6, first=0.0019, gap=0.0025))
+    few = dem(both, 20, first=True)
+    many = dem(both, 60)
+    assert few[1] >= 36 and many[0] > 1.5 * (1.5 * few[0] + 1024)
+
+
+@pytest.mark.parametrize("vertex,edge", [(37, 0), (0, 37), (37, 37), (1, 1)])
+def test_distances_without_room_bitwise(vertex, edge, gpu_lib, oracle_lib):
+    """Near pairs that find no room for their distances, in either list or in
+    both, take the whole narrow phase: the same bits."""
+    from parmec_gb300 import abi
+    both = (mg, eg), _ = pair(pile)
+    eg.attach(mg)
+    mg.engine, mg._dirty = eg, False
+    assert eg.lib.pg_session_mesh_contact_room(eg.sess, 0, vertex, edge) == abi.PG_OK
+    dem(both, 60, first=True)
+    assert dem(both, 100)[1] > 37
