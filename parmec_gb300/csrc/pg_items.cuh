@@ -424,6 +424,11 @@ __device__ __forceinline__ float rb_tolerance(const PgDev &d, const float *c)
 }
 __device__ __forceinline__ bool rb_exact(const PgDev &d, float tol) { return !(tol < 0.02f * (float)d.skin); }
 
+// whether the float distance, squared, keeps a candidate: where the FP64 test
+// follows, unless it is certainly beyond; else only where it is within, so that
+// a NaN sphere is nobody's candidate either way
+__device__ __forceinline__ bool rb_near(float f2, float l2, bool exact) { return exact ? !(f2 >= l2) : f2 < l2; }
+
 // The new list of sphere i with the flags and tangential state of the partners
 // it keeps (both lists in partner order).  The entries before the first
 // difference stay where they are; only the old ones after it are held while
@@ -555,7 +560,7 @@ __device__ __forceinline__ void rb_verlet_item(const PgDev &d, int i, bool valid
         {
           const float f0 = cif[0] - o[q].x, f1 = cif[1] - o[q].y, f2 = cif[2] - o[q].z;
           const float lf = rsf + o[q].w + tol;
-          if (!(b[q] + t < e[q] && p[q].x > pi) || f0*f0 + f1*f1 + f2*f2 >= lf*lf) continue;
+          if (!(b[q] + t < e[q] && p[q].x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, exact))) continue;
           const int j = p[q].y;
           if (exact)
           {
@@ -721,7 +726,7 @@ __device__ __forceinline__ void rb_verlet_group(const PgDev &d, int i, bool vali
           const float f0 = cif[0] - o.x, f1 = cif[1] - o.y, f2 = cif[2] - o.z, lf = rsf + o.w + tol;
           const int2 p = d.pfs[s];
           j = p.y;
-          hit = p.x > pi && !(f0*f0 + f1*f1 + f2*f2 >= lf*lf);
+          hit = p.x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, exact);
           if (hit && exact)
           {
             const double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
