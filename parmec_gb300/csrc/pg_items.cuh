@@ -142,7 +142,7 @@ __device__ __forceinline__ void cell_keys_item(int i, const double *x, const dou
 // product by the reciprocal of a cell 2^-40 larger instead of three divisions
 // (26 FP64 instructions of 42 a sphere): two spheres within a cell's length
 // still lie in adjacent cells, the products being off by less than 2^-43, and
-// the exact tests of the search decide every candidate.
+// the distance tests of the search keep every candidate.
 __device__ __forceinline__ double rb_cell_inverse(const PgDev &d) { return (1.0 - 0x1p-40) / d.cell; }
 
 __device__ __forceinline__ void rb_key_item(const PgDev &d, int i, double inv)
@@ -496,151 +496,158 @@ __device__ __forceinline__ void rb_verlet_item(const PgDev &d, int i, bool valid
     sc = d.escene[i];
   }
   const bool live = sc >= 0 && d.sactive[sc] != 0;
-  if (live)
-  {
-    const unsigned prefix = (unsigned)sc << (3 * d.bits);
-    // the sphere's cell, from the key the key phase computed, instead of
-    // three FP64 divisions again
-    const unsigned cm = d.ekey[i] & ((1u << (3 * d.bits)) - 1u);
-    const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
-    // FP32 prefilter: a neighbour is skipped only when its float distance
-    // exceeds the float limit by tol, more than the rounding of the float
-    // copies and of the float arithmetic can account for, so the FP64 test
-    // below still decides every candidate (the lists are those of the FP64
-    // test alone).  Float coordinates carry at most 2^-24 |c| of error;
-    // tol = 2^-20 (max|c_i| + 2 cell) bounds the distance error 16 times over
-    // for partners within a cell.
-    const float cif[3] = {(float)c[0], (float)c[1], (float)c[2]};
-    const float rsf = (float)ri + (float)d.skin;
-    const float tol = rb_tolerance(d, cif);
-    // where tol is small against the skin the float test's few extra
-    // candidates cost less than the FP64 test, which holds the warp's FP64
-    // pipe for every lane's neighbour in turn (a candidate beyond the limit
-    // is never in contact: the lists decide nothing)
-    const bool exact = rb_exact(d, tol);
-    // a layer of nine cells at a time: their ranges are loaded together, then
-    // the first sphere of each, the second of each, ... (the order in which
-    // candidates are found plays no part).  Every load is issued whether its
-    // cell holds a sphere or not, so that nine are in flight where one cell
-    // after another was a chain of two to four latencies (476 -> 349 us of a
-    // rebuild of 1,270,000 shaken spheres, at one to two spheres a cell)
-    #pragma unroll 1
-    for (int dz = -1; dz <= 1; dz ++)
-    {
-      int b[9], e[9], m = 0;
-      const int z = u[2] + dz;
-      const unsigned mz = spread3((unsigned)z) << 2;
-      #pragma unroll
-      for (int q = 0; q < 9; q ++)
-      {
-        const int x = u[0] + q % 3 - 1, y = u[1] + q / 3 - 1;
-        const bool in = x >= 0 && y >= 0 && z >= 0 && x < d.dim[0] && y < d.dim[1] && z < d.dim[2];
-        const unsigned key = prefix | (in ? spread3((unsigned)x) | (spread3((unsigned)y) << 1) | mz : cm);
-        const int cb = d.cstart[key], ce = d.cend[key];
-        b[q] = in ? cb : 0;
-        e[q] = in ? ce : 0;
-      }
-      #pragma unroll
-      for (int q = 0; q < 9; q ++) m = max(m, e[q] - b[q]);
-      #pragma unroll 1
-      for (int t = 0; t < m; t ++)
-      {
-        // (an entry beyond its cell's range reads the first of all)
-        float4 o[9];
-        int2 p[9];
-        #pragma unroll
-        for (int q = 0; q < 9; q ++)
-        {
-          const int s = b[q] + t < e[q] ? b[q] + t : 0;
-          o[q] = d.cfs[s];
-          p[q] = d.pfs[s];
-        }
-        #pragma unroll
-        for (int q = 0; q < 9; q ++)
-        {
-          const float f0 = cif[0] - o[q].x, f1 = cif[1] - o[q].y, f2 = cif[2] - o[q].z;
-          const float lf = rsf + o[q].w + tol;
-          if (!(b[q] + t < e[q] && p[q].x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, exact))) continue;
-          const int j = p[q].y;
-          if (exact)
-          {
-            double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
-            double lim = ri + d.radii[0][j] + d.skin;
-            if (!(q0*q0 + q1*q1 + q2*q2 < lim*lim)) continue;
-          }
-          if (n < d.kn) codes[n ++] = j;
-          else { over = true; nover ++; }
-        }
-      }
-    }
-    // insertion sort of the sphere partners
-    for (int a = 1; a < n; a ++)
-    {
-      int v = codes[a], b = a - 1;
-      while (b >= 0 && codes[b] > v) { codes[b+1] = codes[b]; b --; }
-      codes[b+1] = v;
-    }
-  }
-  // triangles of the sphere's scene within r + skin (AABB in float, then the
-  // true closest-point distance), in triangle order
-  const float inf = __int_as_float(0x7f800000);
-  float clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
-  if (live)
-  {
-    const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
-    for (int k = 0; k < 3; k ++) { clo[k] = __double2float_rd(c[k]) - rr; chi[k] = __double2float_ru(c[k]) + rr; }
-  }
-  const int T = d.trinum;
-  auto box_apart = [&](int t, const float *lo, const float *hi) {
-    return d.tbox[t] > hi[0] || d.tbox[(size_t)3 * T + t] < lo[0] ||
-           d.tbox[(size_t)T + t] > hi[1] || d.tbox[(size_t)4 * T + t] < lo[1] ||
-           d.tbox[(size_t)2 * T + t] > hi[2] || d.tbox[(size_t)5 * T + t] < lo[2];
-  };
-  auto try_triangle = [&](int t) {
-    if (box_apart(t, clo, chi)) return;
-    double A[3], B[3], C[3], pnt[3], nrm[3];
-    for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
-    // the candidate test uses the true closest point: the reference's region
-    // formula can only report a larger distance, so this set stays a superset
-    double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
-    if (!(depth > -d.skin) && !(depth != depth)) return;
-    ntri ++;
-    if (n < d.kn) codes[n ++] = -(t + 1);
-    else { over = true; nover ++; }
-  };
-  // when every live lane of the warp is in one scene, the warp tests 32
-  // triangles at a time against the box of all its spheres and each lane
-  // then tests its own box against the triangles that box reached
+  const float cif[3] = {(float)c[0], (float)c[1], (float)c[2]}, tol = rb_tolerance(d, cif);
+  // where tol is small against the skin the float test's few extra
+  // candidates cost less than the FP64 test, which holds the warp's FP64
+  // pipe for every lane's neighbour in turn (a candidate beyond the limit
+  // is never in contact: the lists decide nothing).  A list that the extra
+  // candidates fill is made again with the FP64 test.
+  bool exact = rb_exact(d, tol);
   const unsigned full = 0xffffffffu, lm = __ballot_sync(full, live);
   if (!lm) return;
   const int lane = threadIdx.x & 31, sc0 = __shfl_sync(full, sc, __ffs(lm) - 1);
-  if (__all_sync(full, !live || sc == sc0))
+  #pragma unroll 1
+  for (;;)
   {
-    float wlo[3], whi[3];
-    for (int k = 0; k < 3; k ++)
+    n = nover = ntri = 0;
+    over = false;
+    if (live)
     {
-      wlo[k] = clo[k]; whi[k] = chi[k];
-      for (int o = 16; o > 0; o >>= 1)
+      const unsigned prefix = (unsigned)sc << (3 * d.bits);
+      // the sphere's cell, from the key the key phase computed, instead of
+      // three FP64 divisions again
+      const unsigned cm = d.ekey[i] & ((1u << (3 * d.bits)) - 1u);
+      const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
+      // FP32 prefilter: a neighbour is skipped only when its float distance
+      // exceeds the float limit by tol, more than the rounding of the float
+      // copies and of the float arithmetic can account for, so no candidate of
+      // the FP64 test is missed.  Float coordinates carry at most 2^-24 |c| of error;
+      // tol = 2^-20 (max|c_i| + 2 cell) bounds the distance error 16 times over
+      // for partners within a cell.
+      const float rsf = (float)ri + (float)d.skin;
+      // a layer of nine cells at a time: their ranges are loaded together, then
+      // the first sphere of each, the second of each, ... (the order in which
+      // candidates are found plays no part).  Every load is issued whether its
+      // cell holds a sphere or not, so that nine are in flight where one cell
+      // after another was a chain of two to four latencies (476 -> 349 us of a
+      // rebuild of 1,270,000 shaken spheres, at one to two spheres a cell)
+      #pragma unroll 1
+      for (int dz = -1; dz <= 1; dz ++)
       {
-        wlo[k] = fminf(wlo[k], __shfl_xor_sync(full, wlo[k], o));
-        whi[k] = fmaxf(whi[k], __shfl_xor_sync(full, whi[k], o));
+        int b[9], e[9], m = 0;
+        const int z = u[2] + dz;
+        const unsigned mz = spread3((unsigned)z) << 2;
+        #pragma unroll
+        for (int q = 0; q < 9; q ++)
+        {
+          const int x = u[0] + q % 3 - 1, y = u[1] + q / 3 - 1;
+          const bool in = x >= 0 && y >= 0 && z >= 0 && x < d.dim[0] && y < d.dim[1] && z < d.dim[2];
+          const unsigned key = prefix | (in ? spread3((unsigned)x) | (spread3((unsigned)y) << 1) | mz : cm);
+          const int cb = d.cstart[key], ce = d.cend[key];
+          b[q] = in ? cb : 0;
+          e[q] = in ? ce : 0;
+        }
+        #pragma unroll
+        for (int q = 0; q < 9; q ++) m = max(m, e[q] - b[q]);
+        #pragma unroll 1
+        for (int t = 0; t < m; t ++)
+        {
+          // (an entry beyond its cell's range reads the first of all)
+          float4 o[9];
+          int2 p[9];
+          #pragma unroll
+          for (int q = 0; q < 9; q ++)
+          {
+            const int s = b[q] + t < e[q] ? b[q] + t : 0;
+            o[q] = d.cfs[s];
+            p[q] = d.pfs[s];
+          }
+          #pragma unroll
+          for (int q = 0; q < 9; q ++)
+          {
+            const float f0 = cif[0] - o[q].x, f1 = cif[1] - o[q].y, f2 = cif[2] - o[q].z;
+            const float lf = rsf + o[q].w + tol;
+            if (!(b[q] + t < e[q] && p[q].x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, exact))) continue;
+            const int j = p[q].y;
+            if (exact)
+            {
+              double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
+              double lim = ri + d.radii[0][j] + d.skin;
+              if (!(q0*q0 + q1*q1 + q2*q2 < lim*lim)) continue;
+            }
+            if (n < d.kn) codes[n ++] = j;
+            else { over = true; nover ++; }
+          }
+        }
+      }
+      // insertion sort of the sphere partners
+      for (int a = 1; a < n; a ++)
+      {
+        int v = codes[a], b = a - 1;
+        while (b >= 0 && codes[b] > v) { codes[b+1] = codes[b]; b --; }
+        codes[b+1] = v;
       }
     }
-    const int tb = d.stbeg[sc0], te = d.stend[sc0];
-    for (int t0 = tb; t0 < te; t0 += 32)
+    // triangles of the sphere's scene within r + skin (AABB in float, then the
+    // true closest-point distance), in triangle order
+    const float inf = __int_as_float(0x7f800000);
+    float clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
+    if (live)
     {
-      const int t = t0 + lane;
-      unsigned hm = __ballot_sync(full, t < te && !box_apart(t, wlo, whi));
-      while (hm)
+      const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
+      for (int k = 0; k < 3; k ++) { clo[k] = __double2float_rd(c[k]) - rr; chi[k] = __double2float_ru(c[k]) + rr; }
+    }
+    const int T = d.trinum;
+    auto box_apart = [&](int t, const float *lo, const float *hi) {
+      return d.tbox[t] > hi[0] || d.tbox[(size_t)3 * T + t] < lo[0] ||
+             d.tbox[(size_t)T + t] > hi[1] || d.tbox[(size_t)4 * T + t] < lo[1] ||
+             d.tbox[(size_t)2 * T + t] > hi[2] || d.tbox[(size_t)5 * T + t] < lo[2];
+    };
+    auto try_triangle = [&](int t) {
+      if (box_apart(t, clo, chi)) return;
+      double A[3], B[3], C[3], pnt[3], nrm[3];
+      for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
+      // the candidate test uses the true closest point: the reference's region
+      // formula can only report a larger distance, so this set stays a superset
+      double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
+      if (!(depth > -d.skin) && !(depth != depth)) return;
+      ntri ++;
+      if (n < d.kn) codes[n ++] = -(t + 1);
+      else { over = true; nover ++; }
+    };
+    // when every live lane of the warp is in one scene, the warp tests 32
+    // triangles at a time against the box of all its spheres and each lane
+    // then tests its own box against the triangles that box reached
+    if (__all_sync(full, !live || sc == sc0))
+    {
+      float wlo[3], whi[3];
+      for (int k = 0; k < 3; k ++)
       {
-        const int tt = t0 + __ffs(hm) - 1;
-        hm &= hm - 1;
-        if (live) try_triangle(tt);
+        wlo[k] = clo[k]; whi[k] = chi[k];
+        for (int o = 16; o > 0; o >>= 1)
+        {
+          wlo[k] = fminf(wlo[k], __shfl_xor_sync(full, wlo[k], o));
+          whi[k] = fmaxf(whi[k], __shfl_xor_sync(full, whi[k], o));
+        }
+      }
+      const int tb = d.stbeg[sc0], te = d.stend[sc0];
+      for (int t0 = tb; t0 < te; t0 += 32)
+      {
+        const int t = t0 + lane;
+        unsigned hm = __ballot_sync(full, t < te && !box_apart(t, wlo, whi));
+        while (hm)
+        {
+          const int tt = t0 + __ffs(hm) - 1;
+          hm &= hm - 1;
+          if (live) try_triangle(tt);
+        }
       }
     }
+    else if (live)
+      for (int t = d.stbeg[sc]; t < d.stend[sc]; t ++) try_triangle(t);
+    if (!__any_sync(full, over && !exact)) break;
+    exact = true;
   }
-  else if (live)
-    for (int t = d.stbeg[sc]; t < d.stend[sc]; t ++) try_triangle(t);
   // one atomic per warp for the largest list and triangle counts
   {
     const int cmax = __reduce_max_sync(full, live ? n + nover : 0);
@@ -684,100 +691,109 @@ __device__ __forceinline__ void rb_verlet_group(const PgDev &d, int i, bool vali
   }
   const bool live = sc >= 0 && d.sactive[sc] != 0;
   const int kn = d.kn;
-  int n = 0;                                             // entries found (the group's lanes agree)
+  const float cif[3] = {(float)c[0], (float)c[1], (float)c[2]}, tol = rb_tolerance(d, cif);
+  bool exact = rb_exact(d, tol);
+  int n = 0, before_t = 0;                               // entries found, spheres of them (the group's lanes agree)
+  int v[W], rank[W];
   auto append = [&](bool hit, int code) {
     const unsigned m = __ballot_sync(all, hit);
     const int at = n + __popc(m & before);
     if (hit && at < kn) codes[at] = code;
     n += __popc(m & group);
   };
+  #pragma unroll 1
+  for (;;)
   {
-    const unsigned prefix = (unsigned)sc << (3 * d.bits);
-    const unsigned cm = live ? d.ekey[i] & ((1u << (3 * d.bits)) - 1u) : 0u;
-    const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
-    const float cif[3] = {(float)c[0], (float)c[1], (float)c[2]};
-    const float rsf = (float)ri + (float)d.skin, tol = rb_tolerance(d, cif);
-    const bool exact = rb_exact(d, tol);
-    int b[(27 + RB_GROUP - 1) / RB_GROUP], e[(27 + RB_GROUP - 1) / RB_GROUP];
-    #pragma unroll
-    for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
+    n = 0;
     {
-      const int k = l + RB_GROUP * q, x = u[0] + k % 3 - 1, y = u[1] + k / 3 % 3 - 1, z = u[2] + k / 9 - 1;
-      b[q] = e[q] = 0;
-      if (live && k < 27 && x >= 0 && y >= 0 && z >= 0 && x < d.dim[0] && y < d.dim[1] && z < d.dim[2])
+      const unsigned prefix = (unsigned)sc << (3 * d.bits);
+      const unsigned cm = live ? d.ekey[i] & ((1u << (3 * d.bits)) - 1u) : 0u;
+      const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
+      const float rsf = (float)ri + (float)d.skin;
+      int b[(27 + RB_GROUP - 1) / RB_GROUP], e[(27 + RB_GROUP - 1) / RB_GROUP];
+      #pragma unroll
+      for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
       {
-        const unsigned key = prefix | morton(x, y, z);
-        b[q] = d.cstart[key];
-        e[q] = d.cend[key];
-      }
-    }
-    #pragma unroll
-    for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
-    {
-      const int m = __reduce_max_sync(all, e[q] - b[q]);
-      for (int t = 0; t < m; t ++)
-      {
-        const int s = b[q] + t;
-        bool hit = s < e[q];
-        int j = 0;
-        if (hit)
+        const int k = l + RB_GROUP * q, x = u[0] + k % 3 - 1, y = u[1] + k / 3 % 3 - 1, z = u[2] + k / 9 - 1;
+        b[q] = e[q] = 0;
+        if (live && k < 27 && x >= 0 && y >= 0 && z >= 0 && x < d.dim[0] && y < d.dim[1] && z < d.dim[2])
         {
-          const float4 o = d.cfs[s];
-          const float f0 = cif[0] - o.x, f1 = cif[1] - o.y, f2 = cif[2] - o.z, lf = rsf + o.w + tol;
-          const int2 p = d.pfs[s];
-          j = p.y;
-          hit = p.x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, exact);
-          if (hit && exact)
-          {
-            const double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
-            const double lim = ri + d.radii[0][j] + d.skin;
-            hit = q0*q0 + q1*q1 + q2*q2 < lim*lim;
-          }
+          const unsigned key = prefix | morton(x, y, z);
+          b[q] = d.cstart[key];
+          e[q] = d.cend[key];
         }
-        append(hit, j);
+      }
+      #pragma unroll
+      for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
+      {
+        const int m = __reduce_max_sync(all, e[q] - b[q]);
+        for (int t = 0; t < m; t ++)
+        {
+          const int s = b[q] + t;
+          bool hit = s < e[q];
+          int j = 0;
+          if (hit)
+          {
+            const float4 o = d.cfs[s];
+            const float f0 = cif[0] - o.x, f1 = cif[1] - o.y, f2 = cif[2] - o.z, lf = rsf + o.w + tol;
+            const int2 p = d.pfs[s];
+            j = p.y;
+            hit = p.x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, exact);
+            if (hit && exact)
+            {
+              const double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
+              const double lim = ri + d.radii[0][j] + d.skin;
+              hit = q0*q0 + q1*q1 + q2*q2 < lim*lim;
+            }
+          }
+          append(hit, j);
+        }
       }
     }
-  }
-  // the sphere partners in index order
-  __syncwarp();
-  const int ns = n < kn ? n : kn;
-  int v[W], rank[W];
-  #pragma unroll
-  for (int q = 0; q < W; q ++)
-  {
-    const int a = l + RB_GROUP * q;
-    v[q] = a < ns ? codes[a] : 0;
-    rank[q] = 0;
-    if (a < ns) for (int o = 0; o < ns; o ++) rank[q] += codes[o] < v[q];
-  }
-  __syncwarp();
-  #pragma unroll
-  for (int q = 0; q < W; q ++) if (l + RB_GROUP * q < ns) codes[rank[q]] = v[q];
-  // triangles of the sphere's scene, in triangle order
-  const float inf = __int_as_float(0x7f800000);
-  float clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
-  if (live)
-  {
-    const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
-    for (int k = 0; k < 3; k ++) { clo[k] = __double2float_rd(c[k]) - rr; chi[k] = __double2float_ru(c[k]) + rr; }
-  }
-  const int T = d.trinum;
-  auto near = [&](int t) {
-    if (d.tbox[t] > chi[0] || d.tbox[(size_t)3 * T + t] < clo[0] ||
-        d.tbox[(size_t)T + t] > chi[1] || d.tbox[(size_t)4 * T + t] < clo[1] ||
-        d.tbox[(size_t)2 * T + t] > chi[2] || d.tbox[(size_t)5 * T + t] < clo[2]) return false;
-    double A[3], B[3], C[3], pnt[3], nrm[3];
-    for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
-    const double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
-    return depth > -d.skin || depth != depth;
-  };
-  const int tb = live ? d.stbeg[sc] : 0, te = live ? d.stend[sc] : 0;
-  const int before_t = n;
-  const int most = __reduce_max_sync(all, te - tb);
-  for (int t0 = 0; t0 < most; t0 += RB_GROUP)
-  {
-    const int t = tb + t0 + l;
-    append(t < te && near(t), -(t + 1));
+    // the sphere partners in index order
+    __syncwarp();
+    const int ns = n < kn ? n : kn;
+    #pragma unroll
+    for (int q = 0; q < W; q ++)
+    {
+      const int a = l + RB_GROUP * q;
+      v[q] = a < ns ? codes[a] : 0;
+      rank[q] = 0;
+      if (a < ns) for (int o = 0; o < ns; o ++) rank[q] += codes[o] < v[q];
+    }
+    __syncwarp();
+    #pragma unroll
+    for (int q = 0; q < W; q ++) if (l + RB_GROUP * q < ns) codes[rank[q]] = v[q];
+    // triangles of the sphere's scene, in triangle order
+    const float inf = __int_as_float(0x7f800000);
+    float clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
+    if (live)
+    {
+      const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
+      for (int k = 0; k < 3; k ++) { clo[k] = __double2float_rd(c[k]) - rr; chi[k] = __double2float_ru(c[k]) + rr; }
+    }
+    const int T = d.trinum;
+    auto near = [&](int t) {
+      if (d.tbox[t] > chi[0] || d.tbox[(size_t)3 * T + t] < clo[0] ||
+          d.tbox[(size_t)T + t] > chi[1] || d.tbox[(size_t)4 * T + t] < clo[1] ||
+          d.tbox[(size_t)2 * T + t] > chi[2] || d.tbox[(size_t)5 * T + t] < clo[2]) return false;
+      double A[3], B[3], C[3], pnt[3], nrm[3];
+      for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
+      const double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
+      return depth > -d.skin || depth != depth;
+    };
+    const int tb = live ? d.stbeg[sc] : 0, te = live ? d.stend[sc] : 0;
+    before_t = n;
+    const int most = __reduce_max_sync(all, te - tb);
+    for (int t0 = 0; t0 < most; t0 += RB_GROUP)
+    {
+      const int t = tb + t0 + l;
+      append(t < te && near(t), -(t + 1));
+    }
+    // (a list that the extra candidates of the float test fill, as in rb_verlet_item)
+    if (!__any_sync(all, live && n > kn && !exact)) break;
+    exact = true;
+    __syncwarp();
   }
   // statistics: one atomic per warp
   const int cmax = __reduce_max_sync(all, live ? n : 0), tmax = __reduce_max_sync(all, live ? n - before_t : 0);

@@ -27,3 +27,33 @@ def test_nan_spheres_fill_no_list(kn, gpu_lib):
         eng.close()
     for a, b in zip(*out):
         assert np.array_equal(bits(a), bits(b))
+
+
+@pytest.mark.parametrize("kn", [32, 33])
+def test_full_list_with_spheres_just_beyond_it(kn, gpu_lib, oracle_lib):
+    """A sphere with exactly as many partners within the skin as its list holds
+    and eight more a micrometre beyond, inside the margin of the float test
+    (2e-6 m at these coordinates): the list is not out of room."""
+    from parmec_gb300.engine import GpuEngine
+    from parmec_gb300.model import Model
+    from oracle.pyoracle import OracleEngine
+    R, r, skin, c = 0.05, 0.01, 0.003, np.array([2.0, 2.0, 2.0])
+    n = kn + 8
+    k = np.arange(n) + 0.5
+    th, ph = np.arccos(1.0 - 2.0 * k / n), np.pi * (1.0 + 5.0 ** 0.5) * k
+    u = np.stack([np.cos(ph) * np.sin(th), np.sin(ph) * np.sin(th), np.cos(th)], -1)
+    dist = np.where(np.arange(n) % 5 == 4, R + r + skin + 1e-6, R + r + 0.5 * skin)
+    assert (dist > R + r + skin).sum() == 8
+    out = []
+    for eng in (GpuEngine(skin=skin, capacity=(kn, 32)), OracleEngine()):
+        m = Model()
+        mat = m.material(2500.0, 1e9, 0.25)
+        m.spheres(np.concatenate([c[None], c + u * dist[:, None]]), np.array([R] + [r] * n), mat, 1)
+        m.granular(0, 0, 1e6, 0.2, 0.5)
+        dt = 1e-6
+        m.dem(3 * dt, dt, interval=1e9, engine=eng)
+        if isinstance(eng, GpuEngine):
+            assert eng.diagnostics()["max_candidates"] == kn
+        out.append(m)
+    assert_bitwise(*out)
+    assert_spheres_bitwise(*out)
