@@ -358,6 +358,15 @@ PG_DEV bool gyro_settled(const R *O, const R *Tb, double js, double is, double s
   return ok;
 }
 
+// no NaN and no infinity among the nine
+template <class R>
+PG_DEV bool finite_rotation(const R *L)
+{
+  bool ok = true;
+  for (int k = 0; k < 9; k ++) ok = ok && finite_d(L[k]);
+  return ok;
+}
+
 // exp(h 0) L is L, bit for bit: h finite and not negative, L finite without a
 // negative zero (a negative zero plus the zero products would turn positive)
 template <class R>

@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(32) k_integrate_quad(PgDev d, double step, dou
         const double b = iso ? quad_iso(q, js, t) : q.mul(Jr, t);
         T -= q.mul(Lr, b);
       }
-      const bool free_spin = q.every((dbits(T) << 1) == 0);
+      const bool free_spin = q.every((dbits(T) << 1) == 0 && finite_d(Lc[0]) && finite_d(Lc[1]) && finite_d(Lc[2]));
       double Tb = 0.0;
       if (!(iso && free_spin)) Tb = q.mul(Lc, T);
       if (iso && quad_settled(q, O, Tb, js, is, step, half))

@@ -1945,7 +1945,8 @@ __global__ void __launch_bounds__(TPB, PG_INTEGRATE_MINB) k_integrate(PgDev d, d
       }
       f[0] = F[0]; f[1] = F[1]; f[2] = F[2];
       t[0] = T[0]; t[1] = T[1]; t[2] = T[2];
-      const bool free_spin = (dbits(T[0]) << 1 | dbits(T[1]) << 1 | dbits(T[2]) << 1) == 0;
+      // (a rotation that is not finite makes the body-frame torque NaN)
+      const bool free_spin = (dbits(T[0]) << 1 | dbits(T[1]) << 1 | dbits(T[2]) << 1) == 0 && finite_rotation(L1);
       if (iso && free_spin) Tb[0] = Tb[1] = Tb[2] = N(0.0);
       else tvmul(L1, t, Tb);
       if (iso && gyro_settled(O, Tb, js, is, step, half))
