@@ -26,7 +26,7 @@ def test_rotation_that_is_not_finite(n, gpu_lib, oracle_lib):
                                                   (8, np.nan, -0.0), (None, 0.0, 2.0), (None, 0.0, 0.0)]):
             if entry is not None:
                 m.P.rotation[entry, k] = value
-            m.velocity(k, angular=(0.0, spin, 0.5 * spin))
+            m.P.angular[0:3, k] = m.P.angular[3:6, k] = (0.0, spin, 0.5 * spin)   # finite, in both frames
         m.dem(4e-5, 1e-5, interval=1e9, engine=eng)
         out.append(m)
     a, b = out
