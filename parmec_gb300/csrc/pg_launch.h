@@ -11,7 +11,8 @@ void pg_launch_euler(const PgDev &d, cudaStream_t s, double step);
 void pg_launch_shapes(const PgDev &d, cudaStream_t s, bool skip_analytical);
 void pg_launch_obstacles_state(const PgDev &d, cudaStream_t s, double step);   // velocities from obsang/obslin
 void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_step = false);
-int pg_contacts_kernel_count(const PgDev &d);   // launches of one contact evaluation (either form)
+// launches of one contact evaluation (either form), a session's step or not
+int pg_contacts_kernel_count(const PgDev &d, bool adaptive, bool in_step);
 void pg_launch_springs(const PgDev &d, cudaStream_t s, double step, bool in_step = false);
 void pg_launch_spring_runs(const PgDev &d, cudaStream_t s);     // sums of the long flush runs
 void pg_launch_unspring(const PgDev &d, cudaStream_t s);        // UNSPRING rules, after the springs
@@ -36,14 +37,17 @@ void pg_launch_restrain_forces(const PgDev &d, cudaStream_t s);       // drop-in
 void pg_launch_mesh(const PgDev &d, cudaStream_t s);
 void pg_launch_obstacles_tail(const PgDev &d, cudaStream_t s, double step);  // of a step without particles
 void pg_launch_excite(const PgDev &d, cudaStream_t s, double step);
-int  pg_step_kernel_count(const PgDev &d);
+int  pg_step_kernel_count(const PgDev &d, bool adaptive);   // launches of a step beside the rebuild's and the mesh contact's
 void pg_launch_step_end(const PgDev &d, cudaStream_t s, double step);   // where the integration's launch does not
-// whether the integration's launch ends the step: a grid of one wave
 #define PG_MX_BLOCKS 8
 // spheres up to which the mixed contacts take one launch: two warps of 32 a
 // scheduler (152 SMs of four)
 #define PG_MX_FEW (2 * 152 * 4 * 32)
-static inline int pg_ends_step(int blocks, int per_sm) { return blocks <= 152 * per_sm; }
+// the grid of the particle update of either form: blocks of `threads` threads
+// and `per` particles, the first `obstacles` of them for the obstacle triangles
+// (of an update that moves them); it ends the step where it is one wave
+struct PgUpdateGrid { bool quad; int threads, per, obstacles, blocks, ends; };
+PgUpdateGrid pg_update_grid(const PgDev &d, bool fused);
 
 // pg_mixed.cu
 void pg_launch_mx_from64(const PgDev &d, cudaStream_t s, int p0 = 0, int p1 = -1, int e0 = 0, int e1 = -1);

@@ -907,11 +907,12 @@ void pg_tt_count(const PgDev &d, const PgTT &g, int *out2, cudaStream_t s)
   if (d.trinum > 0 && g.np > 0) k_tt_counts<<<nblk(g.np), TPB, 0, s>>>(g, out2);
 }
 
-// kernels of a search and its list, and of one step's contacts and sums
-int pg_tt_search_kernels(const PgTT &g, int trinum)
+// kernels of a search, of its list, and of one step's contacts and sums
+int pg_tt_search_kernels(const PgTT &g, int trinum) { return 4 + pg_sort_kernel_count(trinum, g.passes); }
+
+int pg_tt_list_kernels(const PgTT &g)
 {
-  return 4 + pg_sort_kernel_count(trinum, g.passes) +
-         (g.np > 0 ? 4 + pg_sort_kernel_count(2 * g.np, g.epasses) + (g.nbig > 0 ? 1 : 0) : 0);
+  return g.np > 0 ? 4 + pg_sort_kernel_count(2 * g.np, g.epasses) + (g.nbig > 0 ? 1 : 0) : 0;
 }
 
 int pg_tt_step_kernels(const PgTT &g) { return 2 + (g.np > 0 ? 5 : 0) + (g.nbig > 0 ? 1 : 0); }

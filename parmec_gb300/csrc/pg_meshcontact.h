@@ -95,4 +95,5 @@ void pg_tt_chunk_map(PgTT &g, cudaStream_t s);                            // chu
 void pg_tt_forces(const PgDev &d, const PgTT &g, cudaStream_t s, double step);  // contacts and per-particle sums
 void pg_tt_count(const PgDev &d, const PgTT &g, int *out2, cudaStream_t s);   // overlapping and active pairs
 int pg_tt_search_kernels(const PgTT &g, int trinum);
+int pg_tt_list_kernels(const PgTT &g);
 int pg_tt_step_kernels(const PgTT &g);

@@ -806,8 +806,7 @@ void pg_launch_contacts_mx(const PgDev &d, cudaStream_t s, double step)
 void pg_launch_integrate_mx(const PgDev &d, cudaStream_t s, double step)
 {
   if (!d.parnum) { pg_launch_obstacles_tail(d, s, step); return; }
-  const int ob = d.obsnum ? nblk(d.trinum) : 0;
-  const int nb = ob + nblk(d.parnum), last = pg_ends_step(nb, PG_MX_BLOCKS);
-  k_integrate_mx<<<nb, TPB, 0, s>>>(d, step, ob, last);
-  if (!last) pg_launch_step_end(d, s, step);
+  const PgUpdateGrid g = pg_update_grid(d, true);
+  k_integrate_mx<<<g.blocks, g.threads, 0, s>>>(d, step, g.obstacles, g.ends);
+  if (!g.ends) pg_launch_step_end(d, s, step);
 }

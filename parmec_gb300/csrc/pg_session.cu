@@ -78,6 +78,7 @@ struct pg_session
   double fgraph_step = 0.0;
   int fgraph_chunk = 0, fgraph_ok = 1;
   long long fused_launches = 0;
+  int graph_kernels = 0;                   // kernels of the captured step
 };
 
 // spring force flush events per particle (CSR 'first' over particles), in
@@ -1132,6 +1133,7 @@ int tt_search(pg_session *s)
   for (;;)
   {
     pg_tt_search(d, g, s->stream);
+    s->launches += pg_tt_search_kernels(g, d.trinum);
     CK(cudaMemcpyAsync(s->tt_host, g.moved, 4 * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     if (s->tt_host[0] != 2) break;
@@ -1153,7 +1155,7 @@ int tt_search(pg_session *s)
   g.nchunks = s->tt_host[3];
   if (g.nchunks > g.ccap) TRY(pg_tt_chunk_room(g, g.nchunks, mem));
   pg_tt_chunk_map(g, s->stream);
-  s->launches += pg_tt_search_kernels(g, d.trinum);
+  s->launches += pg_tt_list_kernels(g);
   g.valid = 1;
   return PG_OK;
 }
@@ -1185,6 +1187,23 @@ int tt_stage(pg_session *s, double step)
   return rc;
 }
 
+// kernels of a captured graph
+int count_kernels(cudaGraph_t graph, int *kernels)
+{
+  size_t n = 0;
+  CK(cudaGraphGetNodes(graph, nullptr, &n));
+  std::vector<cudaGraphNode_t> nodes(n);
+  if (n) CK(cudaGraphGetNodes(graph, nodes.data(), &n));
+  *kernels = 0;
+  for (cudaGraphNode_t node : nodes)
+  {
+    cudaGraphNodeType type;
+    CK(cudaGraphNodeGetType(node, &type));
+    *kernels += type == cudaGraphNodeTypeKernel;
+  }
+  return PG_OK;
+}
+
 // capture one step into a CUDA graph (kernel arguments are baked in: the
 // graph is re-captured when a buffer is reallocated or the step changes)
 int capture_step(pg_session *s, double step)
@@ -1196,6 +1215,7 @@ int capture_step(pg_session *s, double step)
   CK(cudaStreamEndCapture(s->stream, &s->graph));
   TRY(rc);
   CK(cudaGraphInstantiate(&s->graph_exec, s->graph, 0));
+  TRY(count_kernels(s->graph, &s->graph_kernels));
   s->graph_step = step;
   s->graph_adapt = 0;
   return PG_OK;
@@ -1225,6 +1245,7 @@ int capture_step_adaptive(pg_session *s)
   enqueue_step_adaptive(s);
   CK(cudaStreamEndCapture(s->stream, &s->graph));
   CK(cudaGraphInstantiate(&s->graph_exec, s->graph, 0));
+  TRY(count_kernels(s->graph, &s->graph_kernels));
   s->graph_adapt = 1;
   return PG_OK;
 }
@@ -1285,20 +1306,6 @@ void enqueue_step_adaptive(pg_session *s)
   pg_launch_adapt_step(d, s->stream, true);
   pg_launch_dynamics_fused(d, s->stream);
   pg_launch_mesh(d, s->stream);
-}
-
-int adaptive_kernel_count(const PgDev &d)
-{
-  int n = pg_rebuild_kernel_count(d) + pg_contacts_kernel_count(d);
-  if (!d.ellnum && !d.sprnum) n += 1;             // excite
-  if (d.sprnum) n += 1 + pg_spring_run_kernel_count(d, true) + (d.unsprnum ? 1 : 0);
-  if (d.trqsprnum) n += 1;
-  // force sums, the minimum with the selection unless they take it, dynamics
-  // with obstacles and tail; without particles the selection and the tail
-  n += d.parnum && !pg_adapt_in_sums(d) ? 3 : 2;
-  if (d.nodnum) n += 1;
-  if (d.facnum) n += 1;
-  return n;
 }
 
 // host step tables of one call -> device (rows [0, n))
@@ -1494,11 +1501,13 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
     if (wait) CK(cudaStreamSynchronize(s->stream));
     return PG_OK;
   }
-  const int per_step = pg_rebuild_kernel_count(d) + pg_step_kernel_count(d);
+  const PgDev live = live_view(s);
+  int per_step = pg_rebuild_kernel_count(live) + pg_step_kernel_count(live, false);
   bool counted = false;
   if (!s->profile && s->use_graph && !d.tt_on)
   {
     TRY(capture_step(s, step));
+    per_step = s->graph_kernels;
     int k = 0;
     if (n >= PG_GRAPH_STEPS)
     {
@@ -1520,7 +1529,7 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
   {
     // groups: 0 rebuild, 1 contacts, 2 springs, 3 integrate (with the obstacles
     // and the tail), 4 mesh, 5 nothing any more
-    const PgDev d = live_view(s);
+    const PgDev &d = live;
     const int G = 6;
     s->ring.resize((size_t)n * (G + 1));
     for (auto &e : s->ring) if (!e) CK(cudaEventCreate(&e));
@@ -1550,7 +1559,7 @@ static int run_steps(pg_session *s, const pg_steptab *tab, double step, bool wai
       CK(cudaEventRecord(ev[6], s->stream));
     }
     CK(cudaStreamSynchronize(s->stream));
-    const int counts[6] = {pg_rebuild_kernel_count(d), pg_contacts_kernel_count(d), d.sprnum ? 1 : 0, d.parnum ? 1 : 0,
+    const int counts[6] = {pg_rebuild_kernel_count(d), pg_contacts_kernel_count(d, false, true), d.sprnum ? 1 : 0, d.parnum ? 1 : 0,
                            (d.nodnum ? 1 : 0) + (d.facnum ? 1 : 0), 0};
     for (int k = 0; k < n; k ++)
     {
@@ -1855,7 +1864,8 @@ int pg_session_run_adaptive(pg_session *s, const pg_steptab *tab, double step0, 
   TRY(h2d(s, s->hs_buf, h3, 3));
   d.hs = s->hs_buf;
   int rc = PG_OK;
-  if (s->use_graph && !s->profile)
+  const bool captured = s->use_graph && !s->profile;
+  if (captured)
   {
     rc = capture_step_adaptive(s);
     for (int k = 0; k < n && rc == PG_OK; k ++)
@@ -1864,7 +1874,7 @@ int pg_session_run_adaptive(pg_session *s, const pg_steptab *tab, double step0, 
   else for (int k = 0; k < n; k ++) enqueue_step_adaptive(s);
   d.hs = nullptr;
   TRY(rc);
-  s->launches += (long long)adaptive_kernel_count(d) * n;
+  s->launches += (long long)(captured ? s->graph_kernels : pg_rebuild_kernel_count(d) + pg_step_kernel_count(d, true)) * n;
   CK(cudaGetLastError());
   if (steps) TRY(d2h(s, steps, d.hrec, (size_t)n));
   CK(cudaStreamSynchronize(s->stream));

@@ -2708,12 +2708,12 @@ void pg_launch_contacts(const PgDev &d, cudaStream_t s, double step, bool in_ste
 // the FP64 form evaluates the lists in three passes with adaptive stepping,
 // two otherwise (one when no work queue is allocated); the mixed form in a
 // sphere and a triangle pass (pg_mixed.cu)
-int pg_contacts_kernel_count(const PgDev &d)
+int pg_contacts_kernel_count(const PgDev &d, bool adaptive, bool in_step)
 {
   if (!d.ellnum) return 0;
   if (d.form == PG_FORM_MIXED) return d.ellnum <= PG_MX_FEW ? 1 : 2;
-  if (!d.cwork || !d.cwork_n) return 1;
-  return (d.ellnum <= PG_SMALL_SCENE ? 1 : 2) + (d.hs ? 1 : 0);
+  if (!d.cwork || !d.cwork_n) return in_step ? 2 : 1;      // with the scene gravities' own
+  return (d.ellnum <= PG_SMALL_SCENE ? 1 : 2) + (adaptive && !(in_step && pg_adapt_in_sums(d)) ? 1 : 0);
 }
 
 // in_step: a session's step; without spheres its scene gravities are taken here
@@ -2775,6 +2775,19 @@ void pg_launch_step_end(const PgDev &d, cudaStream_t s, double step) { k_step_en
 // measures the same on both sides of it (the update 30 us against 29 for one
 // thread a particle with four entries' loads in flight), of 9,261 24 against
 // 28, of 2,197 21 against 28.
+PgUpdateGrid pg_update_grid(const PgDev &d, bool fused)
+{
+  const bool mixed = d.form == PG_FORM_MIXED;
+  PgUpdateGrid g;
+  g.quad = !mixed && d.parnum <= PG_SMALL_SCENE;
+  g.threads = g.quad ? 32 : TPB;
+  g.per = g.quad ? 8 : TPB;
+  g.obstacles = fused && d.obsnum ? (d.trinum + g.threads - 1) / g.threads : 0;
+  g.blocks = g.obstacles + (d.parnum + g.per - 1) / g.per;
+  g.ends = g.blocks <= 152 * (mixed ? PG_MX_BLOCKS : g.quad ? 16 : PG_INTEGRATE_MINB);
+  return g;
+}
+
 template <int MODE>
 static void launch_integrate(const PgDev &d, cudaStream_t s, double step, double half, double hstep, bool masters = false)
 {
@@ -2784,12 +2797,10 @@ static void launch_integrate(const PgDev &d, cudaStream_t s, double step, double
     if (fused) pg_launch_obstacles_tail(d, s, step);
     return;
   }
-  const bool quad = d.parnum <= PG_SMALL_SCENE;
-  const int B = quad ? 32 : TPB, P = quad ? 8 : B;
-  const int ob = fused && d.obsnum ? (d.trinum + B - 1) / B : 0, nb = (d.parnum + P - 1) / P;
-  const int last = fused ? pg_ends_step(ob + nb, quad ? 16 : PG_INTEGRATE_MINB) : masters;
-  if (quad) k_integrate_quad<MODE><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
-  else k_integrate<MODE><<<ob + nb, B, 0, s>>>(d, step, half, hstep, ob, last);
+  const PgUpdateGrid g = pg_update_grid(d, fused);
+  const int last = fused ? g.ends : masters;
+  if (g.quad) k_integrate_quad<MODE><<<g.blocks, g.threads, 0, s>>>(d, step, half, hstep, g.obstacles, last);
+  else k_integrate<MODE><<<g.blocks, g.threads, 0, s>>>(d, step, half, hstep, g.obstacles, last);
   if (fused && !last) pg_launch_step_end(d, s, step);
 }
 
@@ -2870,17 +2881,18 @@ void pg_launch_obstacles_tail(const PgDev &d, cudaStream_t s, double step)
   k_obstacles_tail<<<nb > 0 ? nb : 1, 32, 0, s>>>(d, step);
 }
 
-// launches of a session's step beside the rebuild's
-int pg_step_kernel_count(const PgDev &d)
+// launches of a session's step beside the rebuild's and the mesh contact's
+int pg_step_kernel_count(const PgDev &d, bool adaptive)
 {
-  int n = pg_contacts_kernel_count(d);         // contacts: sphere and triangle passes
+  int n = pg_contacts_kernel_count(d, adaptive, true);
   // the scene gravities have a launch of their own only without both
   if (!d.ellnum && !d.sprnum) n += 1;
-  if (d.sprnum) n += 1 + pg_spring_run_kernel_count(d, false) + (d.unsprnum ? 1 : 0);
+  if (d.sprnum) n += 1 + pg_spring_run_kernel_count(d, adaptive) + (d.unsprnum ? 1 : 0);
   if (d.trqsprnum) n += 1;                     // torsion springs
-  n += 1;                                      // integrate, obstacles and (in small scenes) the step's end
-  const int nb = nblk(d.parnum) + (d.obsnum ? nblk(d.trinum) : 0);
-  if (d.parnum > PG_SMALL_SCENE && !pg_ends_step(nb, d.form == PG_FORM_MIXED ? PG_MX_BLOCKS : PG_INTEGRATE_MINB)) n += 1;
+  // adaptive: the force sums, and the step's choice unless they take it
+  if (adaptive) n += d.parnum ? (pg_adapt_in_sums(d) ? 1 : d.obs_done ? 2 : 3) : 1;
+  n += 1;                                      // the update, with the obstacles
+  if (d.parnum && !pg_update_grid(d, true).ends) n += 1;   // the step's end
   if (d.nodnum) n += 1;
   if (d.facnum) n += 1;
   return n;
