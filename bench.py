@@ -16,6 +16,7 @@ rank's particle-steps over the slowest rank's time.
 --impl reference times the reference's own hot path on all host cores: its
 ISPC sources translated to C++ at gang size one (oracle/ispc_ref.py; the
 ispc compiler is not installed), driven by parmec.cpp's dem() call sequence.
+Where neither the sources nor their translation are on the host it says so.
 """
 import argparse
 import json
@@ -128,6 +129,16 @@ def peaks():
         return 6800.0, "fallback"
 
 
+def reference_library():
+    """(path, None) of the reference's translated hot path, or (None, why)."""
+    try:
+        from oracle import ispc_ref
+        path = ispc_ref.build()
+    except Exception as e:
+        return None, "its translated hot path does not build here: " + " ".join(str(e).split())[:200]
+    return path, None if path else "neither its ISPC sources nor their translation are on this host"
+
+
 def reference_cpu(n_spheres, threads, steps, warmup=1):
     """The reference's own hot path on the host cores: its ISPC sources
     translated to C++ (oracle/ispc_ref.py; tasks spread over `threads`
@@ -137,12 +148,9 @@ def reference_cpu(n_spheres, threads, steps, warmup=1):
     (particle-steps/s, kind, sample description)."""
     from parmec_gb300.scenes import drum
     m, dt, _ = drum(n_spheres)
-    try:
-        from oracle import dem_loop, ispc_ref
-        lib_path = ispc_ref.build()
-    except Exception:
-        lib_path = None
+    lib_path, _ = reference_library()
     if lib_path:
+        from oracle import dem_loop
         lib = dem_loop.library(lib_path)
         host = dem_loop.Host(lib, m, orient=True, ntasks=threads)
         dem_loop.dem(lib, host, warmup * dt - 0.5 * dt, dt)
@@ -438,8 +446,12 @@ def serving_form(args, count):
 def run_reference(args, rank, world):
     """--impl reference: the reference's CPU hot path on all host cores, rank 0
     only, on the same drum, config, metric and unit as the GPU arm; each step
-    is a bounded sample of the workload."""
+    is a bounded sample of the workload.  The oracle never stands in for it."""
     if rank != 0:
+        return 0
+    path, why = reference_library()
+    if not path:
+        print(json.dumps({"impl": "reference", "unavailable": why}))
         return 0
     threads = os.cpu_count() or 1
     from parmec_gb300.scenes import drum
