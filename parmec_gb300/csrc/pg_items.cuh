@@ -848,8 +848,13 @@ __device__ __forceinline__ void rb_verlet_group(const PgDev &d, int i, bool vali
 }
 
 // whether the groups take a scene's lists: its spheres at RB_GROUP lanes each
-// fill no more than a warp a scheduler four times over (152 SMs of four), its
-// lists fit, and its triangles are few (many are scanned better by the warp)
+// are at most eight warps a scheduler (152 SMs of four), its lists fit, and its
+// triangles are few (many are scanned better by the warp).  Rebuilds of moving
+// spheres in a box of 12, 192 and 768 triangles, groups against threads: 216
+// spheres 64, 76, 101 us against 74, 92, 108; 4,096 spheres 104, 118, 143
+// against 116, 130, 153; 12,167 spheres 124, 150, 197 against 124, 141, 162;
+// 17,576 spheres 155, 175, 230 against 157, 166, 191.  At 256 a scene the small
+// scenes keep their gain and the largest lose up to 8% near the line.
 __device__ __forceinline__ bool rb_grouped(const PgDev &d)
 {
   return d.ellnum <= 152 * 4 * 32 && d.kn <= RB_GROUP_KN && d.trinum <= 256 * d.nscene;

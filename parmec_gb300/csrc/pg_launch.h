@@ -41,7 +41,11 @@ int  pg_step_kernel_count(const PgDev &d, bool adaptive);   // launches of a ste
 void pg_launch_step_end(const PgDev &d, cudaStream_t s, double step);   // where the integration's launch does not
 #define PG_MX_BLOCKS 8
 // spheres up to which the mixed contacts take one launch: two warps of 32 a
-// scheduler (152 SMs of four)
+// scheduler (152 SMs of four).  A step in one launch against two: of the drum
+// 5,000 spheres 19.1 us against 20.4, 39,000 22.2 against 23.9, 70,000 24.5
+// against 26.3, 100,000 30.1 against 28.3; of the hopper fill 10,648 spheres 55
+// against 63, 39,304 69 and 69, 97,336 87 against 91.  The line lies on the safe
+// side of where the drum's cross.
 #define PG_MX_FEW (2 * 152 * 4 * 32)
 // the grid of the particle update of either form: blocks of `threads` threads
 // and `per` particles, the first `obstacles` of them for the obstacle triangles
@@ -62,7 +66,7 @@ int  pg_fused_candidates(PgFusedCfg *out, int cap);
 cudaError_t pg_launch_fused_mx(const PgDev &d, cudaStream_t s, double step, int nsteps, const PgFusedCfg &c);
 
 // pg_session.cu
-// spring flush runs longer than this are summed by k_spring_runs
+// spring flush runs longer than this are summed by k_spring_run_groups
 #define PG_SPRING_RUN_LONG 64
 int  pg_spring_run_groups(const std::vector<int4> &big);         // PgDev.nbig_groups
 void pg_spring_events(int P, int S, const int *sj, const int *sk, std::vector<int> &first, std::vector<int4> &ev,

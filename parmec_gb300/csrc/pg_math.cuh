@@ -323,7 +323,7 @@ PG_DEV void spin_iso(R *O, R *Tb, double js, double is, double step, double half
 // takes 9 FP64 instructions then instead of 109 (the map, the products and
 // the cross product feed nothing else).  Of 100 spheres of the drum 99 are
 // settled, of the hopper fill 82 to 93.  With exp_terms and the unturned
-// rotations k_integrate takes 207 FP64 instructions a warp instead of 298:
+// rotations k_integrate takes 183 FP64 instructions a particle instead of 298:
 // 697 -> 547 us on the 1,048,576-sphere drum (480 with register operands),
 // 121 -> 48 us on 207,000 spheres of shaken boxes (most of them not turning
 // yet).

@@ -84,7 +84,7 @@ struct PgTT
   int ccap = 0;
 };
 
-#define PG_TT_CHUNK 1024          // entries one warp sums into one chunk sum
+#define PG_TT_CHUNK 1024          // entries of a chunk: summed by a warp, or by six blocks where a particle has several
 #define PG_TT_TILE 1024           // entries of one tile of the selection of active entries
 
 int pg_tt_key_bits(int ncells);

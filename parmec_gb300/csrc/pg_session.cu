@@ -126,7 +126,8 @@ void pg_spring_events(int P, int S, const int *sj, const int *sk, std::vector<in
   {
     first[ev[q].part + 1] ++;
     evv[q] = ev[q].v;
-    // a long run is summed by its own block beforehand (k_spring_runs); its
+    // a long run is summed beforehand, a warp a group of its chunks and value
+    // (k_spring_run_groups, then k_spring_run_totals or the particle); its
     // index + 1 sits above the run type in .x
     if (ev[q].v.z - ev[q].v.y > PG_SPRING_RUN_LONG)
     {

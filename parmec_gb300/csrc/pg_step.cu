@@ -1759,7 +1759,8 @@ __global__ void __launch_bounds__(TPB, PG_INTEGRATE_MINB) k_integrate(PgDev d, d
         bool started = false;
         if (run >= 0)
         {
-          // a long run, summed in the same order by k_spring_runs
+          // a long run, summed in the same order by k_spring_run_groups and
+          // k_spring_run_totals
           for (int c = 0; c < 3; c ++) { af[c] = d.sbig_sum[6*run + c]; at[c] = d.sbig_sum[6*run + 3 + c]; }
         }
         else
@@ -2771,10 +2772,11 @@ void pg_launch_step_end(const PgDev &d, cudaStream_t s, double step) { k_step_en
 
 // Scenes of up to 19,456 particles take four lanes a particle in blocks of one
 // warp, so that the warps spread over the SMs.  The line is where the four
-// lanes fill every scheduler four warps deep: a step of 17,576 falling spheres
-// measures the same on both sides of it (the update 30 us against 29 for one
-// thread a particle with four entries' loads in flight), of 9,261 24 against
-// 28, of 2,197 21 against 28.
+// lanes fill every scheduler four warps deep, and with it the forms of the
+// contacts change: a step of the hopper fill in the small form takes 45 us
+// against 58 in the large one at 8,000 spheres, 56 against 64 at 12,167, 64
+// against 63 at 17,576, 75 against 76 at 21,952, 86 against 78 at 27,000, 101
+// against 93 at 39,304.
 PgUpdateGrid pg_update_grid(const PgDev &d, bool fused)
 {
   const bool mixed = d.form == PG_FORM_MIXED;

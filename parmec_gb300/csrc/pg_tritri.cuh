@@ -45,9 +45,9 @@ PG_TT void cross(const double *a, const double *b, double *c)
 // device (the FP64 pipe, which issues comparisons too, is the narrow one);
 // each gives the truth value of the IEEE comparison it stands for, NaN
 // operands included.  On the device the bits are taken by a move the
-// compiler cannot fold back into an FP64 comparison.  The plane test and
-// the box keys of the candidate search use them; in the narrow phase, whose
-// branches they reshape, plain comparisons measured faster.
+// compiler cannot fold back into an FP64 comparison.  The plane test, the box
+// keys of the candidate search and the region tests of the vertex-face and
+// edge-edge distances use them.
 PG_TT unsigned long long bits(double x)
 {
   unsigned long long b;
