@@ -366,7 +366,7 @@ def spring_lattice_form(args, n_side):
             leg["mesh_contact"] = {"radius_m": radius, "triangle_pairs_last_step": pairs,
                                    "active_contacts_last_step": active,
                                    "note": "steps with mesh contact run without CUDA graphs (one host wait "
-                                           "per step for the pair count)"}
+                                           "per step: whether a new pair list is due)"}
         out[key] = leg
         out.setdefault("particles", m.parnum)
         out.setdefault("springs", m.sprnum)
