@@ -57,3 +57,31 @@ def test_full_list_with_spheres_just_beyond_it(kn, gpu_lib, oracle_lib):
         out.append(m)
     assert_bitwise(*out)
     assert_spheres_bitwise(*out)
+
+
+@pytest.mark.parametrize("kn", [32, 64])
+@pytest.mark.parametrize("n", [7, 8, 9, 15, 16, 17, 400])
+def test_crowded_cells_bitwise(n, kn, gpu_lib, oracle_lib):
+    """n small spheres in the few cells that a large one sets, rebuilt often,
+    on both sides of the count above which the search walks one cell after
+    another and of its eights."""
+    from parmec_gb300.engine import GpuEngine
+    from parmec_gb300.model import Model
+    from oracle.pyoracle import OracleEngine
+    out = []
+    for eng in (GpuEngine(skin=4e-6, capacity=(kn, 64)), OracleEngine()):
+        rng = np.random.default_rng(n)
+        m = Model()
+        mat = m.material(2500.0, 1e9, 0.25)
+        g = np.stack(np.meshgrid(*(np.arange(8),) * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+        m.spheres(0.05 + g * 2.01e-3 + rng.uniform(-4e-6, 4e-6, size=(n, 3)), np.full(n, 1e-3), mat, 1)
+        m.sphere((0.05 - 0.0111, 0.052, 0.052), 0.01, mat, 1)
+        m.P.linear[:, :n] = rng.normal(0.0, 0.5, size=(3, n))
+        m.granular(0, 0, 1e4, 0.2, 0.5)
+        m.set_gravity(0.0, 0.0, -9.81)
+        m.dem(59.5 * 2e-6, 2e-6, interval=1e9, engine=eng)
+        if isinstance(eng, GpuEngine):
+            assert eng.diagnostics()["rebuilds"] > 10 and len(eng.contacts()["mpart"]) > 0
+        out.append(m)
+    assert_bitwise(*out)
+    assert_spheres_bitwise(*out)
