@@ -6,6 +6,8 @@
 #include "pg_state.h"
 
 #define PG_TT_KMAX 256            // partners one triangle may find (a warp's list in the search)
+#define PG_TT_SOON 4              // steps a list serves at least, or the skin grows
+#define PG_TT_LATE 32             // steps a list serves at most, or a grown skin shrinks
 
 // a pair whose contact a few distances decide: candidates (bits as in
 // pgtf::judge), where their results start, a bound on the smallest
@@ -36,8 +38,11 @@ struct PgTT
   unsigned long long *box[6] = {};
   // the pair list: every pair of triangles whose boxes, widened by half the
   // skin, overlapped at the last search, in (finder, partner) order; valid
-  // while no vertex coordinate has moved by half the skin since
-  double skin = 0.0;
+  // while no vertex coordinate has moved by half the skin since.  The skin
+  // starts at skin0 and doubles, up to skin_most, where a list served fewer than
+  // PG_TT_SOON steps; a grown one halves where it served more than PG_TT_LATE.
+  double skin = 0.0, skin0 = 0.0, skin_most = 0.0;
+  int since = 0;                  // steps the list has served
   int valid = 0;
   int *moved = nullptr;           // [4]: a vertex moved, pairs found, big particles, their chunks
   double *ref[9] = {};            // [trinum] vertices at the last search

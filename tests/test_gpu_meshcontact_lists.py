@@ -147,3 +147,19 @@ def test_distances_without_room_bitwise(vertex, edge, gpu_lib, oracle_lib):
     assert eg.lib.pg_session_mesh_contact_room(eg.sess, 0, vertex, edge) == abi.PG_OK
     dem(both, 60, first=True)
     assert dem(both, 100)[1] > 37
+
+
+def test_fast_meshes_bitwise(gpu_lib, oracle_lib):
+    """A pile whose upper layer flies past and into the lower one at 20 m/s, so
+    that the skin grows, then slowed down, so that it shrinks again."""
+    both = pair(lambda: pile(gap=0.004))
+    for m, _ in both:
+        m.P.linear[:, 10:m.parnum] = np.array([[20.0], [3.0], [-5.0]])
+    dem(both, 60, first=True)
+    assert dem(both, 60)[1] > 0
+    for m, _ in both:
+        m.P.linear[:, 1:m.parnum] *= 0.02
+        m.P.angular[:, 1:m.parnum] *= 0.02
+        m._dirty = True
+    dem(both, 150)
+    dem(both, 300)
