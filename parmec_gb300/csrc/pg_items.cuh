@@ -424,10 +424,66 @@ __device__ __forceinline__ float rb_tolerance(const PgDev &d, const float *c)
 }
 __device__ __forceinline__ bool rb_exact(const PgDev &d, float tol) { return !(tol < 0.02f * (float)d.skin); }
 
-// whether the float distance, squared, keeps a candidate: where the FP64 test
-// follows, unless it is certainly beyond; else only where it is within, so that
-// a NaN sphere is nobody's candidate either way
-__device__ __forceinline__ bool rb_near(float f2, float l2, bool exact) { return exact ? !(f2 >= l2) : f2 < l2; }
+// The float distance, squared, keeps a candidate where it is below the limit's
+// square, a NaN sphere never; `every`: where the float copies overflow, the FP64
+// test decides alone.
+__device__ __forceinline__ bool rb_near(float f2, float l2, bool every) { return f2 < l2 || every; }
+__device__ __forceinline__ bool rb_every(float tol) { return !(tol < __int_as_float(0x7f800000)) && tol == tol; }
+
+// the FP64 test of candidate j of sphere i
+__device__ __forceinline__ bool rb_within(const PgDev &d, const double *c, double ri, int j)
+{
+  const double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
+  const double lim = ri + d.radii[0][j] + d.skin;
+  return q0*q0 + q1*q1 + q2*q2 < lim*lim;
+}
+
+// The list of sphere i by the FP64 tests alone, for one that the extra candidates
+// of the float test have filled: by one thread, out of line (a second pass or a
+// cut in the search itself took 3% of a rebuild, whether a list was full or not).
+// Returns the entries found; codes holds the first d.kn.
+static __device__ __noinline__ int rb_exact_list(const PgDev &d, int i, int *codes)
+{
+  const double c[3] = {d.center[0][i], d.center[1][i], d.center[2][i]}, ri = d.radii[0][i];
+  const int pi = d.part[i], sc = d.escene[i];
+  const unsigned prefix = (unsigned)sc << (3 * d.bits), cm = d.ekey[i] & ((1u << (3 * d.bits)) - 1u);
+  const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
+  int n = 0;
+  for (int q = 0; q < 27; q ++)
+  {
+    const int x = u[0] + q % 3 - 1, y = u[1] + q / 3 % 3 - 1, z = u[2] + q / 9 - 1;
+    if (x < 0 || y < 0 || z < 0 || x >= d.dim[0] || y >= d.dim[1] || z >= d.dim[2]) continue;
+    const unsigned key = prefix | morton(x, y, z);
+    for (int s = d.cstart[key]; s < d.cend[key]; s ++)
+    {
+      const int2 p = d.pfs[s];
+      if (p.x <= pi || !rb_within(d, c, ri, p.y)) continue;
+      int k = n < d.kn ? n : d.kn - 1;                   // in index order
+      if (n < d.kn || codes[k] > p.y)
+      {
+        while (k > 0 && codes[k-1] > p.y) { codes[k] = codes[k-1]; k --; }
+        codes[k] = p.y;
+      }
+      n ++;
+    }
+  }
+  const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
+  const size_t T = d.trinum;
+  for (int t = d.stbeg[sc]; t < d.stend[sc]; t ++)
+  {
+    bool apart = false;
+    for (int k = 0; k < 3; k ++)
+      apart = apart || d.tbox[k * T + t] > __double2float_ru(c[k]) + rr || d.tbox[(3 + k) * T + t] < __double2float_rd(c[k]) - rr;
+    if (apart) continue;
+    double A[3], B[3], C[3], pnt[3], nrm[3];
+    for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
+    const double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
+    if (!(depth > -d.skin) && !(depth != depth)) continue;
+    if (n < d.kn) codes[n] = -(t + 1);
+    n ++;
+  }
+  return n;
+}
 
 // The new list of sphere i with the flags and tangential state of the partners
 // it keeps (both lists in partner order).  The entries before the first
@@ -483,8 +539,8 @@ __device__ __forceinline__ void rb_merge(const PgDev &d, int i, const int *codes
 // particles, their clamped places and the loads of the emptier cells cost more
 // than they hide.  Rebuilds of small spheres in cells of 3, 5, 10 and 20 times
 // their size (20, 94, 750 and all of them a cell), nine at a time against one
-// cell after another: 2,000 spheres 158, 429, 2,094 and 2,210 us against 149,
-// 268, 674 and 564; 60,000 spheres 302, 624 and 3,420 against 288, 443 and 2,008
+// cell after another: 2,000 spheres 158, 429, 2,094 and 2,210 us against 139,
+// 244, 601 and 507; 60,000 spheres 302, 624 and 3,420 against 273, 405 and 1,785
 // of the first three.  At 6 a cell the nine are ahead by a tenth.
 constexpr int RB_CROWDED = 8;
 
@@ -512,184 +568,179 @@ __device__ __forceinline__ void rb_verlet_item(const PgDev &d, int i, bool valid
   // candidates cost less than the FP64 test, which holds the warp's FP64
   // pipe for every lane's neighbour in turn (a candidate beyond the limit
   // is never in contact: the lists decide nothing).  A list that the extra
-  // candidates fill is made again with the FP64 test.
-  bool exact = rb_exact(d, tol);
-  const unsigned full = 0xffffffffu, lm = __ballot_sync(full, live);
-  if (!lm) return;
-  const int lane = threadIdx.x & 31, sc0 = __shfl_sync(full, sc, __ffs(lm) - 1);
-  #pragma unroll 1
-  for (;;)
+  // candidates fill is made anew by the FP64 tests.
+  const bool exact = rb_exact(d, tol), every = rb_every(tol);
+  auto append = [&](int code) {
+    if (n < d.kn) codes[n ++] = code;
+    else { over = true; nover ++; }
+  };
+  if (live)
   {
-    n = nover = ntri = 0;
-    over = false;
-    if (live)
+    const unsigned prefix = (unsigned)sc << (3 * d.bits);
+    // the sphere's cell, from the key the key phase computed, instead of
+    // three FP64 divisions again
+    const unsigned cm = d.ekey[i] & ((1u << (3 * d.bits)) - 1u);
+    const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
+    // FP32 prefilter: a neighbour is skipped only when its float distance
+    // exceeds the float limit by tol, more than the rounding of the float
+    // copies and of the float arithmetic can account for, so no candidate of
+    // the FP64 test is missed.  Float coordinates carry at most 2^-24 |c| of error;
+    // tol = 2^-20 (max|c_i| + 2 cell) bounds the distance error 16 times over
+    // for partners within a cell.
+    const float rsf = (float)ri + (float)d.skin;
+    auto take = [&](int2 p) {
+      if (!exact || rb_within(d, c, ri, p.y)) append(p.y);
+    };
+    // a layer of nine cells at a time: their ranges are loaded together, then
+    // the first sphere of each, the second of each, ... (the order in which
+    // candidates are found plays no part).  Every load is issued whether its
+    // cell holds a sphere or not, so that nine are in flight where one cell
+    // after another was a chain of two to four latencies (476 -> 349 us of a
+    // rebuild of 1,270,000 shaken spheres, at one to two spheres a cell)
+    #pragma unroll 1
+    for (int dz = -1; dz <= 1; dz ++)
     {
-      const unsigned prefix = (unsigned)sc << (3 * d.bits);
-      // the sphere's cell, from the key the key phase computed, instead of
-      // three FP64 divisions again
-      const unsigned cm = d.ekey[i] & ((1u << (3 * d.bits)) - 1u);
-      const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
-      // FP32 prefilter: a neighbour is skipped only when its float distance
-      // exceeds the float limit by tol, more than the rounding of the float
-      // copies and of the float arithmetic can account for, so no candidate of
-      // the FP64 test is missed.  Float coordinates carry at most 2^-24 |c| of error;
-      // tol = 2^-20 (max|c_i| + 2 cell) bounds the distance error 16 times over
-      // for partners within a cell.
-      const float rsf = (float)ri + (float)d.skin;
-      auto take = [&](int2 p) {
-        const int j = p.y;
-        if (exact)
-        {
-          double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
-          double lim = ri + d.radii[0][j] + d.skin;
-          if (!(q0*q0 + q1*q1 + q2*q2 < lim*lim)) return;
-        }
-        if (n < d.kn) codes[n ++] = j;
-        else { over = true; nover ++; }
-      };
-      // a layer of nine cells at a time: their ranges are loaded together, then
-      // the first sphere of each, the second of each, ... (the order in which
-      // candidates are found plays no part).  Every load is issued whether its
-      // cell holds a sphere or not, so that nine are in flight where one cell
-      // after another was a chain of two to four latencies (476 -> 349 us of a
-      // rebuild of 1,270,000 shaken spheres, at one to two spheres a cell)
-      #pragma unroll 1
-      for (int dz = -1; dz <= 1; dz ++)
+      int b[9], e[9], m = 0;
+      const int z = u[2] + dz;
+      const unsigned mz = spread3((unsigned)z) << 2;
+      #pragma unroll
+      for (int q = 0; q < 9; q ++)
       {
-        int b[9], e[9], m = 0;
-        const int z = u[2] + dz;
-        const unsigned mz = spread3((unsigned)z) << 2;
-        #pragma unroll
+        const int x = u[0] + q % 3 - 1, y = u[1] + q / 3 - 1;
+        const bool in = x >= 0 && y >= 0 && z >= 0 && x < d.dim[0] && y < d.dim[1] && z < d.dim[2];
+        const unsigned key = prefix | (in ? spread3((unsigned)x) | (spread3((unsigned)y) << 1) | mz : cm);
+        const int cb = d.cstart[key], ce = d.cend[key];
+        b[q] = in ? cb : 0;
+        e[q] = in ? ce : 0;
+      }
+      #pragma unroll
+      for (int q = 0; q < 9; q ++) m = max(m, e[q] - b[q]);
+      if (m > RB_CROWDED)
+      {
+        #pragma unroll 1
         for (int q = 0; q < 9; q ++)
         {
           const int x = u[0] + q % 3 - 1, y = u[1] + q / 3 - 1;
-          const bool in = x >= 0 && y >= 0 && z >= 0 && x < d.dim[0] && y < d.dim[1] && z < d.dim[2];
-          const unsigned key = prefix | (in ? spread3((unsigned)x) | (spread3((unsigned)y) << 1) | mz : cm);
+          if (x < 0 || y < 0 || z < 0 || x >= d.dim[0] || y >= d.dim[1] || z >= d.dim[2]) continue;
+          const unsigned key = prefix | spread3((unsigned)x) | (spread3((unsigned)y) << 1) | mz;
           const int cb = d.cstart[key], ce = d.cend[key];
-          b[q] = in ? cb : 0;
-          e[q] = in ? ce : 0;
-        }
-        #pragma unroll
-        for (int q = 0; q < 9; q ++) m = max(m, e[q] - b[q]);
-        if (m > RB_CROWDED)
-        {
           #pragma unroll 1
-          for (int q = 0; q < 9; q ++)
+          for (int s = cb; s < ce; s += 8)
           {
-            const int x = u[0] + q % 3 - 1, y = u[1] + q / 3 - 1;
-            if (x < 0 || y < 0 || z < 0 || x >= d.dim[0] || y >= d.dim[1] || z >= d.dim[2]) continue;
-            const unsigned key = prefix | spread3((unsigned)x) | (spread3((unsigned)y) << 1) | mz;
-            const int cb = d.cstart[key], ce = d.cend[key];
-            #pragma unroll 1
-            for (int s = cb; s < ce; s += 8)
+            float4 o[8];
+            #pragma unroll
+            for (int k = 0; k < 8; k ++) o[k] = d.cfs[min(s + k, ce - 1)];
+            #pragma unroll
+            for (int k = 0; k < 8; k ++)
             {
-              float4 o[8];
-              #pragma unroll
-              for (int k = 0; k < 8; k ++) o[k] = d.cfs[min(s + k, ce - 1)];
-              #pragma unroll
-              for (int k = 0; k < 8; k ++)
-              {
-                const float f0 = cif[0] - o[k].x, f1 = cif[1] - o[k].y, f2 = cif[2] - o[k].z;
-                const float lf = rsf + o[k].w + tol;
-                if (s + k >= ce || !rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, exact)) continue;
-                const int2 p = d.pfs[s + k];
-                if (p.x > pi) take(p);
-              }
+              const float f0 = cif[0] - o[k].x, f1 = cif[1] - o[k].y, f2 = cif[2] - o[k].z;
+              const float lf = rsf + o[k].w + tol;
+              if (s + k >= ce || !rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, every)) continue;
+              const int2 p = d.pfs[s + k];
+              if (p.x > pi) take(p);
             }
           }
-          continue;
         }
-        #pragma unroll 1
-        for (int t = 0; t < m; t ++)
-        {
-          // (an entry beyond its cell's range reads the first of all)
-          float4 o[9];
-          int2 p[9];
-          #pragma unroll
-          for (int q = 0; q < 9; q ++)
-          {
-            const int s = b[q] + t < e[q] ? b[q] + t : 0;
-            o[q] = d.cfs[s];
-            p[q] = d.pfs[s];
-          }
-          #pragma unroll
-          for (int q = 0; q < 9; q ++)
-          {
-            const float f0 = cif[0] - o[q].x, f1 = cif[1] - o[q].y, f2 = cif[2] - o[q].z;
-            const float lf = rsf + o[q].w + tol;
-            if (!(b[q] + t < e[q] && p[q].x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, exact))) continue;
-            take(p[q]);
-          }
-        }
+        continue;
       }
-      // insertion sort of the sphere partners
-      for (int a = 1; a < n; a ++)
+      #pragma unroll 1
+      for (int t = 0; t < m; t ++)
       {
-        int v = codes[a], b = a - 1;
-        while (b >= 0 && codes[b] > v) { codes[b+1] = codes[b]; b --; }
-        codes[b+1] = v;
+        // (an entry beyond its cell's range reads the first of all)
+        float4 o[9];
+        int2 p[9];
+        #pragma unroll
+        for (int q = 0; q < 9; q ++)
+        {
+          const int s = b[q] + t < e[q] ? b[q] + t : 0;
+          o[q] = d.cfs[s];
+          p[q] = d.pfs[s];
+        }
+        #pragma unroll
+        for (int q = 0; q < 9; q ++)
+        {
+          const float f0 = cif[0] - o[q].x, f1 = cif[1] - o[q].y, f2 = cif[2] - o[q].z;
+          const float lf = rsf + o[q].w + tol;
+          if (!(b[q] + t < e[q] && p[q].x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, every))) continue;
+          take(p[q]);
+        }
       }
     }
-    // triangles of the sphere's scene within r + skin (AABB in float, then the
-    // true closest-point distance), in triangle order
-    const float inf = __int_as_float(0x7f800000);
-    float clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
-    if (live)
+    // insertion sort of the sphere partners
+    for (int a = 1; a < n; a ++)
     {
-      const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
-      for (int k = 0; k < 3; k ++) { clo[k] = __double2float_rd(c[k]) - rr; chi[k] = __double2float_ru(c[k]) + rr; }
+      int v = codes[a], b = a - 1;
+      while (b >= 0 && codes[b] > v) { codes[b+1] = codes[b]; b --; }
+      codes[b+1] = v;
     }
-    const int T = d.trinum;
-    auto box_apart = [&](int t, const float *lo, const float *hi) {
-      return d.tbox[t] > hi[0] || d.tbox[(size_t)3 * T + t] < lo[0] ||
-             d.tbox[(size_t)T + t] > hi[1] || d.tbox[(size_t)4 * T + t] < lo[1] ||
-             d.tbox[(size_t)2 * T + t] > hi[2] || d.tbox[(size_t)5 * T + t] < lo[2];
-    };
-    auto try_triangle = [&](int t) {
-      if (box_apart(t, clo, chi)) return;
-      double A[3], B[3], C[3], pnt[3], nrm[3];
-      for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
-      // the candidate test uses the true closest point: the reference's region
-      // formula can only report a larger distance, so this set stays a superset
-      double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
-      if (!(depth > -d.skin) && !(depth != depth)) return;
-      ntri ++;
-      if (n < d.kn) codes[n ++] = -(t + 1);
-      else { over = true; nover ++; }
-    };
-    // when every live lane of the warp is in one scene, the warp tests 32
-    // triangles at a time against the box of all its spheres and each lane
-    // then tests its own box against the triangles that box reached
-    if (__all_sync(full, !live || sc == sc0))
-    {
-      float wlo[3], whi[3];
-      for (int k = 0; k < 3; k ++)
-      {
-        wlo[k] = clo[k]; whi[k] = chi[k];
-        for (int o = 16; o > 0; o >>= 1)
-        {
-          wlo[k] = fminf(wlo[k], __shfl_xor_sync(full, wlo[k], o));
-          whi[k] = fmaxf(whi[k], __shfl_xor_sync(full, whi[k], o));
-        }
-      }
-      const int tb = d.stbeg[sc0], te = d.stend[sc0];
-      for (int t0 = tb; t0 < te; t0 += 32)
-      {
-        const int t = t0 + lane;
-        unsigned hm = __ballot_sync(full, t < te && !box_apart(t, wlo, whi));
-        while (hm)
-        {
-          const int tt = t0 + __ffs(hm) - 1;
-          hm &= hm - 1;
-          if (live) try_triangle(tt);
-        }
-      }
-    }
-    else if (live)
-      for (int t = d.stbeg[sc]; t < d.stend[sc]; t ++) try_triangle(t);
-    if (!__any_sync(full, over && !exact)) break;
-    exact = true;
   }
+  // triangles of the sphere's scene within r + skin (AABB in float, then the
+  // true closest-point distance), in triangle order
+  const float inf = __int_as_float(0x7f800000);
+  float clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
+  if (live)
+  {
+    const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
+    for (int k = 0; k < 3; k ++) { clo[k] = __double2float_rd(c[k]) - rr; chi[k] = __double2float_ru(c[k]) + rr; }
+  }
+  const int T = d.trinum;
+  auto box_apart = [&](int t, const float *lo, const float *hi) {
+    return d.tbox[t] > hi[0] || d.tbox[(size_t)3 * T + t] < lo[0] ||
+           d.tbox[(size_t)T + t] > hi[1] || d.tbox[(size_t)4 * T + t] < lo[1] ||
+           d.tbox[(size_t)2 * T + t] > hi[2] || d.tbox[(size_t)5 * T + t] < lo[2];
+  };
+  auto try_triangle = [&](int t) {
+    if (box_apart(t, clo, chi)) return;
+    double A[3], B[3], C[3], pnt[3], nrm[3];
+    for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
+    // the candidate test uses the true closest point: the reference's region
+    // formula can only report a larger distance, so this set stays a superset
+    double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
+    if (!(depth > -d.skin) && !(depth != depth)) return;
+    ntri ++;
+    append(-(t + 1));
+  };
+  const unsigned full = 0xffffffffu, lm = __ballot_sync(full, live);
+  if (!lm) return;
+  const int lane = threadIdx.x & 31, sc0 = __shfl_sync(full, sc, __ffs(lm) - 1);
+  // when every live lane of the warp is in one scene, the warp tests 32
+  // triangles at a time against the box of all its spheres and each lane
+  // then tests its own box against the triangles that box reached
+  if (__all_sync(full, !live || sc == sc0))
+  {
+    float wlo[3], whi[3];
+    for (int k = 0; k < 3; k ++)
+    {
+      wlo[k] = clo[k]; whi[k] = chi[k];
+      for (int o = 16; o > 0; o >>= 1)
+      {
+        wlo[k] = fminf(wlo[k], __shfl_xor_sync(full, wlo[k], o));
+        whi[k] = fmaxf(whi[k], __shfl_xor_sync(full, whi[k], o));
+      }
+    }
+    const int tb = d.stbeg[sc0], te = d.stend[sc0];
+    for (int t0 = tb; t0 < te; t0 += 32)
+    {
+      const int t = t0 + lane;
+      unsigned hm = __ballot_sync(full, t < te && !box_apart(t, wlo, whi));
+      while (hm)
+      {
+        const int tt = t0 + __ffs(hm) - 1;
+        hm &= hm - 1;
+        if (live) try_triangle(tt);
+      }
+    }
+  }
+  else if (live)
+    for (int t = d.stbeg[sc]; t < d.stend[sc]; t ++) try_triangle(t);
+  if (over && !exact)
+  {
+    n = rb_exact_list(d, i, codes);
+    nover = n > d.kn ? n - d.kn : 0;
+    n -= nover;
+    over = nover > 0;
+  }
+  __syncwarp();
   // one atomic per warp for the largest list and triangle counts
   {
     const int cmax = __reduce_max_sync(full, live ? n + nover : 0);
@@ -734,111 +785,103 @@ __device__ __forceinline__ void rb_verlet_group(const PgDev &d, int i, bool vali
   const bool live = sc >= 0 && d.sactive[sc] != 0;
   const int kn = d.kn;
   const float cif[3] = {(float)c[0], (float)c[1], (float)c[2]}, tol = rb_tolerance(d, cif);
-  bool exact = rb_exact(d, tol);
-  int n = 0, before_t = 0;                               // entries found, spheres of them (the group's lanes agree)
-  int v[W], rank[W];
+  const bool exact = rb_exact(d, tol), every = rb_every(tol);
+  int n = 0;                                             // entries found (the group's lanes agree)
   auto append = [&](bool hit, int code) {
     const unsigned m = __ballot_sync(all, hit);
     const int at = n + __popc(m & before);
     if (hit && at < kn) codes[at] = code;
     n += __popc(m & group);
   };
-  #pragma unroll 1
-  for (;;)
   {
-    n = 0;
+    const unsigned prefix = (unsigned)sc << (3 * d.bits);
+    const unsigned cm = live ? d.ekey[i] & ((1u << (3 * d.bits)) - 1u) : 0u;
+    const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
+    const float rsf = (float)ri + (float)d.skin;
+    int b[(27 + RB_GROUP - 1) / RB_GROUP], e[(27 + RB_GROUP - 1) / RB_GROUP];
+    #pragma unroll
+    for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
     {
-      const unsigned prefix = (unsigned)sc << (3 * d.bits);
-      const unsigned cm = live ? d.ekey[i] & ((1u << (3 * d.bits)) - 1u) : 0u;
-      const int u[3] = {(int)compact3(cm), (int)compact3(cm >> 1), (int)compact3(cm >> 2)};
-      const float rsf = (float)ri + (float)d.skin;
-      int b[(27 + RB_GROUP - 1) / RB_GROUP], e[(27 + RB_GROUP - 1) / RB_GROUP];
-      #pragma unroll
-      for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
+      const int k = l + RB_GROUP * q, x = u[0] + k % 3 - 1, y = u[1] + k / 3 % 3 - 1, z = u[2] + k / 9 - 1;
+      b[q] = e[q] = 0;
+      if (live && k < 27 && x >= 0 && y >= 0 && z >= 0 && x < d.dim[0] && y < d.dim[1] && z < d.dim[2])
       {
-        const int k = l + RB_GROUP * q, x = u[0] + k % 3 - 1, y = u[1] + k / 3 % 3 - 1, z = u[2] + k / 9 - 1;
-        b[q] = e[q] = 0;
-        if (live && k < 27 && x >= 0 && y >= 0 && z >= 0 && x < d.dim[0] && y < d.dim[1] && z < d.dim[2])
-        {
-          const unsigned key = prefix | morton(x, y, z);
-          b[q] = d.cstart[key];
-          e[q] = d.cend[key];
-        }
-      }
-      #pragma unroll
-      for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
-      {
-        const int m = __reduce_max_sync(all, e[q] - b[q]);
-        for (int t = 0; t < m; t ++)
-        {
-          const int s = b[q] + t;
-          bool hit = s < e[q];
-          int j = 0;
-          if (hit)
-          {
-            const float4 o = d.cfs[s];
-            const float f0 = cif[0] - o.x, f1 = cif[1] - o.y, f2 = cif[2] - o.z, lf = rsf + o.w + tol;
-            const int2 p = d.pfs[s];
-            j = p.y;
-            hit = p.x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, exact);
-            if (hit && exact)
-            {
-              const double q0 = c[0] - d.center[0][j], q1 = c[1] - d.center[1][j], q2 = c[2] - d.center[2][j];
-              const double lim = ri + d.radii[0][j] + d.skin;
-              hit = q0*q0 + q1*q1 + q2*q2 < lim*lim;
-            }
-          }
-          append(hit, j);
-        }
+        const unsigned key = prefix | morton(x, y, z);
+        b[q] = d.cstart[key];
+        e[q] = d.cend[key];
       }
     }
-    // the sphere partners in index order
-    __syncwarp();
-    const int ns = n < kn ? n : kn;
     #pragma unroll
-    for (int q = 0; q < W; q ++)
+    for (int q = 0; q < (27 + RB_GROUP - 1) / RB_GROUP; q ++)
     {
-      const int a = l + RB_GROUP * q;
-      v[q] = a < ns ? codes[a] : 0;
-      rank[q] = 0;
-      if (a < ns) for (int o = 0; o < ns; o ++) rank[q] += codes[o] < v[q];
+      const int m = __reduce_max_sync(all, e[q] - b[q]);
+      for (int t = 0; t < m; t ++)
+      {
+        const int s = b[q] + t;
+        bool hit = s < e[q];
+        int j = 0;
+        if (hit)
+        {
+          const float4 o = d.cfs[s];
+          const float f0 = cif[0] - o.x, f1 = cif[1] - o.y, f2 = cif[2] - o.z, lf = rsf + o.w + tol;
+          const int2 p = d.pfs[s];
+          j = p.y;
+          hit = p.x > pi && rb_near(f0*f0 + f1*f1 + f2*f2, lf*lf, every);
+          if (hit && exact) hit = rb_within(d, c, ri, j);
+        }
+        append(hit, j);
+      }
     }
-    __syncwarp();
-    #pragma unroll
-    for (int q = 0; q < W; q ++) if (l + RB_GROUP * q < ns) codes[rank[q]] = v[q];
-    // triangles of the sphere's scene, in triangle order
-    const float inf = __int_as_float(0x7f800000);
-    float clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
-    if (live)
-    {
-      const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
-      for (int k = 0; k < 3; k ++) { clo[k] = __double2float_rd(c[k]) - rr; chi[k] = __double2float_ru(c[k]) + rr; }
-    }
-    const int T = d.trinum;
-    auto near = [&](int t) {
-      if (d.tbox[t] > chi[0] || d.tbox[(size_t)3 * T + t] < clo[0] ||
-          d.tbox[(size_t)T + t] > chi[1] || d.tbox[(size_t)4 * T + t] < clo[1] ||
-          d.tbox[(size_t)2 * T + t] > chi[2] || d.tbox[(size_t)5 * T + t] < clo[2]) return false;
-      double A[3], B[3], C[3], pnt[3], nrm[3];
-      for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
-      const double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
-      return depth > -d.skin || depth != depth;
-    };
-    const int tb = live ? d.stbeg[sc] : 0, te = live ? d.stend[sc] : 0;
-    before_t = n;
-    const int most = __reduce_max_sync(all, te - tb);
-    for (int t0 = 0; t0 < most; t0 += RB_GROUP)
-    {
-      const int t = tb + t0 + l;
-      append(t < te && near(t), -(t + 1));
-    }
-    // (a list that the extra candidates of the float test fill, as in rb_verlet_item)
-    if (!__any_sync(all, live && n > kn && !exact)) break;
-    exact = true;
-    __syncwarp();
   }
+  // the sphere partners in index order
+  __syncwarp();
+  const int ns = n < kn ? n : kn;
+  int v[W], rank[W];
+  #pragma unroll
+  for (int q = 0; q < W; q ++)
+  {
+    const int a = l + RB_GROUP * q;
+    v[q] = a < ns ? codes[a] : 0;
+    rank[q] = 0;
+    if (a < ns) for (int o = 0; o < ns; o ++) rank[q] += codes[o] < v[q];
+  }
+  __syncwarp();
+  #pragma unroll
+  for (int q = 0; q < W; q ++) if (l + RB_GROUP * q < ns) codes[rank[q]] = v[q];
+  // triangles of the sphere's scene, in triangle order
+  const float inf = __int_as_float(0x7f800000);
+  float clo[3] = {inf, inf, inf}, chi[3] = {-inf, -inf, -inf};
+  if (live)
+  {
+    const float rr = (float)(ri + d.skin) * 1.0001f + 1e-30f;
+    for (int k = 0; k < 3; k ++) { clo[k] = __double2float_rd(c[k]) - rr; chi[k] = __double2float_ru(c[k]) + rr; }
+  }
+  const int T = d.trinum;
+  auto near = [&](int t) {
+    if (d.tbox[t] > chi[0] || d.tbox[(size_t)3 * T + t] < clo[0] ||
+        d.tbox[(size_t)T + t] > chi[1] || d.tbox[(size_t)4 * T + t] < clo[1] ||
+        d.tbox[(size_t)2 * T + t] > chi[2] || d.tbox[(size_t)5 * T + t] < clo[2]) return false;
+    double A[3], B[3], C[3], pnt[3], nrm[3];
+    for (int q = 0; q < 3; q ++) { A[q] = d.tri[q][t]; B[q] = d.tri[3+q][t]; C[q] = d.tri[6+q][t]; }
+    const double depth = pg::triangle_sphere(A, B, C, c, ri, pnt, nrm, false);
+    return depth > -d.skin || depth != depth;
+  };
+  const int tb = live ? d.stbeg[sc] : 0, te = live ? d.stend[sc] : 0;
+  const int before_t = n;
+  const int most = __reduce_max_sync(all, te - tb);
+  for (int t0 = 0; t0 < most; t0 += RB_GROUP)
+  {
+    const int t = tb + t0 + l;
+    append(t < te && near(t), -(t + 1));
+  }
+  // a list that the extra candidates of the float test fill, by its first lane
+  __syncwarp();
+  int found = n;
+  if (live && n > kn && !exact && l == 0) found = rb_exact_list(d, i, codes);
+  n = __shfl_sync(all, found, g0);
+  __syncwarp();
   // statistics: one atomic per warp
-  const int cmax = __reduce_max_sync(all, live ? n : 0), tmax = __reduce_max_sync(all, live ? n - before_t : 0);
+  const int cmax = __reduce_max_sync(all, live ? n : 0), tmax = __reduce_max_sync(all, live && n > before_t ? n - before_t : 0);
   if (lane == 0)
   {
     if (cmax > 0) atomicMax(&d.stats[1], cmax);

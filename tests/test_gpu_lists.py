@@ -85,3 +85,39 @@ def test_crowded_cells_bitwise(n, kn, gpu_lib, oracle_lib):
         out.append(m)
     assert_bitwise(*out)
     assert_spheres_bitwise(*out)
+
+
+@pytest.mark.parametrize("kn", [32, 33])
+def test_full_list_with_triangles_bitwise(kn, gpu_lib, oracle_lib):
+    """The same with a floor of triangles beside the spheres, so that the last
+    places of a full list hold triangles: what is left must be in order, with
+    the contacts' state in place."""
+    from parmec_gb300.engine import GpuEngine
+    from parmec_gb300.model import Model
+    from parmec_gb300.scenes import box_triangles
+    from oracle.pyoracle import OracleEngine
+    R, r, skin, c = 0.05, 0.01, 3e-4, np.array([2.0, 2.0, 2.0])
+    n = kn - 2 + 6                                       # two triangles of the floor, six spheres too many
+    k = np.arange(n) + 0.5
+    th, ph = np.arccos(1.0 - 1.5 * k / n), np.pi * (1.0 + 5.0 ** 0.5) * k
+    u = np.stack([np.cos(ph) * np.sin(th), np.sin(ph) * np.sin(th), np.cos(th)], -1)
+    dist = np.where(np.arange(n) % 6 == 5, R + r + skin + 1e-6, R + r - 1e-5)
+    dist[np.flatnonzero(np.arange(n) % 6 == 5)[6:]] = R + r - 1e-5
+    assert (dist > R + r + skin).sum() == 6
+    z = 2.0 - R - 1e-4
+    out = []
+    for eng in (GpuEngine(skin=skin, capacity=(kn, 32)), OracleEngine()):
+        m = Model()
+        mat = m.material(2500.0, 1e9, 0.25)
+        m.spheres(np.concatenate([c[None], c + u * dist[:, None]]), np.array([R] + [r] * n), mat, 1)
+        m.obstacle([t for t in box_triangles((1.5, 1.5, z - 0.1), (2.5, 2.5, z)) if t[2] == t[5] == t[8] == z], 2)
+        m.P.linear[:, 1:n + 1] = np.where(dist > R + r + skin, 0.05, 0.0) * u.T      # they never come within
+        m.granular(0, 0, 1e5, 0.2, 0.5)
+        dt = 2e-5
+        m.dem(400.5 * dt, dt, interval=1e9, engine=eng)
+        if isinstance(eng, GpuEngine):
+            d = eng.diagnostics()
+            assert d["max_triangles"] >= 2 and d["rebuilds"] >= 2
+        out.append(m)
+    assert_bitwise(*out)
+    assert_spheres_bitwise(*out)
